@@ -601,6 +601,8 @@ done:
   }
 }
 
+#include "gemm_skinny.cuh"
+
 // ------------------------------------------------------------------ host side
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
                                   const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
@@ -687,6 +689,71 @@ static int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUten
   return SXB_OK;
 }
 
+// Cluster size of the skinny kernel (each side measured, us): enough CTAs for two per SM, at most the portable 8, and
+// powers of two only, because clusters of 6 leave so many SMs of a GPC unused that 48 of them take two waves (6144 x 4096,
+// one token: 16.4 with 6, 13.1 with 4).  Four CTAs want three 64-wide blocks of K each (4096 x 768: 4.7 with 4, 5.2 with 2);
+// eight want eight, or the reduction costs more than the shorter walk saves (2048 x 2048, 48 tokens: 7.4 with 8, 6.5 with 4),
+// unless a smaller cluster would leave half of the chip without work (768 x 2048: 5.9 with 8, 6.3 with 4).
+static int skinny_split(int tiles, int num_kb) {
+  const int sms = num_sms();
+  if (8 * tiles <= 2 * sms && num_kb >= (8 * tiles > sms * 4 / 5 ? 64 : 24)) return 8;
+  if (4 * tiles <= 2 * sms && num_kb >= 12) return 4;
+  return 2 * tiles <= 2 * sms && num_kb >= 4 ? 2 : 1;
+}
+
+// Whether an NT product takes the skinny kernel instead of the persistent ones (measured on projections with N = 768 ..
+// 32000, K = 768 .. 14336; us, persistent | skinny).  Up to 32 tokens always: 4096 x 4096 27.6 | 10.9, 28672 x 4096 43.8 | 42.6.
+// Up to 64 tokens while its 128-row tiles fit the chip once: 16384 x 2048 18.9 | 17.7, but 32000 x 2048 25.7 | 27.4.  More
+// tokens only while the tiles are few for the length of K, which is when the persistent kernels leave SMs without a
+// tile: 4096 x 14336, 512 tokens 68.8 | 58.4; 2048 x 2048, 512 tokens 14.8 | 12.5; 4096 x 768, 256 tokens 8.2 | 9.7;
+// 6144 x 4096, 512 tokens 25.2 | 32.9.
+static bool use_skinny(int M, int N, int K) {
+  if (M <= 32) return true;
+  const long long tiles = (long long)((N + 127) / 128) * ((M + 127) / 128);
+  if (M <= 64 && tiles <= num_sms()) return true;
+  return tiles <= 128 && tiles <= K / 32;
+}
+
+template <int BN, int STAGES>
+static int launch_skinny(const void* A, const void* B, const Params& p, int lda, int ldb, cudaStream_t stream) {
+  using Plan = SkinnyPlan<BN, STAGES>;
+  auto kfn = gemm_skinny_kernel<BN, STAGES>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, Plan::kTotal);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  CUtensorMap tw, tx;
+  const CUtensorMapDataType BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  int rc = make_map_2d(&tw, B, p.N, p.K, ldb, 128, BK, BF, 2);
+  if (rc) return rc;
+  rc = make_map_2d(&tx, A, p.M, p.K, lda, BN, BK, BF, 2);
+  if (rc) return rc;
+  const int tiles_n = (p.N + 127) / 128, tiles_m = (p.M + BN - 1) / BN;
+  const int S = skinny_split(tiles_n * tiles_m, (p.K + BK - 1) / BK);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles_n * S, tiles_m);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = Plan::kTotal;
+  cfg.stream = stream;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = S; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, tw, tx, p, S);
+  if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
+  return SXB_OK;
+}
+
+static int launch_skinny(const void* A, const void* B, const Params& p, int lda, int ldb, cudaStream_t stream) {
+  if (p.M <= 16) return launch_skinny<16, 6>(A, B, p, lda, ldb, stream);
+  if (p.M <= 32) return launch_skinny<32, 5>(A, B, p, lda, ldb, stream);
+  if (p.M <= 64) return launch_skinny<64, 4>(A, B, p, lda, ldb, stream);
+  return launch_skinny<128, 3>(A, B, p, lda, ldb, stream);
+}
+
 }  // namespace gemm
 }  // namespace sxb
 
@@ -698,10 +765,11 @@ SXB_DEFINE_HANG_ACCESSOR(sxb_gemm_hang_info)
 // C[M,N] (+)= alpha * op(A) op(B).  A/B are bf16; C is bf16 or fp32 (c_dtype).
 // lda/ldb/ldc are row pitches in elements of the *stored* matrices.
 // max_ctas: 0 = all SMs; otherwise leaves SMs free for a concurrent comm kernel.
-// 0 = auto (pair kernel for large problems), 1 = force single-CTA kernel, 2 = force pair kernel
+// 0 = auto (pair kernel for large problems), 1 = force single-CTA kernel, 2 = force pair kernel, 3 = force the skinny kernel
+// (NT only)
 static int g_gemm_mode = 0;
 SXB_API int sxb_gemm_set_mode(int mode) {
-  if (mode < 0 || mode > 2) return SXB_ERR_BAD_ARG;
+  if (mode < 0 || mode > 3) return SXB_ERR_BAD_ARG;
   g_gemm_mode = mode;
   return SXB_OK;
 }
@@ -722,6 +790,8 @@ SXB_API int sxb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
   p.M = M; p.N = N; p.K = K; p.layout = layout; p.c_dtype = c_dtype;
   p.accumulate = accumulate ? 1 : 0; p.direct = tma_c ? 0 : 1; p.C = C; p.ldc = ldc;
   p.alpha = alpha;
+  if (layout == NT && (g_gemm_mode == 3 || (g_gemm_mode == 0 && max_ctas <= 0 && use_skinny(M, N, K))))
+    return launch_skinny(A, B, p, lda, ldb, reinterpret_cast<cudaStream_t>(stream));
   const int BNsel = (N > 128) ? 256 : 128;
   CUtensorMap ta, tb, tc;
   int rc;
