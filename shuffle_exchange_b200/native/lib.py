@@ -14,6 +14,7 @@ from pathlib import Path
 from typing import Optional
 
 import torch
+import torch.autograd.forward_ad as _forward_ad
 
 _HERE = Path(__file__).resolve().parent
 _LIB: Optional[ctypes.CDLL] = None
@@ -136,7 +137,22 @@ def ptr(t: Optional[torch.Tensor]):
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current stream of the current device (3.2 us through a ``torch.cuda.Stream`` object, 0.3 us this way)."""
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
+def no_tape(*tensors: Optional[torch.Tensor]) -> bool:
+    """Whether nothing watches an operation on ``tensors``: no gradient is wanted, no forward-mode level is open, nothing is
+    being traced, and no function transform (vmap, grad) or dispatch mode is active.  An operator may then call its kernel
+    without the detour through an autograd function (8 to 15 of a serving layer's 25 us per call)."""
+    if torch.is_grad_enabled():
+        for t in tensors:
+            if t is not None and t.requires_grad:
+                return False
+    return (_forward_ad._current_level < 0 and torch._C._get_tracing_state() is None
+            and torch._C._functorch.peek_interpreter_stack() is None and not torch._C._len_torch_dispatch_stack())
 
 
 def call(name: str, *args):

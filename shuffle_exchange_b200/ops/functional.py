@@ -182,23 +182,30 @@ def _deliver_wgrad(weight, dy2, x2):
     return gemm(dy2, x2, GEMM_TN, out_dtype=weight.dtype)
 
 
+def _linear_fwd(x, x2, weight, bias):
+    # allocate with the final shape so the returned tensor is not a view (in-place consumers
+    # such as RoPE may then modify it)
+    n = weight.shape[0]
+    y = x.new_empty((*x.shape[:-1], n))
+    y2 = y if x.dim() == 2 else y.view(-1, n)
+    gate = getattr(weight, "_sxb_gate", None)
+    if gate is not None:
+        # K2: the weight is still being gathered; the kernel waits for the tiles it needs (ops/gemm_ext.py)
+        from .gemm_ext import gemm_gated
+        gemm_gated(x2, weight, GEMM_NT, gate, out=y2)
+    else:
+        gemm(x2, weight, GEMM_NT, out=y2)
+    if bias is not None:
+        y.add_(bias)
+    _note_use(weight)
+    return y
+
+
 class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias):
         x2 = x.reshape(-1, x.shape[-1])
-        # allocate with the final shape so the returned tensor is not a view (in-place consumers
-        # such as RoPE may then modify it)
-        y = torch.empty((*x.shape[:-1], weight.shape[0]), dtype=x.dtype, device=x.device)
-        gate = getattr(weight, "_sxb_gate", None)
-        if gate is not None:
-            # K2: the weight is still being gathered; the kernel waits for the tiles it needs (ops/gemm_ext.py)
-            from .gemm_ext import gemm_gated
-            gemm_gated(x2, weight, GEMM_NT, gate, out=y.view(-1, weight.shape[0]))
-        else:
-            gemm(x2, weight, GEMM_NT, out=y.view(-1, weight.shape[0]))
-        if bias is not None:
-            y.add_(bias)
-        _note_use(weight)
+        y = _linear_fwd(x, x2, weight, bias)
         ctx.save_for_backward(x2, weight)
         ctx.has_bias = bias is not None
         ctx.xshape = x.shape
@@ -243,6 +250,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
             x = x.contiguous()
         if x.data_ptr() % 16:               # a one-row column slice counts as contiguous wherever it starts
             x = x.clone()
+        if _n.no_tape(x, weight, bias):
+            return _linear_fwd(x, x if x.dim() == 2 else x.reshape(-1, x.shape[-1]), weight, bias)
         return _Linear.apply(x, weight, bias)
     if x.is_cuda:
         # fp16 / fp32 operands or rows that are not 16-byte multiples: the tcgen05 GEMM takes bf16 only, the library
@@ -272,23 +281,26 @@ def rms_norm_ref(x, weight, eps, residual=None):
     return y.to(x.dtype), h
 
 
+def _rms_norm_fwd(x, weight, eps, residual, rstd):
+    """``(norm, x + residual or None)`` of contiguous tensors, in the shape of ``x``; ``rstd`` (fp32, one per row) or None."""
+    H = x.shape[-1]
+    y = torch.empty_like(x)
+    h = torch.empty_like(x) if residual is not None else None
+    _n.call("sxb_rmsnorm_fwd", x.data_ptr(), _n.ptr(residual), weight.data_ptr(), y.data_ptr(), _n.ptr(h), _n.ptr(rstd),
+            x.numel() // H, H, float(eps), _n.dtype_code(x.dtype), _n.stream_ptr())
+    _note_use(weight)
+    return y, h
+
+
 class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, eps, residual):
         H = x.shape[-1]
         x2 = x.reshape(-1, H)
         rows = x2.shape[0]
-        y = torch.empty_like(x2)
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
-        if residual is not None:
-            r2 = residual.reshape(-1, H)
-            h = torch.empty_like(x2)
-        else:
-            r2, h = None, None
-        _n.call("sxb_rmsnorm_fwd", x2.data_ptr(), _n.ptr(r2), weight.data_ptr(), y.data_ptr(),
-                _n.ptr(h), rstd.data_ptr(), rows, H, float(eps), _n.dtype_code(x.dtype), _n.stream_ptr())
+        y, h = _rms_norm_fwd(x2, weight, eps, residual.reshape(-1, H) if residual is not None else None, rstd)
         src = h if h is not None else x2
-        _note_use(weight)
         ctx.save_for_backward(src, weight, rstd)
         ctx.has_res = residual is not None
         ctx.shape = x.shape
@@ -338,7 +350,10 @@ def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
             x = x.contiguous()
         if residual is not None and not residual.is_contiguous():
             residual = residual.contiguous()
-        y, h = _RMSNorm.apply(x, weight, eps, residual)
+        if _n.no_tape(x, weight, residual):
+            y, h = _rms_norm_fwd(x, weight, eps, residual, None)
+        else:
+            y, h = _RMSNorm.apply(x, weight, eps, residual)
         return y, (h if residual is not None else x)
     return rms_norm_ref(x, weight, eps, residual)
 
@@ -462,14 +477,20 @@ def rope(x: torch.Tensor, positions: Optional[torch.Tensor], cos: torch.Tensor, 
 
 
 # ------------------------------------------------------------------- gated activations
+def _gated_fwd(x2, act):
+    rows, F_ = x2.shape[0], x2.shape[1] // 2
+    out = x2.new_empty((rows, F_))
+    _n.call("sxb_gated_act_fwd", x2.data_ptr(), None, out.data_ptr(), rows, F_, act, _n.dtype_code(x2.dtype),
+            _n.stream_ptr())
+    return out
+
+
 class _Gated(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, act):
         F_ = x.shape[-1] // 2
         x2 = x.reshape(-1, 2 * F_)
-        out = torch.empty((x2.shape[0], F_), dtype=x.dtype, device=x.device)
-        _n.call("sxb_gated_act_fwd", x2.data_ptr(), None, out.data_ptr(), x2.shape[0], F_, act,
-                _n.dtype_code(x.dtype), _n.stream_ptr())
+        out = _gated_fwd(x2, act)
         ctx.save_for_backward(x2)
         ctx.act = act
         ctx.shape = x.shape
@@ -492,7 +513,10 @@ def gated_act(x: torch.Tensor, act="silu") -> torch.Tensor:
     """``act(x[..., :F]) * x[..., F:]`` (SwiGLU/GeGLU with concatenated gate|up projection)."""
     code = _act_code(act)
     if x.is_cuda:
-        return _Gated.apply(x.contiguous(), code)
+        x = x.contiguous()
+        if x.dim() == 2 and x.shape[1] % 2 == 0 and _n.no_tape(x):
+            return _gated_fwd(x, code)
+        return _Gated.apply(x, code)
     F_ = x.shape[-1] // 2
     return (_torch_act(x[..., :F_].float(), code) * x[..., F_:].float()).to(x.dtype)
 
