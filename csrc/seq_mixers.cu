@@ -380,7 +380,8 @@ constexpr int kBQ = 64, kBK = 64;    // query rows / keys per tile of the tiled 
 // one 64-key tile of K and V (converted to fp32) and the tile's weights (in the key tile's place, once the scores are
 // done: head sizes up to 128 then leave room for two CTAs per SM) sit in shared memory; 256 threads hold 4x4
 // scores and 4 x (dv/16) outputs each.  Scores, online softmax with the sink logit, and the weighted sum are fp32 FMAs:
-// the weights must stay 32-bit, so the products cannot go through the bf16 tensor path.
+// the weights must stay 32-bit, so the products cannot go through the bf16 tensor path as they are (sink_attention_mma.cuh splits them; this form serves
+// fp32 caches and other head sizes).
 template <typename T, int NV>
 __global__ void __launch_bounds__(256, NV <= 2 ? 2 : 1)
 sink_attention_tile_kernel(const float* __restrict__ q, const T* __restrict__ kcache, const T* __restrict__ vcache,
@@ -540,6 +541,8 @@ sink_attention_tile_kernel(const float* __restrict__ q, const T* __restrict__ kc
       }
   }
 }
+
+#include "sink_attention_mma.cuh"
 
 // One CTA of kAW warps per (token, key/value head): single decode tokens and short portions.  Keys lo..pos of the token's
 // sequence, lo = start of the token's chunk (chunk > 0) or 0; the warps take 32-key tiles in turn (a lane scores one
@@ -1894,6 +1897,22 @@ static int launch_attention_tiles(const void* q, const void* kcache, const void*
   return SXB_OK;
 }
 
+template <int D, int DV>
+static int launch_attention_mma(const void* q, const void* kcache, const void* vcache, const void* sink, void* out,
+                                const void* atoms, int n_long, const void* tables, int max_blocks, int block_size, int Hq,
+                                int G, float scale, int chunk, int window, int kpitch, int vpitch, const void* dist_bias,
+                                int bias_len, const void* gate, long long gate_ld, int gate_heads, long long out_ld,
+                                float out_scale, cudaStream_t s) {
+  using L = SinkMma<D, DV>;
+  cudaError_t e = cudaFuncSetAttribute(sink_attention_mma_kernel<D, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal);
+  if (e != cudaSuccess) return (int)e;
+  sink_attention_mma_kernel<D, DV><<<dim3(Hq, n_long), kSmThreads, L::kTotal, s>>>(
+      (const float*)q, (const __nv_bfloat16*)kcache, (const __nv_bfloat16*)vcache, (const float*)sink, (__nv_bfloat16*)out,
+      (const int*)atoms, (const int*)tables, max_blocks, block_size, Hq, G, scale, chunk, window, kpitch, vpitch,
+      (const float*)dist_bias, bias_len, (const __nv_bfloat16*)gate, gate_ld, gate_heads, out_ld, out_scale);
+  return SXB_OK;
+}
+
 /* The same attention scheduled by attention atoms int32 [n_atoms, 6] = (sequence, first row, queries, first position,
  * -, -), longest first: the first n_long atoms (more than 16 queries, at most 128) run the tiled kernel, 64 queries per
  * CTA; the others one warp per (query, head).  Needs d, dv and both pitches multiples of 4, d and dv at most 256. */
@@ -1914,16 +1933,29 @@ SXB_API int sxb_sink_attention_atoms(const void* q, const void* kcache, const vo
   if (n_long > 0) {
     const int nv = (dv + 63) / 64;
     int rc = SXB_OK;
+    // 16-bit caches with heads of 64 or 128 channels take the tensor-core form: the fp32 FMA form is bound by the FMA lanes (one
+    // prompt of 3000 rows, 16 heads of 128, chunks of 1024: 675 us, 203 on the tensor cores).  Rows are copied 16 bytes at a
+    // time, so pitches are multiples of 8 and the bases 16-byte aligned; fp32 caches and other head sizes keep the FMA form.
+    const bool mma = dtype == kBF16 && n_long <= 65535 && (d == 64 || d == 128) && (dv == 64 || dv == 128) && k_pitch % 8 == 0 && v_pitch % 8 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kcache) |
+                       reinterpret_cast<uintptr_t>(vcache)) & 15) == 0;
+#define MMA(D, DV)                                                                                                    \
+  rc = launch_attention_mma<D, DV>(q, kcache, vcache, sink, out, atoms, n_long, tables, max_blocks, block_size, Hq, G,   \
+                                   scale, chunk, window, k_pitch, v_pitch, dist_bias, bias_len, gate, gate_ld,         \
+                                   gate_heads, out_ld, out_scale, s)
 #define TILES(NV)                                                                                                     \
   SEQMIX_DISPATCH(dtype, (rc = launch_attention_tiles<T, NV>(q, kcache, vcache, sink, out, atoms, n_long, tables,      \
                                                               max_blocks, block_size, Hq, G, d, dv, scale, chunk,      \
                                                               window, k_pitch, v_pitch, dist_bias, bias_len, gate,     \
                                                               gate_ld, gate_heads, out_ld, out_scale, s)))
-    if (nv == 1) TILES(1);
+    if (mma && d == 128) { if (dv == 128) MMA(128, 128); else MMA(128, 64); }
+    else if (mma) { if (dv == 128) MMA(64, 128); else MMA(64, 64); }
+    else if (nv == 1) TILES(1);
     else if (nv == 2) TILES(2);
     else if (nv == 3) TILES(3);
     else TILES(4);
 #undef TILES
+#undef MMA
     if (rc != SXB_OK) return rc;
     SXB_CHECK_LAUNCH();
   }
