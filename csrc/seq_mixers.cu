@@ -965,13 +965,17 @@ channel_decay_gates_kernel(const T* __restrict__ a_raw, long long lda, const T* 
 // ------------------------------------------------------------------------------------------------ recurrence
 // State per (slot, head): dv columns of n floats, stored [dv][n].  Each output column evolves on its own:
 //   s <- a s;  u = b (v_c - [delta] s.k);  s <- s + k u;  o_c = s.q (+ D v_c)
-// A column is held by LPC = 8 lanes (the n-vector as 16-byte chunks, chunk i on lane i mod LPC), 128 / LPC columns per
-// CTA; the CTA walks its sequence's rows in order, staging k and q of TB tokens at a time in shared memory.  (Spreading
+// A column is held by LPC = 8 lanes (the n-vector as 16-byte chunks, chunk i on lane i mod LPC), NC columns per lane,
+// 128 / LPC * NC columns per CTA; the CTA walks its sequence's rows in order, staging k and q of TB tokens at a time in shared memory.  (Spreading
 // a column over a whole warp gives a long sequence four times as many warps, but was measured slower: the work per SM
 // is the same and the longer shuffle trees add instructions.)  The products run as packed pairs (fma.f32x2).
+// What bounds it: with many sequences or heads the words of k and q read from shared memory (halved by NC = 2: 8 sequences,
+// 4096 rows, 32 heads of 128 x 128, 769 us before, 528 now), with few the latency of one token's chain (dot product, three
+// shuffles, update) in the one warp per scheduler.  Taking eight tokens per pass over the state was faster (3 sequences,
+// 2300 rows, 16 heads: 205 us against 277) and is not used: it doubles the rounding error of the read-outs.
 constexpr int kRecThreads = 128, kTB = 8;
 
-template <int R, bool DELTA, int LPC, bool CHAN>
+template <int R, bool DELTA, int LPC, bool CHAN, int NC>
 __global__ void __launch_bounds__(kRecThreads)
 linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict__ qvec, long long ldkq,
                          const float* __restrict__ val, long long ldv, const float* __restrict__ decay,
@@ -984,40 +988,43 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
   // the current ones are walked.  CHAN: the decay is a vector over the key channels (decay [rows, H n]) and follows the
   // scalars as one more [TB][NP] block; the state is multiplied by it chunk by chunk before the delta rule's product.
   // decay_ld 0: the H decays are the same for every row.  beta null: every write strength is one.
-  constexpr int NP = R * LPC, R4 = R / 4, COLS = kRecThreads / LPC;
+  constexpr int NP = R * LPC, R4 = R / 4, COLS = kRecThreads / LPC * NC;
   extern __shared__ __align__(16) float sm[];
   constexpr int stage = (CHAN ? 3 : 2) * kTB * NP + kTB * COLS + 2 * kTB;
   const int* si = seq_info + 4 * blockIdx.z;
   const int first = si[0], rows = si[1], seen = si[2], slot = si[3];
   const int h = blockIdx.y, g = h / (H / G);
   const int lc = threadIdx.x / LPC, l = threadIdx.x % LPC;
-  const int col = blockIdx.x * COLS + lc;
-  const bool live = col < dv;
+  const int col = blockIdx.x * COLS + lc * NC;      // the lane's columns: col .. col + NC - 1
   constexpr int beta0 = 2 * kTB * NP + kTB * COLS + kTB;
   for (int i = threadIdx.x; i < 2 * stage; i += blockDim.x) {                 // the padding stays zero
     const int j = i % stage - beta0;
     sm[i] = (beta == nullptr && j >= 0 && j < kTB) ? 1.f : 0.f;
   }
-  float* sp = state + (((long long)slot * H + h) * dv + (live ? col : 0)) * n;
+  float* sp = state + (((long long)slot * H + h) * dv + col) * n;
   const bool n4 = (n & 3) == 0;
   const bool wide_copy = n4 && (ldkq & 3) == 0 && ((reinterpret_cast<uintptr_t>(kvec) & 15) == 0) &&
                          ((reinterpret_cast<uintptr_t>(qvec) & 15) == 0);
-  float2 S[R / 2];
+  float2 S[NC][R / 2];
 #pragma unroll
-  for (int r4 = 0; r4 < R4; ++r4) {
-    const int i = (r4 * LPC + l) * 4;
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (live && seen > 0) {
-      if (n4 && i < n) {
-        v = *reinterpret_cast<const float4*>(sp + i);
-      } else {
-        if (i < n) v.x = sp[i];
-        if (i + 1 < n) v.y = sp[i + 1];
-        if (i + 2 < n) v.z = sp[i + 2];
-        if (i + 3 < n) v.w = sp[i + 3];
+  for (int c = 0; c < NC; ++c) {
+    const float* sc = sp + (long long)c * n;
+#pragma unroll
+    for (int r4 = 0; r4 < R4; ++r4) {
+      const int i = (r4 * LPC + l) * 4;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (col + c < dv && seen > 0) {
+        if (n4 && i < n) {
+          v = *reinterpret_cast<const float4*>(sc + i);
+        } else {
+          if (i < n) v.x = sc[i];
+          if (i + 1 < n) v.y = sc[i + 1];
+          if (i + 2 < n) v.z = sc[i + 2];
+          if (i + 3 < n) v.w = sc[i + 3];
+        }
       }
+      S[c][2 * r4] = make_float2(v.x, v.y), S[c][2 * r4 + 1] = make_float2(v.z, v.w);
     }
-    S[2 * r4] = make_float2(v.x, v.y), S[2 * r4 + 1] = make_float2(v.z, v.w);
   }
   const float D = skip ? skip[h] : 0.f;
   __syncthreads();
@@ -1045,7 +1052,18 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
         }
       }
     }
-    if (wide_copy) {
+    if (wide_copy && n == NP && kRecThreads % (NP / 4) == 0) {     // a thread copies one chunk of every few rows
+      constexpr int kRows = kRecThreads / (NP / 4) > 0 ? kRecThreads / (NP / 4) : 1;
+      const int c = (threadIdx.x % (NP / 4)) * 4;
+#pragma unroll
+      for (int tt = threadIdx.x / (NP / 4); tt < kTB; tt += kRows) {
+        if (tt < nt) {
+          const long long at = (long long)(first + t0 + tt) * ldkq + g * NP + c;
+          __pipeline_memcpy_async(sk + tt * NP + c, kvec + at, 16);
+          __pipeline_memcpy_async(sq + tt * NP + c, qvec + at, 16);
+        }
+      }
+    } else if (wide_copy) {
       const int nq4 = n >> 2;
       for (int i = threadIdx.x; i < nt * nq4; i += blockDim.x) {
         const int tt = i / nq4, c = (i % nq4) * 4;
@@ -1091,12 +1109,14 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
     // reductions of neighbouring tokens overlap the serial part (the state update, and the dot product before it for
     // the delta rule).
     struct Tok {                      // one token's operands, loaded one token ahead of their use
-      float a, b, v;
+      float a, b, v[NC];
       float4 k[R4], q[R4], g[CHAN ? R4 : 1];
     };
     auto fetch = [&](int tt) {
       Tok t;
-      t.a = CHAN ? 1.f : sa[tt], t.b = sb[tt], t.v = sv[tt * COLS + lc];
+      t.a = CHAN ? 1.f : sa[tt], t.b = sb[tt];
+#pragma unroll
+      for (int c = 0; c < NC; ++c) t.v[c] = sv[tt * COLS + lc * NC + c];
       const float4* kk = reinterpret_cast<const float4*>(sk + tt * NP) + l;
       const float4* qq = reinterpret_cast<const float4*>(sq + tt * NP) + l;
 #pragma unroll
@@ -1108,47 +1128,63 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
       }
       return t;
     };
-    auto step = [&](const Tok& t, float& o_lane) {
-      const float a = t.a, b = t.b, v = t.v;
+    auto step = [&](const Tok& t, float (&o_lane)[NC]) {
+      const float a = t.a, b = t.b;
       const float4* k4 = t.k;
-      float u = b * v;
+      float u[NC];
       if (CHAN) {                      // the decayed state enters the product below: decay first, a stays 1
 #pragma unroll
-        for (int r4 = 0; r4 < R4; ++r4) {
-          S[2 * r4] = __fmul2_rn(S[2 * r4], make_float2(t.g[r4].x, t.g[r4].y));
-          S[2 * r4 + 1] = __fmul2_rn(S[2 * r4 + 1], make_float2(t.g[r4].z, t.g[r4].w));
-        }
+        for (int c = 0; c < NC; ++c)
+#pragma unroll
+          for (int r4 = 0; r4 < R4; ++r4) {
+            S[c][2 * r4] = __fmul2_rn(S[c][2 * r4], make_float2(t.g[r4].x, t.g[r4].y));
+            S[c][2 * r4 + 1] = __fmul2_rn(S[c][2 * r4 + 1], make_float2(t.g[r4].z, t.g[r4].w));
+          }
       }
       if (DELTA) {                     // (a S)^T k = a (S^T k): the decay is folded into the update below
-        float2 d01 = make_float2(0.f, 0.f), d23 = make_float2(0.f, 0.f);
+        float dot[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          float2 d01 = make_float2(0.f, 0.f), d23 = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int r4 = 0; r4 < R4; ++r4) {
+            d01 = __ffma2_rn(S[c][2 * r4], make_float2(k4[r4].x, k4[r4].y), d01);
+            d23 = __ffma2_rn(S[c][2 * r4 + 1], make_float2(k4[r4].z, k4[r4].w), d23);
+          }
+          dot[c] = (d01.x + d01.y) + (d23.x + d23.y);
+        }
+#pragma unroll
+        for (int o = 1; o < LPC; o <<= 1)
+#pragma unroll
+          for (int c = 0; c < NC; ++c) dot[c] += __shfl_xor_sync(0xffffffffu, dot[c], o);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) u[c] = b * (t.v[c] - a * dot[c]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) u[c] = b * t.v[c];
+      }
+      const float2 a2 = make_float2(a, a);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const float2 u2 = make_float2(u[c], u[c]);
+        float2 o01 = make_float2(0.f, 0.f), o23 = make_float2(0.f, 0.f);
 #pragma unroll
         for (int r4 = 0; r4 < R4; ++r4) {
-          d01 = __ffma2_rn(S[2 * r4], make_float2(k4[r4].x, k4[r4].y), d01);
-          d23 = __ffma2_rn(S[2 * r4 + 1], make_float2(k4[r4].z, k4[r4].w), d23);
+          const float4 q4 = t.q[r4];
+          S[c][2 * r4] = __ffma2_rn(make_float2(k4[r4].x, k4[r4].y), u2, CHAN ? S[c][2 * r4] : __fmul2_rn(S[c][2 * r4], a2));
+          S[c][2 * r4 + 1] = __ffma2_rn(make_float2(k4[r4].z, k4[r4].w), u2,
+                                        CHAN ? S[c][2 * r4 + 1] : __fmul2_rn(S[c][2 * r4 + 1], a2));
+          o01 = __ffma2_rn(S[c][2 * r4], make_float2(q4.x, q4.y), o01);
+          o23 = __ffma2_rn(S[c][2 * r4 + 1], make_float2(q4.z, q4.w), o23);
         }
-        float dot = (d01.x + d01.y) + (d23.x + d23.y);
-#pragma unroll
-        for (int o = 1; o < LPC; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        u = b * (v - a * dot);
+        o_lane[c] = (o01.x + o01.y) + (o23.x + o23.y);       // this lane's part of the read-out
       }
-      const float2 a2 = make_float2(a, a), u2 = make_float2(u, u);
-      float2 o01 = make_float2(0.f, 0.f), o23 = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int r4 = 0; r4 < R4; ++r4) {
-        const float4 q4 = t.q[r4];
-        S[2 * r4] = __ffma2_rn(make_float2(k4[r4].x, k4[r4].y), u2, CHAN ? S[2 * r4] : __fmul2_rn(S[2 * r4], a2));
-        S[2 * r4 + 1] = __ffma2_rn(make_float2(k4[r4].z, k4[r4].w), u2,
-                                   CHAN ? S[2 * r4 + 1] : __fmul2_rn(S[2 * r4 + 1], a2));
-        o01 = __ffma2_rn(S[2 * r4], make_float2(q4.x, q4.y), o01);
-        o23 = __ffma2_rn(S[2 * r4 + 1], make_float2(q4.z, q4.w), o23);
-      }
-      o_lane = (o01.x + o01.y) + (o23.x + o23.y);       // this lane's part of the read-out
     };
     if (nt == kTB) {
       // the read-outs of the group are summed over the column's lanes together, off the serial path: TB independent
       // shuffle trees, then lane t of the column writes token t
       static_assert(LPC == kTB, "lane t of a column writes token t of the group");
-      float op[kTB];
+      float op[kTB][NC];
       Tok cur = fetch(0);
 #pragma unroll
       for (int tt = 0; tt < kTB; ++tt) {
@@ -1159,33 +1195,47 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
 #pragma unroll
       for (int x = 1; x < LPC; x <<= 1)
 #pragma unroll
-        for (int tt = 0; tt < kTB; ++tt) op[tt] += __shfl_xor_sync(0xffffffffu, op[tt], x);
-      float mine = op[0];
+        for (int tt = 0; tt < kTB; ++tt)
 #pragma unroll
-      for (int tt = 1; tt < kTB; ++tt) mine = (l == tt) ? op[tt] : mine;
-      if (live) out[(long long)(first + t0 + l) * H * dv + h * dv + col] = mine + D * sv[l * COLS + lc];
+          for (int c = 0; c < NC; ++c) op[tt][c] += __shfl_xor_sync(0xffffffffu, op[tt][c], x);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        float mine = op[0][c];
+#pragma unroll
+        for (int tt = 1; tt < kTB; ++tt) mine = (l == tt) ? op[tt][c] : mine;
+        if (col + c < dv)
+          out[(long long)(first + t0 + l) * H * dv + h * dv + col + c] = mine + D * sv[l * COLS + lc * NC + c];
+      }
     } else {
       for (int tt = 0; tt < nt; ++tt) {
-        float o;
+        float o[NC];
         step(fetch(tt), o);
 #pragma unroll
-        for (int x = 1; x < LPC; x <<= 1) o += __shfl_xor_sync(0xffffffffu, o, x);
-        if (live && l == 0) out[(long long)(first + t0 + tt) * H * dv + h * dv + col] = o + D * sv[tt * COLS + lc];
+        for (int x = 1; x < LPC; x <<= 1)
+#pragma unroll
+          for (int c = 0; c < NC; ++c) o[c] += __shfl_xor_sync(0xffffffffu, o[c], x);
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          if (col + c < dv && l == 0)
+            out[(long long)(first + t0 + tt) * H * dv + h * dv + col + c] = o[c] + D * sv[tt * COLS + lc * NC + c];
       }
     }
     __syncthreads();          // the buffer just walked is the target of the next iteration's copies
   }
-  if (live) {
+#pragma unroll
+  for (int c = 0; c < NC; ++c) {
+    if (col + c >= dv) continue;
+    float* sc = sp + (long long)c * n;
 #pragma unroll
     for (int r4 = 0; r4 < R4; ++r4) {
       const int i = (r4 * LPC + l) * 4;
       if (n4 && i < n) {
-        *reinterpret_cast<float4*>(sp + i) = make_float4(S[2 * r4].x, S[2 * r4].y, S[2 * r4 + 1].x, S[2 * r4 + 1].y);
+        *reinterpret_cast<float4*>(sc + i) = make_float4(S[c][2 * r4].x, S[c][2 * r4].y, S[c][2 * r4 + 1].x, S[c][2 * r4 + 1].y);
       } else {
-        if (i < n) sp[i] = S[2 * r4].x;
-        if (i + 1 < n) sp[i + 1] = S[2 * r4].y;
-        if (i + 2 < n) sp[i + 2] = S[2 * r4 + 1].x;
-        if (i + 3 < n) sp[i + 3] = S[2 * r4 + 1].y;
+        if (i < n) sc[i] = S[c][2 * r4].x;
+        if (i + 1 < n) sc[i + 1] = S[c][2 * r4].y;
+        if (i + 2 < n) sc[i + 2] = S[c][2 * r4 + 1].x;
+        if (i + 3 < n) sc[i + 3] = S[c][2 * r4 + 1].y;
       }
     }
   }
@@ -2052,23 +2102,28 @@ SXB_API int sxb_linear_recurrence(const void* kvec, const void* qvec, long long 
   if (n > 256 || H % G) return SXB_ERR_UNSUPPORTED;
   if (decay_channels && fixed_decay) return SXB_ERR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-#define LAUNCH_REC(R, D, LPC, CH)                                                                                   \
+#define LAUNCH_REC(R, D, LPC, CH, NC)                                                                               \
   do {                                                                                                              \
-    constexpr int cols = kRecThreads / LPC;                                                                         \
+    constexpr int cols = kRecThreads / LPC * NC;                                                                    \
     const size_t smem = (size_t)2 * ((CH ? 3 : 2) * kTB * (R * LPC) + kTB * cols + 2 * kTB) * sizeof(float);        \
     if (smem > 48 * 1024)                                                                                           \
-      cudaFuncSetAttribute(linear_recurrence_kernel<R, D, LPC, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
+      cudaFuncSetAttribute(linear_recurrence_kernel<R, D, LPC, CH, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
                            (int)smem);                                                                              \
-    linear_recurrence_kernel<R, D, LPC, CH><<<dim3((dv + cols - 1) / cols, H, n_seqs), kRecThreads, smem, s>>>(     \
+    linear_recurrence_kernel<R, D, LPC, CH, NC><<<dim3((dv + cols - 1) / cols, H, n_seqs), kRecThreads, smem, s>>>(     \
         (const float*)kvec, (const float*)qvec, ldkq, (const float*)val, ldv, (const float*)decay,                  \
         (const float*)beta, (const float*)skip, (float*)state, (float*)out, (const int*)seq_info, H, G, n, dv,      \
         fixed_decay ? 0 : H);                                                                                       \
   } while (0)
 #define LAUNCH_REC_N(D, CH)                                  \
-  if (n <= 32) LAUNCH_REC(4, D, 8, CH);                      \
-  else if (n <= 64) LAUNCH_REC(8, D, 8, CH);                 \
-  else if (n <= 128) LAUNCH_REC(16, D, 8, CH);               \
-  else LAUNCH_REC(32, D, 8, CH)
+  if (n <= 32) LAUNCH_REC(4, D, 8, CH, 1);                   \
+  else if (n <= 64) { if (two) LAUNCH_REC(8, D, 8, CH, 2); else LAUNCH_REC(8, D, 8, CH, 1); }    \
+  else if (n <= 128) { if (two) LAUNCH_REC(16, D, 8, CH, 2); else LAUNCH_REC(16, D, 8, CH, 1); } \
+  else LAUNCH_REC(32, D, 8, CH, 1)
+  // Two columns per lane share every k and q word that is read from shared memory (and every copy into it); with one column
+  // the chip has twice the warps.  Two win once one column would fill the chip one and a half times (us, one | two columns:
+  // delta rule, 8 sequences, 4096 rows, 32 heads 746 | 528; 3, 2300, 16: 303 | 277; 1, 2000, 32: 512 | 440; 64 decode rows, 16
+  // heads 36 | 26), below that one does (1, 4096, 16: 833 | 892).  Every column's sums are taken in the same order either way.
+  const bool two = (long long)((dv + 15) / 16) * H * n_seqs >= 222;
   if (decay_channels) {
     if (delta) { LAUNCH_REC_N(true, true); } else { LAUNCH_REC_N(false, true); }
   } else {
