@@ -24,6 +24,7 @@
 //   sigmoid_gate_rows, power_norm_act   sigmoid gate per channel or per head in place; p1 z/rms(z) + p2 z^2/rms(z^2) + p3 z^3/rms(z^3) + p0
 #include <algorithm>
 #include "seq_common.cuh"
+#include "mma_sync.cuh"
 #include <cuda_pipeline.h>
 
 namespace sxb {
@@ -380,8 +381,8 @@ constexpr int kBQ = 64, kBK = 64;    // query rows / keys per tile of the tiled 
 // one 64-key tile of K and V (converted to fp32) and the tile's weights (in the key tile's place, once the scores are
 // done: head sizes up to 128 then leave room for two CTAs per SM) sit in shared memory; 256 threads hold 4x4
 // scores and 4 x (dv/16) outputs each.  Scores, online softmax with the sink logit, and the weighted sum are fp32 FMAs:
-// the weights must stay 32-bit, so the products cannot go through the bf16 tensor path as they are (sink_attention_mma.cuh splits them; this form serves
-// fp32 caches and other head sizes).
+// the weights must stay 32-bit, so the products cannot go through the bf16 tensor path as they are (sink_attention_mma.cuh
+// splits them; this form serves fp32 caches and other head sizes).
 template <typename T, int NV>
 __global__ void __launch_bounds__(256, NV <= 2 ? 2 : 1)
 sink_attention_tile_kernel(const float* __restrict__ q, const T* __restrict__ kcache, const T* __restrict__ vcache,

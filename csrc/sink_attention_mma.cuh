@@ -14,19 +14,6 @@
 // the error against 64 bits is that of the 16-bit result (1.7e-3) before and after.
 #pragma once
 
-__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t saddr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr) : "memory");
-}
-__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t saddr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(saddr) : "memory");
-}
-__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
 // Two fp32 numbers as three packed bf16 pairs whose sum is exact (INF: infinities may occur and keep zero rests).
 template <bool INF>
 __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
@@ -40,10 +27,6 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t&
   lo = __byte_perm(__float_as_uint(rx - __uint_as_float(vx & 0xffff0000u)),
                    __float_as_uint(ry - __uint_as_float(vy & 0xffff0000u)), 0x7632);
 }
-// Byte offset of 16-byte chunk `c` of row `r` in a tile of `row_bytes`: the eight rows of a matrix fragment fall on
-// different banks.
-__device__ __forceinline__ uint32_t tile_at(int r, int c, int row_bytes) { return r * row_bytes + ((c ^ (r & 7)) << 4); }
-
 constexpr int kSmQ = 128, kSmThreads = 256;                    // query rows (a whole atom) and threads of a CTA
 
 template <int D, int DV>

@@ -594,6 +594,14 @@ int sxb_lru_scan(const void* a, const void* g, const void* y, long long ldy, con
                  long long ldx, void* state, void* conv_state, const void* seq_info, void* out, long long out_ld,
                  int n_seqs, int N, int keep, float scale, int single_rows, int dtype, void* stream);
 
+/* ---- csrc/attention.cu */
+/* The same with the LAST n_few atoms holding at most 16 / (Hq / Hk) queries each (decode tokens): those run the warp-level
+ * kernel of attention_decode.cu, beside the other atoms' kernel when there are any.  n_packed counts atoms before them. */
+int sxb_attn_fwd_atoms_few(const void* q, const void* cache, void* out, const void* atoms, int n_atoms,
+                           int n_packed, int n_few, const void* block_tables, int max_blocks, int n_blocks,
+                           int block_size, int T, int Hq, int Hk, int D, long long q_stride, long long o_stride,
+                           float scale, void* stream);
+
 #ifdef __cplusplus
 }
 #endif
