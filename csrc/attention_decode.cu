@@ -6,8 +6,9 @@
 // cluster of up to 8 CTAs; partial (maximum, sum, output) are merged in fp32, warps through shared memory, CTAs through
 // distributed shared memory in rank order.
 // What bounds it: the bytes of K and V (two CTAs per SM hold 128 KB of them in flight).  The 128-row tile kernel that served
-// these tokens spent a 128 x 64 MMA and a 64-wide softmax row on four valid rows and gave a sequence one CTA per head:
-// XXMEAS
+// these tokens spent a 128 x 64 MMA and a 64-wide softmax row on four valid rows and gave a sequence one CTA per head: 61
+// requests around 2000 tokens, 32 / 8 heads of 128: 132 us, 104 now (floor 78); 128 of 4000: 323 (floor 319); a few short
+// requests 62 -> 19.
 #include "mma_sync.cuh"
 #include <cuda_pipeline.h>
 
@@ -276,9 +277,10 @@ int paged_decode(const void* q, const void* cache, void* out, const void* atoms,
   p.max_blocks = max_blocks; p.block_size = block_size; p.Hk = Hk; p.group = Hq / Hk;
   p.shift = (block_size & (block_size - 1)) == 0 ? __builtin_ctz(block_size) : -1;
   p.q_stride = q_stride; p.o_stride = o_stride; p.scale = scale; p.after = beside ? 1 : 0;
-  // enough CTAs for two waves of two per SM: contexts differ, and a sequence's CTAs end with its context
+  // enough CTAs for four waves of two per SM: contexts differ, and a sequence's CTAs end with its context (61 requests: 109
+  // us with two waves, 104 with four, 117 with eight, where starting and merging a CTA costs more than the balance gives)
   int S = 8;
-  while (S > 1 && (long long)Hk * n_atoms * S > 4LL * sms) S >>= 1;
+  while (S > 1 && (long long)Hk * n_atoms * S > 8LL * sms) S >>= 1;
   return D == 128 ? decode::launch<128>(p, n_atoms, S, beside, stream) : decode::launch<64>(p, n_atoms, S, beside, stream);
 }
 

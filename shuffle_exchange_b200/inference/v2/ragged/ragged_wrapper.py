@@ -95,10 +95,10 @@ class RaggedBatchWrapper:
             from ..kernels.atom_builder import AtomBuilder
             start, rows, seen = (torch.from_numpy(m[: self._n_seqs]) for m in self._seq_meta)
             _, self._n_atoms = AtomBuilder()(self._host_views[self._turn][5], start, rows, seen, ATOM_Q_BLOCK, ATOM_KV_BLOCK)
-            # longest first: the kernel runs the short tail (decode tokens, chunk remainders) with the GQA group packed
-            # into one tile, and needs those atoms contiguous
+            # longest first: the kernels take the short tail (decode tokens, chunk remainders) on its own and need those
+            # atoms contiguous; among equals the one with most keys first, so that light ones end the grid
             live = self._tables[self._turn][5][: self._n_atoms]
-            live[:] = live[np.argsort(-live[:, 2], kind="stable")]
+            live[:] = live[np.lexsort((-live[:, 5], -live[:, 2]))]
             self._atom_q_lens = live[:, 2].copy()
         self._live = {}
         self._dev.copy_(self._host, non_blocking=True)
