@@ -316,6 +316,22 @@ scale_cast_kernel(const TS* __restrict__ src, TD* __restrict__ dst, long long n,
   }
 }
 
+// x *= *scale (rounded to the type of x first), nothing when it is one: the gradient of a loss that nobody has scaled costs a
+// launch instead of a pass over the logits' gradient.
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+scale_by_kernel(T* __restrict__ x, long long n8, const float* __restrict__ scale) {
+  const float f = to_f32<T>(from_f32<T>(*scale));
+  if (f == 1.f) return;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (long long)gridDim.x * blockDim.x) {
+    float v[8];
+    ld8<T>(x + i * 8, v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] *= f;
+    st8<T>(x + i * 8, v);
+  }
+}
+
 static inline int grid_for(long long work) {
   long long b = (work + kThreads - 1) / kThreads;
   if (b < 1) b = 1;
@@ -404,6 +420,16 @@ SXB_API int sxb_cross_entropy(void* logits, const void* labels, void* loss, void
   DISPATCH_16(dtype, (xent_kernel<T><<<(unsigned)rows, threads, 0, s>>>(
                          (T*)logits, (const long long*)labels, (float*)loss, (float*)lse, V, ld,
                          ignore_index, (const float*)grad_scale, write_grad)));
+  SXB_CHECK_LAUNCH();
+  return SXB_OK;
+}
+
+// x [n] (16-bit, n a multiple of 8, 16-byte aligned) *= *scale (fp32 on the device), in place.
+SXB_API int sxb_scale_by(void* x, long long n, const void* scale, int dtype, void* stream) {
+  if (n <= 0) return SXB_OK;
+  if (n % 8 || (reinterpret_cast<uintptr_t>(x) & 15)) return SXB_ERR_UNSUPPORTED;
+  cudaStream_t s = (cudaStream_t)stream;
+  DISPATCH_16(dtype, (scale_by_kernel<T><<<grid_for(n / 8), kThreads, 0, s>>>((T*)x, n / 8, (const float*)scale)));
   SXB_CHECK_LAUNCH();
   return SXB_OK;
 }

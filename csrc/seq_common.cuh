@@ -76,17 +76,5 @@ __device__ __forceinline__ void store8_f32<__nv_bfloat16>(__nv_bfloat16* p, cons
       make_uint4(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), pack_bf16(o[4], o[5]), pack_bf16(o[6], o[7]));
 }
 
-// Sums of two numbers over the block, both at once (blockDim.x <= 1024 and a multiple of 32).
-__device__ __forceinline__ float2 block_sum2(float a, float b, float2* smem /* >= 32 */) {
-  a = warp_sum(a), b = warp_sum(b);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) smem[w] = make_float2(a, b);
-  __syncthreads();
-  const int nw = (blockDim.x + 31) >> 5;
-  const float2 r = (l < nw) ? smem[l] : make_float2(0.f, 0.f);
-  return make_float2(warp_sum(r.x), warp_sum(r.y));
-}
-
 }  // namespace seqmix
 }  // namespace sxb

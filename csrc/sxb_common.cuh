@@ -423,6 +423,18 @@ __device__ __forceinline__ float block_max(float v, float* smem) {
   return r;
 }
 
+// Sums of two numbers over the block, both at once (blockDim.x <= 1024 and a multiple of 32).
+__device__ __forceinline__ float2 block_sum2(float a, float b, float2* smem /* >= 32 */) {
+  a = warp_sum(a), b = warp_sum(b);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  __syncthreads();
+  if (l == 0) smem[w] = make_float2(a, b);
+  __syncthreads();
+  const int nw = (blockDim.x + 31) >> 5;
+  const float2 r = (l < nw) ? smem[l] : make_float2(0.f, 0.f);
+  return make_float2(warp_sum(r.x), warp_sum(r.y));
+}
+
 template <typename T>
 __device__ __forceinline__ float to_f32(T v);
 template <>

@@ -602,6 +602,10 @@ int sxb_attn_fwd_atoms_few(const void* q, const void* cache, void* out, const vo
                            int block_size, int T, int Hq, int Hk, int D, long long q_stride, long long o_stride,
                            float scale, void* stream);
 
+/* ---- csrc/elementwise.cu */
+/* x [n] (16-bit, n a multiple of 8, 16-byte aligned) *= *scale (fp32 on the device), in place. */
+int sxb_scale_by(void* x, long long n, const void* scale, int dtype, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

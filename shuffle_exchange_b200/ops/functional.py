@@ -578,7 +578,11 @@ class _CrossEntropy(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss):
         (g,) = ctx.saved_tensors
-        g.mul_(dloss.to(g.dtype))  # in place: the saved buffer is the (consumed) logits tensor
+        # in place: the saved buffer is the (consumed) logits tensor
+        if dloss.dtype == torch.float32 and dloss.device == g.device and g.is_contiguous() and _n.no_tape(dloss, g):
+            _n.call("sxb_scale_by", g.data_ptr(), g.numel(), dloss.data_ptr(), _n.dtype_code(g.dtype), _n.stream_ptr())
+        else:
+            g.mul_(dloss.to(g.dtype))
         return g.view(ctx.shape), None, None
 
 
