@@ -126,6 +126,47 @@ gated_fwd_kernel(const T* __restrict__ in, const T* __restrict__ bias, T* __rest
     st8<T>(out + r * F + c, o);
   }
 }
+// The same for the routed rows of an expert layer only: group g of `in` / `out` starts at row offsets[g] and holds counts[g]
+// routed rows, the rest of its (256-row aligned) room is padding that nothing reads.  blockIdx.x counts the routed rows of
+// all groups; rows behind them are left as they are.
+template <typename T>
+__global__ void __launch_bounds__(kThreads)
+gated_groups_kernel(const T* __restrict__ in, T* __restrict__ out, const int* __restrict__ offsets,
+                    const int* __restrict__ counts, int groups, int F, int act) {
+  __shared__ int row_s;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x, i = blockIdx.x;
+    int base = 0, row = -1;
+    for (int g0 = 0; g0 < groups; g0 += 32) {
+      const int own = g0 + lane < groups ? counts[g0 + lane] : 0;
+      int incl = own;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      const unsigned hit = __ballot_sync(0xffffffffu, base + incl > i);
+      if (hit) {
+        const int src = __ffs(hit) - 1;
+        row = offsets[g0 + src] + i - base - (__shfl_sync(0xffffffffu, incl, src) - __shfl_sync(0xffffffffu, own, src));
+        break;
+      }
+      base += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) row_s = row;
+  }
+  __syncthreads();
+  const long long r = row_s;
+  if (r < 0) return;
+  for (int c = (blockIdx.y * kThreads + threadIdx.x) * 8; c < F; c += gridDim.y * kThreads * 8) {
+    float g[8], u[8], o[8];
+    ld8<T>(in + r * 2 * F + c, g);
+    ld8<T>(in + r * 2 * F + F + c, u);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) o[k] = act_fwd(g[k], act) * u[k];
+    st8<T>(out + r * F + c, o);
+  }
+}
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 gated_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ in, T* __restrict__ din,
@@ -375,6 +416,20 @@ SXB_API int sxb_gated_act_fwd(const void* in, const void* bias, void* out, long 
   cudaStream_t s = (cudaStream_t)stream;
   DISPATCH_16(dtype, (gated_fwd_kernel<T><<<grid_for(rows * (F / 8)), kThreads, 0, s>>>(
                          (const T*)in, (const T*)bias, (T*)out, rows, F, act)));
+  SXB_CHECK_LAUNCH();
+  return SXB_OK;
+}
+// act(gate) * up for the routed rows of grouped expert rows: in [capacity, 2F], out [capacity, F]; offsets / counts int32
+// [groups] (first row and routed rows of every group); n_rows = sum of the counts.  Other rows of out are not written.
+SXB_API int sxb_gated_act_groups(const void* in, void* out, const void* offsets, const void* counts, int groups, int n_rows,
+                                 int F, int act, int dtype, void* stream) {
+  if (n_rows <= 0 || groups <= 0) return SXB_OK;
+  if (F % 8) return SXB_ERR_UNSUPPORTED;
+  cudaStream_t s = (cudaStream_t)stream;
+  const int parts = (F / 8 + kThreads - 1) / kThreads;        // a word per thread while the rows are few
+  const dim3 grid(n_rows, n_rows >= 148 * 16 ? 1 : parts);
+  DISPATCH_16(dtype, (gated_groups_kernel<T><<<grid, kThreads, 0, s>>>((const T*)in, (T*)out, (const int*)offsets,
+                                                                     (const int*)counts, groups, F, act)));
   SXB_CHECK_LAUNCH();
   return SXB_OK;
 }

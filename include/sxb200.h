@@ -606,6 +606,12 @@ int sxb_attn_fwd_atoms_few(const void* q, const void* cache, void* out, const vo
 /* x [n] (16-bit, n a multiple of 8, 16-byte aligned) *= *scale (fp32 on the device), in place. */
 int sxb_scale_by(void* x, long long n, const void* scale, int dtype, void* stream);
 
+/* ---- csrc/elementwise.cu */
+/* act(gate) * up for the routed rows of grouped expert rows: in [capacity, 2F], out [capacity, F]; offsets / counts int32
+ * [groups] (first row and routed rows of every group); n_rows = sum of the counts.  Other rows of out are not written. */
+int sxb_gated_act_groups(const void* in, void* out, const void* offsets, const void* counts, int groups,
+                         int n_rows, int F, int act, int dtype, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

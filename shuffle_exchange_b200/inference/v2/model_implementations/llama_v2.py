@@ -60,7 +60,7 @@ class RaggedLlamaModel:
         from ....moe import fused_ep
         if fused_ep.grouped_inference_ok(x, moe["w_gate_up"], moe["w_down"]):
             return fused_ep.grouped_experts_inference(x, scores, assign, offsets, counts, moe["w_gate_up"],
-                                                      moe["w_down"], F.swiglu, self.top_k)
+                                                      moe["w_down"], F.swiglu, self.top_k, gate_act="silu")
         moe_in, cumsum, slots = moe_ops.moe_scatter(x, assign, offsets, counts)
         ends = cumsum.tolist()
         out = torch.empty_like(moe_in)

@@ -347,7 +347,9 @@ class DSMultiGemmMoE(DSMoEBase):
             self._output = fused_ep.grouped_experts_inference(
                 hidden_states, scores, assign, offsets, counts, mlp_1_w, mlp_2_w,
                 lambda t: _apply_activation(t, None, c.activation, c.activation_limit), c.top_k,
-                weight_input=c.weight_input, n_identity=n_id)
+                weight_input=c.weight_input, n_identity=n_id,
+                gate_act=_act_name(c.activation) if is_gated(c.activation)
+                and ActivationType(c.activation) != ActivationType.CLAMPED_SWIGLU else None)
             return self._output
         if c.weight_input:
             moe_in, cumsum, slots = moe_ops.moe_scatter_scaled(hidden_states, scores, assign, offsets, counts)

@@ -39,6 +39,7 @@ _n.register({
     "sxb_moe_ep_push": "ppii" "pppp" "ppp" "iiiii" "i" "i" "pi" "p",
     "sxb_moe_ep_pull": "ppii" "ppp" "ppp" "iiiii" "i" "i" "pi" "p",
     "sxb_moe_ep_hang_info": "p",
+    "sxb_gated_act_groups": "pppp" "iiiii" "p",
 })
 
 CH_PLAN, CH_LANDED, CH_READY, CH_PULLED = 8, 9, 10, 11
@@ -238,11 +239,13 @@ def make_plan(ep: FusedEP, counts, assign, offsets) -> EPPlan:
 
 @torch.no_grad()
 def grouped_experts_inference(x, scores, assign, offsets, counts, w1, w2, activation, top_k: int,
-                              weight_input: bool = False, n_identity: int = 0):
+                              weight_input: bool = False, n_identity: int = 0, gate_act=None):
     """Inference MoE body without a host synchronisation: expert-contiguous rows through the plan / push kernels (one
     rank: every "peer" access is local), ONE grouped GEMM per projection over the 256-aligned groups, weighted
     un-permute through the pull kernel.  ``w1`` ``[E, N1, H]``, ``w2`` ``[E, H, F]`` (stacked expert weights),
-    ``activation``: callable on the first projection's output (e.g. SwiGLU).  ``weight_input``: the routing weight
+    ``activation``: callable on the first projection's output (e.g. SwiGLU); ``gate_act``: its name ("silu", "gelu", "relu")
+    where it is ``act(gate) * up`` of the two halves -- it then runs on the routed rows only, not on the capacity and its
+    alignment padding (200 tokens, 8 experts of 14336: 74 us before, 12 now).  ``weight_input``: the routing weight
     scales the rows on their way INTO the experts (the push kernel multiplies) and the outputs are summed unweighted.
     ``n_identity``: the assignments run over ``E + n_identity`` experts of which the last ``n_identity`` have no weights
     and return their input: their row groups skip both products and are copied from the receive to the return buffer.
@@ -255,7 +258,15 @@ def grouped_experts_inference(x, scores, assign, offsets, counts, w1, w2, activa
     plan = make_plan(ep, counts, assign, offsets)
     wts = scores.to(torch.float32).contiguous()
     ep.push(x.contiguous(), plan, weights=wts if weight_input else None)
-    h = activation(grouped_gemm_nt(ep.recv_rows, w1, plan.group_offsets))
+    h = grouped_gemm_nt(ep.recv_rows, w1, plan.group_offsets)
+    if gate_act is not None and h.shape[1] % 16 == 0:
+        from ..ops.functional import _act_code
+        a = h.new_empty((h.shape[0], h.shape[1] // 2))
+        _n.call("sxb_gated_act_groups", h.data_ptr(), a.data_ptr(), plan.group_offsets.data_ptr(), counts.data_ptr(), E,
+                T * top_k, a.shape[1], _act_code(gate_act), _n.dtype_code(h.dtype), _n.stream_ptr())
+        h = a
+    else:
+        h = activation(h)
     grouped_gemm_nt(h, w2, plan.group_offsets, out=ep.ret_rows)
     if n_identity > 0:
         from ..ops.moe_ops import copy_group_rows_

@@ -1,8 +1,10 @@
-"""The scaled gradient of the loss and norm backward with its partial sums in registers: sizes at the edges of their blocks,
-against 64-bit references."""
+"""The scaled gradient of the loss, norm backward with its partial sums in registers, and the routed rows' activation: sizes
+at the edges of their blocks, against 64-bit references."""
 import pytest
 import torch
 
+from shuffle_exchange_b200.moe import fused_ep  # noqa: F401  (declares the routed rows' entry point)
+from shuffle_exchange_b200.native import lib
 from shuffle_exchange_b200.ops import functional as F
 
 pytestmark = pytest.mark.gpu
@@ -55,3 +57,22 @@ def test_norm_backward(rows, H, layer):
     torch.autograd.backward([yd, hd], [dy.double(), dh.double()])
     for a, c in zip(ins[: 4 if layer else 3], ref):
         assert float((a.grad.double() - c.grad).norm() / c.grad.norm()) < 4e-3          # one rounding to 16 bits (1.7e-3)
+
+
+@pytest.mark.parametrize("counts", [[3, 0, 5], [0, 0, 1], [1] * 40, [300, 2]])
+@pytest.mark.parametrize("width", [16, 2056, 4096])
+def test_routed_rows_activation(counts, width):
+    offs, at = [], 0
+    for c in counts:
+        offs.append(at)
+        at += (c + 255) // 256 * 256
+    x = torch.randn(max(at, 256), 2 * width, device="cuda").bfloat16()
+    out = torch.full((x.shape[0], width), 5.0, device="cuda", dtype=torch.bfloat16)
+    o, c = (torch.tensor(t, dtype=torch.int32, device="cuda") for t in (offs, counts))
+    lib.call("sxb_gated_act_groups", x.data_ptr(), out.data_ptr(), o.data_ptr(), c.data_ptr(), len(counts), sum(counts) + 2, width,
+             3, lib.dtype_code(x.dtype), lib.stream_ptr())
+    want = F.swiglu(x)
+    used = torch.zeros(x.shape[0], dtype=torch.bool, device="cuda")
+    for a, n in zip(offs, counts):
+        used[a: a + n] = True
+    assert torch.equal(out[used], want[used]) and bool((out[~used] == 5.0).all())
