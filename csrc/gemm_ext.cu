@@ -57,6 +57,7 @@ struct XParams {
   // ---- groups
   int group_mode, num_groups;
   const int* offsets;  // device, num_groups + 1 row offsets
+  const int* used;     // USED kernels: rows in use at the start of every group (the rest of its room is padding)
   int b_group_rows;    // rows of one group's matrix inside the stacked B tensor map
   long long c_group_stride;  // ragged-K: elements between the C matrices of consecutive groups
   // ---- fp8 scales (may be null)
@@ -188,7 +189,11 @@ __device__ __forceinline__ void umma_f8_pair(uint32_t d_tmem, uint64_t a_desc, u
       : "memory");
 }
 
-template <bool FP8>
+// USED (ragged-M, NT): only the rows in use of a group's last tile are loaded (in boxes of 64) and stored.  Experts that serve a
+// decode batch hold a few dozen rows in a 256-row tile; with the whole tile every weight byte came with as many bytes of
+// padding through L2, and the padding's results went to memory (200 tokens, 8 experts of 4096 x 14336, both projections: 538 us
+// before, 523 now, 430 for the weights at copy speed; what is left is the reading itself and the last wave of tiles).
+template <bool FP8, bool USED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_pair_x_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    const __grid_constant__ CUtensorMap tmC, const XParams p) {
@@ -257,6 +262,12 @@ gemm_pair_x_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       const int m0 = ti.m0 + int(cta) * 128;   // this CTA's 128 rows of A
       const int nb = ti.n0 + int(cta) * 128;   // this CTA's 128 rows/columns of B
       const int b_goff = (p.group_mode == kRaggedM) ? ti.g * p.b_group_rows : 0;
+      int boxes = 2, boxes_pair = 4;           // 64-row boxes of A in use: this CTA's, both CTAs'
+      if (USED) {
+        const int n = min(p.used[ti.g] - (ti.m0 - p.offsets[ti.g]), 256);
+        boxes_pair = max(0, (n + 63) / 64);
+        boxes = min(max(boxes_pair - 2 * (int)cta, 0), 2);
+      }
       for (int kb = 0; kb < ti.num_kb; ++kb) {
         const int k0 = kb * BKE;
         if (gate_on && (b_mn || kb == 0)) {
@@ -285,8 +296,11 @@ gemm_pair_x_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         if (elected) {
           uint8_t* sa = smem + stage * Plan::kStage;
           uint8_t* sb = sa + Plan::kA;
-          if (leader) mbar_expect_tx(&full_bar[stage], 2 * Plan::kStage);
-          if (!a_mn) {
+          if (leader) mbar_expect_tx(&full_bar[stage], USED ? 2 * Plan::kB + boxes_pair * (64 * 128) : 2 * Plan::kStage);
+          if (USED) {
+            if (boxes > 0) tma_load_2d_pair(sa, &tmA, &full_bar[stage], k0, m0);
+            if (boxes > 1) tma_load_2d_pair(sa + 64 * 128, &tmA, &full_bar[stage], k0, m0 + 64);
+          } else if (!a_mn) {
             tma_load_2d_pair(sa, &tmA, &full_bar[stage], k0, m0);
           } else {
             const int kr = ti.k_row0 + k0;
@@ -397,6 +411,17 @@ gemm_pair_x_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
       }
       if (!mbar_wait_to(&tfull_bar[acc], acc_phase, 44, t)) goto done;
       tc_fence_after();
+      const int mine = USED ? p.used[ti.g] - (m0 - p.offsets[ti.g]) : 128;      // rows in use of this CTA's 128
+      if (USED && mine <= 0) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_leader(&tempty_bar[acc]);
+        if (++acc == 2) {
+          acc = 0;
+          acc_phase ^= 1;
+        }
+        continue;
+      }
       float sa = 1.f;
       if (FP8 && p.scale_a != nullptr && gr < m_end) sa = p.scale_a[gr];
       const float* sbp = (FP8 && p.scale_b != nullptr) ? p.scale_b + (long long)ti.g * p.scale_b_group_stride : nullptr;
@@ -441,6 +466,7 @@ gemm_pair_x_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
           asm volatile("bar.sync 1, 128;" ::: "memory");
           if (et == 0) {
             if (half_valid && gc0 < p.N) tma_store_2d(&tmC, stage_c + buf * kStageC, gc0, c_row_tma);
+            if (USED && mine > 64 && gc0 < p.N) tma_store_2d(&tmC, stage_c + buf * kStageC + 64 * 128, gc0, c_row_tma + 64);
             tma_store_commit();
           }
           buf ^= 1;
@@ -620,7 +646,7 @@ SXB_API int sxb_gemm_ext(const void* A, const void* B, void* C, int M, int N, in
     tc = ta;
   }
   static bool configured[2] = {false, false};
-  const void* kfn = fp8 ? (const void*)gemm_pair_x_kernel<true> : (const void*)gemm_pair_x_kernel<false>;
+  const void* kfn = fp8 ? (const void*)gemm_pair_x_kernel<true, false> : (const void*)gemm_pair_x_kernel<false, false>;
   if (!configured[fp8 ? 1 : 0]) {
     cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, Plan::kTotal);
     if (e != cudaSuccess) return (int)e;
@@ -634,8 +660,40 @@ SXB_API int sxb_gemm_ext(const void* A, const void* B, void* C, int M, int N, in
   }
   if (grid < 2) grid = 2;
   cudaStream_t s = (cudaStream_t)stream;
-  if (fp8) gemm_pair_x_kernel<true><<<grid, kThreads, Plan::kTotal, s>>>(ta, tb, tc, p);
-  else gemm_pair_x_kernel<false><<<grid, kThreads, Plan::kTotal, s>>>(ta, tb, tc, p);
+  if (fp8) gemm_pair_x_kernel<true, false><<<grid, kThreads, Plan::kTotal, s>>>(ta, tb, tc, p);
+  else gemm_pair_x_kernel<false, false><<<grid, kThreads, Plan::kTotal, s>>>(ta, tb, tc, p);
+  SXB_CHECK_LAUNCH();
+  return SXB_OK;
+}
+
+// Ragged-M NT product in bf16 whose groups use only their first counts[g] rows (device, int32): rows behind them are neither
+// read nor defined in C.  A, C [total_rows, K | N] with row pitches lda, ldc; B [num_groups * N, K]; offsets as above.
+SXB_API int sxb_gemm_grouped_used(const void* A, const void* B, void* C, int N, int K, long long lda, long long ldb,
+                                  long long ldc, int num_groups, const void* offsets, const void* counts,
+                                  long long total_rows, void* stream) {
+  if (offsets == nullptr || counts == nullptr || num_groups < 1 || total_rows <= 0) return SXB_ERR_BAD_ARG;
+  if (N <= 0 || K <= 0) return SXB_OK;
+  if ((lda % 8) || (ldb % 8) || (ldc % 8) ||
+      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15))
+    return SXB_ERR_UNSUPPORTED;
+  XParams p{};
+  p.N = N; p.K = K; p.layout = NT; p.c_dtype = kBF16; p.C = C; p.ldc = (int)ldc; p.alpha = 1.f; p.ldb_bytes = ldb * 2;
+  p.group_mode = kRaggedM; p.num_groups = num_groups; p.offsets = (const int*)offsets; p.used = (const int*)counts;
+  p.scale_b_group_stride = N; p.b_group_rows = N; p.b_rows = N;
+  CUtensorMap ta, tb, tc;
+  int rc;
+  if ((rc = make_map(&ta, A, total_rows, K, lda, 64, 2))) return rc;
+  if ((rc = make_map(&tb, B, (unsigned long long)num_groups * N, K, ldb, 128, 2))) return rc;
+  if ((rc = make_map(&tc, C, total_rows, N, ldc, 64, 2))) return rc;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_pair_x_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         Plan::kTotal);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  const int grid = num_sms() & ~1;
+  gemm_pair_x_kernel<false, true><<<grid < 2 ? 2 : grid, kThreads, Plan::kTotal, (cudaStream_t)stream>>>(ta, tb, tc, p);
   SXB_CHECK_LAUNCH();
   return SXB_OK;
 }
@@ -668,7 +726,7 @@ SXB_API int sxb_gemm_scatter(const void* A, const void* B, int M, int N, int K, 
   if ((rc = make_map(&tb, B, b_rows, b_cols, ldb, (layout == NT) ? 128 : 64, 2))) return rc;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_pair_x_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_pair_x_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          Plan::kTotal);
     if (e != cudaSuccess) return (int)e;
     configured = true;
@@ -678,7 +736,7 @@ SXB_API int sxb_gemm_scatter(const void* A, const void* B, int M, int N, int K, 
   const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
   if (2 * tiles < grid) grid = (int)(2 * tiles);
   if (grid < 2) grid = 2;
-  gemm_pair_x_kernel<false><<<grid, kThreads, Plan::kTotal, (cudaStream_t)stream>>>(ta, tb, ta, p);
+  gemm_pair_x_kernel<false, false><<<grid, kThreads, Plan::kTotal, (cudaStream_t)stream>>>(ta, tb, ta, p);
   SXB_CHECK_LAUNCH();
   return SXB_OK;
 }

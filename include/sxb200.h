@@ -612,6 +612,13 @@ int sxb_scale_by(void* x, long long n, const void* scale, int dtype, void* strea
 int sxb_gated_act_groups(const void* in, void* out, const void* offsets, const void* counts, int groups,
                          int n_rows, int F, int act, int dtype, void* stream);
 
+/* ---- csrc/gemm_ext.cu */
+/* Ragged-M NT product in bf16 whose groups use only their first counts[g] rows (device, int32): rows behind them are neither
+ * read nor defined in C.  A, C [total_rows, K | N] with row pitches lda, ldc; B [num_groups * N, K]; offsets as above. */
+int sxb_gemm_grouped_used(const void* A, const void* B, void* C, int N, int K, long long lda, long long ldb,
+                          long long ldc, int num_groups, const void* offsets, const void* counts,
+                          long long total_rows, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -251,14 +251,15 @@ def grouped_experts_inference(x, scores, assign, offsets, counts, w1, w2, activa
     and return their input: their row groups skip both products and are copied from the receive to the return buffer.
     Replaces the per-expert loop over
     ``cumsum.tolist()`` (reference: ``inference/v2/kernels/cutlass_ops/moe_gemm``)."""
-    from ..ops.gemm_ext import grouped_gemm_nt
+    from ..ops.gemm_ext import grouped_gemm_nt_used
     T, H = x.shape
     E = w1.shape[0]
     ep = FusedEP.get(None, H, E + n_identity, T, top_k, 1.0)
     plan = make_plan(ep, counts, assign, offsets)
     wts = scores.to(torch.float32).contiguous()
     ep.push(x.contiguous(), plan, weights=wts if weight_input else None)
-    h = grouped_gemm_nt(ep.recv_rows, w1, plan.group_offsets)
+    counts = counts.contiguous()
+    h = grouped_gemm_nt_used(ep.recv_rows, w1, plan.group_offsets, counts)
     if gate_act is not None and h.shape[1] % 16 == 0:
         from ..ops.functional import _act_code
         a = h.new_empty((h.shape[0], h.shape[1] // 2))
@@ -267,7 +268,7 @@ def grouped_experts_inference(x, scores, assign, offsets, counts, w1, w2, activa
         h = a
     else:
         h = activation(h)
-    grouped_gemm_nt(h, w2, plan.group_offsets, out=ep.ret_rows)
+    grouped_gemm_nt_used(h, w2, plan.group_offsets, counts, out=ep.ret_rows)
     if n_identity > 0:
         from ..ops.moe_ops import copy_group_rows_
         copy_group_rows_(ep.ret_rows, ep.recv_rows, plan.group_offsets, E, E + n_identity)

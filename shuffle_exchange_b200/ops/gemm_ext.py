@@ -27,6 +27,7 @@ GROUP_ALIGN_K = 64
 
 _n.register({
     "sxb_gemm_ext": "ppp" "iiii" "lll" "iii" "f" "pilll" "iipll" "pp" "i" "p",
+    "sxb_gemm_grouped_used": "ppp" "ii" "lll" "ipp" "l" "p",
     "sxb_gemmx_hang_info": "p",
     "sxb_stream_write_u32": "pip",
     "sxb_fp8_rowwise_quant": "ppp" "li" "ll" "p",
@@ -166,6 +167,19 @@ def grouped_gemm_nt(x, w, offsets, out=None, scale_x=None, qw=None, scale_w=None
         _call(x.data_ptr(), qw.data_ptr(), out.data_ptr(), 0, N, K, GEMM_NT, x.stride(0), qw.stride(1), out.stride(0),
               _n.FP8E4M3, _n.dtype_code(out.dtype), False, 1.0, None, None, RAGGED_M, G, offsets, R, 0,
               scale_x, scale_w.reshape(-1))
+    return out
+
+
+def grouped_gemm_nt_used(x, w, offsets, counts, out=None):
+    """:func:`grouped_gemm_nt` in bf16 for groups that use only their first ``counts[g]`` rows (int32, device): the rows of
+    padding behind them are neither read nor defined in the result."""
+    G, N, K = w.shape
+    if out is None:
+        out = torch.empty((x.shape[0], N), dtype=torch.bfloat16, device=x.device)
+    if not x.is_cuda or K == 0 or out.dtype != torch.bfloat16 or out.stride(0) % 8 or out.data_ptr() % 16:
+        return grouped_gemm_nt(x, w, offsets, out=out)       # the stores of single elements stay there
+    _n.call("sxb_gemm_grouped_used", x.data_ptr(), w.data_ptr(), out.data_ptr(), N, K, x.stride(0), w.stride(1), out.stride(0), G,
+            offsets.data_ptr(), counts.data_ptr(), x.shape[0], _n.stream_ptr())
     return out
 
 
