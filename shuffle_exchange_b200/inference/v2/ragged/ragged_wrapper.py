@@ -96,9 +96,10 @@ class RaggedBatchWrapper:
             start, rows, seen = (torch.from_numpy(m[: self._n_seqs]) for m in self._seq_meta)
             _, self._n_atoms = AtomBuilder()(self._host_views[self._turn][5], start, rows, seen, ATOM_Q_BLOCK, ATOM_KV_BLOCK)
             # longest first: the kernels take the short tail (decode tokens, chunk remainders) on its own and need those
-            # atoms contiguous; among equals the one with most keys first, so that light ones end the grid
+            # atoms contiguous; among equal short ones the one with most keys first, so that light ones end the grid
+            # (the kernel for the long ones walks them from the end: a sequence's later tiles have more keys)
             live = self._tables[self._turn][5][: self._n_atoms]
-            live[:] = live[np.lexsort((-live[:, 5], -live[:, 2]))]
+            live[:] = live[np.lexsort((np.where(live[:, 2] <= 16, -live[:, 5], 0), -live[:, 2]))]
             self._atom_q_lens = live[:, 2].copy()
         self._live = {}
         self._dev.copy_(self._host, non_blocking=True)
