@@ -36,7 +36,7 @@ from ..ops.gemm_ext import GROUP_ALIGN_M
 
 _n.register({
     "sxb_moe_ep_plan": "ppii" "pp" "iii" "iii" "p",
-    "sxb_moe_ep_push": "ppii" "pppp" "ppp" "iiiii" "i" "i" "pi" "p",
+    "sxb_moe_ep_push": "ppii" "pppp" "ppp" "iiiii" "i" "i" "pii" "p",
     "sxb_moe_ep_pull": "ppii" "ppp" "ppp" "iiiii" "i" "i" "pi" "p",
     "sxb_moe_ep_hang_info": "p",
     "sxb_gated_act_groups": "pppp" "iiiii" "p",
@@ -137,22 +137,25 @@ class FusedEP:
             self._overflow_sources.append(tables)
         return tables
 
-    def push(self, x, plan: EPPlan, weights=None, pulled=None, d_scores=None):
+    def push(self, x, plan: EPPlan, weights=None, pulled=None, d_scores=None, zero_pad=True):
         """Rows of ``x`` -> peers' receive buffers (after :meth:`plan` of this epoch); then wait until every peer's rows
-        for ME have landed."""
+        for ME have landed (one rank: the order of the stream says so).  ``zero_pad=False``: nothing reads the rows between an
+        expert's last one and its aligned end, and they keep what they held."""
         _n.call("sxb_moe_ep_push", self.recv.bufs, self.ret.sigs, self.rank, self.world, x.data_ptr(),
                 _n.ptr(weights), _n.ptr(pulled), _n.ptr(d_scores), plan.assign.data_ptr(), plan.offsets.data_ptr(),
                 plan.tables.data_ptr(), plan.T, plan.K, self.H, self.E, self.L, self.cap_rows, self.epoch,
-                self.sg._ctr(3), 0, _n.stream_ptr())
-        _n.call("sxb_symm_wait", self.ret.bufs, self.ret.sigs, self.rank, self.world, CH_LANDED, self.epoch,
-                _n.stream_ptr())
+                self.sg._ctr(3), 0, int(zero_pad), _n.stream_ptr())
+        if self.world > 1:
+            _n.call("sxb_symm_wait", self.ret.bufs, self.ret.sigs, self.rank, self.world, CH_LANDED, self.epoch,
+                    _n.stream_ptr())
 
     def pull(self, out, plan: EPPlan, weights=None, keep=None):
         """Announce that my return buffer holds this epoch's rows, wait for every peer's, then gather-reduce."""
-        _n.call("sxb_symm_signal", self.ret.bufs, self.ret.sigs, self.rank, self.world, CH_READY, self.epoch,
-                _n.stream_ptr())
-        _n.call("sxb_symm_wait", self.ret.bufs, self.ret.sigs, self.rank, self.world, CH_READY, self.epoch,
-                _n.stream_ptr())
+        if self.world > 1:
+            _n.call("sxb_symm_signal", self.ret.bufs, self.ret.sigs, self.rank, self.world, CH_READY, self.epoch,
+                    _n.stream_ptr())
+            _n.call("sxb_symm_wait", self.ret.bufs, self.ret.sigs, self.rank, self.world, CH_READY, self.epoch,
+                    _n.stream_ptr())
         _n.call("sxb_moe_ep_pull", self.ret.bufs, self.ret.sigs, self.rank, self.world, out.data_ptr(),
                 _n.ptr(weights), _n.ptr(keep), plan.assign.data_ptr(), plan.offsets.data_ptr(),
                 plan.tables.data_ptr(), plan.T, plan.K, self.H, self.E, self.L, self.cap_rows, self.epoch,
@@ -257,7 +260,7 @@ def grouped_experts_inference(x, scores, assign, offsets, counts, w1, w2, activa
     ep = FusedEP.get(None, H, E + n_identity, T, top_k, 1.0)
     plan = make_plan(ep, counts, assign, offsets)
     wts = scores.to(torch.float32).contiguous()
-    ep.push(x.contiguous(), plan, weights=wts if weight_input else None)
+    ep.push(x.contiguous(), plan, weights=wts if weight_input else None, zero_pad=False)
     counts = counts.contiguous()
     h = grouped_gemm_nt_used(ep.recv_rows, w1, plan.group_offsets, counts)
     if gate_act is not None and h.shape[1] % 16 == 0:
