@@ -33,6 +33,10 @@ int sxb_attn_hang_info(unsigned int* out_host);
  * kernel family (1 = 2-CTA multicast, 0 = single CTA) sxb_attn_fwd / the dQ pass would take for these K/V. */
 int sxb_register_foreign_range(const void* p, long long bytes);
 int sxb_range_is_local(const void* p, long long bytes);
+/* Tells how many ranks the program has (sxb_attn_*: multicast kernels are for programs of one rank; WORLD_SIZE of a launcher
+ * counts from the start).  Once it was more than one they stay off for the rest of the process.  Returns 1 while they are
+ * open, 0 otherwise. */
+int sxb_attn_note_ranks(int world);
 int sxb_attn_would_multicast(const void* k, const void* v, int B, int S, int Hq, int Hk, int D, long long k_stride,
                              long long v_stride);
 

@@ -23,6 +23,7 @@ import torch
 import torch.distributed as tdist
 
 from ..device import get_accelerator
+from ..native.lib import note_ranks
 from ..utils.comms_logging import CommsLogger
 from ..utils.logging import logger
 from .reduce_op import ReduceOp
@@ -153,6 +154,8 @@ def init_distributed(dist_backend: Optional[str] = None, auto_mpi_discovery: boo
     if dist_init_required is None:
         dist_init_required = not is_initialized()
     if dist_init_required is False or is_initialized():
+        if is_initialized():
+            note_ranks(get_world_size())
         return
     need = ("RANK", "WORLD_SIZE", "MASTER_ADDR", "MASTER_PORT")
     if auto_mpi_discovery and not all(k in os.environ for k in need):
@@ -181,6 +184,7 @@ def init_distributed(dist_backend: Optional[str] = None, auto_mpi_discovery: boo
         except Exception:
             pass
     tdist.init_process_group(**kw)
+    note_ranks(tdist.get_world_size())
     _initialized_here = True
 
 

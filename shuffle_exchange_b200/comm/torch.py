@@ -10,6 +10,7 @@ import torch
 import torch.distributed as tdist
 
 from . import comm as _c
+from ..native.lib import note_ranks
 from .backend import Backend
 from .constants import NCCL_BACKEND
 from .reduce_op import ReduceOp
@@ -85,6 +86,7 @@ class TorchBackend(Backend):
         self.using_mpi = tdist.get_backend() == "mpi"
         self.world_group = tdist.group.WORLD
         self.world_rank, self.world_size = tdist.get_rank(), tdist.get_world_size()
+        note_ranks(self.world_size)
         self.initialized = True
 
     # ---- collectives

@@ -132,7 +132,7 @@ def paged_attention_atoms(q: torch.Tensor, cache: torch.Tensor, atoms: torch.Ten
     n_kv = cache.shape[3]
     scale = 1.0 / math.sqrt(D) if scale is None else scale
     out = torch.empty(T, n_q, D, dtype=q.dtype, device=q.device)
-    _lib.call("sxb_attn_fwd_atoms_few", q.data_ptr(), cache.data_ptr(), out.data_ptr(), atoms.data_ptr(), atoms.shape[0],
+    _lib.attn_call("sxb_attn_fwd_atoms_few", q.data_ptr(), cache.data_ptr(), out.data_ptr(), atoms.data_ptr(), atoms.shape[0],
               int(n_packed), int(n_few), block_tables.data_ptr(), block_tables.shape[1], cache.shape[0], cache.shape[1], T, n_q, n_kv, D,
               q.stride(0), out.stride(0), float(scale), _lib.stream_ptr())
     return out

@@ -15,9 +15,11 @@ from typing import Optional
 
 import torch
 import torch.autograd.forward_ad as _forward_ad
+import torch.distributed as _dist
 
 _HERE = Path(__file__).resolve().parent
 _LIB: Optional[ctypes.CDLL] = None
+_RANKS = 1                       # ranks of the program as far as known
 _HOST: Optional[ctypes.CDLL] = None
 _LOCK = threading.Lock()
 
@@ -66,6 +68,7 @@ SIGNATURES = {
     "sxb_gemm_hang_info": "p",
     "sxb_gemm_set_mode": "i",
     "sxb_attn_hang_info": "p",
+    "sxb_attn_note_ranks": "i",
 }
 _LONG_RETURN = {"sxb_norm_bwd_scratch_elems"}
 
@@ -115,8 +118,20 @@ def load() -> ctypes.CDLL:
                               "shuffle_exchange_b200.native.build`")
         lib = ctypes.CDLL(str(path), mode=ctypes.RTLD_GLOBAL)
         _bind(lib, SIGNATURES)
+        if _RANKS > 1:
+            lib.sxb_attn_note_ranks(_RANKS)
         _LIB = lib
         return lib
+
+
+def note_ranks(world: int) -> None:
+    """Tell the library that the program has ``world`` ranks: with more than one, attention keeps to the kernels without TMA
+    multicast for the rest of the process (``sxb_attn_note_ranks``)."""
+    global _RANKS
+    if world > _RANKS:
+        _RANKS = world
+        if _LIB is not None:
+            _LIB.sxb_attn_note_ranks(world)
 
 
 def register(table) -> None:
@@ -171,6 +186,13 @@ def call(name: str, *args):
                   -4: "driver entry point unavailable"}.get(rc, "error")
         raise NativeError(f"{name} rejected the call: {reason} ({rc})")
     return 0
+
+
+def attn_call(name: str, *args):
+    """:func:`call` of an attention kernel, which has to know of every process group, whoever made it (:func:`note_ranks`)."""
+    if _RANKS == 1 and _dist.is_available() and _dist.is_initialized():
+        note_ranks(_dist.get_world_size())
+    return call(name, *args)
 
 
 def hang_info(kind: str = "attn"):

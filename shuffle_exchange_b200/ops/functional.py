@@ -662,7 +662,7 @@ class _FlashAttn(torch.autograd.Function):
         lse = torch.empty((B, Hq, S), dtype=torch.float32, device=q.device)
         if flop_sink is not None:
             flop_sink("attention", 4.0 * B * Hq * S * S * D * (0.5 if causal else 1.0))
-        _n.call("sxb_attn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
+        _n.attn_call("sxb_attn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
                 B, S, Hq, Hk, D, q.stride(1), k.stride(1), v.stride(1), out.stride(1), int(causal),
                 float(scale), _n.stream_ptr())
         ctx.save_for_backward(q, k, v, out, lse)
@@ -682,7 +682,7 @@ class _FlashAttn(torch.autograd.Function):
         dk = dqkv[..., Hq * D: (Hq + Hk) * D].view(B, S, Hk, D)
         dv = dqkv[..., (Hq + Hk) * D:].view(B, S, Hk, D)
         delta = torch.empty((B, Hq, S), dtype=torch.float32, device=q.device)
-        _n.call("sxb_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
+        _n.attn_call("sxb_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
                 lse.data_ptr(), delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                 B, S, Hq, Hk, D, q.stride(1), k.stride(1), v.stride(1), out.stride(1), dout.stride(1),
                 dq.stride(1), dk.stride(1), dv.stride(1), int(ctx.causal), float(ctx.scale), _n.stream_ptr())
@@ -702,7 +702,7 @@ class _FlashAttnQKV(torch.autograd.Function):
         lse = torch.empty((B, Hq, S), dtype=torch.float32, device=qkv.device)
         if flop_sink is not None:
             flop_sink("attention", 4.0 * B * Hq * S * S * D * (0.5 if causal else 1.0))
-        _n.call("sxb_attn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
+        _n.attn_call("sxb_attn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
                 B, S, Hq, Hk, D, C, C, C, out.stride(1), int(causal), float(scale), _n.stream_ptr())
         ctx.save_for_backward(qkv, out, lse)
         ctx.meta = (Hq, Hk, D, causal, scale)
@@ -719,7 +719,7 @@ class _FlashAttnQKV(torch.autograd.Function):
         dqkv = torch.empty_like(qkv)
         dq, dk, dv = _split_qkv(dqkv, Hq, Hk, D)
         delta = torch.empty((B, Hq, S), dtype=torch.float32, device=qkv.device)
-        _n.call("sxb_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
+        _n.attn_call("sxb_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
                 lse.data_ptr(), delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                 B, S, Hq, Hk, D, C, C, C, out.stride(1), dout.stride(1), C, C, C, int(causal), float(scale),
                 _n.stream_ptr())
@@ -757,7 +757,7 @@ def attention_fwd_lse(q, k, v, causal: bool, scale: float):
         q, k, v = (t if _attn_layout_ok(t) else t.contiguous() for t in (q, k, v))
         out = torch.empty((B, S, Hq, D), dtype=q.dtype, device=q.device)
         lse = torch.empty((B, Hq, S), dtype=torch.float32, device=q.device)
-        _n.call("sxb_attn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
+        _n.attn_call("sxb_attn_fwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
                 B, S, Hq, k.shape[2], D, q.stride(1), k.stride(1), v.stride(1), out.stride(1), int(causal),
                 float(scale), _n.stream_ptr())
         return out, lse
@@ -784,7 +784,7 @@ def attention_bwd_raw(q, k, v, out, dout, lse, causal: bool, scale: float):
         dk = torch.empty_like(k)
         dv = torch.empty_like(v)
         delta = torch.empty((B, Hq, S), dtype=torch.float32, device=q.device)
-        _n.call("sxb_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
+        _n.attn_call("sxb_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
                 lse.data_ptr(), delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                 B, S, Hq, Hk, D, q.stride(1), k.stride(1), v.stride(1), out.stride(1), dout.stride(1),
                 dq.stride(1), dk.stride(1), dv.stride(1), int(causal), float(scale), _n.stream_ptr())
@@ -828,7 +828,7 @@ class _FlashAttnKeyBias(torch.autograd.Function):
         Hk = k.shape[2]
         out = torch.empty((B, S, Hq, D), dtype=q.dtype, device=q.device)
         lse = torch.empty((B, Hq, S), dtype=torch.float32, device=q.device)
-        _n.call("sxb_attn_fwd_kbias", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
+        _n.attn_call("sxb_attn_fwd_kbias", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
                 kb_raw.data_ptr(), int(kb_raw.dim() == 3), B, S, Hq, Hk, D, q.stride(1), k.stride(1), v.stride(1),
                 out.stride(1), int(causal), float(scale), _n.stream_ptr())
         ctx.save_for_backward(q, k, v, out, lse, kb_raw)
@@ -844,7 +844,7 @@ class _FlashAttnKeyBias(torch.autograd.Function):
             dout = dout.contiguous()
         dq, dk, dv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
         delta = torch.empty((B, Hq, S), dtype=torch.float32, device=q.device)
-        _n.call("sxb_attn_bwd_kbias", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
+        _n.attn_call("sxb_attn_bwd_kbias", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
                 lse.data_ptr(), delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), kb_raw.data_ptr(),
                 int(kb_raw.dim() == 3), B, S, Hq, Hk, D, q.stride(1), k.stride(1), v.stride(1), out.stride(1), dout.stride(1),
                 dq.stride(1), dk.stride(1), dv.stride(1), int(ctx.causal), float(ctx.scale), _n.stream_ptr())
@@ -909,7 +909,7 @@ class _FlashAttnVarlen(torch.autograd.Function):
         nseq = cu_seqlens.numel() - 1
         out = torch.empty((T, Hq, D), dtype=q.dtype, device=q.device)
         lse = torch.empty((Hq, T), dtype=torch.float32, device=q.device)
-        _n.call("sxb_attn_fwd_varlen", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
+        _n.attn_call("sxb_attn_fwd_varlen", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), lse.data_ptr(),
                 cu_seqlens.data_ptr(), nseq, int(max_seqlen), T, Hq, Hk, D, q.stride(0), k.stride(0), v.stride(0),
                 out.stride(0), int(causal), float(scale), _n.stream_ptr())
         ctx.save_for_backward(q, k, v, out, lse, cu_seqlens)
@@ -929,7 +929,7 @@ class _FlashAttnVarlen(torch.autograd.Function):
         dk = dqkv[:, Hq * D: (Hq + Hk) * D].view(T, Hk, D)
         dv = dqkv[:, (Hq + Hk) * D:].view(T, Hk, D)
         delta = torch.empty((Hq, T), dtype=torch.float32, device=q.device)
-        _n.call("sxb_attn_bwd_varlen", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
+        _n.attn_call("sxb_attn_bwd_varlen", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
                 lse.data_ptr(), delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(), cu.data_ptr(),
                 cu.numel() - 1, max_seqlen, T, Hq, Hk, D, q.stride(0), k.stride(0), v.stride(0), out.stride(0),
                 dout.stride(0), dq.stride(0), dk.stride(0), dv.stride(0), int(causal), float(scale), _n.stream_ptr())

@@ -184,7 +184,7 @@ class _Stage:
         self.lse = torch.empty((1, up.hq, S), dtype=torch.float32, device=qkv.device)
         q, k, v = self._qkv_views()
         kk, pp = _ptrs(up.peers("ctx"), r * up.hq * D)
-        _n.call("sxb_attn_fwd_scatter", q.data_ptr(), k.data_ptr(), v.data_ptr(), pp, up.world, up.S_local,
+        _n.attn_call("sxb_attn_fwd_scatter", q.data_ptr(), k.data_ptr(), v.data_ptr(), pp, up.world, up.S_local,
                 self.o_keep.data_ptr(), self.o_keep.stride(0), self.lse.data_ptr(), 1, S, up.hq, up.hk, D,
                 qkv.stride(0), qkv.stride(0), qkv.stride(0), up.Hq * D, int(self.causal), float(self.scale),
                 _n.stream_ptr())
@@ -215,7 +215,7 @@ class _Stage:
         delta = torch.empty((1, up.hq, S), dtype=torch.float32, device=dctx.device)
         kq, pq = _ptrs(up.peers("dqkv"), r * up.hq * D)
         kk, pk = _ptrs(up.peers("dqkv"), up.Hq * D + r * up.hk * D)
-        _n.call("sxb_attn_bwd_scatter", q.data_ptr(), k.data_ptr(), v.data_ptr(), self.o_keep.data_ptr(),
+        _n.attn_call("sxb_attn_bwd_scatter", q.data_ptr(), k.data_ptr(), v.data_ptr(), self.o_keep.data_ptr(),
                 dctx.data_ptr(), self.lse.data_ptr(), delta.data_ptr(), pq, pk, up.Hk * D, up.world, up.S_local,
                 1, S, up.hq, up.hk, D, self.qkv.stride(0), self.qkv.stride(0), self.qkv.stride(0),
                 self.o_keep.stride(0), dctx.stride(0), up.C_all, up.C_all, up.C_all, int(self.causal),
