@@ -400,10 +400,11 @@ SXB_API int sxb_moe_ep_plan_emu(const void* const* counts, const void* const* si
   return launch_emu((const void*)plan_emu_kernel, A, world, 1, (cudaStream_t)stream);
 }
 
-SXB_API int sxb_moe_ep_push(const void* const* recv, const void* const* sigs, int rank, int world, const void* x,
-                            const void* weights, const void* pulled, void* d_scores, const void* assign,
-                            const void* offsets, const void* tables, int T, int K, int H, int E, int L,
-                            int cap_rows, unsigned int epoch, void* counter, int max_ctas, int zero_pad, void* stream) {
+// zero_pad 0: the padding rows behind an expert's last one keep what they held (nothing reads them).
+SXB_API int sxb_moe_ep_push_rows(const void* const* recv, const void* const* sigs, int rank, int world, const void* x,
+                                 const void* weights, const void* pulled, void* d_scores, const void* assign,
+                                 const void* offsets, const void* tables, int T, int K, int H, int E, int L, int cap_rows,
+                                 unsigned int epoch, void* counter, int max_ctas, int zero_pad, void* stream) {
   PushArgs A;
   int rc = fill_peers(A.P, recv, nullptr, nullptr, sigs, rank, world);
   if (rc) return rc;
@@ -417,6 +418,14 @@ SXB_API int sxb_moe_ep_push(const void* const* recv, const void* const* sigs, in
   push_kernel<<<row_grid((long long)T * K * A.parts + (long long)L * A.pad_rows, max_ctas), 256, 0, (cudaStream_t)stream>>>(A);
   SXB_CHECK_LAUNCH();
   return SXB_OK;
+}
+// The same with the padding rows zeroed.
+SXB_API int sxb_moe_ep_push(const void* const* recv, const void* const* sigs, int rank, int world, const void* x,
+                            const void* weights, const void* pulled, void* d_scores, const void* assign,
+                            const void* offsets, const void* tables, int T, int K, int H, int E, int L,
+                            int cap_rows, unsigned int epoch, void* counter, int max_ctas, void* stream) {
+  return sxb_moe_ep_push_rows(recv, sigs, rank, world, x, weights, pulled, d_scores, assign, offsets, tables, T, K, H, E, L,
+                              cap_rows, epoch, counter, max_ctas, 1, stream);
 }
 SXB_API int sxb_moe_ep_push_emu(const void* const* recv, const void* const* sigs, int world, const void* const* x,
                                 const void* const* weights, const void* const* pulled, void* const* d_scores,

@@ -235,7 +235,12 @@ int sxb_moe_ep_plan_emu(const void* const* counts, const void* const* sigs, int 
 int sxb_moe_ep_push(const void* const* recv, const void* const* sigs, int rank, int world, const void* x,
                     const void* weights, const void* pulled, void* d_scores, const void* assign,
                     const void* offsets, const void* tables, int T, int K, int H, int E, int L, int cap_rows,
-                    unsigned int epoch, void* counter, int max_ctas, int zero_pad, void* stream);
+                    unsigned int epoch, void* counter, int max_ctas, void* stream);
+/* zero_pad 0: the padding rows behind an expert's last one keep what they held (nothing reads them); 1: as sxb_moe_ep_push. */
+int sxb_moe_ep_push_rows(const void* const* recv, const void* const* sigs, int rank, int world, const void* x,
+                         const void* weights, const void* pulled, void* d_scores, const void* assign,
+                         const void* offsets, const void* tables, int T, int K, int H, int E, int L, int cap_rows,
+                         unsigned int epoch, void* counter, int max_ctas, int zero_pad, void* stream);
 int sxb_moe_ep_push_emu(const void* const* recv, const void* const* sigs, int world, const void* const* x,
                         const void* const* weights, const void* const* pulled, void* const* d_scores,
                         const void* const* assign, const void* const* offsets, const void* const* tables, int T,

@@ -36,7 +36,8 @@ from ..ops.gemm_ext import GROUP_ALIGN_M
 
 _n.register({
     "sxb_moe_ep_plan": "ppii" "pp" "iii" "iii" "p",
-    "sxb_moe_ep_push": "ppii" "pppp" "ppp" "iiiii" "i" "i" "pii" "p",
+    "sxb_moe_ep_push": "ppii" "pppp" "ppp" "iiiii" "i" "i" "pi" "p",
+    "sxb_moe_ep_push_rows": "ppii" "pppp" "ppp" "iiiii" "i" "i" "pii" "p",
     "sxb_moe_ep_pull": "ppii" "ppp" "ppp" "iiiii" "i" "i" "pi" "p",
     "sxb_moe_ep_hang_info": "p",
     "sxb_gated_act_groups": "pppp" "iiiii" "p",
@@ -141,7 +142,7 @@ class FusedEP:
         """Rows of ``x`` -> peers' receive buffers (after :meth:`plan` of this epoch); then wait until every peer's rows
         for ME have landed (one rank: the order of the stream says so).  ``zero_pad=False``: nothing reads the rows between an
         expert's last one and its aligned end, and they keep what they held."""
-        _n.call("sxb_moe_ep_push", self.recv.bufs, self.ret.sigs, self.rank, self.world, x.data_ptr(),
+        _n.call("sxb_moe_ep_push_rows", self.recv.bufs, self.ret.sigs, self.rank, self.world, x.data_ptr(),
                 _n.ptr(weights), _n.ptr(pulled), _n.ptr(d_scores), plan.assign.data_ptr(), plan.offsets.data_ptr(),
                 plan.tables.data_ptr(), plan.T, plan.K, self.H, self.E, self.L, self.cap_rows, self.epoch,
                 self.sg._ctr(3), 0, int(zero_pad), _n.stream_ptr())

@@ -144,3 +144,9 @@ def test_host_library_signatures_match_the_header():
                     if k.value in header and sig != header[k.value]:
                         bad.append((f, k.value, sig, header[k.value]))
     assert seen >= 20 and not bad, (seen, bad)
+
+
+def test_entry_points_of_this_abi_version_keep_their_parameters():
+    """A program that was compiled against an earlier header of the same ``sxb_abi_version`` passes what that header declared:
+    a further parameter needs an entry point of its own."""
+    assert "".join(_header_params()["sxb_moe_ep_push"]) == "ppii" "pppp" "ppp" "iiiii" "i" "i" "pi" "p"
