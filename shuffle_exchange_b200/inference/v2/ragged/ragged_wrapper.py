@@ -74,6 +74,10 @@ class RaggedBatchWrapper:
         ids, t2s, pos, last, tables, _, info = self._tables[self._turn]
         i, seen = self._n_seqs, seq_descriptor.seen_tokens
         a, b = self._n_tokens, self._n_tokens + n
+        blocks = seq_descriptor.kv_blocks()
+        if (tokens.dim() > 1 and tokens.shape[-1] != n) or b > self.max_tokens or blocks.numel() > self.max_blocks:
+            raise RuntimeError(f"tokens {tuple(tokens.shape)} at row {a} with {blocks.numel()} blocks do not fit a batch of "
+                               f"{self.max_tokens} rows of tokens and {self.max_blocks} blocks per sequence")
         self._seq_meta[:, i] = (a, n, seen)
         ids[a:b] = tokens.to(device="cpu", dtype=torch.int32).reshape(-1).numpy()
         t2s[a:b] = i
@@ -85,7 +89,6 @@ class RaggedBatchWrapper:
             last[self._n_logit_rows] = a + r
             self._n_logit_rows += 1
         info[i] = (a, n, seen, getattr(seq_descriptor, "state_slot", -1))
-        blocks = seq_descriptor.kv_blocks()
         tables[i, : blocks.numel()] = blocks.cpu().numpy()
         self._n_tokens, self._n_seqs = b, i + 1
         self._live = {}

@@ -34,6 +34,18 @@ def test_wrapper_cuts_atoms_on_cpu():
     assert w.atoms().shape[0] == 0
 
 
+def test_what_does_not_fit_a_batch_is_refused():
+    one = torch.arange(1)
+    for tokens, blocks in ((torch.zeros(3, 1, dtype=torch.int64), [0]), (torch.zeros(2, 2, dtype=torch.int64), [0]),
+                           (one, list(range(5))), (torch.arange(9), [0])):
+        w = RaggedBatchWrapper(8, 2, 4, device="cpu")
+        with pytest.raises(RuntimeError):
+            w.insert_sequence(_Seq(0, blocks), tokens, do_checks=False)
+        w.insert_sequence(_Seq(4, [2]), one[None])                     # one row of tokens; nothing of the refused ones is left
+        w.finalize()
+        assert w.input_ids().tolist() == [0] and w.seq_info().tolist() == [[0, 1, 4, -1]]
+
+
 def _rel_err(a, b):
     return ((a.float() - b.float()).norm() / b.float().norm().clamp_min(1e-9)).item()
 
