@@ -60,8 +60,9 @@ def _stale(src: Path, obj: Path, extra_deps, flags) -> bool:
     return sha.read_text().strip() != _digest(src, extra_deps, flags)
 
 
-def _stamp(src: Path, obj: Path, extra_deps, flags):
-    obj.with_suffix(obj.suffix + ".sha").write_text(_digest(src, extra_deps, flags))
+def _stamp(obj: Path, digest: str):
+    """``digest`` was taken before the compiler ran: a source that changes meanwhile leaves the object stale."""
+    obj.with_suffix(obj.suffix + ".sha").write_text(digest)
 
 
 def _run(cmd):
@@ -87,14 +88,14 @@ def build_cuda(verbose: bool = False, force: bool = False) -> Path:
             if verbose:
                 cmd.insert(1, "-Xptxas=-v")
             jobs.append(cmd)
-            rebuilt.append((s, o))
+            rebuilt.append((o, _digest(s, headers, NVCC_FLAGS)))
     if jobs:
         with cf.ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
             for out in ex.map(_run, jobs):
                 if verbose and out:
                     print(out)
-        for s, o in rebuilt:
-            _stamp(s, o, headers, NVCC_FLAGS)
+        for o, digest in rebuilt:
+            _stamp(o, digest)
     lib = OUT_DIR / "libsxb200.so"
     if jobs or not lib.exists():
         _run([nvcc, "-shared", "-o", str(lib), *map(str, objs), "-gencode", "arch=compute_100a,code=sm_100a",
@@ -113,12 +114,12 @@ def build_host(verbose: bool = False, force: bool = False) -> Path:
         objs.append(o)
         if force or _stale(s, o, headers, HOST_FLAGS):
             jobs.append([gxx, *HOST_FLAGS, "-I", str(ROOT / "include"), "-c", str(s), "-o", str(o)])
-            rebuilt.append((s, o))
+            rebuilt.append((o, _digest(s, headers, HOST_FLAGS)))
     if jobs:
         with cf.ThreadPoolExecutor(max_workers=min(8, len(jobs))) as ex:
             list(ex.map(_run, jobs))
-        for s, o in rebuilt:
-            _stamp(s, o, headers, HOST_FLAGS)
+        for o, digest in rebuilt:
+            _stamp(o, digest)
     lib = OUT_DIR / "libsxb200_host.so"
     if srcs and (jobs or not lib.exists()):
         _run([gxx, "-shared", "-o", str(lib), *map(str, objs), "-fopenmp", "-pthread", "-ldl"])
