@@ -581,6 +581,7 @@ class _CrossEntropy(torch.autograd.Function):
         # in place: the saved buffer is the (consumed) logits tensor
         if dloss.dtype == torch.float32 and dloss.device == g.device and g.is_contiguous() and _n.no_tape(dloss, g):
             _n.call("sxb_scale_by", g.data_ptr(), g.numel(), dloss.data_ptr(), _n.dtype_code(g.dtype), _n.stream_ptr())
+            torch.autograd.graph.increment_version(g)       # a second pass would scale it again: autograd refuses that
         else:
             g.mul_(dloss.to(g.dtype))
         return g.view(ctx.shape), None, None

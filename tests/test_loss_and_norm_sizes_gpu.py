@@ -35,6 +35,23 @@ def test_scale_that_is_not_a_number_reaches_the_gradient():
     assert bool(x.grad.isnan().all())
 
 
+@pytest.mark.parametrize("scale", [1.0, 0.5])
+def test_second_pass_through_a_loss_is_refused(scale):
+    """The first pass scales the gradient where it is saved; a second one would scale it again."""
+    x = torch.randn(5, 1024, device="cuda").bfloat16().requires_grad_()
+    labels = torch.arange(5, device="cuda")
+    loss = F.cross_entropy(x * 1, labels) * scale
+    loss.backward(retain_graph=True)
+    first = x.grad.clone()
+    with pytest.raises(RuntimeError, match="inplace"):
+        loss.backward()
+    assert torch.equal(x.grad, first)
+    loss = F.cross_entropy(x * 1, labels) * scale
+    torch.autograd.grad(loss, x, retain_graph=True)
+    with pytest.raises(RuntimeError, match="inplace"):
+        torch.autograd.grad(loss, x)
+
+
 @pytest.mark.parametrize("rows", [1, 7, 296, 297, 1500])
 @pytest.mark.parametrize("H", [8, 768, 2048, 2056, 4096, 5120, 8192, 16384])
 @pytest.mark.parametrize("layer", [False, True])
