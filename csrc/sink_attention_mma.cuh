@@ -27,6 +27,66 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t& hi, uint32_t&
   lo = __byte_perm(__float_as_uint(rx - __uint_as_float(vx & 0xffff0000u)),
                    __float_as_uint(ry - __uint_as_float(vy & 0xffff0000u)), 0x7632);
 }
+// One row by fp32 FMAs, a whole warp on it: the sums of the tiled form (64 keys from the first key `kbeg` of the row's 64-query
+// half), over the keys that the row sees.  For rows whose products met an infinity: three terms cannot carry it, since
+// 0 * inf of a term that is zero is not a number (the weight of the largest key is 1 = 1 + 0 + 0).  Rows that the tensor
+// cores give as finite numbers are right: a term's rests have its sign, so an infinity stays one or becomes NaN.
+template <int D, int DV>
+__device__ __noinline__ void sink_row_plain(const float* q, float scale, const __nv_bfloat16* kc, const __nv_bfloat16* vc,
+                                            const int* tab, int block_size, int kpitch, int vpitch, int kbeg, int lo, int qp,
+                                            const float* sink, const float* bias, int bias_len, const __nv_bfloat16* gate,
+                                            int gate_heads, __nv_bfloat16* out, float out_scale) {
+  constexpr int C = DV / 32;                                    // value channels of a lane: C lane .. + C - 1
+  const int lane = threadIdx.x & 31;
+  auto slot_of = [&](int pos) { return (long long)tab[pos / block_size] * block_size + pos % block_size; };
+  float m = sink ? *sink : -INFINITY, l = sink ? 1.f : 0.f, acc[C];
+#pragma unroll
+  for (int i = 0; i < C; ++i) acc[i] = 0.f;
+  for (int k0 = kbeg; k0 <= qp; k0 += kBK) {
+    float s[2], mt = -INFINITY, ps = 0.f;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int kj = k0 + lane + 32 * j;
+      s[j] = -INFINITY;
+      if (kj <= qp && kj >= lo) {
+        const __nv_bfloat16* k = kc + slot_of(kj) * kpitch;
+        float x = 0.f, y = 0.f;
+        for (int c = 0; c < D; c += 2) {
+          x = fmaf(q[c] * scale, __bfloat162float(k[c]), x);
+          y = fmaf(q[c + 1] * scale, __bfloat162float(k[c + 1]), y);
+        }
+        s[j] = x + y;
+        if (bias != nullptr) s[j] += bias[min(qp - kj, bias_len - 1)];
+      }
+      mt = fmaxf(mt, s[j]);
+    }
+    const float mn = fmaxf(m, warp_max(mt));
+    const float corr = mn == -INFINITY ? 1.f : expf(m - mn);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      s[j] = s[j] == -INFINITY ? 0.f : expf(s[j] - mn);
+      ps += s[j];
+    }
+    l = l * corr + warp_sum(ps);
+    m = mn;
+#pragma unroll
+    for (int i = 0; i < C; ++i) acc[i] *= corr;
+    for (int j = max(0, lo - k0); j < min(kBK, qp - k0 + 1); ++j) {
+      const float p = __shfl_sync(0xffffffffu, j < 32 ? s[0] : s[1], j & 31);
+      const __nv_bfloat16* v = vc + slot_of(k0 + j) * vpitch + lane * C;
+#pragma unroll
+      for (int i = 0; i < C; ++i) acc[i] = fmaf(p, __bfloat162float(v[i]), acc[i]);
+    }
+  }
+  const float inv = l > 0.f ? 1.f / l : 0.f;
+#pragma unroll
+  for (int i = 0; i < C; ++i) {
+    const int c = lane * C + i;
+    float x = acc[i] * inv;
+    if (gate != nullptr) x *= sigmoid_f(__bfloat162float(gate[gate_heads ? 0 : c]));
+    out[c] = __float2bfloat16_rn(x * out_scale);
+  }
+}
 constexpr int kSmQ = 128, kSmThreads = 256;                    // query rows (a whole atom) and threads of a CTA
 
 template <int D, int DV>
@@ -234,12 +294,20 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
     __syncthreads();                                            // the tile just read is the target of the next copies
   }
   if (!busy) return;
+  unsigned again = 0u;                                          // bit 4 j + i: row warp * 16 + j + 8 i is not finite
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
     l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
     const int r = r0 + 8 * i;
-    if (r >= nq) continue;
+    bool bad = !(fabsf(l[i]) < INFINITY);
+#pragma unroll
+    for (int n = 0; n < DV / 8; ++n) bad |= !(fabsf(acc[n][2 * i]) < INFINITY) || !(fabsf(acc[n][2 * i + 1]) < INFINITY);
+    unsigned b = __ballot_sync(0xffffffffu, bad && r < nq);
+    b |= b >> 1;
+    b = (b | b >> 2) & 0x11111111u;
+    again |= b << i;
+    if (r >= nq || (b >> (lane & ~3) & 1u)) continue;
     const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
     const __nv_bfloat16* gr = gate ? gate + (long long)(row0 + r) * gate_ld + (gate_heads ? h : h * DV) : nullptr;
     __nv_bfloat16* orow = out + (long long)(row0 + r) * out_ld + h * DV;
@@ -262,5 +330,13 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
         orow[c + 1] = __float2bfloat16_rn(y);
       }
     }
+  }
+  for (; again != 0u; again &= again - 1u) {
+    const int bit = __ffs(again) - 1, r = warp * 16 + (bit >> 2) + 8 * (bit & 1), qp = pos0 + r;
+    sink_row_plain<D, DV>(q + ((long long)(row0 + r) * Hq + h) * D, scale, kcache + g * D, vcache + g * DV, tab, block_size,
+                          kpitch, vpitch, first_key(pos0 + r / kBQ * kBQ, chunk, window), first_key(qp, chunk, window), qp,
+                          sink ? sink + h : nullptr, dist_bias ? dist_bias + (long long)h * bias_len : nullptr, bias_len,
+                          gate ? gate + (long long)(row0 + r) * gate_ld + (gate_heads ? h : h * DV) : nullptr, gate_heads,
+                          out + (long long)(row0 + r) * out_ld + h * DV, out_scale);
   }
 }

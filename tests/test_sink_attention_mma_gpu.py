@@ -119,3 +119,28 @@ def test_as_close_as_the_32_bit_form():
     e16, e32 = ((t.double() - want).norm() / want.norm() for t in (y16, y32.bfloat16()))
     assert float(e16) <= 1.01 * float(e32)
     assert float((y16 != y32.bfloat16().double()).double().mean()) < 0.01      # they round differently at ties only
+
+
+def test_infinite_keys_and_values():
+    """What a plain softmax gives: an infinite value comes out infinite wherever its weight is not zero (the weight of the
+    largest key is exactly one), a key whose score is minus infinity has no weight, and rows that do not see them are untouched."""
+    plan, page, Hq, G, d = [(0, 150), (70, 40)], 64, 4, 2, 128
+    b, pages = _batch(plan, page)
+    g = torch.Generator(device="cuda").manual_seed(8)
+    q = torch.randn(190, Hq, d, generator=g, device="cuda")
+    kc, vc = (torch.randn(pages, page, G, d, generator=g, device="cuda").bfloat16() for _ in range(2))
+    at = lambda i, j: (b.block_tables()[i, j // page].long(), j % page)  # noqa: E731
+    q[3, 1], q[3, 1, 0] = 0.0, 64.0                    # row 3 of head 1: its own key takes weight one
+    kc[at(0, 3)][0, 0] = 64.0
+    vc[at(0, 3)][0, 5] = float("inf")
+    vc[at(0, 90)][1, 7], vc[at(0, 91)][1, 8] = float("-inf"), float("inf")
+    kc[at(1, 80)][0, 2] = float("inf")                 # a score of plus infinity (not a number) or minus infinity (no weight)
+    vc[at(1, 100)][1, 9] = float("nan")
+    args = lambda dev: (b.token_to_seq().to(dev), b.token_positions().to(dev), b.block_tables().to(dev), d ** -0.5, 0)  # noqa: E731
+    y = M.sink_attention(q, kc, vc, None, *args("cuda"), torch.bfloat16, b.atoms(), b.atoms_longer_than(M.SHORT_ATOM)).cpu()
+    want = M.sink_attention(q.cpu(), kc.cpu(), vc.cpu(), None, *args("cpu"), torch.float32)
+    assert bool(want.isinf().any()) and bool(want.isnan().any()) and bool(want.view(190, Hq, d)[3, 1, 5].isinf())
+    assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.isinf(), want.isinf())
+    assert torch.equal(y[want.isinf()].float(), want[want.isinf()])
+    ok = want.isfinite()
+    assert bool(((y.float() - want)[ok].abs() <= 2.0 ** -8 * want[ok].abs() + 1e-4).all())
