@@ -1,7 +1,7 @@
 """Per-shape GEMM table on the Llama-3-8B / Mixtral shapes: the base CTA-pair tcgen05 kernel, the extended kernel
 (ungated, gated with all flags set, fp8 forward), and cuBLAS (torch.matmul) on the same box.
 
-    python tools/gemm_table.py            # writes gpurun_out/gemm_table.{json,md}
+    python tools/gemm_table.py            # writes build/reports/gemm_table.{json,md}
 
 Timing: CUDA events around each launch, 3 warm-ups, 10 timed iterations, L2 flushed (a 256 MB write) before every timed
 launch; reported = median.  TFLOP/s = 2MNK / time."""
@@ -69,15 +69,15 @@ def main():
                 r[k.replace("_ms", "_tflops")] = fl / r[k] / 1e9
         rows.append(r)
         del a, b, out
-    os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-    json.dump(rows, open(os.path.join(ROOT, "gpurun_out", "gemm_table.json"), "w"), indent=1)
+    os.makedirs(os.path.join(ROOT, "build/reports"), exist_ok=True)
+    json.dump(rows, open(os.path.join(ROOT, "build/reports", "gemm_table.json"), "w"), indent=1)
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
     except Exception:
         pass
     peak = peaks.get("bf16_tflops", 1590.0)
-    with open(os.path.join(ROOT, "gpurun_out", "gemm_table.md"), "w") as f:
+    with open(os.path.join(ROOT, "build/reports", "gemm_table.md"), "w") as f:
         f.write(f"# GEMM table (TFLOP/s; bf16 peak of measured = {peak:.0f}, L2 flushed between launches)\n\n")
         f.write("| op | layout | M | N | K | base pair | ext | ext gated | cuBLAS | base/cuBLAS | base of measured | fp8 ext |\n")
         f.write("|---|---|---|---|---|---|---|---|---|---|---|---|\n")
@@ -86,7 +86,7 @@ def main():
                     f"{r['ext_tflops']:.0f} | {r.get('ext_gated_tflops', float('nan')):.0f} | {r['cublas_tflops']:.0f} | "
                     f"{r['base_tflops'] / r['cublas_tflops']:.2f} | {r['base_tflops'] / peak:.2f} | "
                     f"{r.get('fp8_tflops', float('nan')):.0f} |\n")
-    print(open(os.path.join(ROOT, "gpurun_out", "gemm_table.md")).read())
+    print(open(os.path.join(ROOT, "build/reports", "gemm_table.md")).read())
 
 
 if __name__ == "__main__":

@@ -1,5 +1,5 @@
 """Run every kernel check in its own subprocess (a hang or a fault in one kernel must not hide
-the others) and write ``gpurun_out/selftest.json``.
+the others) and write ``build/reports/selftest.json``.
 
     python tools/gpu_selftest.py            # all checks
     python tools/gpu_selftest.py gemm attn  # only checks whose name contains one of the words
@@ -650,7 +650,7 @@ def main():
         return
     words = [a for a in sys.argv[1:] if not a.startswith("-")]
     names = [n for n in CHECKS if not words or any(w in n for w in words)]
-    os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
+    os.makedirs(os.path.join(ROOT, "build/reports"), exist_ok=True)
     results = {}
     for name in names:
         t0 = time.time()
@@ -676,7 +676,7 @@ def main():
             results[name]["ok"] = False
             results[name]["error"] = f"numerical error {err} >= {tol}"
         print(name, json.dumps(results[name], default=float)[:600], flush=True)
-        with open(os.path.join(ROOT, "gpurun_out", "selftest.json"), "w") as f:
+        with open(os.path.join(ROOT, "build/reports", "selftest.json"), "w") as f:
             json.dump(results, f, indent=1, default=float)
     bad = [n for n, r in results.items() if not r.get("ok")]
     print("FAILED:", bad)

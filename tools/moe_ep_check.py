@@ -66,8 +66,8 @@ def main():
     res["watchdog"] = n.hang_info("moe_ep")
     res["ok"] = all(v.get("ok", True) for v in res.values() if isinstance(v, dict)) and res["watchdog"] is None
     if rank == 0:
-        os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-        json.dump(res, open(os.path.join(ROOT, "gpurun_out", "moe_ep_check.json"), "w"), indent=1)
+        os.makedirs(os.path.join(ROOT, "build/reports"), exist_ok=True)
+        json.dump(res, open(os.path.join(ROOT, "build/reports", "moe_ep_check.json"), "w"), indent=1)
         print(json.dumps(res))
     td.barrier()
     td.destroy_process_group()

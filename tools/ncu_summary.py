@@ -1,7 +1,7 @@
 #!/usr/bin/env python
 """Summarise ``.ncu-rep`` files into a small JSON/markdown table (the kept artefacts live in profiles/).
 
-    python tools/ncu_summary.py gpurun_out/prof_gemm.ncu-rep ... > profiles/ncu_summary_<tag>.md
+    python tools/ncu_summary.py build/reports/prof_gemm.ncu-rep ... > profiles/ncu_summary_<tag>.md
 """
 import csv
 import io

@@ -2,7 +2,7 @@
 
     python tools/ncu_targets.py && ncu --set full --clock-control none \
         -k regex:'gemm_pair_x_kernel|gemm_pair_kernel|rs_adam_emu|push_emu|pull_emu|attn_fwd_kernel|attn_bwd|all_gather_emu|fp_gemv' \
-        -s 36 -c 18 -o gpurun_out/prof_r2 python tools/ncu_targets.py
+        -s 36 -c 18 -o build/reports/prof_r2 python tools/ncu_targets.py
 
 Kernels: base pair GEMM (qkv fwd shape), extended GEMM gated NN / grouped NT / fp8 NT, emulated (4 logical ranks) fused
 reduce-scatter+AdamW, all-gather with flags, MoE push / pull, attention forward with the row-scatter epilogue."""

@@ -1,5 +1,5 @@
 """Prefill / mixed-batch timing of the ragged attention: atom-scheduled tcgen05 kernel vs the per-token SIMT kernel.
-Writes gpurun_out/paged_attn_bench.json (CUDA events, 3 warm-ups, 10 timed calls)."""
+Writes build/reports/paged_attn_bench.json (CUDA events, 3 warm-ups, 10 timed calls)."""
 import json
 import os
 import sys
@@ -57,8 +57,8 @@ def main():
            case("chunked prefill 512 @ 8192 seen", [(8192, 512)]),
            case("decode 64 seqs @ 2048", [(2048, 1)] * 64),
            case("mixed: prefill 2048 + 32 decodes @ 1024", [(0, 2048)] + [(1024, 1)] * 32)]
-    os.makedirs("gpurun_out", exist_ok=True)
-    json.dump(out, open("gpurun_out/paged_attn_bench.json", "w"), indent=1)
+    os.makedirs("build/reports", exist_ok=True)
+    json.dump(out, open("build/reports/paged_attn_bench.json", "w"), indent=1)
     for r in out:
         print(json.dumps(r))
 

@@ -1,6 +1,6 @@
 """Pipeline parallelism on real GPUs (torchrun, 2 or 4 ranks): PP=2 over NCCL p2p, DP = world / 2 with ZeRO-`--zero`
 inside each stage.  Compares the first batches' losses with a sequential fp32-master oracle on the same data and writes
-gpurun_out/pipe_gpu_check.json.
+build/reports/pipe_gpu_check.json.
 
     torchrun --nproc-per-node 2 tools/pipe_gpu_check.py --zero 1
     torchrun --nproc-per-node 4 tools/pipe_gpu_check.py --zero 3"""
@@ -84,8 +84,8 @@ def main():
                "ok": ok, "ms_total": e0.elapsed_time(e1), "backend": torch.distributed.get_backend()}
         print(json.dumps(out))
         if rank == 0:
-            os.makedirs("gpurun_out", exist_ok=True)
-            json.dump(out, open(f"gpurun_out/pipe_gpu_check_zero{a.zero}.json", "w"), indent=1)
+            os.makedirs("build/reports", exist_ok=True)
+            json.dump(out, open(f"build/reports/pipe_gpu_check_zero{a.zero}.json", "w"), indent=1)
     assert ok, (losses, want)
 
 

@@ -4,7 +4,7 @@ re-creating NCCL process groups (deepspeed/runtime/zero/stage_1_and_2.py:698-711
 
     python -m torch.distributed.run --nproc-per-node 8 --master-addr 127.0.0.1 --master-port 29565 tools/replica_avg_bench.py
 
-Device-timed (CUDA events), max over ranks; writes gpurun_out/replica_avg_bench.json."""
+Device-timed (CUDA events), max over ranks; writes build/reports/replica_avg_bench.json."""
 import json
 import os
 import sys
@@ -111,8 +111,8 @@ def main():
         sch.reshuffle()
     res["table_reshuffle_ms"] = (time.perf_counter() - t0) * 10
     if rank == 0:
-        os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-        json.dump(res, open(os.path.join(ROOT, "gpurun_out", "replica_avg_bench.json"), "w"), indent=1)
+        os.makedirs(os.path.join(ROOT, "build/reports"), exist_ok=True)
+        json.dump(res, open(os.path.join(ROOT, "build/reports", "replica_avg_bench.json"), "w"), indent=1)
         print(json.dumps(res))
     td.barrier()
     td.destroy_process_group()

@@ -18,7 +18,7 @@ def main():
     ap.add_argument("--layers", type=int, default=2)
     ap.add_argument("--seq", type=int, default=8192)
     ap.add_argument("--steps", type=int, default=2)
-    ap.add_argument("--out", default="gpurun_out/step_profile.json")
+    ap.add_argument("--out", default="build/reports/step_profile.json")
     ap.add_argument("--gaps", action="store_true", help="report idle gaps of the busiest stream and what ran meanwhile")
     ap.add_argument("--trace-kernel", default="", help="comma-separated kernel-name substrings: report which CPU ops launch them")
     a = ap.parse_args()

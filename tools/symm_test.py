@@ -2,7 +2,7 @@
 
     python -m torch.distributed.run --nproc-per-node 2 --master-addr 127.0.0.1 --master-port 29555 tools/symm_test.py
 
-Each rank prints nothing; rank 0 writes gpurun_out/symm_test.json (numerics + device-timed ms, max over ranks).
+Each rank prints nothing; rank 0 writes build/reports/symm_test.json (numerics + device-timed ms, max over ranks).
 """
 import json
 import os
@@ -136,8 +136,8 @@ def main():
     res["a2a_bytes_per_rank_out"] = rows_per * (world - 1) * M * 2
     res["watchdog"] = n.hang_info("symm")
     if rank == 0:
-        os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-        with open(os.path.join(ROOT, "gpurun_out", "symm_test.json"), "w") as f:
+        os.makedirs(os.path.join(ROOT, "build/reports"), exist_ok=True)
+        with open(os.path.join(ROOT, "build/reports", "symm_test.json"), "w") as f:
             json.dump(res, f, indent=1)
         print(json.dumps(res))
     td.barrier()

@@ -44,8 +44,8 @@ def int_layers():
                             "speedup": t_deq / t_fused, "gemv_weight_TBps": packed / t_fused / 1e9})
                 print(json.dumps(out[-1]))
             del q
-    os.makedirs("gpurun_out", exist_ok=True)
-    json.dump(out, open("gpurun_out/int_gemv_bench.json", "w"), indent=1)
+    os.makedirs("build/reports", exist_ok=True)
+    json.dump(out, open("build/reports/int_gemv_bench.json", "w"), indent=1)
 
 
 def main():
@@ -65,8 +65,8 @@ def main():
             out.append({"N": N, "K": K, "rows": rows, "fused_ms": t_fused, "dequant_gemm_ms": t_deq,
                         "speedup": t_deq / t_fused, "fused_weight_TBps": packed / t_fused / 1e9})
             print(json.dumps(out[-1]))
-    os.makedirs("gpurun_out", exist_ok=True)
-    json.dump(out, open("gpurun_out/w6a16_bench.json", "w"), indent=1)
+    os.makedirs("build/reports", exist_ok=True)
+    json.dump(out, open("build/reports/w6a16_bench.json", "w"), indent=1)
 
 
 if __name__ == "__main__":

@@ -67,8 +67,8 @@ def main():
         out["oracle_error"] = oracle_err
         out["ok"] = out["max_rel_diff_fused_vs_nccl"] < 2e-2
     if int(os.environ["RANK"]) == 0:
-        os.makedirs(os.path.join(ROOT, "gpurun_out"), exist_ok=True)
-        json.dump(out, open(os.path.join(ROOT, "gpurun_out", "z3_fused_check.json"), "w"), indent=1)
+        os.makedirs(os.path.join(ROOT, "build/reports"), exist_ok=True)
+        json.dump(out, open(os.path.join(ROOT, "build/reports", "z3_fused_check.json"), "w"), indent=1)
         print(json.dumps(out))
 
 
