@@ -10,6 +10,7 @@
 // Reference behaviour: deepspeed/inference/v2/kernels/core_ops/cuda_rms_norm/rms_norm_cuda.cu:19,84
 // (rms_norm / pre_rms_norm) and cuda_layer_norm/layer_norm_cuda.cu:31,220 (fused_ln /
 // fused_residual_ln) — forward only there; the training backward is new.
+#include <type_traits>
 #include "sxb_common.cuh"
 
 namespace sxb {
@@ -234,18 +235,28 @@ norm_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __re
     }
   }
   float* prow = partial + (long long)blockIdx.x * (kLayer ? 2 : 1) * H;
+  auto put = [&](auto wide) {
 #pragma unroll
-  for (int it = 0; it < ITERS; ++it) {
-    const int vi = threadIdx.x + it * kThreads;
-    if (vi < nvec) {
+    for (int it = 0; it < ITERS; ++it) {
+      const int vi = threadIdx.x + it * kThreads;
+      if (vi < nvec) {
 #pragma unroll
-      for (int k = 0; k < 8; k += 4) {
-        *reinterpret_cast<float4*>(prow + vi * 8 + k) = make_float4(dw_acc[it][k], dw_acc[it][k + 1], dw_acc[it][k + 2], dw_acc[it][k + 3]);
-        if (kLayer)
-          *reinterpret_cast<float4*>(prow + H + vi * 8 + k) = make_float4(db_acc[it][k], db_acc[it][k + 1], db_acc[it][k + 2], db_acc[it][k + 3]);
+        for (int hf = 0; hf < 2; ++hf) {
+          const int k = 4 * hf;
+          float* p = prow + vi * 8 + k;
+          float4 v = make_float4(dw_acc[it][k], dw_acc[it][k + 1], dw_acc[it][k + 2], dw_acc[it][k + 3]);
+#pragma unroll
+          for (int b = 0; b < (kLayer ? 2 : 1); ++b) {
+            if (b) v = make_float4(db_acc[it][k], db_acc[it][k + 1], db_acc[it][k + 2], db_acc[it][k + 3]), p += H;
+            if constexpr (decltype(wide)::value) *reinterpret_cast<float4*>(p) = v;
+            else p[0] = v.x, p[1] = v.y, p[2] = v.z, p[3] = v.w;
+          }
+        }
       }
     }
-  }
+  };
+  if ((reinterpret_cast<uintptr_t>(partial) & 15) == 0) put(std::true_type());
+  else put(std::false_type());               // the caller's scratch may start anywhere
 }
 
 // out[j] (+)= sum_b partial[b, j].  CTA: 32 channels x 8 runs of rows, merged in run order.

@@ -76,6 +76,29 @@ def test_norm_backward(rows, H, layer):
         assert float((a.grad.double() - c.grad).norm() / c.grad.norm()) < 4e-3          # one rounding to 16 bits (1.7e-3)
 
 
+@pytest.mark.parametrize("H", [768, 8192, 8200])
+@pytest.mark.parametrize("layer", [False, True])
+def test_norm_backward_with_scratch_that_starts_anywhere(H, layer):
+    rows = 300
+    mk = lambda *s: torch.randn(*s, device="cuda").bfloat16()  # noqa: E731
+    dy, x, w = mk(rows, H), mk(rows, H), mk(H)
+    mean, rstd = torch.zeros(rows, device="cuda"), torch.ones(rows, device="cuda")
+    room = torch.empty(lib.call("sxb_norm_bwd_scratch_elems", rows, H, int(layer)) + 4, device="cuda")
+    got = []
+    for at in range(4):
+        dx, dw, db = torch.empty_like(x), torch.empty_like(w), torch.empty_like(w)
+        tail = (room[at:].data_ptr(), rows, H, lib.dtype_code(x.dtype), 0, lib.stream_ptr())
+        if layer:
+            lib.call("sxb_layernorm_bwd", dy.data_ptr(), x.data_ptr(), w.data_ptr(), mean.data_ptr(), rstd.data_ptr(), None,
+                     dx.data_ptr(), dw.data_ptr(), db.data_ptr(), *tail)
+        else:
+            lib.call("sxb_rmsnorm_bwd", dy.data_ptr(), x.data_ptr(), w.data_ptr(), rstd.data_ptr(), None, dx.data_ptr(),
+                     dw.data_ptr(), *tail)
+        got.append((dx, dw, db) if layer else (dx, dw))
+    for other in got[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(got[0], other))
+
+
 @pytest.mark.parametrize("counts", [[3, 0, 5], [0, 0, 1], [1] * 40, [300, 2]])
 @pytest.mark.parametrize("width", [16, 2056, 4096])
 def test_routed_rows_activation(counts, width):
