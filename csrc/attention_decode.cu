@@ -270,7 +270,7 @@ static int launch(const Params& p, int n_atoms, int S, bool beside, cudaStream_t
 // its successor start early and shares no output with this one.
 int paged_decode(const void* q, const void* cache, void* out, const void* atoms, int n_atoms, const void* tables,
                  int max_blocks, int block_size, int Hq, int Hk, int D, long long q_stride, long long o_stride, float scale,
-                 bool beside, int sms, cudaStream_t stream) {
+                 bool beside, cudaStream_t stream) {
   decode::Params p;
   p.q = (const __nv_bfloat16*)q; p.cache = (const __nv_bfloat16*)cache; p.out = (__nv_bfloat16*)out;
   p.atoms = (const int*)atoms; p.tables = (const int*)tables;
@@ -280,7 +280,7 @@ int paged_decode(const void* q, const void* cache, void* out, const void* atoms,
   // enough CTAs for four waves of two per SM: contexts differ, and a sequence's CTAs end with its context (61 requests: 109
   // us with two waves, 104 with four, 117 with eight, where starting and merging a CTA costs more than the balance gives)
   int S = 8;
-  while (S > 1 && (long long)Hk * n_atoms * S > 8LL * sms) S >>= 1;
+  while (S > 1 && (long long)Hk * n_atoms * S > 8LL * num_sms()) S >>= 1;
   return D == 128 ? decode::launch<128>(p, n_atoms, S, beside, stream) : decode::launch<64>(p, n_atoms, S, beside, stream);
 }
 

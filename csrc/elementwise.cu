@@ -427,7 +427,7 @@ SXB_API int sxb_gated_act_groups(const void* in, void* out, const void* offsets,
   if (F % 8) return SXB_ERR_UNSUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
   const int parts = (F / 8 + kThreads - 1) / kThreads;        // a word per thread while the rows are few
-  const dim3 grid(n_rows, n_rows >= 148 * 16 ? 1 : parts);
+  const dim3 grid(n_rows, n_rows >= 16 * num_sms() ? 1 : parts);
   DISPATCH_16(dtype, (gated_groups_kernel<T><<<grid, kThreads, 0, s>>>((const T*)in, (T*)out, (const int*)offsets,
                                                                      (const int*)counts, groups, F, act)));
   SXB_CHECK_LAUNCH();

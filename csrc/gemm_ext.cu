@@ -556,17 +556,6 @@ static int make_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t col
   return encode_tensor_map(m, esize == 2 ? kBF16 : kU8, 2, ptr, dims, strides, box, 128);
 }
 
-static int num_sms() {
-  static int n = 0;
-  if (!n) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (n <= 0) n = 148;
-  }
-  return n;
-}
-
 }  // namespace gemmx
 }  // namespace sxb
 

@@ -638,17 +638,6 @@ static int make_map_2d(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t 
   return r == CUDA_SUCCESS ? SXB_OK : SXB_ERR_DRIVER;
 }
 
-static int g_num_sms = 0;
-static int num_sms() {
-  if (!g_num_sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev);
-    if (g_num_sms <= 0) g_num_sms = 148;
-  }
-  return g_num_sms;
-}
-
 template <int BN, int STAGES>
 static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc,
                   const Params& p, int max_ctas, cudaStream_t stream) {

@@ -359,7 +359,7 @@ static int row_grid(long long items, int max_ctas) {
 // 8.2 now (its padding rows are left alone there), pull 16.9 us, 7.2 now.
 static int row_parts(long long rows, int H) {
   int parts = 1;
-  while (parts < 16 && rows * parts * 2 <= 148 * 2 * 8 && H >= parts * 2 * 256) parts *= 2;
+  while (parts < 16 && rows * parts * 2 <= 2 * 8 * num_sms() && H >= parts * 2 * 256) parts *= 2;
   return parts;
 }
 

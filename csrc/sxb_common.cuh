@@ -515,6 +515,16 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // true only for ordinary allocations of the current device, whole extent inside one allocation, not registered as
 // foreign (tensormap.cu) — the precondition for covering a range with a TMA multicast tensor map
 bool range_is_local(const void* p, long long bytes);
+// SMs of the current device (asked once).
+static inline int num_sms() {
+  static const int n = [] {
+    int dev = 0, v = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    return v > 0 ? v : 148;
+  }();
+  return n;
+}
 int encode_tensor_map(CUtensorMap* m, int dtype_code, int rank, const void* ptr,
                       const unsigned long long* dims, const unsigned long long* strides_bytes,
                       const unsigned int* box, int swizzle_bytes);
