@@ -2122,9 +2122,12 @@ SXB_API int sxb_linear_recurrence(const void* kvec, const void* qvec, long long 
   else LAUNCH_REC(32, D, 8, CH, 1)
   // Two columns per lane share every k and q word that is read from shared memory (and every copy into it); with one column
   // the chip has twice the warps.  Two win once one column would fill the chip one and a half times (us, one | two columns:
-  // delta rule, 8 sequences, 4096 rows, 32 heads 746 | 528; 3, 2300, 16: 303 | 277; 1, 2000, 32: 512 | 440; 64 decode rows, 16
-  // heads 36 | 26), below that one does (1, 4096, 16: 833 | 892).  Every column's sums are taken in the same order either way.
-  const bool two = (long long)((dv + 15) / 16) * H * n_seqs >= 222;
+  // delta rule, 8 sequences, 4096 rows, 32 heads 746 | 528; 3, 2300, 16: 303 | 277; 1, 2000, 32: 512 | 440), below that one
+  // does (1, 4096, 16: 833 | 892), and where the columns fill blocks of 32: lanes without a column walk along (16 sequences
+  // of 256 rows, 16 heads, keys of 64: dv = 16 58 | 79, 32 79 | 77, 48 106 | 112).  Every column's sums are taken in the same
+  // order either way.
+  const int blocks = (dv + 15) / 16;
+  const bool two = blocks % 2 == 0 && 2LL * blocks * H * n_seqs >= 3LL * num_sms();
   if (decay_channels) {
     if (delta) { LAUNCH_REC_N(true, true); } else { LAUNCH_REC_N(false, true); }
   } else {
