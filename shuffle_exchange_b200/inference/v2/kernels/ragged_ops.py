@@ -5,6 +5,7 @@ Every wrapper has a PyTorch branch with identical semantics (CPU execution and t
 """
 from __future__ import annotations
 
+import functools
 import math
 
 import torch
@@ -138,6 +139,11 @@ def paged_attention_atoms(q: torch.Tensor, cache: torch.Tensor, atoms: torch.Ten
     return out
 
 
+@functools.lru_cache(None)
+def _sm_count(device: int) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
 def ragged_attention(q: torch.Tensor, cache: torch.Tensor, batch, scale: float = None) -> torch.Tensor:
     """Attention of a finalized ragged batch: atoms on the tensor cores where the layout allows, else per token."""
     atoms = batch.atoms() if hasattr(batch, "atoms") else None
@@ -147,9 +153,15 @@ def ragged_attention(q: torch.Tensor, cache: torch.Tensor, batch, scale: float =
         if hasattr(batch, "atoms_longer_than"):
             if group <= 16 and (q.data_ptr() | cache.data_ptr()) % 16 == 0:
                 n_few = atoms.shape[0] - batch.atoms_longer_than(16 // group)
-            if group > 1 and 128 % group == 0 and batch.atoms_longer_than(128 // group) == 0:
-                # the remainders of longer portions run with them: two of them alone held the chip for 46 of 160 us
-                n_packed = atoms.shape[0] - n_few
+            n_long = batch.atoms_longer_than(128 // group) if group > 1 and 128 % group == 0 else atoms.shape[0]
+            short = atoms.shape[0] - n_few - n_long
+            # Short atoms (chunk remainders, drafts under verification, decode tokens of groups beyond 16) have a tile per
+            # key/value head in a launch of their own, and walk their keys there once.  A few of them beside longer atoms run
+            # with those, a tile per query head, as long as their tiles fit the chip once (two per SM): 32/8 heads, one
+            # portion of 777 rows beside n of 20 behind 1500 keys, own launch | with it, us: n = 2 75 | 40, 8 89 | 67, 16
+            # 95 | 101, 64 153 | 298; 64/2 heads, a portion of 200 and 24 decode tokens 69 | 208.
+            if n_long == 0 or short * q.shape[1] > 2 * _sm_count(q.device.index):
+                n_packed = max(short, 0)
         return paged_attention_atoms(q, cache, atoms, batch.block_tables(), scale, n_packed, n_few)
     return paged_attention(q, cache, batch.token_to_seq(), batch.token_positions(), batch.block_tables(), scale)
 

@@ -92,3 +92,28 @@ def test_captured_step_keeps_its_order():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(twice, first)
+
+
+PACKED = [
+    # plan, page, query heads, kv heads, head size, atoms packed into the tile with their group, atoms of the decode kernel
+    ([(40, 20), (0, 32), (300, 9)], 64, 8, 2, 128, 3, 0),
+    ([(40, 20), (0, 32), (300, 9)], 64, 8, 2, 64, 3, 0),
+    ([(40, 20), (0, 32), (700, 1), (300, 9), (5, 1)], 64, 8, 2, 128, 3, 2),
+    ([(31, 17), (700, 1), (64, 64)], 32, 8, 4, 64, 2, 1),
+    ([(0, 200)] + [(50 + 90 * i, 8 + i) for i in range(10)] + [(333, 1)], 64, 32, 8, 128, 10, 1),
+    ([(0, 200)] + [(50 + 90 * i, 8 + i) for i in range(9)] + [(333, 1)], 64, 32, 8, 128, 0, 1),
+    ([(100 + 61 * i, 1) for i in range(12)], 64, 32, 1, 128, 12, 0),
+    ([(0, 150)] + [(100 + 61 * i, 1 + i % 4) for i in range(12)], 64, 32, 1, 64, 12, 0),
+    ([(0, 150)] + [(100 + 61 * i, 1) for i in range(4)], 64, 32, 1, 128, 0, 0),
+]
+
+
+@pytest.mark.parametrize("plan,page,Hq,Hk,D,n_packed,n_few", PACKED)
+def test_which_atoms_share_a_tile(plan, page, Hq, Hk, D, n_packed, n_few, monkeypatch):
+    """Short atoms have a launch of their own when they are alone or many, run with the longer ones when they are few, and
+    decode tokens have theirs in either case; all of it against the oracle."""
+    seen, run = [], R.paged_attention_atoms
+    monkeypatch.setattr(R, "paged_attention_atoms", lambda *a: (seen.append(a[5:7]), run(*a))[1])
+    monkeypatch.setattr(R, "_sm_count", lambda device: 148)
+    test_against_the_oracle(plan, page, Hq, Hk, D)
+    assert set(seen) == {(n_packed, n_few)}
