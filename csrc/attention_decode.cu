@@ -7,8 +7,8 @@
 // distributed shared memory in rank order.
 // What bounds it: the bytes of K and V (two CTAs per SM hold 128 KB of them in flight).  The 128-row tile kernel that served
 // these tokens spent a 128 x 64 MMA and a 64-wide softmax row on four valid rows and gave a sequence one CTA per head: 61
-// requests around 2000 tokens, 32 / 8 heads of 128: 132 us, 104 now (floor 78); 128 of 4000: 323 (floor 319); a few short
-// requests 62 -> 19.
+// requests around 2000 tokens, 32 / 8 heads of 128: 127 us, 80 now (floor 78); 100 of 4000: 336, 242; 8 of 500: 17.7, 8.5; 40
+// of 100: 14.5, 9.2.
 #include "mma_sync.cuh"
 #include <cuda_pipeline.h>
 
@@ -267,20 +267,26 @@ static int launch(const Params& p, int n_atoms, int S, bool beside, cudaStream_t
 }  // namespace decode
 
 // Attention atoms of at most 16 / group queries each (see the file's head).  `beside`: the stream's previous kernel lets
-// its successor start early and shares no output with this one.
+// its successor start early and shares no output with this one.  `keys`, `most`: keys of all atoms together and of the longest
+// one, 0 where the caller does not know.
 int paged_decode(const void* q, const void* cache, void* out, const void* atoms, int n_atoms, const void* tables,
                  int max_blocks, int block_size, int Hq, int Hk, int D, long long q_stride, long long o_stride, float scale,
-                 bool beside, cudaStream_t stream) {
+                 long long keys, int most, bool beside, cudaStream_t stream) {
   decode::Params p;
   p.q = (const __nv_bfloat16*)q; p.cache = (const __nv_bfloat16*)cache; p.out = (__nv_bfloat16*)out;
   p.atoms = (const int*)atoms; p.tables = (const int*)tables;
   p.max_blocks = max_blocks; p.block_size = block_size; p.Hk = Hk; p.group = Hq / Hk;
   p.shift = (block_size & (block_size - 1)) == 0 ? __builtin_ctz(block_size) : -1;
   p.q_stride = q_stride; p.o_stride = o_stride; p.scale = scale; p.after = beside ? 1 : 0;
-  // enough CTAs for four waves of two per SM: contexts differ, and a sequence's CTAs end with its context (61 requests: 109
-  // us with two waves, 104 with four, 117 with eight, where starting and merging a CTA costs more than the balance gives)
+  // CTAs per sequence: as many as keep the grid within one and a half waves of two per SM, since starting and merging a CTA
+  // costs 4 us of a wave (us, up to one and a half | four waves: 61 requests of 2048 80 | 94, 40 of 100 9 | 16, 24 of 6000 93 |
+  // 101), and no more than have a step each (4 requests of 40 keys, 32 key/value heads: 4.3 with one, 8.0 with eight).
+  // More, up to four waves, only where one context would be walked long after the others: its warps have twenty steps or more, and
+  // half as many again as the average of the chip's (50 requests of 30 keys beside 3 of 8000: 125 with one, 71 with two).
+  const long long ctas = (long long)Hk * n_atoms, sms = num_sms(), slots = (D == 128 ? 2 : 4) * sms;
   int S = 8;
-  while (S > 1 && (long long)Hk * n_atoms * S > 8LL * num_sms()) S >>= 1;
+  while (S > 1 && (ctas * S > 3 * sms || (most > 0 && S / 2 * decode::kWarps * decode::kKeys >= most))) S >>= 1;
+  while (S < 8 && 2 * S * ctas <= 8 * sms && most >= 20 * S * decode::kWarps * decode::kKeys && 2 * most * slots > 3 * S * keys * Hk) S <<= 1;
   return D == 128 ? decode::launch<128>(p, n_atoms, S, beside, stream) : decode::launch<64>(p, n_atoms, S, beside, stream);
 }
 

@@ -610,6 +610,12 @@ int sxb_attn_fwd_atoms_few(const void* q, const void* cache, void* out, const vo
                            int n_packed, int n_few, const void* block_tables, int max_blocks, int n_blocks,
                            int block_size, int T, int Hq, int Hk, int D, long long q_stride, long long o_stride,
                            float scale, void* stream);
+/* The same; few_keys, few_most: keys that the last n_few atoms see together and that the one with most of them sees (how many
+ * CTAs share a sequence); 0 where the caller does not know. */
+int sxb_attn_fwd_atoms_keys(const void* q, const void* cache, void* out, const void* atoms, int n_atoms, int n_packed,
+                            int n_few, long long few_keys, int few_most, const void* block_tables, int max_blocks,
+                            int n_blocks, int block_size, int T, int Hq, int Hk, int D, long long q_stride,
+                            long long o_stride, float scale, void* stream);
 
 /* ---- csrc/elementwise.cu */
 /* x [n] (16-bit, n a multiple of 8, 16-byte aligned) *= *scale (fp32 on the device), in place. */

@@ -19,6 +19,7 @@ _lib.register({
     "sxb_paged_attention": "pppppp" "iiiiii" "l" "f" "p",
     "sxb_attn_fwd_atoms": "ppp" "pii" "piii" "iiii" "ll" "f" "p",
     "sxb_attn_fwd_atoms_few": "ppp" "piii" "piii" "iiii" "ll" "f" "p",
+    "sxb_attn_fwd_atoms_keys": "ppp" "piii" "li" "piii" "iiii" "ll" "f" "p",
 })
 
 
@@ -121,20 +122,21 @@ def atoms_supported(q: torch.Tensor, cache: torch.Tensor) -> bool:
 
 
 def paged_attention_atoms(q: torch.Tensor, cache: torch.Tensor, atoms: torch.Tensor, block_tables: torch.Tensor,
-                          scale: float = None, n_packed: int = 0, n_few: int = 0) -> torch.Tensor:
+                          scale: float = None, n_packed: int = 0, n_few: int = 0, few_keys=(0, 0)) -> torch.Tensor:
     """The same attention as :func:`paged_attention`, scheduled by attention atoms on the tcgen05 flash kernel: one CTA
     per (atom, q head) runs 128 queries of one sequence against that sequence's pages, K/V tiles fetched by TMA through
-    the block table (``csrc/attention.cu``: ``sxb_attn_fwd_atoms``).  Prefill re-reads K/V once per 128 queries instead
+    the block table (``csrc/attention.cu``: ``sxb_attn_fwd_atoms_keys``).  Prefill re-reads K/V once per 128 queries instead
     of once per query.  ``n_packed``: that many atoms at the end have at most ``128 // (n_q // n_kv)`` queries and run
     with the GQA group packed into the tile (K/V read once per KV head).  ``n_few``: that many atoms behind them have at
     most ``16 // (n_q // n_kv)`` queries and run one warp per 16 keys, their keys dealt out over a cluster of CTAs (decode
-    tokens; ``csrc/attention_decode.cu``)."""
+    tokens; ``csrc/attention_decode.cu``).  ``few_keys``: the keys that those see together and that the longest of them sees,
+    zeros where the caller does not know."""
     T, n_q, D = q.shape
     n_kv = cache.shape[3]
     scale = 1.0 / math.sqrt(D) if scale is None else scale
     out = torch.empty(T, n_q, D, dtype=q.dtype, device=q.device)
-    _lib.attn_call("sxb_attn_fwd_atoms_few", q.data_ptr(), cache.data_ptr(), out.data_ptr(), atoms.data_ptr(), atoms.shape[0],
-              int(n_packed), int(n_few), block_tables.data_ptr(), block_tables.shape[1], cache.shape[0], cache.shape[1], T, n_q, n_kv, D,
+    _lib.attn_call("sxb_attn_fwd_atoms_keys", q.data_ptr(), cache.data_ptr(), out.data_ptr(), atoms.data_ptr(), atoms.shape[0],
+              int(n_packed), int(n_few), *few_keys, block_tables.data_ptr(), block_tables.shape[1], cache.shape[0], cache.shape[1], T, n_q, n_kv, D,
               q.stride(0), out.stride(0), float(scale), _lib.stream_ptr())
     return out
 
@@ -149,10 +151,11 @@ def ragged_attention(q: torch.Tensor, cache: torch.Tensor, batch, scale: float =
     atoms = batch.atoms() if hasattr(batch, "atoms") else None
     if atoms is not None and atoms.shape[0] > 0 and atoms_supported(q, cache):
         group = q.shape[1] // cache.shape[3]
-        n_packed = n_few = 0
+        n_packed, n_few, few_keys = 0, 0, (0, 0)
         if hasattr(batch, "atoms_longer_than"):
             if group <= 16 and (q.data_ptr() | cache.data_ptr()) % 16 == 0:
                 n_few = atoms.shape[0] - batch.atoms_longer_than(16 // group)
+                few_keys = batch.last_atoms_keys(n_few) if hasattr(batch, "last_atoms_keys") else (0, 0)
             n_long = batch.atoms_longer_than(128 // group) if group > 1 and 128 % group == 0 else atoms.shape[0]
             short = atoms.shape[0] - n_few - n_long
             # Short atoms (chunk remainders, drafts under verification, decode tokens of groups beyond 16) have a tile per
@@ -162,7 +165,7 @@ def ragged_attention(q: torch.Tensor, cache: torch.Tensor, batch, scale: float =
             # 95 | 101, 64 153 | 298; 64/2 heads, a portion of 200 and 24 decode tokens 69 | 208.
             if n_long == 0 or short * q.shape[1] > 2 * _sm_count(q.device.index):
                 n_packed = max(short, 0)
-        return paged_attention_atoms(q, cache, atoms, batch.block_tables(), scale, n_packed, n_few)
+        return paged_attention_atoms(q, cache, atoms, batch.block_tables(), scale, n_packed, n_few, few_keys)
     return paged_attention(q, cache, batch.token_to_seq(), batch.token_positions(), batch.block_tables(), scale)
 
 

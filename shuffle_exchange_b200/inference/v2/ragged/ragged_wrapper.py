@@ -6,7 +6,7 @@ per-sequence info]`` and
 is uploaded with a single ``cudaMemcpyAsync`` in ``finalize`` (the reference uses three pinned "fast host buffers",
 ``ragged/csrc/fast_host_buffer.cu``).  The attention atoms (one per 128-query tile of a sequence, with the KV extent
 it attends to) are cut by the native scheduler ``sxbh_build_atoms`` (``csrc/host/ragged_host.cpp``) at ``finalize``
-and consumed by the tensor-core paged attention kernel (``sxb_attn_fwd_atoms``).
+and consumed by the tensor-core paged attention kernels (``sxb_attn_fwd_atoms_keys``).
 
 The upload is asynchronous and forwards may be queued without a synchronisation between them, so the batches take turns over
 ``STAGING_BUFFERS`` pinned buffers; a buffer is written again only when the upload that read it has completed.
@@ -103,7 +103,8 @@ class RaggedBatchWrapper:
             # (the kernel for the long ones walks them from the end: a sequence's later tiles have more keys)
             live = self._tables[self._turn][5][: self._n_atoms]
             live[:] = live[np.lexsort((np.where(live[:, 2] <= 16, -live[:, 5], 0), -live[:, 2]))]
-            self._atom_q_lens = live[:, 2].copy()
+            self._atom_q_lens, self._atom_keys = live[:, 2].copy(), live[:, 5].copy()
+            self._last_keys = {}
         self._live = {}
         self._dev.copy_(self._host, non_blocking=True)
         if self._dev.is_cuda:
@@ -148,6 +149,17 @@ class RaggedBatchWrapper:
     def atoms_longer_than(self, q_len: int) -> int:
         """How many (leading) atoms have more than ``q_len`` queries; host-side, no synchronisation."""
         return int(np.count_nonzero(self._atom_q_lens > q_len)) if self._n_atoms else 0
+
+    def last_atoms_keys(self, n: int):
+        """``(keys that the last n atoms see together, keys that the longest of them sees)``; host-side, looked up once per
+        batch."""
+        if not self._n_atoms or n <= 0:
+            return 0, 0
+        got = self._last_keys.get(n)
+        if got is None:
+            keys = self._atom_keys[-n:]
+            got = self._last_keys[n] = int(keys.sum(dtype=np.int64)), int(keys.max())
+        return got
 
     def single_rows(self) -> bool:
         """Whether every sequence of the batch brings exactly one token (a pure decode step); host-side."""

@@ -105,6 +105,9 @@ PACKED = [
     ([(100 + 61 * i, 1) for i in range(12)], 64, 32, 1, 128, 12, 0),
     ([(0, 150)] + [(100 + 61 * i, 1 + i % 4) for i in range(12)], 64, 32, 1, 64, 12, 0),
     ([(0, 150)] + [(100 + 61 * i, 1) for i in range(4)], 64, 32, 1, 128, 0, 0),
+    ([(9 * i, 1) for i in range(8)], 64, 32, 2, 128, 0, 8),
+    ([(30, 1)] * 20 + [(5000, 1), (2700, 1)], 64, 32, 8, 128, 0, 22),            # few long contexts beside short ones
+    ([(11 * i, 1) for i in range(60)], 64, 32, 8, 64, 0, 60),
 ]
 
 
