@@ -690,15 +690,22 @@ static int skinny_split(int tiles, int num_kb) {
   return 2 * tiles <= 2 * sms && num_kb >= 4 ? 2 : 1;
 }
 
-// Whether an NT product takes the skinny kernel instead of the persistent ones (measured on projections with N = 768 ..
-// 32000, K = 768 .. 14336; us, persistent | skinny).  Up to 32 tokens always: 4096 x 4096 27.6 | 10.9, 28672 x 4096 43.8 | 42.6.
+// Whether an NT product takes the skinny kernel instead of the persistent ones (measured on N = 64 .. 32000, K = 64 .. 14336; us,
+// persistent | skinny).  Never where K is too short for its fixed cost, which grows with its token tile (4 us for 16 tokens, 5 for
+// 32, 6 for 64, 7 to 9 for 128), while the persistent kernels' is 3.5 to 4.5 and grows with K, less so with the narrow tile of
+// N <= 128: 4096 x 64, 32 tokens 4.7 | 5.0, 128 tokens 4.8 | 8.9; 2048 x 256, 64 tokens 5.5 | 6.1; 2048 x 512, 64 tokens 7.2 | 6.7;
+// 14336 x 512, 64 tokens 8.7 | 9.4; 64 x 256, 32 tokens 4.2 | 4.8, 256 tokens 4.3 | 7.7; 64 x 1536, 256 tokens 8.5 | 6.5.
+// Beyond that up to 32 tokens always: 4096 x 4096 27.6 | 10.9, 28672 x 4096 43.8 | 42.6.
 // Up to 64 tokens while its 128-row tiles fit the chip once: 16384 x 2048 18.9 | 17.7, but 32000 x 2048 25.7 | 27.4.  More
 // tokens only while the tiles are few for the length of K, which is when the persistent kernels leave SMs without a
 // tile: 4096 x 14336, 512 tokens 68.8 | 58.4; 2048 x 2048, 512 tokens 14.8 | 12.5; 4096 x 768, 256 tokens 8.2 | 9.7;
 // 6144 x 4096, 512 tokens 25.2 | 32.9.
 static bool use_skinny(int M, int N, int K) {
-  if (M <= 32) return true;
   const long long tiles = (long long)((N + 127) / 128) * ((M + 127) / 128);
+  const int BN = M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
+  const bool wide = tiles > (BN == 16 ? num_sms() : num_sms() / 2);
+  if (K < (N <= 128 ? (BN <= 32 ? 16 : 12) * BN : wide ? 12 * BN : BN == 16 ? 0 : 6 * BN)) return false;
+  if (M <= 32) return true;
   if (M <= 64 && tiles <= num_sms()) return true;
   return tiles <= 128 && tiles <= K / 32;
 }
