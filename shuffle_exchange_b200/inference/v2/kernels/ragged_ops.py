@@ -162,7 +162,7 @@ def ragged_attention(q: torch.Tensor, cache: torch.Tensor, batch, scale: float =
             # key/value head in a launch of their own, and walk their keys there once.  A few of them beside longer atoms run
             # with those, a tile per query head, as long as their tiles fit the chip once (two per SM): 32/8 heads, one
             # portion of 777 rows beside n of 20 behind 1500 keys, own launch | with it, us: n = 2 75 | 40, 8 89 | 67, 16
-            # 95 | 101, 64 153 | 298; 64/2 heads, a portion of 200 and 24 decode tokens 69 | 208.
+            # 90 | 101, 64 142 | 298; 64/2 heads, a portion of 200 and 24 decode tokens 69 | 208.
             if n_long == 0 or short * q.shape[1] > 2 * _sm_count(q.device.index):
                 n_packed = max(short, 0)
         return paged_attention_atoms(q, cache, atoms, batch.block_tables(), scale, n_packed, n_few, few_keys)
