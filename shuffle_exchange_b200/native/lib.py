@@ -118,9 +118,9 @@ def load() -> ctypes.CDLL:
                               "shuffle_exchange_b200.native.build`")
         lib = ctypes.CDLL(str(path), mode=ctypes.RTLD_GLOBAL)
         _bind(lib, SIGNATURES)
-        if _RANKS > 1:
-            lib.sxb_attn_note_ranks(_RANKS)
         _LIB = lib
+        if _RANKS > 1:                  # behind the line above: a count that arrives meanwhile is told by one side or both
+            lib.sxb_attn_note_ranks(_RANKS)
         return lib
 
 
