@@ -686,7 +686,8 @@ class _FlashAttn(torch.autograd.Function):
         _n.attn_call("sxb_attn_bwd", q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), dout.data_ptr(),
                 lse.data_ptr(), delta.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr(),
                 B, S, Hq, Hk, D, q.stride(1), k.stride(1), v.stride(1), out.stride(1), dout.stride(1),
-                dq.stride(1), dk.stride(1), dv.stride(1), int(ctx.causal), float(ctx.scale), _n.stream_ptr())
+                *(dqkv.stride(1),) * 3,      # not that of the views, which is another one where S = 1
+                int(ctx.causal), float(ctx.scale), _n.stream_ptr())
         return dq, dk, dv, None, None
 
 
