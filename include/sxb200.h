@@ -31,7 +31,7 @@ int sxb_attn_hang_info(unsigned int* out_host);
  * across a cluster only do so when the tensor map covers this GPU's memory alone: ordinary allocation of the
  * current device, whole extent inside one allocation, not registered here.  comm/symm.py registers every peer /
  * multicast mapping of symmetric memory.  sxb_range_is_local returns 1/0; sxb_attn_would_multicast reports which
- * kernel family (1 = 2-CTA multicast, 0 = single CTA) sxb_attn_fwd / the dQ pass would take for these K/V. */
+ * kernel family (1 = 2-CTA multicast, 0 = single CTA) sxb_attn_fwd would take for these K/V. */
 int sxb_register_foreign_range(const void* p, long long bytes);
 int sxb_range_is_local(const void* p, long long bytes);
 /* Tells how many ranks the program has (sxb_attn_*: multicast kernels are for programs of one rank; WORLD_SIZE of a launcher
