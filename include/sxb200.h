@@ -281,6 +281,26 @@ int sxb_paged_attention(const void* q, void* out, const void* cache, const void*
                         const void* block_tables, int n_tokens, int max_blocks, int block_size, int Hq, int Hk,
                         int D, long long q_stride, float scale, void* stream);
 
+/* One forward of a dense Llama (RMS norms, rotary, grouped attention, gated SiLU) over a ragged batch: the launches of
+ * sxb_ragged_embed ... sxb_gemm_bf16 that its operators would make, from one call.  Fields of 8 bytes throughout; bf16 weights with
+ * unit inner stride and 16-byte aligned rows; every buffer is the caller's and is written whole before it is read. */
+struct sxb_ragged_llama {
+  const void *ids, *tok_seq, *tok_pos, *block_tables, *last_token, *atoms; /* the batch's tables (int32) */
+  const void *embed, *norm, *head;
+  void* buf[3];                                   /* [T, H] each */
+  void *x, *qkv, *ctx, *gate_up, *act, *rows;     /* [T, H], [T, (Hq + 2 Hk) D], [T, Hq D], [T, 2 F], [T, F], [n_rows, H] */
+  void* logits;                                   /* [n_rows, vocab] */
+  long long ld_head, T, H, Hq, Hk, D, F, vocab, n_rows, max_blocks, n_blocks, block_size;
+  long long n_atoms, n_packed, n_few, few_keys, few_most; /* as for sxb_attn_fwd_atoms_keys */
+};
+struct sxb_ragged_llama_layer {
+  const void *ln1, *wqkv, *wo, *ln2, *w_gate_up, *w_down;
+  void* cache;                                    /* [n_blocks, block_size, 2, Hk, D] */
+  long long ld_qkv, ld_o, ld_gate_up, ld_down;
+};
+int sxb_ragged_llama_forward(const struct sxb_ragged_llama* m, const struct sxb_ragged_llama_layer* layers,
+                             int n_layers, float eps, float theta, float scale, void* stream);
+
 /* ---- csrc/quantize.cu */
 /* Grouped integer quantisation.  in: [groups, group_size] of `dtype`; q: groups*group_size*bits/8 bytes;
  * scales: fp32 [groups] (symmetric) or [groups, 2] = (scale, min) (asymmetric).  nodes/devs > 1 select the

@@ -19,6 +19,7 @@ _lib.register({
     "sxb_paged_attention": "pppppp" "iiiiii" "l" "f" "p",
     "sxb_attn_fwd_atoms": "ppp" "pii" "piii" "iiii" "ll" "f" "p",
     "sxb_attn_fwd_atoms_few": "ppp" "piii" "piii" "iiii" "ll" "f" "p",
+    "sxb_ragged_llama_forward": "pp" "i" "fff" "p",
     "sxb_attn_fwd_atoms_keys": "ppp" "piii" "li" "piii" "iiii" "ll" "f" "p",
 })
 
@@ -113,12 +114,17 @@ def paged_attention(q: torch.Tensor, cache: torch.Tensor, tok_seq: torch.Tensor,
     return out
 
 
+def atoms_layout_ok(cache: torch.Tensor, head_dim: int) -> bool:
+    """Whether the tensor-core atom kernel takes this cache."""
+    bs = cache.shape[1]
+    return (cache.is_cuda and cache.dtype == torch.bfloat16 and head_dim in (64, 128) and cache.is_contiguous()
+            and bs % 8 == 0 and (64 % bs == 0 if bs < 64 else bs % 64 == 0))
+
+
 def atoms_supported(q: torch.Tensor, cache: torch.Tensor) -> bool:
     """Whether the tensor-core atom kernel takes this query / cache layout."""
-    bs = cache.shape[1]
-    return (q.is_cuda and q.dtype == torch.bfloat16 and cache.dtype == torch.bfloat16 and q.shape[-1] in (64, 128)
-            and q.stride(2) == 1 and q.stride(1) == q.shape[-1] and q.stride(0) % 8 == 0 and cache.is_contiguous()
-            and bs % 8 == 0 and (64 % bs == 0 if bs < 64 else bs % 64 == 0))
+    return (q.is_cuda and q.dtype == torch.bfloat16 and q.stride(2) == 1 and q.stride(1) == q.shape[-1]
+            and q.stride(0) % 8 == 0 and atoms_layout_ok(cache, q.shape[-1]))
 
 
 def paged_attention_atoms(q: torch.Tensor, cache: torch.Tensor, atoms: torch.Tensor, block_tables: torch.Tensor,
@@ -146,25 +152,34 @@ def _sm_count(device: int) -> int:
     return torch.cuda.get_device_properties(device).multi_processor_count
 
 
+def atoms_split(batch, n_atoms: int, n_q: int, n_kv: int, aligned: bool, device: int):
+    """``(n_packed, n_few, few_keys)`` of :func:`paged_attention_atoms` for a batch's atoms; ``aligned``: queries and cache
+    start on 16 bytes."""
+    if not hasattr(batch, "atoms_longer_than"):
+        return 0, 0, (0, 0)
+    group = n_q // n_kv
+    n_packed, n_few, few_keys = 0, 0, (0, 0)
+    if group <= 16 and aligned:
+        n_few = n_atoms - batch.atoms_longer_than(16 // group)
+        few_keys = batch.last_atoms_keys(n_few) if hasattr(batch, "last_atoms_keys") else (0, 0)
+    n_long = batch.atoms_longer_than(128 // group) if group > 1 and 128 % group == 0 else n_atoms
+    short = n_atoms - n_few - n_long
+    # Short atoms (chunk remainders, drafts under verification, decode tokens of groups beyond 16) have a tile per
+    # key/value head in a launch of their own, and walk their keys there once.  A few of them beside longer atoms run
+    # with those, a tile per query head, as long as their tiles fit the chip once (two per SM): 32/8 heads, one
+    # portion of 777 rows beside n of 20 behind 1500 keys, own launch | with it, us: n = 2 75 | 40, 8 89 | 67, 16
+    # 90 | 101, 64 142 | 298; 64/2 heads, a portion of 200 and 24 decode tokens 69 | 208.
+    if n_long == 0 or short * n_q > 2 * _sm_count(device):
+        n_packed = max(short, 0)
+    return n_packed, n_few, few_keys
+
+
 def ragged_attention(q: torch.Tensor, cache: torch.Tensor, batch, scale: float = None) -> torch.Tensor:
     """Attention of a finalized ragged batch: atoms on the tensor cores where the layout allows, else per token."""
     atoms = batch.atoms() if hasattr(batch, "atoms") else None
     if atoms is not None and atoms.shape[0] > 0 and atoms_supported(q, cache):
-        group = q.shape[1] // cache.shape[3]
-        n_packed, n_few, few_keys = 0, 0, (0, 0)
-        if hasattr(batch, "atoms_longer_than"):
-            if group <= 16 and (q.data_ptr() | cache.data_ptr()) % 16 == 0:
-                n_few = atoms.shape[0] - batch.atoms_longer_than(16 // group)
-                few_keys = batch.last_atoms_keys(n_few) if hasattr(batch, "last_atoms_keys") else (0, 0)
-            n_long = batch.atoms_longer_than(128 // group) if group > 1 and 128 % group == 0 else atoms.shape[0]
-            short = atoms.shape[0] - n_few - n_long
-            # Short atoms (chunk remainders, drafts under verification, decode tokens of groups beyond 16) have a tile per
-            # key/value head in a launch of their own, and walk their keys there once.  A few of them beside longer atoms run
-            # with those, a tile per query head, as long as their tiles fit the chip once (two per SM): 32/8 heads, one
-            # portion of 777 rows beside n of 20 behind 1500 keys, own launch | with it, us: n = 2 75 | 40, 8 89 | 67, 16
-            # 90 | 101, 64 142 | 298; 64/2 heads, a portion of 200 and 24 decode tokens 69 | 208.
-            if n_long == 0 or short * q.shape[1] > 2 * _sm_count(q.device.index):
-                n_packed = max(short, 0)
+        n_packed, n_few, few_keys = atoms_split(batch, atoms.shape[0], q.shape[1], cache.shape[3],
+                                                (q.data_ptr() | cache.data_ptr()) % 16 == 0, q.device.index)
         return paged_attention_atoms(q, cache, atoms, batch.block_tables(), scale, n_packed, n_few, few_keys)
     return paged_attention(q, cache, batch.token_to_seq(), batch.token_positions(), batch.block_tables(), scale)
 

@@ -12,10 +12,13 @@ Weights come from a training :class:`~shuffle_exchange_b200.models.llama.LlamaFo
 """
 from __future__ import annotations
 
+import array
+import math
 from typing import List, Optional
 
 import torch
 
+from ....native import lib as _n
 from ....ops import functional as F
 from ....ops import moe_ops
 from ..kernels import ragged_ops as R
@@ -72,11 +75,87 @@ class RaggedLlamaModel:
             lo = hi
         return moe_ops.moe_gather(out, scores, slots)
 
+    def _native_plan(self, batch):
+        """Operands of ``sxb_ragged_llama_forward`` for ``batch``, looked at afresh in every call, or None where the operators
+        below would not all run on the kernels that it issues (or have more to do than launch them)."""
+        c, m = self.cfg, self.lm.model
+        H, nq, nkv, d = c.hidden_size, c.num_attention_heads, c.num_key_value_heads, c.head_dim
+        Fw, bf16, dev = c.intermediate_size, torch.bfloat16, m.embed_tokens.device
+        if (self.moe_layers is not None or F.flop_sink is not None or dev.type != "cuda" or not hasattr(batch, "atoms")
+                or batch.current_tokens == 0 or batch.atoms().shape[0] == 0 or H % 8 or Fw % 8 or not _n.no_tape()):
+            return None
+        head = self.lm.head_weight()
+        ptrs = 0
+
+        def matrix(w, n, k):
+            nonlocal ptrs
+            if (w.dtype != bf16 or w.device != dev or w.shape != (n, k) or w.stride(1) != 1 or w.stride(0) % 8
+                    or hasattr(w, "_sxb_gate") or hasattr(w, "_sxb_grad_ready")):
+                return None
+            p = w.data_ptr()
+            ptrs |= p
+            return p
+
+        def vector(w):
+            return (w.data_ptr() if w.dtype == bf16 and w.device == dev and w.shape == (H,) and w.stride(0) == 1
+                    and not hasattr(w, "_sxb_grad_ready") else None)
+
+        rows = []
+        for li, layer in enumerate(m.layers):
+            cache = self.state_manager.get_cache(li)
+            if (not isinstance(cache, torch.Tensor) or cache.device != dev or not R.atoms_layout_ok(cache, d)
+                    or cache.shape[3:] != (nkv, d)):
+                return None
+            wqkv, wo, gu, down = layer.wqkv, layer.wo, layer.w_gate_up, layer.w_down
+            row = [vector(layer.input_layernorm), matrix(wqkv, (nq + 2 * nkv) * d, H), matrix(wo, H, nq * d),
+                   vector(layer.post_attention_layernorm), matrix(gu, 2 * Fw, H), matrix(down, H, Fw), cache.data_ptr()]
+            ptrs |= row[-1]
+            if None in row:
+                return None
+            rows += row
+            rows += [wqkv.stride(0), wo.stride(0), gu.stride(0), down.stride(0)]
+        emb = m.embed_tokens
+        top = [matrix(emb, emb.shape[0], H), vector(m.norm), matrix(head, head.shape[0], H)]
+        if not rows or None in top or not emb.is_contiguous() or head.shape[0] % 8 or ptrs % 16:
+            return None
+        return rows, top, head, cache
+
+    def _native_forward(self, batch, plan) -> torch.Tensor:
+        layers, (embed, norm, head_ptr), head, cache = plan
+        c = self.cfg
+        H, nq, nkv, d, Fw = c.hidden_size, c.num_attention_heads, c.num_key_value_heads, c.head_dim, c.intermediate_size
+        T, last, tables, atoms = batch.current_tokens, batch.last_token_index(), batch.block_tables(), batch.atoms()
+        n_rows, vocab, dev = last.shape[0], head.shape[0], head.device
+        # activations of one layer after the other in one allocation; those of attention and feed-forward take turns
+        sizes = [T * H] * 4 + [n_rows * H, T * (nq + 2 * nkv) * d, T * nq * d]
+        wide = (T * 2 * Fw + 127) // 128 * 128
+        at = [0]
+        for n in sizes:
+            at.append(at[-1] + (n + 127) // 128 * 128)
+        work = torch.empty(max(at[-1], at[5] + wide + T * Fw), dtype=torch.bfloat16, device=dev)
+        b0, b1, b2, x, rows, qkv, ctx = (work.data_ptr() + 2 * a for a in at[:-1])
+        logits = torch.empty((n_rows, vocab), dtype=torch.bfloat16, device=dev)
+        n_packed, n_few, few_keys = R.atoms_split(batch, atoms.shape[0], nq, nkv, True, dev.index)
+        model = array.array("q", [
+            batch.input_ids().data_ptr(), batch.token_to_seq().data_ptr(), batch.token_positions().data_ptr(), tables.data_ptr(),
+            last.data_ptr(), atoms.data_ptr(), embed, norm, head_ptr, b0, b1, b2, x, qkv, ctx, qkv, qkv + 2 * wide, rows,
+            logits.data_ptr(), head.stride(0), T, H, nq, nkv, d, Fw, vocab, n_rows, tables.shape[1], cache.shape[0],
+            cache.shape[1], atoms.shape[0], n_packed, n_few, *few_keys])
+        table = array.array("q", layers)
+        n_layers = len(layers) // 11
+        _n.attn_call("sxb_ragged_llama_forward", model.buffer_info()[0], table.buffer_info()[0], n_layers,
+                     float(c.rms_norm_eps), float(c.rope_theta), 1.0 / math.sqrt(d), _n.stream_ptr())
+        _n.launch_count += 9 * n_layers + 3        # the entry points that the call stands for, itself among them
+        return logits
+
     @torch.no_grad()
     def forward(self, batch) -> torch.Tensor:
         """``batch``: finalized :class:`RaggedBatchWrapper`.  Returns logits [n_seqs, vocab] of every sequence's last
         in-flight token."""
         c, m = self.cfg, self.lm.model
+        plan = self._native_plan(batch)
+        if plan is not None:
+            return self._native_forward(batch, plan)
         ids, t2s, pos = batch.input_ids(), batch.token_to_seq(), batch.token_positions()
         tables = batch.block_tables()
         h = R.ragged_embed(ids, m.embed_tokens)

@@ -1,0 +1,82 @@
+"""The forward of a dense Llama issued by one native call: the same bits as operator by operator, and what it does not take goes
+there."""
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(hidden, heads, kv, ff, vocab, layers=2, page=64, tie=False):
+    import torch
+    from shuffle_exchange_b200.inference.v2.config_v2 import RaggedInferenceEngineConfig
+    from shuffle_exchange_b200.inference.v2.engine_factory import build_engine_from_model
+    from shuffle_exchange_b200.inference.v2.ragged.manager_configs import DSStateManagerConfig
+    from shuffle_exchange_b200.models.llama import LlamaForCausalLM, llama_config
+    torch.manual_seed(0)
+    cfg = llama_config("llama-tiny", hidden_size=hidden, num_hidden_layers=layers, num_attention_heads=heads,
+                       num_key_value_heads=kv, intermediate_size=ff, vocab_size=vocab, activation_checkpointing=False,
+                       tie_word_embeddings=tie)
+    model = LlamaForCausalLM(cfg, device="cuda", dtype=torch.bfloat16).eval()
+    sm = DSStateManagerConfig(max_tracked_sequences=8, max_ragged_sequence_count=8, max_ragged_batch_size=2048, max_context=1024,
+                              num_kv_blocks=64 * 64 // page)
+    return model, build_engine_from_model(model, RaggedInferenceEngineConfig(state_manager=sm, kv_block_size=page))
+
+
+STEPS = [[5], [1], [300, 1, 17, 130], [1, 1, 1, 1], [1, 64, 1]]
+
+
+def _serve(eng, native, monkeypatch, **kw):
+    import torch
+    from shuffle_exchange_b200.inference.v2.model_implementations.llama_v2 import RaggedLlamaModel
+    used = []
+    if native:
+        real = RaggedLlamaModel._native_forward
+        monkeypatch.setattr(RaggedLlamaModel, "_native_forward", lambda s, b, p: used.append(1) or real(s, b, p))
+    else:
+        monkeypatch.setattr(RaggedLlamaModel, "_native_plan", lambda s, b: None)
+    g = torch.Generator().manual_seed(1)
+    out = []
+    for lens in STEPS:
+        toks = [torch.randint(0, 256, (n,), generator=g, dtype=torch.int32) for n in lens]
+        out.append(eng.put(range(len(lens)), toks, **{k: v[: len(lens)] for k, v in kw.items()}).clone())
+    for u in range(4):
+        eng.flush(u)
+    monkeypatch.undo()
+    return out, len(used)
+
+
+@pytest.mark.parametrize("hidden,heads,kv,ff,vocab,layers,page,tie", [
+    (512, 4, 2, 1024, 1024, 2, 64, False), (512, 8, 8, 776, 512, 1, 16, True), (768, 6, 1, 2048, 1000, 3, 128, False)])
+def test_same_bits_as_operator_by_operator(hidden, heads, kv, ff, vocab, layers, page, tie, monkeypatch):
+    import torch
+    model, eng = _engine(hidden, heads, kv, ff, vocab, layers, page, tie)
+    got, n = _serve(eng, True, monkeypatch)
+    want, _ = _serve(eng, False, monkeypatch)
+    assert n == len(STEPS)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b) and torch.isfinite(a).all()
+    (a, _), (b, _) = (_serve(eng, x, monkeypatch, logit_positions=[[0], [], [0], [0]]) for x in (True, False))
+    assert all(torch.equal(x, y) for x, y in zip(a, b))
+
+
+def test_what_it_does_not_take(monkeypatch):
+    """Odd vocabulary, head size of 32, weights of another type: operator by operator, as ever."""
+    import torch
+    for kw in (dict(vocab=1001, heads=4, kv=2), dict(vocab=1024, heads=16, kv=16)):
+        model, eng = _engine(512, kw["heads"], kw["kv"], 1024, kw["vocab"])
+        got, n = _serve(eng, True, monkeypatch)
+        want, _ = _serve(eng, False, monkeypatch)
+        assert n == 0 and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_replaced_weights_are_seen(monkeypatch):
+    import torch
+    model, eng = _engine(512, 4, 2, 1024, 1024)
+    before, _ = _serve(eng, True, monkeypatch)
+    layer = model.model.layers[1]
+    layer.wqkv = torch.nn.Parameter(layer.wqkv.detach() * 0.5)
+    layer.w_down.data = torch.cat([layer.w_down.data, layer.w_down.data], 1)[:, 512: 1536]       # another pitch
+    got, n = _serve(eng, True, monkeypatch)
+    want, _ = _serve(eng, False, monkeypatch)
+    assert n == len(STEPS) and all(torch.equal(a, b) for a, b in zip(got, want))
+    assert not torch.equal(got[0], before[0])
