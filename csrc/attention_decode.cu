@@ -28,6 +28,7 @@ struct Params {
   long long q_stride, o_stride;
   float scale;
   int after;                       // launched beside an earlier kernel of the stream: leave only behind it
+  int chain;                       // launched while the kernel that makes its queries may still run
 };
 
 template <int D>
@@ -54,6 +55,8 @@ paged_decode_kernel(const Params p, const int S) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = blockIdx.x % S, hk = blockIdx.x / S;
+  chain_next();
+  if (p.chain) chain_wait();
   const int* a = p.atoms + 6 * (int)blockIdx.y;
   const int q_row0 = a[1], nq = a[2], q_pos0 = a[3], kv_len = a[5];
   const int* pages = p.tables + (long long)a[0] * p.max_blocks;
@@ -258,7 +261,7 @@ static int launch(const Params& p, int n_atoms, int S, bool beside, cudaStream_t
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = beside ? 2 : 1;
+  cfg.numAttrs = beside || p.chain ? 2 : 1;
   e = cudaLaunchKernelEx(&cfg, k, p, S);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
   return SXB_OK;
@@ -278,6 +281,7 @@ int paged_decode(const void* q, const void* cache, void* out, const void* atoms,
   p.max_blocks = max_blocks; p.block_size = block_size; p.Hk = Hk; p.group = Hq / Hk;
   p.shift = (block_size & (block_size - 1)) == 0 ? __builtin_ctz(block_size) : -1;
   p.q_stride = q_stride; p.o_stride = o_stride; p.scale = scale; p.after = beside ? 1 : 0;
+  p.chain = !beside && chained() ? 1 : 0;
   // CTAs per sequence: as many as keep the grid within one and a half waves of two per SM, since starting and merging a CTA
   // costs 4 us of a wave (us, up to one and a half | four waves: 61 requests of 2048 80 | 94, 40 of 100 9 | 16, 24 of 6000 93 |
   // 101), and no more than have a step each (4 requests of 40 keys, 32 key/value heads: 4.3 with one, 8.0 with eight).

@@ -105,6 +105,8 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads)
 gated_fwd_kernel(const T* __restrict__ in, const T* __restrict__ bias, T* __restrict__ out,
                  long long rows, int F, int act) {
+  chain_next();
+  chain_wait();
   const int vpr = F >> 3;
   const long long total = rows * vpr;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
@@ -414,10 +416,10 @@ SXB_API int sxb_gated_act_fwd(const void* in, const void* bias, void* out, long 
   if (rows <= 0) return SXB_OK;
   if (F % 8) return SXB_ERR_UNSUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
-  DISPATCH_16(dtype, (gated_fwd_kernel<T><<<grid_for(rows * (F / 8)), kThreads, 0, s>>>(
-                         (const T*)in, (const T*)bias, (T*)out, rows, F, act)));
-  SXB_CHECK_LAUNCH();
-  return SXB_OK;
+  int rc = SXB_OK;
+  DISPATCH_16(dtype, rc = launch_chained(gated_fwd_kernel<T>, dim3(grid_for(rows * (F / 8))), kThreads, s, (const T*)in,
+                                         (const T*)bias, (T*)out, rows, F, act));
+  return rc;
 }
 // act(gate) * up for the routed rows of grouped expert rows: in [capacity, 2F], out [capacity, F]; offsets / counts int32
 // [groups] (first row and routed rows of every group); n_rows = sum of the counts.  Other rows of out are not written.

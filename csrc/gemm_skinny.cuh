@@ -10,7 +10,8 @@
 // fp32, 1.6e-5 without the cut.
 // Measured (weights from HBM, us before -> after, floor): 1 x 28672 x 4096 53.9 -> 40.2, 35.9; 48 x 4096 x 4096 27.5 -> 11.7,
 // 5.2; 24 x 2048 x 8192 49.6 -> 11.7, 5.2; 128 x 4096 x 14336 84.1 -> 29.0, 18.6; 1 x 768 x 768 7.9 -> 4.7, 0.2.  What is left
-// on the large ones is DRAM time, on the small ones launch, tensor-map fetch, TMEM allocation and two cluster barriers.
+// on the large ones is DRAM time, on the small ones launch, tensor-map fetch, TMEM allocation and two cluster barriers; in a chain of
+// launches those, and the first turn of the weight ring, run beside the kernel before (ragged_llama.cu).
 #pragma once
 
 template <int BN, int STAGES>
@@ -38,7 +39,7 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t saddr, uint32_t rank) {
 template <int BN, int STAGES>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p,
-                   const int S) {
+                   const int S, const int chain) {
   using Plan = SkinnyPlan<BN, STAGES>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -71,6 +72,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (chain) chain_next();                  // behind the tensor memory, so that no later kernel takes it first
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t sbase = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
   const uint32_t tbase = __shfl_sync(0xffffffffu, tmem_base, 0);
@@ -78,14 +80,25 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (warp == 0) {
     const bool elected = elect_one();
+    // in a chain the weights of a first turn of the ring are on their way while the kernel that makes the tokens still runs
+    const int ahead = chain ? min(kb1, kb0 + STAGES) : kb0;
+    if (elected)
+      for (int kb = kb0; kb < ahead; ++kb) {
+        mbar_expect_tx(&full_bar[kb - kb0], Plan::kStage);
+        tma_load_2d(smem + (kb - kb0) * Plan::kStage, &tmW, &full_bar[kb - kb0], kb * BK, n0);
+      }
+    __syncwarp();
+    if (chain) chain_wait();
     int stage = 0;
     uint32_t phase = 0;
     for (int kb = kb0; kb < kb1; ++kb) {
       if (!__all_sync(0xffffffffu, mbar_wait_to(&empty_bar[stage], phase ^ 1, 41, kb))) break;
       if (elected) {
         uint8_t* sa = smem + stage * Plan::kStage;
-        mbar_expect_tx(&full_bar[stage], Plan::kStage);
-        tma_load_2d(sa, &tmW, &full_bar[stage], kb * BK, n0);
+        if (kb >= ahead) {
+          mbar_expect_tx(&full_bar[stage], Plan::kStage);
+          tma_load_2d(sa, &tmW, &full_bar[stage], kb * BK, n0);
+        }
         tma_load_2d(sa + Plan::kA, &tmX, &full_bar[stage], kb * BK, m0);
       }
       __syncwarp();

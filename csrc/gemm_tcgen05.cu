@@ -733,12 +733,14 @@ static int launch_skinny(const void* A, const void* B, const Params& p, int lda,
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = Plan::kTotal;
   cfg.stream = stream;
-  cudaLaunchAttribute at;
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = S; at.val.clusterDim.y = 1; at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, tw, tx, p, S);
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = chained() ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, tw, tx, p, S, chained() ? 1 : 0);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
   return SXB_OK;
 }

@@ -431,6 +431,8 @@ logits_gather_kernel(const uint4* __restrict__ hidden, const int* __restrict__ l
                      int row_vec) {
   const int s = blockIdx.x;
   const uint4* src = hidden + (long long)last_token[s] * row_vec;
+  chain_next();
+  chain_wait();
   for (int i = threadIdx.x; i < row_vec; i += blockDim.x) out[(long long)s * row_vec + i] = src[i];
 }
 
@@ -446,19 +448,22 @@ __global__ void kv_rotary_blocked_kernel(__nv_bfloat16* __restrict__ qkv, __nv_b
                                          int Hk, int D, int rot_dim, float log2_theta) {
   const int t = blockIdx.x, head = blockIdx.y, i = threadIdx.x;  // i in [0, D/2)
   const int pos = tok_pos[t];
+  const bool is_k = head >= Hq;
+  const int blk = is_k ? block_tables[(long long)tok_seq[t] * max_blocks + pos / block_size] : 0;
+  chain_next();
   const long long row = (long long)t * (Hq + 2 * Hk) * D;
   __nv_bfloat16* h = qkv + row + (long long)head * D;            // q heads then k heads are contiguous
   const int half = rot_dim / 2;
-  float x0, x1;
+  float x0, x1, sn = 0.f, cs = 1.f;
+  if (i < half) sincosf(pos * exp2f(-(2.0f * i / rot_dim) * log2_theta), &sn, &cs);
+  chain_wait();                                                  // the position and its angle are the batch's own
   int i0, i1;
   if (i < half) { i0 = i; i1 = i + half; } else { i0 = half + i; i1 = -1; }  // beyond rot_dim: pass-through pairs
   if (i < half) {
     x0 = __bfloat162float(h[i0]);
     x1 = __bfloat162float(h[i1]);
-    const float inv_freq = exp2f(-(2.0f * i / rot_dim) * log2_theta);
-    float sn, cs;
-    sincosf(pos * inv_freq, &sn, &cs);
-    const float y0 = x0 * cs - x1 * sn, y1 = x1 * cs + x0 * sn;
+    // which product is rounded is said here, so that it does not hang on the code around
+    const float y0 = __fmaf_rn(x0, cs, -__fmul_rn(x1, sn)), y1 = __fmaf_rn(x1, cs, __fmul_rn(x0, sn));
     x0 = y0; x1 = y1;
   } else {
     // unrotated tail [rot_dim, D): two elements per thread
@@ -467,13 +472,11 @@ __global__ void kv_rotary_blocked_kernel(__nv_bfloat16* __restrict__ qkv, __nv_b
     x0 = i0 < D ? __bfloat162float(h[i0]) : 0.f;
     x1 = i1 < D ? __bfloat162float(h[i1]) : 0.f;
   }
-  const bool is_k = head >= Hq;
   if (!is_k) {
     if (i < half) { h[i0] = __float2bfloat16_rn(x0); h[i1] = __float2bfloat16_rn(x1); }
     return;
   }
   const int kh = head - Hq;
-  const int blk = block_tables[(long long)tok_seq[t] * max_blocks + pos / block_size];
   const long long slot = ((long long)blk * block_size + pos % block_size) * 2 * Hk * D;
   __nv_bfloat16* kdst = cache + slot + (long long)kh * D;
   __nv_bfloat16* vdst = cache + slot + (long long)(Hk + kh) * D;
@@ -718,11 +721,9 @@ SXB_API int sxb_logits_gather(const void* hidden_states, const void* last_token,
                               void* stream) {
   if (n_seqs <= 0) return SXB_OK;
   if ((hidden * 2) % 16) return SXB_ERR_UNSUPPORTED;
-  ragged::logits_gather_kernel<<<n_seqs, 128, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(hidden_states), static_cast<const int*>(last_token), static_cast<uint4*>(out),
-      hidden * 2 / 16);
-  SXB_CHECK_LAUNCH();
-  return SXB_OK;
+  return launch_chained(ragged::logits_gather_kernel, dim3(n_seqs), 128, reinterpret_cast<cudaStream_t>(stream),
+                        static_cast<const uint4*>(hidden_states), static_cast<const int*>(last_token), static_cast<uint4*>(out),
+                        hidden * 2 / 16);
 }
 
 SXB_API int sxb_kv_rotary_blocked(void* qkv, void* cache, const void* tok_seq, const void* tok_pos,
@@ -731,12 +732,10 @@ SXB_API int sxb_kv_rotary_blocked(void* qkv, void* cache, const void* tok_seq, c
   if (n_tokens <= 0) return SXB_OK;
   if (D % 2 || D > 256 || rot_dim > D || rot_dim % 2) return SXB_ERR_UNSUPPORTED;
   dim3 grid(n_tokens, Hq + Hk);
-  ragged::kv_rotary_blocked_kernel<<<grid, D / 2, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(cache), static_cast<const int*>(tok_seq),
-      static_cast<const int*>(tok_pos), static_cast<const int*>(block_tables), max_blocks, block_size, Hq, Hk, D,
-      rot_dim, log2f(theta));
-  SXB_CHECK_LAUNCH();
-  return SXB_OK;
+  return launch_chained(ragged::kv_rotary_blocked_kernel, grid, D / 2, reinterpret_cast<cudaStream_t>(stream),
+                        static_cast<__nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(cache), static_cast<const int*>(tok_seq),
+                        static_cast<const int*>(tok_pos), static_cast<const int*>(block_tables), max_blocks, block_size, Hq, Hk, D,
+                        rot_dim, log2f(theta));
 }
 
 SXB_API int sxb_paged_attention(const void* q, void* out, const void* cache, const void* tok_seq, const void* tok_pos,

@@ -72,6 +72,8 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ res, const T* __r
                 const T* __restrict__ b, T* __restrict__ y, T* __restrict__ res_out,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int H, float eps) {
   __shared__ float red[32];
+  chain_next();
+  chain_wait();
   const long long row = blockIdx.x;
   const T* xr = x + row * H;
   const int nvec = H >> 3;
@@ -88,9 +90,10 @@ norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ res, const T* __r
 #pragma unroll
         for (int k = 0; k < 8; ++k) vals[it][k] += r[k];
         if (res_out) {
-          // round-trip through T so the normalised value matches what backward re-reads
+          // rounded to T so the normalised value matches what backward re-reads
           st8<T>(res_out + row * H + vi * 8, vals[it]);
-          ld8<T>(res_out + row * H + vi * 8, vals[it]);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) vals[it][k] = to_f32<T>(from_f32<T>(vals[it][k]));
         }
       }
 #pragma unroll
@@ -325,10 +328,10 @@ static int norm_fwd(const void* x, const void* res, const void* w, const void* b
   if (rows <= 0) return SXB_OK;
   if (!norm_ok(H)) return SXB_ERR_UNSUPPORTED;
   const int iters = (H / 8 + kThreads - 1) / kThreads;
+  int rc = SXB_OK;
 #define LI(T, I)                                                                                  \
-  norm_fwd_kernel<T, kLayer, I><<<(unsigned)rows, kThreads, 0, s>>>(                              \
-      (const T*)x, (const T*)res, (const T*)w, (const T*)b, (T*)y, (T*)res_out, (float*)mean,      \
-      (float*)rstd, H, eps)
+  rc = launch_chained(norm_fwd_kernel<T, kLayer, I>, dim3((unsigned)rows), kThreads, s, (const T*)x, (const T*)res,   \
+                      (const T*)w, (const T*)b, (T*)y, (T*)res_out, (float*)mean, (float*)rstd, H, eps)
 #define L(T)                                                                                      \
   do {                                                                                            \
     if (iters <= 1) LI(T, 1); else if (iters <= 2) LI(T, 2); else if (iters <= 4) LI(T, 4);       \
@@ -340,8 +343,7 @@ static int norm_fwd(const void* x, const void* res, const void* w, const void* b
   else return SXB_ERR_BAD_ARG;
 #undef L
 #undef LI
-  SXB_CHECK_LAUNCH();
-  return SXB_OK;
+  return rc;
 }
 
 template <bool kLayer>

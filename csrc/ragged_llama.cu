@@ -3,6 +3,8 @@
 // The kernels are those of the operators' own entry points, in the same order and on the same operands: this entry only takes the
 // way from one launch to the next out of Python, which a decode step of a few requests spends its time on (4 layers of 2048, 4
 // requests, prompts and six decode steps: 5.53 ms from Python, 2.88 this way, 2.4 of device work).  Nothing is kept between calls.
+// The launches form a chain (sxb_common.cuh): a kernel comes onto the SMs while the one before it still runs, so that its launch, its
+// set-up and a product's first weights are behind it when its operands are there: 2.88 -> 2.40 ms.
 #include "sxb_common.cuh"
 #include "sxb200.h"
 
@@ -29,6 +31,7 @@ SXB_API int sxb_ragged_llama_forward(const struct sxb_ragged_llama* m, const str
     return SXB_OK;
   };
   if ((rc = sxb_ragged_embed(m->ids, nullptr, m->embed, nullptr, h, T, H, 0, stream))) return rc;
+  const ChainScope chain;      // everything below reads only what kernels above wrote, the batch's tables and the weights
   for (int i = 0; i < n_layers; ++i) {
     const struct sxb_ragged_llama_layer& l = layers[i];
     if ((rc = norm(l.ln1))) return rc;

@@ -528,6 +528,35 @@ static inline int num_sms() {
 int encode_tensor_map(CUtensorMap* m, int dtype_code, int rank, const void* ptr,
                       const unsigned long long* dims, const unsigned long long* strides_bytes,
                       const unsigned int* box, int swizzle_bytes);
+
+// A chain of launches (set for the calls that a host thread makes meanwhile): each kernel may be brought onto the SMs while the one
+// before it still runs, as far as that one leaves room.  A kernel launched so calls chain_wait() ahead of everything that it
+// shares with earlier kernels, reads and writes; what none of them writes (weights, a batch's tables) it may fetch before.
+bool& chained();
+struct ChainScope {
+  bool before;
+  ChainScope() : before(chained()) { chained() = true; }
+  ~ChainScope() { chained() = before; }
+};
+// Every earlier kernel of the stream is done (at once in a kernel that was launched behind them anyway).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel may come beside this one, once every CTA of this grid has said so.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+template <typename K, typename... Args>
+static int launch_chained(K kernel, dim3 grid, int threads, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = chained() ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+  if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
+  return SXB_OK;
+}
 }  // namespace sxb
 
 // ---- appended: bounded mbarrier wait + hang diagnostics -----------------------------------
