@@ -23,8 +23,8 @@
 //   channel_decay_gates   decay per (head, key channel) pair for linear_recurrence (its per-channel form), sigmoid write strength
 //   sigmoid_gate_rows, power_norm_act   sigmoid gate per channel or per head in place; p1 z/rms(z) + p2 z^2/rms(z^2) + p3 z^3/rms(z^3) + p0
 #include <algorithm>
+#include <type_traits>
 #include "seq_common.cuh"
-#include "mma_sync.cuh"
 #include <cuda_pipeline.h>
 
 namespace sxb {
@@ -1684,6 +1684,8 @@ mlstm_output_kernel(const float* __restrict__ o, const float* __restrict__ mt, c
 using namespace sxb;
 using namespace sxb::seqmix;
 
+SXB_DEFINE_HANG_ACCESSOR(sxb_seqmix_hang_info)
+
 /* out fp32 [n_tokens, width] = table[ids[t]] * scale + p, p[2i] = sin(pos * base^(-2i/width)), p[2i+1] = cos(same);
  * base <= 0: p = 0.  table: `dtype` [vocab, width]. */
 SXB_API int sxb_embed_sinusoid(const void* ids, const void* pos, const void* table, void* out, int n_tokens, int width,
@@ -1985,7 +1987,7 @@ SXB_API int sxb_sink_attention_atoms(const void* q, const void* kcache, const vo
     const int nv = (dv + 63) / 64;
     int rc = SXB_OK;
     // 16-bit caches with heads of 64 or 128 channels take the tensor-core form: the fp32 FMA form is bound by the FMA lanes (one
-    // prompt of 3000 rows, 16 heads of 128, chunks of 1024: 675 us, 203 on the tensor cores).  Rows are copied 16 bytes at a
+    // prompt of 3000 rows, 16 heads of 128, chunks of 1024: 675 us, 80 on the tensor cores).  Rows are copied 16 bytes at a
     // time, so pitches are multiples of 8 and the bases 16-byte aligned; fp32 caches and other head sizes keep the FMA form.
     const bool mma = dtype == kBF16 && n_long <= 65535 && (d == 64 || d == 128) && (dv == 64 || dv == 128) && k_pitch % 8 == 0 && v_pitch % 8 == 0 &&
                      ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(kcache) |

@@ -7,11 +7,16 @@
 // the tensor cores' truncating adders: every tile's P V starts from zero and joins the output by one fp32 FMA together
 // with the softmax rescale, and a score's two small terms have an accumulator of their own.
 //
-// One CTA of eight warps per (atom, query head); a warp owns 16 query rows and all 64 keys of a tile, so the softmax needs
-// two shuffles and no barrier.  Q takes 96 KB (three terms, head size 128), two K/V tiles (cp.async) 64 KB.  What bounds it:
-// the 384 MMAs of a warp and tile, then the softmax and the split of the weights (tensor pipe 44 % active with two warps per
-// scheduler, 255 registers each).  One prompt of 3000 rows, 16 query heads of 128, chunks of 1024: 675 us with fp32 FMAs, 203 now;
-// the error against 64 bits is that of the 16-bit result (1.7e-3) before and after.
+// One CTA per (atom, query head) over tiles of 64 keys: eight row warps (two per lane quadrant of tensor memory, each with 32 of a
+// tile's keys and half of the value channels), two that copy K and V (cp.async: keys begin anywhere in a page), one that issues
+// the MMAs.  Q's three terms take 96 KB of shared memory, a ring of three K/V tiles 96 KB (head size 128).  Tensor memory: scores of
+// even tiles 0..127 (leading term, rests), of odd tiles 128..255, the tile's output 256..383, the weights' three terms 384..479 (A
+// operand).  The scores of the next tile are computed while the rows work on this one, its P V while they work on the next.
+// What bounds it: the row warps (some 25 instructions per score for expf and the split: 2600 cycles a tile) and the 36 MMAs of a tile
+// beside them (2350); 3500 cycles a tile all told.  Against the same three terms on mma.sync, one warp per 16 rows, us: one prompt of 3000
+// rows, 16 heads of 128, chunks of 1024 202 -> 80 (675 with fp32 FMAs); 4096 rows, 32 heads, one chunk 1468 -> 470; four prompts
+// of 750 behind 700, window of 512 201 -> 80; one of 100 rows, 8 heads, 23 both.  K and V in rings of their own matter: 109 with one
+// ring for both.  The error against 64 bits is that of the 16-bit result (1.656e-3) all along.
 #pragma once
 
 // Two fp32 numbers as three packed bf16 pairs whose sum is exact (INF: infinities may occur and keep zero rests).
@@ -87,14 +92,18 @@ __device__ __noinline__ void sink_row_plain(const float* q, float scale, const _
     out[c] = __float2bfloat16_rn(x * out_scale);
   }
 }
-constexpr int kSmQ = 128, kSmThreads = 256;                    // query rows (a whole atom) and threads of a CTA
+constexpr int kSmQ = 128, kSmThreads = 352;                    // query rows (a whole atom) and threads of a CTA
 
 template <int D, int DV>
 struct SinkMma {
+  static constexpr int kStages = 3;
   static constexpr int kQ = kSmQ * D * 2;                     // one term
   static constexpr int kK = kBK * D * 2, kV = kBK * DV * 2;
-  static constexpr int oK = 3 * kQ, oV = oK + 2 * kK;
-  static constexpr int kTotal = oV + 2 * kV;
+  static constexpr int oK = 3 * kQ, oV = oK + kStages * kK;
+  static constexpr int oRow = oV + kStages * kV;              // floats [2][2][128]: the halves' maxima of even / odd tiles; sums [2][128]
+  static constexpr int oBad = oRow + 3072;                    // uint32 [2 halves][4 quadrants]: rows that are not finite
+  static constexpr int oBar = oBad + 64;
+  static constexpr int kTotal = oBar + 192 + 1024;
 };
 
 template <int D, int DV>
@@ -107,7 +116,21 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
                           const __nv_bfloat16* __restrict__ gate, long long gate_ld, int gate_heads, long long out_ld,
                           float out_scale) {
   using L = SinkMma<D, DV>;
-  extern __shared__ __align__(128) uint8_t smb[];
+  constexpr int NS = L::kStages;
+  extern __shared__ __align__(128) uint8_t smb_raw[];
+  uint8_t* smb = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smb_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smb + L::oBar);
+  uint64_t* k_full = bars + 0;     // [NS]
+  uint64_t* k_empty = bars + 3;    // [NS] the tile's scores are there
+  uint64_t* v_full = bars + 6;     // [NS]
+  uint64_t* v_empty = bars + 9;    // [NS] P V of the tile retired
+  uint64_t* q_full = bars + 12;    // Q's terms in place (one arrival per row warp)
+  uint64_t* s_full = bars + 13;    // [2]
+  uint64_t* s_free = bars + 15;    // [2] scores read (one arrival per row warp)
+  uint64_t* p_full = bars + 17;    // weights in place and the output of the tile before read (one arrival per row warp)
+  uint64_t* o_full = bars + 18;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 19);
+
   // later positions first: they tend to see more keys, so light tiles end the grid
   const int* a = atoms + 6 * (gridDim.y - 1 - blockIdx.y);
   const int nq = min(a[2], kSmQ);
@@ -116,227 +139,277 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
   const int h = blockIdx.x, g = h / (Hq / G);
   const int* tab = tables + (long long)a[0] * max_blocks;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t base = smem_u32(smb);
   const int last = pos0 + nq - 1;
   const int kbeg = first_key(pos0, chunk, window);
+  const int n_tiles = (last - kbeg) / kBK + 1;
 
-  const int shift = (block_size & (block_size - 1)) == 0 ? 31 - __clz(block_size) : -1;
-  auto slot_of = [&](int pos) {
-    const int blk = shift >= 0 ? pos >> shift : pos / block_size;
-    return (long long)tab[blk] * block_size + (pos - blk * block_size);
-  };
-  auto load_tile = [&](int buf, int k0) {           // rows behind the last query are zeros, as are their weights
-    constexpr int KC = D / 8, VC = DV / 8;
-#pragma unroll
-    for (int i = 0; i < kBK * KC / kSmThreads; ++i) {
-      const int r = tid / KC + i * (kSmThreads / KC), c = tid % KC, kj = k0 + r, zero = kj <= last ? 0 : 16;
-      const long long slot = slot_of(min(kj, last));
-      __pipeline_memcpy_async(smb + L::oK + buf * L::kK + tile_at(r, c, D * 2), kcache + slot * kpitch + g * D + c * 8, 16, zero);
-      if (DV == D)
-        __pipeline_memcpy_async(smb + L::oV + buf * L::kV + tile_at(r, c, DV * 2), vcache + slot * vpitch + g * DV + c * 8, 16,
-                                zero);
+  if (warp == 8) {
+    if (lane == 0) {
+      for (int i = 0; i < NS; ++i) {
+        mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1);
+      }
+      for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 8); }
+      mbar_init(q_full, 8); mbar_init(p_full, 8); mbar_init(o_full, 1);
+      mbar_fence_init();
     }
-    if (DV != D) {
+    __syncwarp();
+    tmem_alloc(tmem_slot, 512);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp >= 9) {
+    // ---- one warp copies K, one V, in the layout of 128-byte swizzled operands: K is used up long before the V of its tile.  Rows
+    // behind the last query are zeros, as are their weights.  A lane looks up the slots of two of a tile's rows; the copies
+    // take them from there, a row or more at a time.
+    const bool is_k = warp == 9;
+    const int shift = (block_size & (block_size - 1)) == 0 ? 31 - __clz(block_size) : -1;
+    uint64_t *full = is_k ? k_full : v_full, *empty = is_k ? k_empty : v_empty;
+    auto copy = [&](auto width, const __nv_bfloat16* src, int pitch, uint8_t* dst, const int (&slot)[2], int k0) {
+      constexpr int C = decltype(width)::value, R = 32 / C;       // 16-byte chunks of a row, rows at a time
+      const int c = lane % C;
 #pragma unroll
-      for (int i = 0; i < kBK * VC / kSmThreads; ++i) {
-        const int r = tid / VC + i * (kSmThreads / VC), c = tid % VC, kj = k0 + r;
-        __pipeline_memcpy_async(smb + L::oV + buf * L::kV + tile_at(r, c, DV * 2),
-                                vcache + slot_of(min(kj, last)) * vpitch + g * DV + c * 8, 16, kj <= last ? 0 : 16);
+      for (int hf = 0; hf < 2; ++hf)
+#pragma unroll 4
+        for (int i = 0; i < C; ++i) {
+          const int rr = i * R + lane / C, r = hf * 32 + rr;
+          const long long sl = __shfl_sync(0xffffffffu, slot[hf], rr);
+          __pipeline_memcpy_async(dst + (c >> 3) * (kBK * 128) + r * 128 + (((c & 7) ^ (r & 7)) << 4), src + sl * pitch + c * 8, 16,
+                                  k0 + r <= last ? 0 : 16);
+        }
+    };
+    auto load_tile = [&](int j) {
+      const int k0 = kbeg + j * kBK, st = j % NS;
+      int slot[2];
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        const int pos = min(k0 + hf * 32 + lane, last);
+        const int blk = shift >= 0 ? pos >> shift : pos / block_size;
+        slot[hf] = tab[blk] * block_size + (pos - blk * block_size);
+      }
+      if (is_k) copy(std::integral_constant<int, D / 8>(), kcache + g * D, kpitch, smb + L::oK + st * L::kK, slot, k0);
+      else copy(std::integral_constant<int, DV / 8>(), vcache + g * DV, vpitch, smb + L::oV + st * L::kV, slot, k0);
+      __pipeline_commit();
+    };
+    // two tiles under way; one is handed over before the wait for the slot of another
+    load_tile(0);
+    if (n_tiles > 1) load_tile(1);
+    for (int j = 0; j < n_tiles; ++j) {
+      if (j + 1 < n_tiles) __pipeline_wait_prior(1);
+      else __pipeline_wait_prior(0);
+      fence_async_smem();            // for the MMAs, too
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&full[j % NS]);
+      const int n = j + 2;
+      if (n < n_tiles) {
+        if (!__all_sync(0xffffffffu, mbar_wait_to(&empty[n % NS], ((n / NS) & 1) ^ 1, 120, n))) goto done;
+        load_tile(n);
       }
     }
-    __pipeline_commit();
-  };
-  load_tile(0, kbeg);
-  for (int i = tid; i < kSmQ * (D / 8); i += kSmThreads) {
-    const int r = i / (D / 8), c = i % (D / 8);
-    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    if (r < nq) load8_f32<float>(q + ((long long)(row0 + r) * Hq + h) * D + c * 8, v);
-    uint32_t t[3][4];
+  } else if (warp == 8) {
+    const bool elected = elect_one();
+    const uint32_t sbase = __shfl_sync(0xffffffffu, smem_u32(smb), 0);
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const uint32_t idesc_s = make_idesc(kSmQ, kBK, 1, 1, 0, 0);
+    const uint32_t idesc_o = make_idesc(kSmQ, DV, 1, 1, 0, 1);
+    auto issue_s = [&](int j) -> bool {
+      if (!__all_sync(0xffffffffu, mbar_wait_to(&k_full[j % NS], (j / NS) & 1, 121, j))) return false;
+      if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait_to(&s_free[j & 1], ((j >> 1) - 1) & 1, 122, j))) return false;
+      tc_fence_after();
+      const uint32_t sK = sbase + L::oK + (j % NS) * L::kK, tS = tm + (j & 1) * 128;
+      if (elected) {
+        // the leading term has an accumulator of its own (columns 0..63); the rests, smallest first, share the other
 #pragma unroll
-    for (int j = 0; j < 4; ++j) split3<true>(v[2 * j] * scale, v[2 * j + 1] * scale, t[0][j], t[1][j], t[2][j]);
+        for (int i = 0; i < 3; ++i) {
+          const int term = 2 - i;
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
-      *reinterpret_cast<uint4*>(smb + j * L::kQ + tile_at(r, c, D * 2)) = make_uint4(t[j][0], t[j][1], t[j][2], t[j][3]);
-  }
-
-  const int t2 = (lane & 3) * 2, mi = lane >> 3, mr = lane & 7;
-  const int r0 = warp * 16 + (lane >> 2);                       // the thread's rows: r0 and r0 + 8
-  const bool busy = warp * 16 < nq;
-  float m[2], l[2], acc[DV / 8][4];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    m[i] = sink ? sink[h] : -INFINITY;
-    l[i] = sink && (lane & 3) == 0 ? 1.f : 0.f;                 // a quarter of the row's sum; the sink counts once
-  }
-#pragma unroll
-  for (int n = 0; n < DV / 8; ++n)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
-  const int lo[2] = {first_key(pos0 + r0, chunk, window), first_key(pos0 + r0 + 8, chunk, window)};
-
-  int buf = 0;
-  for (int k0 = kbeg; k0 <= last; k0 += kBK, buf ^= 1) {
-    const bool more = k0 + kBK <= last;
-    if (more) load_tile(buf ^ 1, k0 + kBK);
-    if (more) __pipeline_wait_prior(1);
-    else __pipeline_wait_prior(0);
-    __syncthreads();
-    // rows above the tile's first key, and chunks or windows that begin behind its last one, have nothing here
-    if (busy && k0 <= pos0 + min(warp * 16 + 15, nq - 1) && k0 + kBK > first_key(pos0 + warp * 16, chunk, window)) {
-      const uint32_t sk = base + L::oK + buf * L::kK, sv = base + L::oV + buf * L::kV;
-      float s[8][4], s2[8][4];                                  // products with the leading term; with the two rests
-#pragma unroll
-      for (int n = 0; n < 8; ++n)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) s[n][i] = s2[n][i] = 0.f;
-#pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk) {
-        uint32_t ah[4], am[4], al[4];
-        const uint32_t qa = base + tile_at(warp * 16 + (mi & 1) * 8 + mr, kk * 2 + (mi >> 1), D * 2);
-        ldsm4(ah, qa);
-        ldsm4(am, qa + L::kQ);
-        ldsm4(al, qa + 2 * L::kQ);
-        uint32_t b[4][4];
-#pragma unroll
-        for (int np = 0; np < 4; ++np)
-          ldsm4(b[np], sk + tile_at(np * 16 + (mi >> 1) * 8 + mr, kk * 2 + (mi & 1), D * 2));
-        // one term over all eight key columns at a time: eight independent accumulators between two uses of one
-#pragma unroll
-        for (int n = 0; n < 8; ++n) mma_bf16(s2[n], al, b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
-#pragma unroll
-        for (int n = 0; n < 8; ++n) mma_bf16(s[n], ah, b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
-#pragma unroll
-        for (int n = 0; n < 8; ++n) mma_bf16(s2[n], am, b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
+          for (int kk = 0; kk < D / 16; ++kk)
+            umma_f16(tS + (term == 0 ? 0 : 64),
+                     make_smem_desc(sbase + term * L::kQ + (kk >> 2) * (kSmQ * 128) + (kk & 3) * 32, 16, 1024, 2),
+                     make_smem_desc(sK + (kk >> 2) * (kBK * 128) + (kk & 3) * 32, 16, 1024, 2), idesc_s,
+                     kk != 0 || term == 1);
+        }
+        umma_commit(&s_full[j & 1]);
+        umma_commit(&k_empty[j % NS]);
       }
-      float corr[2];
-      // a tile that all rows see whole needs no look at positions
-      const bool whole = k0 + kBK - 1 <= pos0 + warp * 16 && k0 >= first_key(last, chunk, window) && dist_bias == nullptr;
+      __syncwarp();
+      return true;
+    };
+    if (!__all_sync(0xffffffffu, mbar_wait_to(q_full, 0, 123))) goto done;
+    if (!issue_s(0)) goto done;
+    for (int j = 0; j < n_tiles; ++j) {
+      if (j + 1 < n_tiles && !issue_s(j + 1)) goto done;
+      if (!__all_sync(0xffffffffu, mbar_wait_to(&v_full[j % NS], (j / NS) & 1, 127, j))) goto done;
+      if (!__all_sync(0xffffffffu, mbar_wait_to(p_full, j & 1, 124, j))) goto done;
+      tc_fence_after();
+      const uint32_t sV = sbase + L::oV + (j % NS) * L::kV;
+      if (elected) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)                             // the weights' smallest term first
+#pragma unroll
+          for (int kk = 0; kk < kBK / 16; ++kk)
+            umma_f16_ts(tm + 256, tm + 384 + (2 - i) * 32 + kk * 8, make_smem_desc(sV + kk * 2048, kBK * 128, 1024, 2), idesc_o,
+                        (i | kk) != 0);
+        umma_commit(&v_empty[j % NS]);
+        umma_commit(o_full);
+      }
+      __syncwarp();
+    }
+  } else {
+    const int quad = warp & 3, half = warp >> 2;                // lane quadrant; keys 32 half .. and value channels DV/2 half ..
+    const int r = quad * 32 + lane, qp = pos0 + r;              // this thread's row
+    const uint32_t lane_off = uint32_t(quad * 32) << 16;
+    float* xch = reinterpret_cast<float*>(smb + L::oRow) + r;
+    for (int i = tid; i < kSmQ * (D / 8); i += 256) {
+      const int qr = i / (D / 8), c = i % (D / 8);
+      float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (qr < nq) load8_f32<float>(q + ((long long)(row0 + qr) * Hq + h) * D + c * 8, v);
+      uint32_t w[3][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) split3<true>(v[2 * j] * scale, v[2 * j + 1] * scale, w[0][j], w[1][j], w[2][j]);
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        *reinterpret_cast<uint4*>(smb + j * L::kQ + (c >> 3) * (kSmQ * 128) + qr * 128 + (((c & 7) ^ (qr & 7)) << 4)) =
+            make_uint4(w[j][0], w[j][1], w[j][2], w[j][3]);
+    }
+    fence_async_smem();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(q_full);
+
+    constexpr int CV = DV / 2;                                  // value channels of this thread
+    float m = sink ? sink[h] : -INFINITY, l = sink && half == 0 ? 1.f : 0.f, corr_prev = 1.f, acc[CV];
+#pragma unroll
+    for (int i = 0; i < CV; ++i) acc[i] = 0.f;
+    const int lo = first_key(qp, chunk, window), lo_last = first_key(last, chunk, window);
+    auto add_output = [&](int j) -> bool {                      // acc = acc * corr(j) + output of tile j
+      if (!mbar_wait_to(o_full, j & 1, 125, j)) return false;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < CV / 32; ++c) {
+        uint32_t o[32];
+        tmem_ld_32x32(tmem + 256 + half * CV + c * 32 + lane_off, o);
+        tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc[c * 32 + i] = fmaf(acc[c * 32 + i], corr_prev, __uint_as_float(o[i]));
+      }
+      return true;
+    };
+    for (int j = 0; j < n_tiles; ++j) {
+      const int k0 = kbeg + j * kBK + half * 32;
+      if (!mbar_wait_to(&s_full[j & 1], (j >> 1) & 1, 126, j)) goto done;
+      tc_fence_after();
+      float s[32];
+      {
+        uint32_t x[32], y[32];
+        const uint32_t tS = tmem + (j & 1) * 128 + half * 32 + lane_off;
+        tmem_ld_32x32(tS, x);
+        tmem_ld_32x32(tS + 64, y);
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_free[j & 1]);
+#pragma unroll
+        for (int c = 0; c < 32; ++c) s[c] = __uint_as_float(x[c]) + __uint_as_float(y[c]);
+      }
+      // a tile that all rows of the warp see whole needs no look at positions
+      const bool whole = k0 + 31 <= pos0 + quad * 32 && k0 >= lo_last && dist_bias == nullptr;
       if (!whole) {
+        const int c0 = lo - k0, c1 = r < nq ? qp - k0 : -1;     // columns c0 .. c1 are visible
+        if (dist_bias != nullptr) {
+          const float* db = dist_bias + (long long)h * bias_len;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          const int qp = pos0 + r0 + 8 * i;
-          const bool row_ok = r0 + 8 * i < nq;
-#pragma unroll
-          for (int n = 0; n < 8; ++n)
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              float x = s[n][2 * i + e] + s2[n][2 * i + e];
-              const int kj = k0 + n * 8 + t2 + e;
-              const bool ok = row_ok && kj <= qp && kj >= lo[i];
-              if (ok && dist_bias != nullptr) x += __ldg(dist_bias + (long long)h * bias_len + min(qp - kj, bias_len - 1));
-              s[n][2 * i + e] = ok ? x : -INFINITY;
-            }
+          for (int c = 0; c < 32; ++c)
+            if (c >= c0 && c <= c1) s[c] += __ldg(db + min(c1 - c, bias_len - 1));
         }
-      } else {
 #pragma unroll
-        for (int n = 0; n < 8; ++n)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) s[n][i] += s2[n][i];
+        for (int c = 0; c < 32; ++c) s[c] = c >= c0 && c <= c1 ? s[c] : -INFINITY;
       }
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        float mt = -INFINITY;
+      for (int c = 0; c < 32; ++c) mx[c & 3] = fmaxf(mx[c & 3], s[c]);
+      float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+      float* xm = xch + (j & 1) * 256;
+      xm[half * 128] = mt;
+      named_bar_sync(1 + quad, 64);
+      mt = fmaxf(mt, xm[(half ^ 1) * 128]);
+      const float mn = fmaxf(m, mt);
+      const float corr = (mn == -INFINITY) ? 1.f : expf(m - mn);
+      float ps[4] = {0.f, 0.f, 0.f, 0.f};
+      const float mu = (mn == -INFINITY) ? 0.f : mn;            // what is masked becomes expf(-inf) = 0 either way
 #pragma unroll
-        for (int n = 0; n < 8; ++n) mt = fmaxf(mt, fmaxf(s[n][2 * i], s[n][2 * i + 1]));
-        mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 1));
-        mt = fmaxf(mt, __shfl_xor_sync(0xffffffffu, mt, 2));
-        const float mn = fmaxf(m[i], mt);
-        corr[i] = (mn == -INFINITY) ? 1.f : expf(m[i] - mn);
-        float ps = 0.f;
+      for (int c = 0; c < 32; ++c) { s[c] = expf(s[c] - mu); ps[c & 3] += s[c]; }
+      l = l * corr + ((ps[0] + ps[1]) + (ps[2] + ps[3]));
+      m = mn;
+      if (j > 0 && !add_output(j - 1)) goto done;
+      corr_prev = corr;
+      {
+        uint32_t w[3][16];                                      // the weights' terms over those of the tile before, which are used up
 #pragma unroll
-        for (int n = 0; n < 8; ++n)
+        for (int i = 0; i < 16; ++i) split3<false>(s[2 * i], s[2 * i + 1], w[0][i], w[1][i], w[2][i]);
 #pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            const float x = s[n][2 * i + e];
-            const float p = (x == -INFINITY) ? 0.f : expf(x - mn);
-            ps += p;
-            s[n][2 * i + e] = p;
-          }
-        l[i] = l[i] * corr[i] + ps;
-        m[i] = mn;
+        for (int i = 0; i < 3; ++i) tmem_st_32x16(tmem + 384 + i * 32 + half * 16 + lane_off, w[i]);
       }
-      uint32_t ph[4][4], pm[4][4], pl[4][4];                    // the weights as A fragments of 16 keys each
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+    }
+    if (!add_output(n_tiles - 1)) goto done;
+    float* xs = xch + 512;
+    xs[half * 128] = l;
+    bool bad = false;
 #pragma unroll
-      for (int kb = 0; kb < 4; ++kb)
+    for (int i = 0; i < CV; ++i) bad |= !(fabsf(acc[i]) < INFINITY);
+    uint32_t* bad_rows = reinterpret_cast<uint32_t*>(smb + L::oBad);
+    {
+      const uint32_t b = __ballot_sync(0xffffffffu, bad);
+      if (lane == 0) bad_rows[half * 4 + quad] = b;
+    }
+    named_bar_sync(1 + quad, 64);
+    l = xs[0] + xs[128];
+    unsigned again = __ballot_sync(0xffffffffu, (bad_rows[quad] | bad_rows[4 + quad]) >> lane & 1u || !(fabsf(l) < INFINITY));
+    if (r < nq && !(again >> lane & 1u)) {
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      const __nv_bfloat16* gr = gate ? gate + (long long)(row0 + r) * gate_ld + (gate_heads ? h : h * DV + half * CV) : nullptr;
+      __nv_bfloat16* orow = out + (long long)(row0 + r) * out_ld + h * DV + half * CV;
+      const float gh = gate && gate_heads ? sigmoid_f(__bfloat162float(gr[0])) : 1.f;
+      const bool wide = (reinterpret_cast<uintptr_t>(orow) & 15) == 0;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int n = 2 * kb + (i >> 1), e = (i & 1) * 2;
-          split3<false>(s[n][e], s[n][e + 1], ph[kb][i], pm[kb][i], pl[kb][i]);
+      for (int c = 0; c < CV; c += 8) {
+        float x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          x[i] = acc[c + i] * inv;
+          if (gate != nullptr) x[i] *= gate_heads ? gh : sigmoid_f(__bfloat162float(gr[c + i]));
+          x[i] *= out_scale;
         }
-      constexpr int kPart = 8;                                  // value columns in parts of 64
+        if (wide) {
+          *reinterpret_cast<uint4*>(orow + c) = make_uint4(pack_bf16(x[0], x[1]), pack_bf16(x[2], x[3]), pack_bf16(x[4], x[5]),
+                                                           pack_bf16(x[6], x[7]));
+        } else {
 #pragma unroll
-      for (int part = 0; part < DV / 8 / kPart; ++part) {
-        float o[kPart][4];
-#pragma unroll
-        for (int n = 0; n < kPart; ++n)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) o[n][i] = 0.f;
-#pragma unroll
-        for (int kb = 0; kb < 4; ++kb) {
-          uint32_t b[kPart / 2][4];
-#pragma unroll
-          for (int np = 0; np < kPart / 2; ++np)
-            ldsm4_t(b[np], sv + tile_at(kb * 16 + (mi & 1) * 8 + mr, (part * kPart + np * 2) + (mi >> 1), DV * 2));
-#pragma unroll
-          for (int n = 0; n < kPart; ++n) mma_bf16(o[n], pl[kb], b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
-#pragma unroll
-          for (int n = 0; n < kPart; ++n) mma_bf16(o[n], pm[kb], b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
-#pragma unroll
-          for (int n = 0; n < kPart; ++n) mma_bf16(o[n], ph[kb], b[n >> 1][(n & 1) * 2], b[n >> 1][(n & 1) * 2 + 1]);
+          for (int i = 0; i < 8; ++i) orow[c + i] = __float2bfloat16_rn(x[i]);
         }
-#pragma unroll
-        for (int n = 0; n < kPart; ++n)
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            acc[part * kPart + n][i] = fmaf(acc[part * kPart + n][i], corr[i >> 1], o[n][i]);
       }
     }
-    __syncthreads();                                            // the tile just read is the target of the next copies
-  }
-  if (!busy) return;
-  unsigned again = 0u;                                          // bit 4 j + i: row warp * 16 + j + 8 i is not finite
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
-    l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
-    const int r = r0 + 8 * i;
-    bool bad = !(fabsf(l[i]) < INFINITY);
-#pragma unroll
-    for (int n = 0; n < DV / 8; ++n) bad |= !(fabsf(acc[n][2 * i]) < INFINITY) || !(fabsf(acc[n][2 * i + 1]) < INFINITY);
-    unsigned b = __ballot_sync(0xffffffffu, bad && r < nq);
-    b |= b >> 1;
-    b = (b | b >> 2) & 0x11111111u;
-    again |= b << i;
-    if (r >= nq || (b >> (lane & ~3) & 1u)) continue;
-    const float inv = l[i] > 0.f ? 1.f / l[i] : 0.f;
-    const __nv_bfloat16* gr = gate ? gate + (long long)(row0 + r) * gate_ld + (gate_heads ? h : h * DV) : nullptr;
-    __nv_bfloat16* orow = out + (long long)(row0 + r) * out_ld + h * DV;
-    const float gh = gate && gate_heads ? sigmoid_f(__bfloat162float(gr[0])) : 1.f;
-    const bool pairs = (reinterpret_cast<uintptr_t>(orow) & 3) == 0;
-#pragma unroll
-    for (int n = 0; n < DV / 8; ++n) {
-      const int c = n * 8 + t2;
-      float x = acc[n][2 * i] * inv, y = acc[n][2 * i + 1] * inv;
-      if (gate != nullptr) {
-        x *= gate_heads ? gh : sigmoid_f(__bfloat162float(gr[c]));
-        y *= gate_heads ? gh : sigmoid_f(__bfloat162float(gr[c + 1]));
-      }
-      x *= out_scale;
-      y *= out_scale;
-      if (pairs) {
-        *reinterpret_cast<uint32_t*>(orow + c) = pack_bf16(x, y);
-      } else {
-        orow[c] = __float2bfloat16_rn(x);
-        orow[c + 1] = __float2bfloat16_rn(y);
-      }
+    // rows that are not finite, taken in turn by the two warps that share them
+    again &= nq >= quad * 32 + 32 ? 0xffffffffu : nq <= quad * 32 ? 0u : (1u << (nq - quad * 32)) - 1u;
+    for (again &= half == 0 ? 0x55555555u : 0xaaaaaaaau; again != 0u; again &= again - 1u) {
+      const int br = quad * 32 + __ffs(again) - 1, bp = pos0 + br;
+      sink_row_plain<D, DV>(q + ((long long)(row0 + br) * Hq + h) * D, scale, kcache + g * D, vcache + g * DV, tab, block_size,
+                            kpitch, vpitch, first_key(pos0 + br / kBQ * kBQ, chunk, window), first_key(bp, chunk, window), bp,
+                            sink ? sink + h : nullptr, dist_bias ? dist_bias + (long long)h * bias_len : nullptr, bias_len,
+                            gate ? gate + (long long)(row0 + br) * gate_ld + (gate_heads ? h : h * DV) : nullptr, gate_heads,
+                            out + (long long)(row0 + br) * out_ld + h * DV, out_scale);
     }
   }
-  for (; again != 0u; again &= again - 1u) {
-    const int bit = __ffs(again) - 1, r = warp * 16 + (bit >> 2) + 8 * (bit & 1), qp = pos0 + r;
-    sink_row_plain<D, DV>(q + ((long long)(row0 + r) * Hq + h) * D, scale, kcache + g * D, vcache + g * DV, tab, block_size,
-                          kpitch, vpitch, first_key(pos0 + r / kBQ * kBQ, chunk, window), first_key(qp, chunk, window), qp,
-                          sink ? sink + h : nullptr, dist_bias ? dist_bias + (long long)h * bias_len : nullptr, bias_len,
-                          gate ? gate + (long long)(row0 + r) * gate_ld + (gate_heads ? h : h * DV) : nullptr, gate_heads,
-                          out + (long long)(row0 + r) * out_ld + h * DV, out_scale);
+done:
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 8) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
   }
 }

@@ -27,6 +27,7 @@ int sxb_gemm_hang_info(unsigned int* out_host);
  * 2 = force CTA-pair, 3 = force the skinny kernel (NT). */
 int sxb_gemm_set_mode(int mode);
 int sxb_attn_hang_info(unsigned int* out_host);
+int sxb_seqmix_hang_info(unsigned int* out_host);
 /* Local-ownership registry for TMA multicast (no counterpart in the reference).  Kernels that multicast a tile
  * across a cluster only do so when the tensor map covers this GPU's memory alone: ordinary allocation of the
  * current device, whole extent inside one allocation, not registered here.  comm/symm.py registers every peer /
