@@ -982,7 +982,7 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
                          const float* __restrict__ val, long long ldv, const float* __restrict__ decay,
                          const float* __restrict__ beta, const float* __restrict__ skip, float* __restrict__ state,
                          float* __restrict__ out, const int* __restrict__ seq_info, int H, int G, int n, int dv,
-                         int decay_ld) {
+                         int decay_ld, bool longest_first) {
   // Lane l of a column holds the float4 chunks l, l + LPC, l + 2 LPC, ... of the column's n-vector (padded with zeros
   // to NP = LPC R), so k, q and the state move as 16-byte words without bank conflicts.  Two staging buffers, each
   // k [TB][NP] | q [TB][NP] | v [TB][COLS] | decay [TB] | beta [TB]: the next TB tokens are copied in (cp.async) while
@@ -992,8 +992,36 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
   constexpr int NP = R * LPC, R4 = R / 4, COLS = kRecThreads / LPC * NC;
   extern __shared__ __align__(16) float sm[];
   constexpr int stage = (CHAN ? 3 : 2) * kTB * NP + kTB * COLS + 2 * kTB;
-  const int* si = seq_info + 4 * blockIdx.z;
-  const int first = si[0], rows = si[1], seen = si[2], slot = si[3];
+  // The plain delta rule at two columns per lane takes up to 32 sequences longest first, whatever their order: a CTA walks its
+  // sequence alone and there are only a few per SM, so a long one that starts late ends late (us as they come | longest
+  // first: 3 sequences, 2300 rows, 16 heads 277 | 254; 4, 1500, 32: 254 | 222; 6, 3000, 32: 449 | 381; 8, 1500, 16: 130 | 111;
+  // 7, 1500, 16: 126 | 126; shortest first 313 for the first).  Not where little more than one CTA per SM is launched, since then
+  // the longest would be the ones that share (5, 1500, 8, 160 CTAs: 101 | 109).  The other forms keep the order of the batch:
+  // they gain as much with 3, 4 and 6 sequences and lose with 5 and 7 (one column, 5 of 8 heads 124 | 135; two, 7 of 16 heads:
+  // state space 103 | 106, channel decay 164 | 166).  Running every second round of CTAs backwards, to pair long with short, was
+  // worse (3 sequences, 32 heads: no gain; 5, 16: none).
+  // A lane holds the four numbers of one sequence.
+  constexpr bool kSorted = DELTA && !CHAN && NC == 2;
+  auto info = [&](int i) {                 // (four words: the table need not start on 16 bytes)
+    const int* p = seq_info + 4 * i;
+    return make_int4(p[0], p[1], p[2], p[3]);
+  };
+  int4 si;
+  if (kSorted && longest_first) {         // at most 32 sequences
+    const int i = threadIdx.x % 32, count = gridDim.z;
+    si = i < count ? info(i) : make_int4(0, -1, 0, 0);
+    int rank = 0;
+    for (int j = 0; j < count; ++j) {
+      const int other = __shfl_sync(0xffffffffu, si.y, j);
+      rank += other > si.y || (other == si.y && j < i);
+    }
+    const int z = __ffs(__ballot_sync(0xffffffffu, i < count && rank == (int)blockIdx.z)) - 1;
+    si = make_int4(__shfl_sync(0xffffffffu, si.x, z), __shfl_sync(0xffffffffu, si.y, z), __shfl_sync(0xffffffffu, si.z, z),
+                   __shfl_sync(0xffffffffu, si.w, z));
+  } else {
+    si = info(blockIdx.z);
+  }
+  const int first = si.x, rows = si.y, seen = si.z, slot = si.w;
   const int h = blockIdx.y, g = h / (H / G);
   const int lc = threadIdx.x / LPC, l = threadIdx.x % LPC;
   const int col = blockIdx.x * COLS + lc * NC;      // the lane's columns: col .. col + NC - 1
@@ -2115,7 +2143,7 @@ SXB_API int sxb_linear_recurrence(const void* kvec, const void* qvec, long long 
     linear_recurrence_kernel<R, D, LPC, CH, NC><<<dim3((dv + cols - 1) / cols, H, n_seqs), kRecThreads, smem, s>>>(     \
         (const float*)kvec, (const float*)qvec, ldkq, (const float*)val, ldv, (const float*)decay,                  \
         (const float*)beta, (const float*)skip, (float*)state, (float*)out, (const int*)seq_info, H, G, n, dv,      \
-        fixed_decay ? 0 : H);                                                                                       \
+        fixed_decay ? 0 : H, n_seqs <= 32 && 4LL * ((dv + cols - 1) / cols) * H * n_seqs >= 5LL * num_sms());       \
   } while (0)
 #define LAUNCH_REC_N(D, CH)                                  \
   if (n <= 32) LAUNCH_REC(4, D, 8, CH, 1);                   \
