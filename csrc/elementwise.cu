@@ -246,29 +246,46 @@ bias_act_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* 
 // One CTA per token row.  loss[row] = lse - logit[label]; logits are overwritten by
 // dlogits = (softmax - onehot) * (*grad_scale) so the [T,V] tensor is touched twice
 // and never duplicated.  Rows with label == ignore_index get loss 0 / grad 0.
-template <typename T>
-__global__ void __launch_bounds__(1024)
+// What bounds it: bytes under way.  A row's second reading comes from L2 (two CTAs per SM of 256 KB rows are 76 MB), so four
+// words of a thread are asked for before the first is used (bf16, us with one word | four: 2048 rows of 128256 254 | 242,
+// 1024 of 50304 61 | 55, 4096 of 32000 127 | 115, 2048 of 32000 72 | 64; one reading and one writing of the first
+// take 158).
+template <typename T, int THREADS, int CTAS>
+__global__ void __launch_bounds__(THREADS, CTAS)
 xent_kernel(T* __restrict__ logits, const long long* __restrict__ labels,
             float* __restrict__ loss, float* __restrict__ lse_out, int V, long long ld,
             long long ignore_index, const float* __restrict__ grad_scale, int write_grad) {
   __shared__ float red[32];
+  constexpr int U = 4;
   const long long row = blockIdx.x;
   T* lr = logits + row * ld;
   const long long label = labels[row];
   const int nvec = V >> 3;
   float mx = -INFINITY, sum = 0.f;
-  for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
-    float v[8];
-    ld8<T>(lr + vi * 8, v);
-    float lm = v[0];
+  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
+    uint4 raw[U];
 #pragma unroll
-    for (int k = 1; k < 8; ++k) lm = fmaxf(lm, v[k]);
-    const float nm = fmaxf(mx, lm);
-    float acc = 0.f;
+    for (int j = 0; j < U; ++j) {
+      const int vi = v0 + j * THREADS;
+      if (vi < nvec) raw[j] = *reinterpret_cast<const uint4*>(lr + (long long)vi * 8);
+    }
 #pragma unroll
-    for (int k = 0; k < 8; ++k) acc += __expf(v[k] - nm);
-    sum = sum * __expf(mx - nm) + acc;
-    mx = nm;
+    for (int j = 0; j < U; ++j) {
+      if (v0 + j * THREADS >= nvec) break;
+      const T* h = reinterpret_cast<const T*>(&raw[j]);
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = to_f32<T>(h[k]);
+      float lm = v[0];
+#pragma unroll
+      for (int k = 1; k < 8; ++k) lm = fmaxf(lm, v[k]);
+      const float nm = fmaxf(mx, lm);
+      float acc = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) acc += __expf(v[k] - nm);
+      sum = sum * __expf(mx - nm) + acc;
+      mx = nm;
+    }
   }
   for (int j = (nvec << 3) + threadIdx.x; j < V; j += blockDim.x) {
     const float v = to_f32<T>(lr[j]);
@@ -288,16 +305,27 @@ xent_kernel(T* __restrict__ logits, const long long* __restrict__ labels,
   if (!write_grad) return;
   __syncthreads();
   const float gs = ignored ? 0.f : (grad_scale ? *grad_scale : 1.f);
-  for (int vi = threadIdx.x; vi < nvec; vi += blockDim.x) {
-    float v[8];
-    ld8<T>(lr + vi * 8, v);
+  for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
+    uint4 raw[U];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      float pr = __expf(v[k] - lse);
-      if ((long long)(vi * 8 + k) == label) pr -= 1.f;
-      v[k] = pr * gs;
+    for (int j = 0; j < U; ++j) {
+      const int vi = v0 + j * THREADS;
+      if (vi < nvec) raw[j] = *reinterpret_cast<const uint4*>(lr + (long long)vi * 8);
     }
-    st8<T>(lr + vi * 8, v);
+#pragma unroll
+    for (int j = 0; j < U; ++j) {
+      const int vi = v0 + j * THREADS;
+      if (vi >= nvec) break;
+      const T* h = reinterpret_cast<const T*>(&raw[j]);
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        float pr = __expf(to_f32<T>(h[k]) - lse);
+        if ((long long)(vi * 8 + k) == label) pr -= 1.f;
+        v[k] = pr * gs;
+      }
+      st8<T>(lr + (long long)vi * 8, v);
+    }
   }
   for (int j = (nvec << 3) + threadIdx.x; j < V; j += blockDim.x) {
     float pr = __expf(to_f32<T>(lr[j]) - lse);
@@ -473,10 +501,16 @@ SXB_API int sxb_cross_entropy(void* logits, const void* labels, void* loss, void
   if (rows <= 0) return SXB_OK;
   if (ld % 8 || (reinterpret_cast<uintptr_t>(logits) & 15)) return SXB_ERR_UNSUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
-  const int threads = V >= 32768 ? 1024 : 256;
-  DISPATCH_16(dtype, (xent_kernel<T><<<(unsigned)rows, threads, 0, s>>>(
-                         (T*)logits, (const long long*)labels, (float*)loss, (float*)lse, V, ld,
-                         ignore_index, (const float*)grad_scale, write_grad)));
+  // Short rows: 256 threads.  Long ones 512, two CTAs per SM, so that one reads while the other waits in its reductions;
+  // 1024 while no SM has more than one row (64 rows, 128256 columns: 24.6 us, 26.6 with 512; 512 rows: 77.8 and 73.7).
+#define LAUNCH_XENT(THREADS, CTAS)                                                                                            \
+  DISPATCH_16(dtype, (xent_kernel<T, THREADS, CTAS><<<(unsigned)rows, THREADS, 0, s>>>(                                       \
+                         (T*)logits, (const long long*)labels, (float*)loss, (float*)lse, V, ld, ignore_index,                \
+                         (const float*)grad_scale, write_grad)))
+  if (V < 32768) LAUNCH_XENT(256, 4);
+  else if (rows > num_sms()) LAUNCH_XENT(512, 2);
+  else LAUNCH_XENT(1024, 1);
+#undef LAUNCH_XENT
   SXB_CHECK_LAUNCH();
   return SXB_OK;
 }
