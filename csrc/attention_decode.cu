@@ -28,7 +28,7 @@ struct Params {
   long long q_stride, o_stride;
   float scale;
   int after;                       // launched beside an earlier kernel of the stream: leave only behind it
-  int chain;                       // launched while the kernel that makes its queries may still run
+  int chain;                       // the kernel's CHAIN
 };
 
 template <int D>
@@ -47,7 +47,9 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t saddr, uint32_t rank) {
 }
 
 // grid (Hk * S, atoms), clusters of S along x.
-template <int D>
+// CHAIN: launched while the kernel that makes its queries may still run (its own instance: the waits between the set-up and the first
+// loads cost a launch by itself 0.6 of 88 us, 61 requests of 2048 keys).
+template <int D, bool CHAIN>
 __global__ void __launch_bounds__(32 * kWarps, 2)
 paged_decode_kernel(const Params p, const int S) {
   using L = Smem<D>;
@@ -55,8 +57,10 @@ paged_decode_kernel(const Params p, const int S) {
   extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = blockIdx.x % S, hk = blockIdx.x / S;
-  chain_next();
-  if (p.chain) chain_wait();
+  if constexpr (CHAIN) {
+    chain_next();
+    chain_wait();
+  }
   const int* a = p.atoms + 6 * (int)blockIdx.y;
   const int q_row0 = a[1], nq = a[2], q_pos0 = a[3], kv_len = a[5];
   const int* pages = p.tables + (long long)a[0] * p.max_blocks;
@@ -247,7 +251,7 @@ paged_decode_kernel(const Params p, const int S) {
 
 template <int D>
 static int launch(const Params& p, int n_atoms, int S, bool beside, cudaStream_t stream) {
-  auto k = paged_decode_kernel<D>;
+  auto k = p.chain ? paged_decode_kernel<D, true> : paged_decode_kernel<D, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<D>::kTotal);
   if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};

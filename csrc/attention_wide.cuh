@@ -83,14 +83,14 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::oBar);
   uint64_t* q_full = bars + 0;
   uint64_t* kv_full = bars + 1;    // [NS]
-  uint64_t* kv_empty = bars + 4;   // [NS] dQ of the block retired in every CTA of the cluster
+  uint64_t* kv_empty = bars + 4;   // [NS] dQ of the block retired
   uint64_t* s_full = bars + 7;
   uint64_t* s_free = bars + 8;     // S copied into registers (one arrival per row warp)
   uint64_t* dp_full = bars + 9;
   uint64_t* ds_full = bars + 15;   // [2] dS of the first / second 32 keys of each half in place (one arrival per row warp)
   uint64_t* dq_done = bars + 11;
   uint64_t* qa_full = bars + 12;   // Q / dO parked (one arrival per row warp)
-  uint64_t* qa_all = bars + 13;    // ... in every CTA of the cluster
+  uint64_t* qa_all = bars + 13;    // ... and seen there by the MMA warp
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
