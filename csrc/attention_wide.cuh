@@ -13,7 +13,7 @@
 namespace sxb {
 namespace attn {
 
-constexpr int WB = 128;              // block of the inner loop (keys in forward / dQ, queries in dK / dV)
+constexpr int WB = 128;              // block of the inner loop (keys in dQ, queries in dK / dV)
 constexpr int kWideTile = WB * 128 * 2;   // bytes of a [128 x 128] bf16 tile
 
 // exp2, free to be scheduled among other work
@@ -44,6 +44,12 @@ __device__ __forceinline__ F2 mul2(F2 a, F2 b) {
       "mul.rn.f32x2 d, a, b;\n\tmov.b64 {%0, %1}, d;\n\t}" : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
   return d;
 }
+// A block is two groups of 64 columns; of each, the row warps of half h have columns 32 h .. 32 h + 31, and dS / P^T (bf16) goes over
+// the first 16 of the columns that it was made from.  So what a row warp delivers first belongs to the first 64 keys or queries, and
+// the sums run in the order of keys and queries, step by step of 16, whatever the blocks.
+// The A operand of step kk (16 columns of the block) among such columns:
+__device__ __forceinline__ uint32_t a_step(int kk) { return (kk >> 1) * 32 + (kk & 1) * 8; }
+
 // Rows [row, row + 128) of a sequence that begins at `off` into one [128 x 128] tile, in boxes of 64 rows x 64 columns.  A box that
 // lies wholly behind the sequence re-reads the last one that does not (`last64`: its first row), so nothing is touched that blocks
 // of 64 rows would not touch; its products are masked.
@@ -87,7 +93,7 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   uint64_t* s_full = bars + 7;
   uint64_t* s_free = bars + 8;     // S copied into registers (one arrival per row warp)
   uint64_t* dp_full = bars + 9;
-  uint64_t* ds_full = bars + 15;   // [2] dS of the first / second 32 keys of each half in place (one arrival per row warp)
+  uint64_t* ds_full = bars + 15;   // [2] dS of the first / second 64 keys in place (one arrival per row warp)
   uint64_t* dq_done = bars + 11;
   uint64_t* qa_full = bars + 12;   // Q / dO parked (one arrival per row warp)
   uint64_t* qa_all = bars + 13;    // ... and seen there by the MMA warp
@@ -136,7 +142,7 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     for (int j = 0; j < nblk; ++j) {
       const int st = j % NS;
       if (!__all_sync(0xffffffffu, mbar_wait_to(&kv_empty[st], ((j / NS) & 1) ^ 1, 70, j))) goto done;
-      // the last stage: free once Q and dO are parked in every CTA whose ring this load fills
+      // the last stage: free once Q and dO are parked
       if (j == NS - 1 && !__all_sync(0xffffffffu, mbar_wait_to(qa_all, 0, 71))) goto done;
       if (elected) {
         mbar_expect_tx(&kv_full[st], 2 * kWideTile);
@@ -189,15 +195,13 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
       const uint32_t sK = sbase + L::offK(st);
 #pragma unroll
-      for (int q4 = 0; q4 < 2; ++q4) {
-        if (!__all_sync(0xffffffffu, mbar_wait_to(&ds_full[q4], j & 1, 75, j))) goto done;
+      for (int g = 0; g < 2; ++g) {
+        if (!__all_sync(0xffffffffu, mbar_wait_to(&ds_full[g], j & 1, 75, j))) goto done;
         tc_fence_after();
         if (elected) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {   // dS of keys [64 hf, 64 hf + 64) sits on the first 32 of that half's own dP columns
-            const int kk = (i >> 1) * 4 + q4 * 2 + (i & 1);
-            umma_f16_ts(tm_u + 384, tm_u + 256 + (kk >> 2) * 64 + (kk & 3) * 8, desc_mnmajor(sK, WB, kk), idesc_dq, (j | q4 | i) != 0);
-          }
+          for (int kk = 4 * g; kk < 4 * g + 4; ++kk)
+            umma_f16_ts(tm_u + 384, tm_u + 256 + a_step(kk), desc_mnmajor(sK, WB, kk), idesc_dq, (j | kk) != 0);
         }
         __syncwarp();
       }
@@ -210,7 +214,7 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
   } else {
     const int quad = warp & 3;                 // TMEM lane quadrant (hardware: warp id mod 4)
-    const int half = (warp - 2) >> 2;          // which 64 of the block's 128 key columns
+    const int half = (warp - 2) >> 2;          // which 32 of each 64 key columns
     const int row = quad * 32 + lane;
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
     const int qpos = q0 + row;
@@ -238,34 +242,37 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       __syncwarp();
       if (lane == 0) mbar_arrive(qa_full);
     }
-    const uint32_t tSh = tS + lane_off + half * 64, tDPh = tDP + lane_off + half * 64;
+    const uint32_t tSh = tS + lane_off + half * 32, tDPh = tDP + lane_off + half * 32;
     for (int j = 0; j < nblk; ++j) {
       if (!mbar_wait_to(s_full, j & 1, 77, j)) goto done;
       tc_fence_after();
-      float s[64];
-      ld_row64(tSh, s);
+      float s[64];                             // [32 g + c]: column 64 g + 32 half + c of the block
+      ld_row64(tSh, s, 64);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(s_free);
-      const int k0 = j * WB + half * 64;
+      const int k0 = j * WB + half * 32;
       if (p.kbias != nullptr) {
         const float4* kb = reinterpret_cast<const float4*>(p.kbias + b * p.kbias_bstride + h * p.kbias_hstride + k0);
-        const int nv = min(16, (S_ - k0 + 3) >> 2);
 #pragma unroll
         for (int c4 = 0; c4 < 16; ++c4) {
-          if (c4 < nv) {
-            const float4 t = __ldg(kb + c4);
+          const int k4 = (c4 >> 3) * 16 + (c4 & 7);
+          if (k0 + 4 * k4 < S_) {
+            const float4 t = __ldg(kb + k4);
             s[c4 * 4 + 0] += t.x; s[c4 * 4 + 1] += t.y; s[c4 * 4 + 2] += t.z; s[c4 * 4 + 3] += t.w;
           }
         }
       }
-      const bool need_mask = (p.causal && (k0 + 63 > q0)) || (k0 + 64 > S_) || (q0 + BQ > S_);
+      const bool need_mask = (p.causal && (k0 + 95 > q0)) || (k0 + 96 > S_) || (q0 + BQ > S_);
       if (need_mask) {
 #pragma unroll
-        for (int c = 0; c < 64; ++c) {
-          const int kp = k0 + c;
-          const bool ok = (kp < S_) && (!p.causal || kp <= qpos) && (qpos < S_);
-          s[c] = ok ? ex2(fmaf(s[c], sc, -lse2)) : 0.f;
+        for (int g = 0; g < 2; ++g) {
+#pragma unroll
+          for (int c = 32 * g; c < 32 * g + 32; ++c) {
+            const int kp = k0 + 32 * g + c;
+            const bool ok = (kp < S_) && (!p.causal || kp <= qpos) && (qpos < S_);
+            s[c] = ok ? ex2(fmaf(s[c], sc, -lse2)) : 0.f;
+          }
         }
       } else {
 #pragma unroll
@@ -276,23 +283,22 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       }
       if (!mbar_wait_to(dp_full, j & 1, 78, j)) goto done;
       tc_fence_after();
-      // dS (bf16) over the first half of this warp's own dP columns
       float dp[64];
-      ld_row64(tDPh, dp);
+      ld_row64(tDPh, dp, 64);
 #pragma unroll
-      for (int q4 = 0; q4 < 2; ++q4) {
+      for (int g = 0; g < 2; ++g) {
         uint32_t pk[16];
 #pragma unroll
         for (int c = 0; c < 16; ++c) {
-          const int i = q4 * 32 + 2 * c;
+          const int i = g * 32 + 2 * c;
           const F2 d = mul2(mul2(F2{s[i], s[i + 1]}, add2(F2{dp[i], dp[i + 1]}, F2{-dlt, -dlt})), F2{p.scale, p.scale});
           pk[c] = pack_bf16(d.x, d.y);
         }
-        tmem_st_32x16(tDPh + q4 * 16, pk);
+        tmem_st_32x16(tDPh + g * 64, pk);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&ds_full[q4]);
+        if (lane == 0) mbar_arrive(&ds_full[g]);
       }
     }
     if (!mbar_wait_to(dq_done, 0, 79)) goto done;
@@ -358,7 +364,7 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   uint64_t* do_empty = bars + 7;   // [NS]  dV of the block retired
   uint64_t* s_full = bars + 9;
   uint64_t* dp_full = bars + 10;
-  uint64_t* p_full = bars + 17;    // [2] P^T of the first / second 32 queries of each half in place (one arrival per row warp)
+  uint64_t* p_full = bars + 17;    // [2] P^T of the first / second 64 queries in place (one arrival per row warp)
   uint64_t* ds_full = bars + 12;   // dS^T in place (one arrival per row warp)
   uint64_t* acc_done = bars + 13;
   uint64_t* stat_full = bars + 14; // [NS]
@@ -493,15 +499,13 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       // runs in order
       const uint32_t sQ = sbase + L::oQ + st * kWideTile, sDO = sbase + L::oDO + st * kWideTile;
 #pragma unroll
-      for (int q4 = 0; q4 < 2; ++q4) {
-        if (!__all_sync(0xffffffffu, mbar_wait_to(&p_full[q4], it & 1, 105, it))) goto done;
+      for (int g = 0; g < 2; ++g) {
+        if (!__all_sync(0xffffffffu, mbar_wait_to(&p_full[g], it & 1, 105, it))) goto done;
         tc_fence_after();
         if (elected) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {      // P^T of queries [64 hf, 64 hf + 64) sits on the first 32 of that half's own columns
-            const int kk = (i >> 1) * 4 + q4 * 2 + (i & 1);
-            umma_f16_ts(tm_u + 256, tm_u + (kk >> 2) * 64 + (kk & 3) * 8, desc_mnmajor(sDO, WB, kk), idesc_acc, (it | q4 | i) != 0);
-          }
+          for (int kk = 4 * g; kk < 4 * g + 4; ++kk)
+            umma_f16_ts(tm_u + 256, tm_u + a_step(kk), desc_mnmajor(sDO, WB, kk), idesc_acc, (it | kk) != 0);
         }
         __syncwarp();
       }
@@ -513,7 +517,7 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       if (elected) {
 #pragma unroll
         for (int kk = 0; kk < WB / 16; ++kk)
-          umma_f16_ts(tm_u + 384, tm_u + 128 + (kk >> 2) * 64 + (kk & 3) * 8, desc_mnmajor(sQ, WB, kk), idesc_acc, (it | kk) != 0);
+          umma_f16_ts(tm_u + 384, tm_u + 128 + a_step(kk), desc_mnmajor(sQ, WB, kk), idesc_acc, (it | kk) != 0);
         umma_commit(&q_empty[st]);
         if (it == niter - 1) umma_commit(acc_done);
       }
@@ -522,7 +526,7 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     }
   } else {
     const int quad = warp & 3;
-    const int half = (warp - 2) >> 2;          // which 64 of the block's 128 query columns
+    const int half = (warp - 2) >> 2;          // which 32 of each 64 query columns
     const int row = quad * 32 + lane;
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
     const int kpos = n0 + row;
@@ -532,79 +536,78 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     int hrel = 0, qrel = 0, st = 0;
     float kb2 = kb_row ? kb_row[(long long)(hk * group) * p.kbias_hstride] * sc : 0.f;
     uint32_t ph = 0;
-    const uint32_t stat_u = smem_u32(smem + L::oStat) + half * 256;   // this warp's 64 of the 128 queries
-    const uint32_t tSh = tmem + half * 64 + lane_off, tDPh = tSh + 128;
+    const uint32_t stat_u = smem_u32(smem + L::oStat) + half * 128;   // this warp's 32 of the first 64 queries
+    const uint32_t tSh = tmem + half * 32 + lane_off, tDPh = tSh + 128;
     for (int it = 0; it < niter; ++it) {
-      const int qb = (i_start + qrel) * WB + half * 64;
+      const int qb = (i_start + qrel) * WB + half * 32;
       const uint32_t sstat = stat_u + st * 1024;
-      const bool need_mask = (p.causal && (n0 + BQ - 1 > qb)) || (qb + 64 > S_) || (n0 + BQ > S_);
+      const bool need_mask = (p.causal && (n0 + BQ - 1 > qb)) || (qb + 96 > S_) || (n0 + BQ > S_);
       if (!mbar_wait_to(&stat_full[st], ph, 107, it)) goto done;
       if (!mbar_wait_to(s_full, it & 1, 108, it)) goto done;
       tc_fence_after();
-      float s[64];
-      auto p_half_done = [&](int q4) {
+      float s[64];                             // [32 g + c]: query column 64 g + 32 half + c of the block
+      auto p_half_done = [&](int g) {
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&p_full[q4]);
+        if (lane == 0) mbar_arrive(&p_full[g]);
       };
-      // P^T (bf16) over the first 32 of this warp's own S^T columns
-      ld_row64(tSh, s);
+      ld_row64(tSh, s, 64);
       if (!need_mask && p.kbias == nullptr) {      // apart from the other form: branches among the exponentials part them
 #pragma unroll
-        for (int q4 = 0; q4 < 2; ++q4) {
+        for (int g = 0; g < 2; ++g) {
           uint32_t pk[16];
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4) {
-            const float4 nl = lds128(sstat + q4 * 128 + c4 * 16);           // -lse * log2e, warp-broadcast
-            float* o = s + q4 * 32 + c4 * 4;
+            const float4 nl = lds128(sstat + g * 256 + c4 * 16);           // -lse * log2e, warp-broadcast
+            float* o = s + g * 32 + c4 * 4;
             const F2 a = fma2(F2{o[0], o[1]}, F2{sc, sc}, F2{nl.x, nl.y}), d = fma2(F2{o[2], o[3]}, F2{sc, sc}, F2{nl.z, nl.w});
             o[0] = ex2(a.x); o[1] = ex2(a.y); o[2] = ex2(d.x); o[3] = ex2(d.y);
             pk[c4 * 2] = pack_bf16(o[0], o[1]);
             pk[c4 * 2 + 1] = pack_bf16(o[2], o[3]);
           }
-          tmem_st_32x16(tSh + q4 * 16, pk);
-          p_half_done(q4);
+          tmem_st_32x16(tSh + g * 64, pk);
+          p_half_done(g);
         }
       } else {
-        const int first = (kpos < S_) ? (p.causal ? kpos - qb : 0) : 64, end = S_ - qb;     // columns of this key that count
+        const int first = (kpos < S_) ? (p.causal ? kpos - qb : 0) : WB, end = S_ - qb;     // columns of this key that count
 #pragma unroll
-        for (int q4 = 0; q4 < 2; ++q4) {
+        for (int g = 0; g < 2; ++g) {
           uint32_t pk[16];
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4) {
-            const float4 nl = lds128(sstat + q4 * 128 + c4 * 16);
+            const float4 nl = lds128(sstat + g * 256 + c4 * 16);
             const float off[4] = {nl.x + kb2, nl.y + kb2, nl.z + kb2, nl.w + kb2};
-            float* o = s + q4 * 32 + c4 * 4;
+            float* o = s + g * 32 + c4 * 4;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              const int col = q4 * 32 + c4 * 4 + i;
+              const int col = g * 64 + c4 * 4 + i;
               o[i] = (col >= first && col < end) ? ex2(fmaf(o[i], sc, off[i])) : 0.f;
             }
             pk[c4 * 2] = pack_bf16(o[0], o[1]);
             pk[c4 * 2 + 1] = pack_bf16(o[2], o[3]);
           }
-          tmem_st_32x16(tSh + q4 * 16, pk);
-          p_half_done(q4);
+          tmem_st_32x16(tSh + g * 64, pk);
+          p_half_done(g);
         }
       }
       if (!mbar_wait_to(dp_full, it & 1, 109, it)) goto done;
       tc_fence_after();
       float dp[64];
-      ld_row64(tDPh, dp);
+      ld_row64(tDPh, dp, 64);
 #pragma unroll
-      for (int q4 = 0; q4 < 2; ++q4) {
+      for (int g = 0; g < 2; ++g) {
         uint32_t pk[16];
 #pragma unroll
         for (int c4 = 0; c4 < 8; ++c4) {
-          const float4 nd = lds128(sstat + 512 + q4 * 128 + c4 * 16);     // -delta
-          const float *o = s + q4 * 32 + c4 * 4, *x = dp + q4 * 32 + c4 * 4;
+          const float4 nd = lds128(sstat + 512 + g * 256 + c4 * 16);     // -delta
+          const float *o = s + g * 32 + c4 * 4, *x = dp + g * 32 + c4 * 4;
           const F2 a = mul2(mul2(F2{o[0], o[1]}, F2{p.scale, p.scale}), add2(F2{x[0], x[1]}, F2{nd.x, nd.y}));
           const F2 d = mul2(mul2(F2{o[2], o[3]}, F2{p.scale, p.scale}), add2(F2{x[2], x[3]}, F2{nd.z, nd.w}));
           pk[c4 * 2] = pack_bf16(a.x, a.y);
           pk[c4 * 2 + 1] = pack_bf16(d.x, d.y);
         }
-        tmem_st_32x16(tDPh + q4 * 16, pk);
+        tmem_st_32x16(tDPh + g * 64, pk);
       }
       tmem_st_wait();
       tc_fence_before();

@@ -80,3 +80,24 @@ def test_packed_sequences_and_what_lies_behind_them(causal):
     for i in (0, 2, 4, 6):
         r = slice(at[i], at[i + 1])
         _close([x.grad[None, r] for x in t], _reference(q[None, r], k[None, r], v[None, r], do[None, r], causal))
+
+
+@pytest.mark.parametrize("first", range(0, 15))
+def test_sums_run_in_the_order_of_keys_and_queries(first):
+    """Every weight is one, and 2^30 comes and goes in two neighbouring steps of 16 rows: ones that are added between them are lost
+    to the 24 bits of a sum, those behind them are not."""
+    import torch
+    from shuffle_exchange_b200.ops import functional as F
+    S = 256
+    c = torch.zeros(S, device="cuda", dtype=torch.bfloat16)
+    c[16 * first: 16 * first + 16], c[16 * first + 16: 16 * first + 32], c[16 * first + 32:] = 2.0 ** 30, -2.0 ** 30, 1.0
+    want = float(max(0, S - 16 * first - 32))
+    zero, unit = torch.zeros(1, S, 1, 128, device="cuda", dtype=torch.bfloat16), torch.zeros(1, S, 1, 128, device="cuda", dtype=torch.bfloat16)
+    unit[..., 0] = 1.0
+    rows = c[None, :, None, None].expand(1, S, 1, 128).contiguous()
+    grad = rows.clone()
+    grad[..., 0] = 1.0
+    lse = torch.zeros(1, 1, S, device="cuda")
+    dq, _, _ = F.attention_bwd_raw(zero, rows, unit, zero, unit, lse, False, 1.0)
+    _, dk, dv = F.attention_bwd_raw(rows, zero, unit, zero, grad, lse, False, 1.0)
+    assert (dq == want).all() and (dk == want).all() and (dv[..., 1:] == want).all()
