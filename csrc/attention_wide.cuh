@@ -46,19 +46,21 @@ __device__ __forceinline__ F2 mul2(F2 a, F2 b) {
 }
 // A block is two groups of 64 columns; of each, the row warps of half h have columns 32 h .. 32 h + 31, and dS / P^T (bf16) goes over
 // the first 16 of the columns that it was made from.  So what a row warp delivers first belongs to the first 64 keys or queries, and
-// the sums run in the order of keys and queries, step by step of 16, whatever the blocks.
+// the sums run in the order of keys and queries, step by step of 16, whatever the blocks.  A block with at most 64 rows left is
+// narrow: one group, MMAs of 64 columns, half the copies; what lies behind the last row is not read a second time to fill the block,
+// where an infinity would meet a weight of zero.  Delta, dQ, dK and dV, us, blocks of 64 | 128 throughout | narrow ones at the end:
+// 64 sequences of 64 rows, 32 heads of Q, K and V 179 | 192 | 173, 4 of 64, 32 / 8 heads 20.7 | 22.6 | 18.7, packed ones of 17 to 64
+// rows, 4096 in all 212 | 210 | 184, 16 of 192 rows 98 | 93 | 88.
 // The A operand of step kk (16 columns of the block) among such columns:
 __device__ __forceinline__ uint32_t a_step(int kk) { return (kk >> 1) * 32 + (kk & 1) * 8; }
 
-// Rows [row, row + 128) of a sequence that begins at `off` into one [128 x 128] tile, in boxes of 64 rows x 64 columns.  A box that
-// lies wholly behind the sequence re-reads the last one that does not (`last64`: its first row), so nothing is touched that blocks
-// of 64 rows would not touch; its products are masked.
+// Rows [row, row + 64 groups) of a sequence that begins at `off` into a [128 x 128] tile, in boxes of 64 rows x 64 columns.  A box that
+// lies wholly behind the sequence re-reads the last one that does not (`last64`: its first row).
 __device__ __forceinline__ void load_tile(const CUtensorMap* tm, uint8_t* dst, uint64_t* bar, int head, int off, int row, int last64,
-                                          int tb) {
+                                          int tb, int groups) {
 #pragma unroll
   for (int c = 0; c < 2; ++c)
-#pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < groups; ++r)
       tma_load_4d(dst + c * (WB * 128) + r * (64 * 128), tm, bar, c * 64, head, off + min(row + r * 64, last64), tb);
 }
 
@@ -109,6 +111,7 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   if (q0 >= S_) return;
   const int kv_len = p.causal ? min(S_, q0 + BQ) : S_;
   const int nblk = (kv_len + WB - 1) / WB, last64 = (kv_len - 1) / 64 * 64;
+  auto narrow = [&](int j) { return kv_len - j * WB <= 64; };      // the last block, if any
 
   if (warp == 1) {
     if (lane == 0) {
@@ -145,9 +148,10 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // the last stage: free once Q and dO are parked
       if (j == NS - 1 && !__all_sync(0xffffffffu, mbar_wait_to(qa_all, 0, 71))) goto done;
       if (elected) {
-        mbar_expect_tx(&kv_full[st], 2 * kWideTile);
-        load_tile(&tmK, smem + L::offK(st), &kv_full[st], hk, w.off, j * WB, last64, w.tb);
-        load_tile(&tmV, smem + L::offV(st), &kv_full[st], hk, w.off, j * WB, last64, w.tb);
+        const int groups = narrow(j) ? 1 : 2;
+        mbar_expect_tx(&kv_full[st], groups * kWideTile);
+        load_tile(&tmK, smem + L::offK(st), &kv_full[st], hk, w.off, j * WB, last64, w.tb, groups);
+        load_tile(&tmV, smem + L::offV(st), &kv_full[st], hk, w.off, j * WB, last64, w.tb, groups);
       }
       __syncwarp();
     }
@@ -155,24 +159,24 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const bool elected = elect_one();
     const uint32_t sbase = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
     const uint32_t tm_u = __shfl_sync(0xffffffffu, tmem, 0);
-    const uint32_t idesc_s = make_idesc(BQ, WB, 1, 1, 0, 0);
+    const uint32_t idesc_s = make_idesc(BQ, WB, 1, 1, 0, 0), idesc_s64 = make_idesc(BQ, 64, 1, 1, 0, 0);
     const uint32_t idesc_dq = make_idesc(BQ, D, 1, 1, 0, 1);
     auto issue_s = [&](int j) {
-      const uint32_t sK = sbase + L::offK(j % NS);
+      const uint32_t sK = sbase + L::offK(j % NS), idesc = narrow(j) ? idesc_s64 : idesc_s;
       if (elected) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16_ts(tm_u + 128, tm_u + kk * 8, desc_kmajor_d(sK, WB, kk), idesc_s, kk != 0);
+          umma_f16_ts(tm_u + 128, tm_u + kk * 8, desc_kmajor_d(sK, WB, kk), idesc, kk != 0);
         umma_commit(s_full);
       }
       __syncwarp();
     };
     auto issue_dp = [&](int j) {
-      const uint32_t sV = sbase + L::offV(j % NS);
+      const uint32_t sV = sbase + L::offV(j % NS), idesc = narrow(j) ? idesc_s64 : idesc_s;
       if (elected) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16_ts(tm_u + 256, tm_u + 64 + kk * 8, desc_kmajor_d(sV, WB, kk), idesc_s, kk != 0);
+          umma_f16_ts(tm_u + 256, tm_u + 64 + kk * 8, desc_kmajor_d(sV, WB, kk), idesc, kk != 0);
         umma_commit(dp_full);
       }
       __syncwarp();
@@ -196,6 +200,7 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       const uint32_t sK = sbase + L::offK(st);
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
+        if (g == 1 && narrow(j)) break;
         if (!__all_sync(0xffffffffu, mbar_wait_to(&ds_full[g], j & 1, 75, j))) goto done;
         tc_fence_after();
         if (elected) {
@@ -267,6 +272,7 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (need_mask) {
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
+          if (g == 1 && narrow(j)) break;
 #pragma unroll
           for (int c = 32 * g; c < 32 * g + 32; ++c) {
             const int kp = k0 + 32 * g + c;
@@ -287,6 +293,7 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       ld_row64(tDPh, dp, 64);
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
+        if (g == 1 && narrow(j)) break;
         uint32_t pk[16];
 #pragma unroll
         for (int c = 0; c < 16; ++c) {
@@ -385,6 +392,7 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   const int per_head = (S_ + WB - 1) / WB - i_start;
   const int niter = per_head * group;
   const int last64 = (S_ - 1) / 64 * 64;
+  auto narrow = [&](int qrel) { return S_ - (i_start + qrel) * WB <= 64; };       // the last block of each head, if any
 
   if (warp == 1) {
     if (lane == 0) {
@@ -408,8 +416,8 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const bool elected = elect_one();
     if (elected) {
       mbar_expect_tx(kv_full, 2 * kWideTile);
-      load_tile(&tmK, smem + L::oK, kv_full, hk, w.off, n0, last64, w.tb);
-      load_tile(&tmV, smem + L::oV, kv_full, hk, w.off, n0, last64, w.tb);
+      load_tile(&tmK, smem + L::oK, kv_full, hk, w.off, n0, last64, w.tb, 2);
+      load_tile(&tmV, smem + L::oV, kv_full, hk, w.off, n0, last64, w.tb, 2);
     }
     __syncwarp();
     // The statistics of each block's queries (-lse * log2e and -delta) go next to its Q tile: loaded one block ahead, written
@@ -431,8 +439,10 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     for (int it = 0; it < niter; ++it) {
       if (!__all_sync(0xffffffffu, mbar_wait_to(&q_empty[st], ph, 100, it))) goto done;
       if (elected) {
-        mbar_expect_tx(&q_full[st], kWideTile);
-        load_tile(&tmQ, smem + L::oQ + st * kWideTile, &q_full[st], hk * group + hrel, w.off, (i_start + qrel) * WB, last64, w.tb);
+        const int groups = narrow(qrel) ? 1 : 2;
+        mbar_expect_tx(&q_full[st], groups * (kWideTile / 2));
+        load_tile(&tmQ, smem + L::oQ + st * kWideTile, &q_full[st], hk * group + hrel, w.off, (i_start + qrel) * WB, last64, w.tb,
+                  groups);
       }
       float* sp = stat + st * 256;
 #pragma unroll
@@ -450,8 +460,10 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     for (int it = 0; it < niter; ++it) {
       if (!__all_sync(0xffffffffu, mbar_wait_to(&do_empty[st], ph, 101, it))) goto done;
       if (elected) {
-        mbar_expect_tx(&do_full[st], kWideTile);
-        load_tile(&tmDO, smem + L::oDO + st * kWideTile, &do_full[st], hk * group + hrel, w.off, (i_start + qrel) * WB, last64, w.tb);
+        const int groups = narrow(qrel) ? 1 : 2;
+        mbar_expect_tx(&do_full[st], groups * (kWideTile / 2));
+        load_tile(&tmDO, smem + L::oDO + st * kWideTile, &do_full[st], hk * group + hrel, w.off, (i_start + qrel) * WB, last64, w.tb,
+                  groups);
       }
       __syncwarp();
       if (++qrel == per_head) { qrel = 0; ++hrel; }
@@ -461,40 +473,44 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const bool elected = elect_one();
     const uint32_t sbase = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
     const uint32_t tm_u = __shfl_sync(0xffffffffu, tmem, 0);
-    const uint32_t idesc_s = make_idesc(BQ, WB, 1, 1, 0, 0);
+    const uint32_t idesc_s = make_idesc(BQ, WB, 1, 1, 0, 0), idesc_s64 = make_idesc(BQ, 64, 1, 1, 0, 0);
     const uint32_t idesc_acc = make_idesc(BQ, D, 1, 1, 0, 1);
-    auto issue_s = [&](int it) -> bool {
+    auto issue_s = [&](int it, bool nar) -> bool {
       const int st = it % NS;
       if (!__all_sync(0xffffffffu, mbar_wait_to(&q_full[st], (it / NS) & 1, 102, it))) return false;
       tc_fence_after();
-      const uint32_t sK = sbase + L::oK, sQ = sbase + L::oQ + st * kWideTile;
+      const uint32_t sK = sbase + L::oK, sQ = sbase + L::oQ + st * kWideTile, idesc = nar ? idesc_s64 : idesc_s;
       if (elected) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16(tm_u, desc_kmajor_d(sK, BQ, kk), desc_kmajor_d(sQ, WB, kk), idesc_s, kk != 0);
+          umma_f16(tm_u, desc_kmajor_d(sK, BQ, kk), desc_kmajor_d(sQ, WB, kk), idesc, kk != 0);
         umma_commit(s_full);
       }
       __syncwarp();
       return true;
     };
-    auto issue_dp = [&](int it) -> bool {
+    auto issue_dp = [&](int it, bool nar) -> bool {
       const int st = it % NS;
       if (!__all_sync(0xffffffffu, mbar_wait_to(&do_full[st], (it / NS) & 1, 103, it))) return false;
       tc_fence_after();
-      const uint32_t sV = sbase + L::oV, sDO = sbase + L::oDO + st * kWideTile;
+      const uint32_t sV = sbase + L::oV, sDO = sbase + L::oDO + st * kWideTile, idesc = nar ? idesc_s64 : idesc_s;
       if (elected) {
 #pragma unroll
         for (int kk = 0; kk < D / 16; ++kk)
-          umma_f16(tm_u + 128, desc_kmajor_d(sV, BQ, kk), desc_kmajor_d(sDO, WB, kk), idesc_s, kk != 0);
+          umma_f16(tm_u + 128, desc_kmajor_d(sV, BQ, kk), desc_kmajor_d(sDO, WB, kk), idesc, kk != 0);
         umma_commit(dp_full);
       }
       __syncwarp();
       return true;
     };
+    int qrel = 0;
+    bool nar = narrow(0);
     if (!__all_sync(0xffffffffu, mbar_wait_to(kv_full, 0, 104))) goto done;
-    if (!issue_s(0) || !issue_dp(0)) goto done;
+    if (!issue_s(0, nar) || !issue_dp(0, nar)) goto done;
     for (int it = 0; it < niter; ++it) {
       const int st = it % NS;
+      if (++qrel == per_head) qrel = 0;
+      const bool nar_next = narrow(qrel);
       // S^T(it + 1) overwrites P^T(it), dP^T(it + 1) dS^T(it): behind the MMAs that read them in this thread's stream, which
       // runs in order
       const uint32_t sQ = sbase + L::oQ + st * kWideTile, sDO = sbase + L::oDO + st * kWideTile;
@@ -502,7 +518,7 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       for (int g = 0; g < 2; ++g) {
         if (!__all_sync(0xffffffffu, mbar_wait_to(&p_full[g], it & 1, 105, it))) goto done;
         tc_fence_after();
-        if (elected) {
+        if (elected && !(g == 1 && nar)) {
 #pragma unroll
           for (int kk = 4 * g; kk < 4 * g + 4; ++kk)
             umma_f16_ts(tm_u + 256, tm_u + a_step(kk), desc_mnmajor(sDO, WB, kk), idesc_acc, (it | kk) != 0);
@@ -511,18 +527,21 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       }
       if (elected) umma_commit(&do_empty[st]);
       __syncwarp();
-      if (it + 1 < niter && !issue_s(it + 1)) goto done;
+      if (it + 1 < niter && !issue_s(it + 1, nar_next)) goto done;
       if (!__all_sync(0xffffffffu, mbar_wait_to(ds_full, it & 1, 106, it))) goto done;
       tc_fence_after();
       if (elected) {
 #pragma unroll
-        for (int kk = 0; kk < WB / 16; ++kk)
+        for (int kk = 0; kk < WB / 16; ++kk) {
+          if (kk == 4 && nar) break;
           umma_f16_ts(tm_u + 384, tm_u + 128 + a_step(kk), desc_mnmajor(sQ, WB, kk), idesc_acc, (it | kk) != 0);
+        }
         umma_commit(&q_empty[st]);
         if (it == niter - 1) umma_commit(acc_done);
       }
       __syncwarp();
-      if (it + 1 < niter && !issue_dp(it + 1)) goto done;
+      if (it + 1 < niter && !issue_dp(it + 1, nar_next)) goto done;
+      nar = nar_next;
     }
   } else {
     const int quad = warp & 3;
@@ -540,6 +559,7 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     const uint32_t tSh = tmem + half * 32 + lane_off, tDPh = tSh + 128;
     for (int it = 0; it < niter; ++it) {
       const int qb = (i_start + qrel) * WB + half * 32;
+      const bool nar = narrow(qrel);
       const uint32_t sstat = stat_u + st * 1024;
       const bool need_mask = (p.causal && (n0 + BQ - 1 > qb)) || (qb + 96 > S_) || (n0 + BQ > S_);
       if (!mbar_wait_to(&stat_full[st], ph, 107, it)) goto done;
@@ -573,21 +593,23 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         const int first = (kpos < S_) ? (p.causal ? kpos - qb : 0) : WB, end = S_ - qb;     // columns of this key that count
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
-          uint32_t pk[16];
+          if (!(g == 1 && nar)) {
+            uint32_t pk[16];
 #pragma unroll
-          for (int c4 = 0; c4 < 8; ++c4) {
-            const float4 nl = lds128(sstat + g * 256 + c4 * 16);
-            const float off[4] = {nl.x + kb2, nl.y + kb2, nl.z + kb2, nl.w + kb2};
-            float* o = s + g * 32 + c4 * 4;
+            for (int c4 = 0; c4 < 8; ++c4) {
+              const float4 nl = lds128(sstat + g * 256 + c4 * 16);
+              const float off[4] = {nl.x + kb2, nl.y + kb2, nl.z + kb2, nl.w + kb2};
+              float* o = s + g * 32 + c4 * 4;
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const int col = g * 64 + c4 * 4 + i;
-              o[i] = (col >= first && col < end) ? ex2(fmaf(o[i], sc, off[i])) : 0.f;
+              for (int i = 0; i < 4; ++i) {
+                const int col = g * 64 + c4 * 4 + i;
+                o[i] = (col >= first && col < end) ? ex2(fmaf(o[i], sc, off[i])) : 0.f;
+              }
+              pk[c4 * 2] = pack_bf16(o[0], o[1]);
+              pk[c4 * 2 + 1] = pack_bf16(o[2], o[3]);
             }
-            pk[c4 * 2] = pack_bf16(o[0], o[1]);
-            pk[c4 * 2 + 1] = pack_bf16(o[2], o[3]);
+            tmem_st_32x16(tSh + g * 64, pk);
           }
-          tmem_st_32x16(tSh + g * 64, pk);
           p_half_done(g);
         }
       }
@@ -597,6 +619,7 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       ld_row64(tDPh, dp, 64);
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
+        if (g == 1 && nar) break;
         uint32_t pk[16];
 #pragma unroll
         for (int c4 = 0; c4 < 8; ++c4) {

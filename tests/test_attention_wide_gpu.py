@@ -101,3 +101,18 @@ def test_sums_run_in_the_order_of_keys_and_queries(first):
     dq, _, _ = F.attention_bwd_raw(zero, rows, unit, zero, unit, lse, False, 1.0)
     _, dk, dv = F.attention_bwd_raw(rows, zero, unit, zero, grad, lse, False, 1.0)
     assert (dq == want).all() and (dk == want).all() and (dv[..., 1:] == want).all()
+
+
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("S,Hq,Hk", [(1, 2, 1), (16, 2, 1), (33, 4, 2), (64, 4, 1), (130, 4, 1), (192, 6, 2), (193, 2, 1), (320, 4, 4)])
+def test_infinite_last_row_stays_where_it_is(S, Hq, Hk, causal):
+    """Blocks with at most 64 rows left have nothing behind those rows: an infinity of the last row of dO meets its own weights only,
+    which are not zero, and is never read a second time with weight zero."""
+    import torch
+    from shuffle_exchange_b200.ops import functional as F
+    q, k, v, do = _tensors((1, S, Hq, 128), (1, S, Hk, 128), (1, S, Hk, 128), (1, S, Hq, 128))
+    do[0, -1, :, 5] = float("inf")
+    t = [x.clone().requires_grad_() for x in (q, k, v)]
+    F.flash_attention(*t, causal=causal).backward(do)
+    dv = t[2].grad[0]
+    assert (dv[:, :, 5] == float("inf")).all() and torch.isfinite(dv[:, :, :5]).all() and torch.isfinite(dv[:, :, 6:]).all()
