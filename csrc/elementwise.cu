@@ -7,6 +7,7 @@
 //   rotary            deepspeed/sequence/layer.py:84-103, deepspeed/sequence/fpdt_layer.py:26-37
 //   vocab-parallel CE deepspeed/sequence/cross_entropy.py:13-58
 //   ragged embed      deepspeed/inference/v2/kernels/ragged_ops/embed/embed_cuda.cu:19-90
+#include <cfloat>
 #include "sxb_common.cuh"
 
 namespace sxb {
@@ -261,7 +262,8 @@ xent_kernel(T* __restrict__ logits, const long long* __restrict__ labels,
   T* lr = logits + row * ld;
   const long long label = labels[row];
   const int nvec = V >> 3;
-  float mx = -INFINITY, sum = 0.f;
+  // a finite lowest value: -inf minus it is -inf, so words of masked columns alone leave a sum of 0, not NaN
+  float mx = -FLT_MAX, sum = 0.f;
   for (int v0 = threadIdx.x; v0 < nvec; v0 += U * THREADS) {
     uint4 raw[U];
 #pragma unroll
@@ -294,8 +296,7 @@ xent_kernel(T* __restrict__ logits, const long long* __restrict__ labels,
     mx = nm;
   }
   const float gmx = block_max(mx, red);
-  sum = (mx == -INFINITY) ? 0.f : sum * __expf(mx - gmx);
-  sum = block_sum(sum, red);
+  sum = block_sum(sum * __expf(mx - gmx), red);
   const float lse = gmx + __logf(sum);
   const bool ignored = (label == ignore_index);
   if (threadIdx.x == 0) {

@@ -29,3 +29,56 @@ def test_against_float64(rows, vocab):
     assert abs(got.double() * n - want).item() <= n * (eps + 40 * 2.0 ** -22) + 3 * want.item() * 2.0 ** -24
     err = (leaf.grad.double() * n - y.grad).abs()
     assert (err <= y.grad.abs() * (2.0 ** -8 + 2 * eps) + 2 * eps + 2.0 ** -20).all()
+
+
+def _masked(rows, vocab, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = (4 * torch.randn(rows, vocab, generator=g, device="cuda")).bfloat16()
+    lo, hi, inf = vocab // 2, vocab - vocab // 4, float("-inf")
+    x[0, :lo], x[1, hi:], x[2, : vocab - 1], x[3, lo + 1:], x[3, :lo] = inf, inf, inf, inf, inf
+    x[4, :lo] = torch.finfo(torch.bfloat16).min            # the lowest number there is
+    x[5::7, ::2] = inf
+    labels = torch.full((rows,), vocab - 1, device="cuda")
+    labels[1], labels[3] = 0, lo
+    return x, labels
+
+
+def _check(grad, loss, x, labels, gs):
+    y = x.double().requires_grad_()
+    want = torch.nn.functional.cross_entropy(y, labels, reduction="none")
+    want.sum().backward()
+    eps = (x.shape[1] / 256 + 8 + 11) * 2.0 ** -24 + 2.0 ** -17         # as above
+    assert ((loss.double() - want).abs() <= eps + 3 * want.abs() * 2.0 ** -24 + 40 * 2.0 ** -22).all()
+    err = (grad.double() / gs - y.grad).abs()
+    assert (err <= y.grad.abs() * (2.0 ** -8 + 2 * eps) + 2 * eps + 2.0 ** -20).all()
+
+
+@pytest.mark.parametrize("rows", [6, 300])
+@pytest.mark.parametrize("vocab", [8, 2048, 8192, 24584, 32768, 49160, 98312])
+def test_masked_columns(rows, vocab):
+    """Columns at -inf, whole words and whole threads of them, weigh nothing wherever they stand."""
+    x, labels = _masked(rows, vocab, vocab)
+    for r in range(rows):                                  # a label is one of the columns that count
+        if not torch.isfinite(x[r, labels[r]]):
+            labels[r] = int(torch.isfinite(x[r]).nonzero()[0])
+    leaf = x.clone().requires_grad_()
+    loss = F.cross_entropy(leaf * 1, labels)
+    loss.backward()
+    y = x.double()
+    rows_loss = torch.logsumexp(y, 1) - y.gather(1, labels[:, None])[:, 0]
+    assert abs(loss.double().item() - rows_loss.mean().item()) <= 2.0 ** -15 * max(1.0, rows_loss.mean().item())
+    _check(leaf.grad, rows_loss, x, labels, 1.0 / rows)
+
+
+@pytest.mark.parametrize("vocab", [5, 13, 2051, 32771])
+def test_masked_columns_and_a_last_partial_word(vocab):
+    from shuffle_exchange_b200.native import lib
+    ld = (vocab + 7) // 8 * 8
+    x, labels = _masked(6, vocab, vocab)
+    wide = torch.zeros(6, ld, device="cuda", dtype=torch.bfloat16)
+    wide[:, :vocab] = x
+    loss = torch.empty(6, device="cuda")
+    labels[5] = int(torch.isfinite(x[5]).nonzero()[0])
+    lib.call("sxb_cross_entropy", wide.data_ptr(), labels.data_ptr(), loss.data_ptr(), None, 6, vocab, ld, -100, None, 1,
+             lib.dtype_code(torch.bfloat16), lib.stream_ptr())
+    _check(wide[:, :vocab], loss, x, labels, 1.0)
