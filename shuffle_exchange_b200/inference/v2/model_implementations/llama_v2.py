@@ -81,7 +81,9 @@ class RaggedLlamaModel:
         c, m = self.cfg, self.lm.model
         H, nq, nkv, d = c.hidden_size, c.num_attention_heads, c.num_key_value_heads, c.head_dim
         Fw, bf16, dev = c.intermediate_size, torch.bfloat16, m.embed_tokens.device
-        if (self.moe_layers is not None or F.flop_sink is not None or dev.type != "cuda" or not hasattr(batch, "atoms")
+        # (a subclass or an object with a feed-forward of its own has it called)
+        if (self.moe_layers is not None or getattr(self._mlp, "__func__", None) is not RaggedLlamaModel._mlp
+                or F.flop_sink is not None or dev.type != "cuda" or not hasattr(batch, "atoms")
                 or batch.current_tokens == 0 or batch.atoms().shape[0] == 0 or H % 8 or Fw % 8 or not _n.no_tape()):
             return None
         head = self.lm.head_weight()

@@ -83,3 +83,25 @@ def test_replaced_weights_are_seen(monkeypatch):
     want, _ = _serve(eng, False, monkeypatch)
     assert n == len(STEPS) and all(torch.equal(a, b) for a, b in zip(got, want))
     assert not torch.equal(got[0], before[0])
+
+
+def test_a_feed_forward_of_its_own_is_called(monkeypatch):
+    import torch
+    from shuffle_exchange_b200.inference.v2.model_implementations.llama_v2 import RaggedLlamaModel
+    model, eng = _engine(512, 4, 2, 1024, 1024)
+    plain, n = _serve(eng, True, monkeypatch)
+    assert n == len(STEPS)
+    ragged = next(x for x in vars(eng).values() if isinstance(x, RaggedLlamaModel))
+
+    class Halved(RaggedLlamaModel):
+        def _mlp(self, layer_idx, layer, x):
+            return super()._mlp(layer_idx, layer, x) * 0.5
+
+    ragged.__class__ = Halved
+    got, n = _serve(eng, True, monkeypatch)
+    want, _ = _serve(eng, False, monkeypatch)
+    assert n == 0 and all(torch.equal(a, b) for a, b in zip(got, want)) and not torch.equal(got[0], plain[0])
+    ragged.__class__ = RaggedLlamaModel
+    ragged._mlp = lambda layer_idx, layer, x: RaggedLlamaModel._mlp(ragged, layer_idx, layer, x) * 0.5
+    again, n = _serve(eng, True, monkeypatch)
+    assert n == 0 and all(torch.equal(a, b) for a, b in zip(again, want))
