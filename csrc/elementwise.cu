@@ -104,7 +104,7 @@ __device__ __forceinline__ float act_bwd(float x, int act) {
 // out[T,F] = act(in[:, :F] (+bias)) * (in[:, F:] (+bias))       (concatenated gate|up layout)
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
-gated_fwd_kernel(const T* __restrict__ in, const T* __restrict__ bias, T* __restrict__ out,
+gated_fwd_kernel(const T* in, const T* __restrict__ bias, T* __restrict__ out,
                  long long rows, int F, int act) {
   chain_next();
   chain_wait();

@@ -427,7 +427,7 @@ ragged_embed_kernel(const int* __restrict__ ids, const int* __restrict__ pos, co
 
 // out[s, :] = hidden[last_token[s], :]     one CTA per sequence
 __global__ void __launch_bounds__(128)
-logits_gather_kernel(const uint4* __restrict__ hidden, const int* __restrict__ last_token, uint4* __restrict__ out,
+logits_gather_kernel(const uint4* hidden, const int* __restrict__ last_token, uint4* __restrict__ out,
                      int row_vec) {
   const int s = blockIdx.x;
   const uint4* src = hidden + (long long)last_token[s] * row_vec;
@@ -442,7 +442,7 @@ logits_gather_kernel(const uint4* __restrict__ hidden, const int* __restrict__ l
 //   tok_seq  [T] sequence slot of the token ; tok_pos [T] absolute position in its sequence
 //   block_tables [n_seqs, max_blocks]
 // grid (T, Hq + Hk), block D/2 threads: thread i rotates the pair (i, i + rot/2) of one head (HF "rotate_half").
-__global__ void kv_rotary_blocked_kernel(__nv_bfloat16* __restrict__ qkv, __nv_bfloat16* __restrict__ cache,
+__global__ void kv_rotary_blocked_kernel(__nv_bfloat16* qkv, __nv_bfloat16* cache,
                                          const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
                                          const int* __restrict__ block_tables, int max_blocks, int block_size, int Hq,
                                          int Hk, int D, int rot_dim, float log2_theta) {

@@ -68,7 +68,7 @@ __device__ __forceinline__ void st8(T* p, const float (&o)[8]) {
 // kLayer: LayerNorm (mean subtraction + bias) vs RMSNorm.
 template <typename T, bool kLayer, int ITERS>
 __global__ void __launch_bounds__(kThreads)
-norm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ res, const T* __restrict__ w,
+norm_fwd_kernel(const T* x, const T* res, const T* __restrict__ w,
                 const T* __restrict__ b, T* __restrict__ y, T* __restrict__ res_out,
                 float* __restrict__ mean_out, float* __restrict__ rstd_out, int H, float eps) {
   __shared__ float red[32];

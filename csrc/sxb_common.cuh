@@ -532,6 +532,8 @@ int encode_tensor_map(CUtensorMap* m, int dtype_code, int rank, const void* ptr,
 // A chain of launches (set for the calls that a host thread makes meanwhile): each kernel may be brought onto the SMs while the one
 // before it still runs, as far as that one leaves room.  A kernel launched so calls chain_wait() ahead of everything that it
 // shares with earlier kernels, reads and writes; what none of them writes (weights, a batch's tables) it may fetch before.
+// Pointers to what they do write are not __restrict__ where the kernel reads through them: that would promise data that stands still
+// while the kernel runs, and allow loads ahead of the wait or through the read-only path.
 bool& chained();
 struct ChainScope {
   bool before;
