@@ -229,7 +229,7 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const float dlt = p.delta[stat_idx];
     {
       // half 0 copies its Q rows, half 1 its dO rows: undo the 128B swizzle, 16 bytes = 4 packed columns at a time
-      if (!mbar_wait_to(q_full, 0, 76)) goto done;
+      mbar_wait_on(q_full, 0, 76);
       const uint8_t* tile = smem + (half == 0 ? L::oQ : L::oDO) + row * 128;
       const uint32_t tA = tmem + half * 64 + lane_off;
 #pragma unroll
@@ -249,7 +249,7 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
     const uint32_t tSh = tS + lane_off + half * 32, tDPh = tDP + lane_off + half * 32;
     for (int j = 0; j < nblk; ++j) {
-      if (!mbar_wait_to(s_full, j & 1, 77, j)) goto done;
+      mbar_wait_on(s_full, j & 1, 77, j);
       tc_fence_after();
       float s[64];                             // [32 g + c]: column 64 g + 32 half + c of the block
       ld_row64(tSh, s, 64);
@@ -287,7 +287,7 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           s[c] = ex2(x.x); s[c + 1] = ex2(x.y);
         }
       }
-      if (!mbar_wait_to(dp_full, j & 1, 78, j)) goto done;
+      mbar_wait_on(dp_full, j & 1, 78, j);
       tc_fence_after();
       float dp[64];
       ld_row64(tDPh, dp, 64);
@@ -308,7 +308,7 @@ attn_bwd_dq128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (lane == 0) mbar_arrive(&ds_full[g]);
       }
     }
-    if (!mbar_wait_to(dq_done, 0, 79)) goto done;
+    mbar_wait_on(dq_done, 0, 79);
     tc_fence_after();
     __nv_bfloat16* orow = out_row_ptr(p, false, w.tb, w.off + min(qpos, S_ - 1)) + (long long)h * D;
 #pragma unroll 1
@@ -562,8 +562,8 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const bool nar = narrow(qrel);
       const uint32_t sstat = stat_u + st * 1024;
       const bool need_mask = (p.causal && (n0 + BQ - 1 > qb)) || (qb + 96 > S_) || (n0 + BQ > S_);
-      if (!mbar_wait_to(&stat_full[st], ph, 107, it)) goto done;
-      if (!mbar_wait_to(s_full, it & 1, 108, it)) goto done;
+      mbar_wait_on(&stat_full[st], ph, 107, it);
+      mbar_wait_on(s_full, it & 1, 108, it);
       tc_fence_after();
       float s[64];                             // [32 g + c]: query column 64 g + 32 half + c of the block
       auto p_half_done = [&](int g) {
@@ -613,7 +613,7 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
           p_half_done(g);
         }
       }
-      if (!mbar_wait_to(dp_full, it & 1, 109, it)) goto done;
+      mbar_wait_on(dp_full, it & 1, 109, it);
       tc_fence_after();
       float dp[64];
       ld_row64(tDPh, dp, 64);
@@ -644,7 +644,7 @@ attn_bwd_dkv128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       }
       if (++st == NS) { st = 0; ph ^= 1; }
     }
-    if (!mbar_wait_to(acc_done, 0, 110)) goto done;
+    mbar_wait_on(acc_done, 0, 110);
     tc_fence_after();
     // half 0 drains dV, half 1 drains dK
     const bool is_dv = (half == 0);

@@ -409,7 +409,7 @@ gemm_pair_x_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         }
         continue;
       }
-      if (!mbar_wait_to(&tfull_bar[acc], acc_phase, 44, t)) goto done;
+      mbar_wait_on(&tfull_bar[acc], acc_phase, 44, t);
       tc_fence_after();
       const int mine = USED ? p.used[ti.g] - (m0 - p.offsets[ti.g]) : 128;      // rows in use of this CTA's 128
       if (USED && mine <= 0) {

@@ -212,7 +212,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       int tm, tn;
       tile_coord(t, tm, tn);
       const int m0 = tm * BM, n0 = tn * BN;
-      if (!mbar_wait_to(&tfull_bar[acc], acc_phase, 4, t)) goto done;
+      mbar_wait_on(&tfull_bar[acc], acc_phase, 4, t);
       tc_fence_after();
       const uint32_t t_row = tmem_base + acc * BN + (uint32_t(quad * 32) << 16);
 #pragma unroll 1
@@ -501,7 +501,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int tm, tn;
       tile_coord(t, tm, tn);
       const int m0 = tm * 256 + int(cta) * 128, n0 = tn * BN;
-      if (!mbar_wait_to(&tfull_bar[acc], acc_phase, 14, t)) goto done;
+      mbar_wait_on(&tfull_bar[acc], acc_phase, 14, t);
       tc_fence_after();
       const uint32_t t_row = tmem_base + acc * BN + (uint32_t(quad * 32) << 16);
 #pragma unroll 1

@@ -283,8 +283,8 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
 #pragma unroll
     for (int i = 0; i < CV; ++i) acc[i] = 0.f;
     const int lo = first_key(qp, chunk, window), lo_last = first_key(last, chunk, window);
-    auto add_output = [&](int j) -> bool {                      // acc = acc * corr(j) + output of tile j
-      if (!mbar_wait_to(o_full, j & 1, 125, j)) return false;
+    auto add_output = [&](int j) {                              // acc = acc * corr(j) + output of tile j
+      mbar_wait_on(o_full, j & 1, 125, j);
       tc_fence_after();
 #pragma unroll
       for (int c = 0; c < CV / 32; ++c) {
@@ -294,11 +294,10 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
 #pragma unroll
         for (int i = 0; i < 32; ++i) acc[c * 32 + i] = fmaf(acc[c * 32 + i], corr_prev, __uint_as_float(o[i]));
       }
-      return true;
     };
     for (int j = 0; j < n_tiles; ++j) {
       const int k0 = kbeg + j * kBK + half * 32;
-      if (!mbar_wait_to(&s_full[j & 1], (j >> 1) & 1, 126, j)) goto done;
+      mbar_wait_on(&s_full[j & 1], (j >> 1) & 1, 126, j);
       tc_fence_after();
       float s[32];
       {
@@ -342,7 +341,7 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
       for (int c = 0; c < 32; ++c) { s[c] = expf(s[c] - mu); ps[c & 3] += s[c]; }
       l = l * corr + ((ps[0] + ps[1]) + (ps[2] + ps[3]));
       m = mn;
-      if (j > 0 && !add_output(j - 1)) goto done;
+      if (j > 0) add_output(j - 1);
       corr_prev = corr;
       {
         uint32_t w[3][16];                                      // the weights' terms over those of the tile before, which are used up
@@ -356,7 +355,7 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
     }
-    if (!add_output(n_tiles - 1)) goto done;
+    add_output(n_tiles - 1);
     float* xs = xch + 512;
     xs[half * 128] = l;
     bool bad = false;
