@@ -320,7 +320,7 @@ def run_ours(args):
     for i in range(args.warmup):
         step_device(i)
     barrier_sync()
-    hang = nlib.hang_info("gemm") or nlib.hang_info("attn")
+    hang = nlib.hang_any()
     if hang:
         raise RuntimeError(f"kernel watchdog fired during warm-up: {hang}")
     sampler = ClockSampler(local)
@@ -364,7 +364,7 @@ def run_ours(args):
     if not args.no_extras and not is_moe and sp == 1:
         extras = secondary_measurements(args, engine, cfg, step_device, barrier_sync, max_over_ranks, dev, world, ms / args.steps,
                                         B, S)
-    hang = nlib.hang_info("gemm") or nlib.hang_info("attn")
+    hang = nlib.hang_any()
     if rank == 0:
         flops = cfg.flops_per_token(args.seq) * tokens_per_step / world
         out = {
@@ -481,8 +481,13 @@ def main():
     if args.serve:
         from shuffle_exchange_b200.inference.v2 import serve_bench
         sizes = list(serve_bench.SIZES) if args.serve == "all" else args.serve.split(",")
-        print(json.dumps(serve_bench.run(sizes, args.serve_prefill, args.serve_batch, args.serve_context, args.steps,
-                                         args.warmup, chunk=args.serve_chunk, model=args.serve_model)))
+        from shuffle_exchange_b200.native import lib as nlib
+        out = serve_bench.run(sizes, args.serve_prefill, args.serve_batch, args.serve_context, args.steps, args.warmup,
+                              chunk=args.serve_chunk, model=args.serve_model)
+        hang = nlib.hang_any()
+        if hang:
+            raise RuntimeError(f"kernel watchdog fired: {hang}")
+        print(json.dumps(out))
         return
     if args.impl == "reference":
         try:

@@ -195,8 +195,17 @@ def attn_call(name: str, *args):
     return call(name, *args)
 
 
+HANG_KINDS = ("attn", "gemm", "gemmx", "moe_ep", "seqmix", "symm")      # kernel families whose waits can give up
+
+
+def hang_any():
+    """``{kind: record}`` of every kernel family that abandoned a wait since it was last asked (its results are garbage), or None."""
+    found = {kind: info for kind in HANG_KINDS if (info := hang_info(kind)) is not None}
+    return found or None
+
+
 def hang_info(kind: str = "attn"):
-    """Read-and-clear the pipeline watchdog record of a kernel family (``gemm`` | ``attn`` | ...).
+    """Read-and-clear the pipeline watchdog record of a kernel family (one of :data:`HANG_KINDS`).
 
     Returns ``None`` when no wait was abandoned since the last call, else a dict naming the
     barrier tag and the block/thread that gave up (see ``mbar_wait_to`` in csrc/sxb_common.cuh).
