@@ -63,7 +63,7 @@ def test_same_bits_as_operator_by_operator(hidden, heads, kv, ff, vocab, layers,
 
 
 def test_what_it_does_not_take(monkeypatch):
-    """Odd vocabulary, head size of 32, weights of another type: operator by operator, as ever."""
+    """Odd vocabulary, head size of 32: operator by operator, as ever."""
     import torch
     for kw in (dict(vocab=1001, heads=4, kv=2), dict(vocab=1024, heads=16, kv=16)):
         model, eng = _engine(512, kw["heads"], kw["kv"], 1024, kw["vocab"])
@@ -105,3 +105,88 @@ def test_a_feed_forward_of_its_own_is_called(monkeypatch):
     ragged._mlp = lambda layer_idx, layer, x: RaggedLlamaModel._mlp(ragged, layer_idx, layer, x) * 0.5
     again, n = _serve(eng, True, monkeypatch)
     assert n == 0 and all(torch.equal(a, b) for a, b in zip(again, want))
+
+
+def test_operands_that_the_plan_refuses(monkeypatch):
+    """Types, pitches, addresses, watchers and layouts that the native call has no check for are turned down before it."""
+    import contextlib
+
+    import torch
+    from torch.utils._python_dispatch import TorchDispatchMode
+    from shuffle_exchange_b200.inference.v2.model_implementations.llama_v2 import RaggedLlamaModel
+    from shuffle_exchange_b200.ops import functional as F
+    model, eng = _engine(512, 4, 2, 1024, 1024)
+    m, layer, P = model.model, model.model.layers[1], torch.nn.Parameter
+
+    @contextlib.contextmanager
+    def put(obj, name, value):
+        old = getattr(obj, name)
+        setattr(obj, name, value)
+        try:
+            yield
+        finally:
+            setattr(obj, name, old)
+
+    @contextlib.contextmanager
+    def mark(w, name):
+        setattr(w, name, None)
+        try:
+            yield
+        finally:
+            delattr(w, name)
+
+    def pitched(w, pitch, shift=0):
+        room = torch.zeros(w.shape[0] * pitch + 8, device="cuda", dtype=w.dtype)
+        return P(torch.as_strided(room, w.shape, (pitch, 1), shift))
+
+    class Watcher(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    ragged = eng._model
+    cache = ragged.state_manager.get_cache(1)
+    every = lambda c: lambda li: c if li == 1 else type(ragged.state_manager).get_cache(ragged.state_manager, li)  # noqa: E731
+    cases = {}
+    for name in ("wqkv", "wo", "w_gate_up", "w_down"):
+        w = getattr(layer, name)
+        cases.update({
+            f"{name} fp32": put(layer, name, P(w.detach().float())),
+            f"{name} fp16": put(layer, name, P(w.detach().half())),
+            f"{name} pitch": put(layer, name, pitched(w, w.shape[1] + 4)),
+            f"{name} base": put(layer, name, pitched(w, w.shape[1], 1)),
+            f"{name} inner stride": put(layer, name, P(w.detach().t().contiguous().t())),
+            f"{name} shape": put(layer, name, P(torch.zeros(0, device="cuda", dtype=w.dtype))),
+            f"{name} device": put(layer, name, P(w.detach().cpu())),
+            f"{name} gated": mark(w, "_sxb_gate"),
+            f"{name} main gradient": mark(w, "_sxb_grad_ready")})
+    norms = [(layer, "input_layernorm"), (layer, "post_attention_layernorm"), (m, "norm")]
+    for obj, name in norms:
+        w = getattr(obj, name)
+        cases.update({
+            f"{name} fp32": put(obj, name, P(w.detach().float())),
+            f"{name} stride": put(obj, name, P(torch.as_strided(torch.ones(2 * 512, device="cuda", dtype=w.dtype), (512,), (2,)))),
+            f"{name} shape": put(obj, name, P(torch.ones(256, device="cuda", dtype=w.dtype)))})
+    cases.update({
+        "embedding pitch": put(m, "embed_tokens", pitched(m.embed_tokens, 520)),
+        "experts": put(ragged, "moe_layers", [{}, {}]),
+        "flops counted": put(F, "flop_sink", lambda *a: None),
+        "cache fp32": put(ragged.state_manager, "get_cache", every(cache.float())),
+        "cache strided": put(ragged.state_manager, "get_cache", every(torch.cat([cache, cache], -1)[..., : cache.shape[-1]])),
+        "cache elsewhere": put(ragged.state_manager, "get_cache", every(cache.cpu())),
+        "cache in parts": put(ragged.state_manager, "get_cache", every((cache, cache))),
+        "dispatch mode": Watcher()})
+    taken, real = [], RaggedLlamaModel._native_plan
+
+    def spy(self, batch):
+        assert real(self, batch) is not None
+        for what, change in cases.items():
+            with change:
+                if real(self, batch) is not None:
+                    taken.append(what)
+        plan = real(self, batch)
+        assert plan is not None
+        return plan
+
+    monkeypatch.setattr(RaggedLlamaModel, "_native_plan", spy)
+    eng.put([0, 1], [torch.arange(5, dtype=torch.int32), torch.arange(70, dtype=torch.int32)])
+    assert not taken, taken

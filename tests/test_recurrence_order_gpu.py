@@ -25,7 +25,8 @@ def test_every_sequence_by_itself(rows, shift):
     got = M.linear_recurrence(k, q, v, decay, beta, None, got_state, table, H, H, n, dv, True)
     for i, (first, r, _, slot) in enumerate(info):         # one at a time: the order of the sums is the same
         one = state.clone()
-        if r:
-            want = M.linear_recurrence(k, q, v, decay, beta, None, one, table[i: i + 1].clone(), H, H, n, dv, True)
-            assert torch.equal(got[first: first + r], want[first: first + r])
-            assert torch.equal(got_state[slot], one[slot])
+        want = M.linear_recurrence(k, q, v, decay, beta, None, one, table[i: i + 1].clone(), H, H, n, dv, True)
+        assert torch.equal(got[first: first + r], want[first: first + r])
+        assert torch.equal(got_state[slot], one[slot])         # without rows, too: kept, or zero where nothing was seen
+        if r == 0:
+            assert torch.equal(one[slot], state[slot] if i % 2 else torch.zeros_like(state[slot])), i
