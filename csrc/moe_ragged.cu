@@ -442,6 +442,9 @@ logits_gather_kernel(const uint4* hidden, const int* __restrict__ last_token, ui
 //   tok_seq  [T] sequence slot of the token ; tok_pos [T] absolute position in its sequence
 //   block_tables [n_seqs, max_blocks]
 // grid (T, Hq + Hk), block D/2 threads: thread i rotates the pair (i, i + rot/2) of one head (HF "rotate_half").
+// CHAIN: launched while the kernel that makes qkv may still run, so position, angle and page come first.  Without a wait between them the
+// angle is worked out while the pair is on its way; with one, 4000 tokens of 16 + 4 heads take 84 us and not 44.
+template <bool CHAIN>
 __global__ void kv_rotary_blocked_kernel(__nv_bfloat16* qkv, __nv_bfloat16* cache,
                                          const int* __restrict__ tok_seq, const int* __restrict__ tok_pos,
                                          const int* __restrict__ block_tables, int max_blocks, int block_size, int Hq,
@@ -449,19 +452,25 @@ __global__ void kv_rotary_blocked_kernel(__nv_bfloat16* qkv, __nv_bfloat16* cach
   const int t = blockIdx.x, head = blockIdx.y, i = threadIdx.x;  // i in [0, D/2)
   const int pos = tok_pos[t];
   const bool is_k = head >= Hq;
-  const int blk = is_k ? block_tables[(long long)tok_seq[t] * max_blocks + pos / block_size] : 0;
-  chain_next();
+  int blk = 0;
+  auto page = [&] { if (is_k) blk = block_tables[(long long)tok_seq[t] * max_blocks + pos / block_size]; };
   const long long row = (long long)t * (Hq + 2 * Hk) * D;
   __nv_bfloat16* h = qkv + row + (long long)head * D;            // q heads then k heads are contiguous
   const int half = rot_dim / 2;
   float x0, x1, sn = 0.f, cs = 1.f;
-  if (i < half) sincosf(pos * exp2f(-(2.0f * i / rot_dim) * log2_theta), &sn, &cs);
-  chain_wait();                                                  // the position and its angle are the batch's own
+  auto angle = [&] { sincosf(pos * exp2f(-(2.0f * i / rot_dim) * log2_theta), &sn, &cs); };
+  if constexpr (CHAIN) {                                         // all of this is the batch's own
+    page();
+    chain_next();
+    if (i < half) angle();
+    chain_wait();
+  }
   int i0, i1;
   if (i < half) { i0 = i; i1 = i + half; } else { i0 = half + i; i1 = -1; }  // beyond rot_dim: pass-through pairs
   if (i < half) {
     x0 = __bfloat162float(h[i0]);
     x1 = __bfloat162float(h[i1]);
+    if constexpr (!CHAIN) angle();
     // which product is rounded is said here, so that it does not hang on the code around
     const float y0 = __fmaf_rn(x0, cs, -__fmul_rn(x1, sn)), y1 = __fmaf_rn(x1, cs, __fmul_rn(x0, sn));
     x0 = y0; x1 = y1;
@@ -476,6 +485,7 @@ __global__ void kv_rotary_blocked_kernel(__nv_bfloat16* qkv, __nv_bfloat16* cach
     if (i < half) { h[i0] = __float2bfloat16_rn(x0); h[i1] = __float2bfloat16_rn(x1); }
     return;
   }
+  if constexpr (!CHAIN) page();
   const int kh = head - Hq;
   const long long slot = ((long long)blk * block_size + pos % block_size) * 2 * Hk * D;
   __nv_bfloat16* kdst = cache + slot + (long long)kh * D;
@@ -732,10 +742,17 @@ SXB_API int sxb_kv_rotary_blocked(void* qkv, void* cache, const void* tok_seq, c
   if (n_tokens <= 0) return SXB_OK;
   if (D % 2 || D > 256 || rot_dim > D || rot_dim % 2) return SXB_ERR_UNSUPPORTED;
   dim3 grid(n_tokens, Hq + Hk);
-  return launch_chained(ragged::kv_rotary_blocked_kernel, grid, D / 2, reinterpret_cast<cudaStream_t>(stream),
-                        static_cast<__nv_bfloat16*>(qkv), static_cast<__nv_bfloat16*>(cache), static_cast<const int*>(tok_seq),
-                        static_cast<const int*>(tok_pos), static_cast<const int*>(block_tables), max_blocks, block_size, Hq, Hk, D,
-                        rot_dim, log2f(theta));
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  const float lt = log2f(theta);
+  auto *x = static_cast<__nv_bfloat16*>(qkv), *c = static_cast<__nv_bfloat16*>(cache);
+  auto *seq = static_cast<const int*>(tok_seq), *pos = static_cast<const int*>(tok_pos), *tables = static_cast<const int*>(block_tables);
+  // in a chain ahead of the kernel before, as long as its CTAs come all at once (32 per SM): behind them there is nothing to be ahead of
+  if (chained() && (long long)n_tokens * (Hq + Hk) <= 32LL * num_sms())
+    return launch_chained(ragged::kv_rotary_blocked_kernel<true>, grid, D / 2, s, x, c, seq, pos, tables, max_blocks, block_size, Hq, Hk,
+                          D, rot_dim, lt);
+  ragged::kv_rotary_blocked_kernel<false><<<grid, D / 2, 0, s>>>(x, c, seq, pos, tables, max_blocks, block_size, Hq, Hk, D, rot_dim, lt);
+  SXB_CHECK_LAUNCH();
+  return SXB_OK;
 }
 
 SXB_API int sxb_paged_attention(const void* q, void* out, const void* cache, const void* tok_seq, const void* tok_pos,
