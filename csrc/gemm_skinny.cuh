@@ -36,10 +36,12 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t saddr, uint32_t rank) {
 }
 
 // grid (tiles of 128 weight rows * S, ceil(M / BN)); clusters of S CTAs along x share one tile.
-template <int BN, int STAGES>
+// CHAIN: launched while the kernel that makes the tokens may still run (its own instance: asked at run time, the question cost a product
+// outside a chain up to half a microsecond, 16 x 768 x 768 7.6 -> 8.2 us).
+template <int BN, int STAGES, bool CHAIN>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p,
-                   const int S, const int chain) {
+                   const int S) {
   using Plan = SkinnyPlan<BN, STAGES>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -72,7 +74,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (chain) chain_next();                  // behind the tensor memory, so that no later kernel takes it first
+  if constexpr (CHAIN) chain_next();        // behind the tensor memory, so that no later kernel takes it first
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t sbase = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
   const uint32_t tbase = __shfl_sync(0xffffffffu, tmem_base, 0);
@@ -80,22 +82,24 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (warp == 0) {
     const bool elected = elect_one();
-    // in a chain the weights of a first turn of the ring are on their way while the kernel that makes the tokens still runs
-    const int ahead = chain ? min(kb1, kb0 + STAGES) : kb0;
-    if (elected)
-      for (int kb = kb0; kb < ahead; ++kb) {
-        mbar_expect_tx(&full_bar[kb - kb0], Plan::kStage);
-        tma_load_2d(smem + (kb - kb0) * Plan::kStage, &tmW, &full_bar[kb - kb0], kb * BK, n0);
-      }
-    __syncwarp();
-    if (chain) chain_wait();
+    int ahead = kb0;
+    if constexpr (CHAIN) {                  // the weights of a first turn of the ring are on their way while that kernel runs
+      ahead = min(kb1, kb0 + STAGES);
+      if (elected)
+        for (int kb = kb0; kb < ahead; ++kb) {
+          mbar_expect_tx(&full_bar[kb - kb0], Plan::kStage);
+          tma_load_2d(smem + (kb - kb0) * Plan::kStage, &tmW, &full_bar[kb - kb0], kb * BK, n0);
+        }
+      __syncwarp();
+      chain_wait();
+    }
     int stage = 0;
     uint32_t phase = 0;
     for (int kb = kb0; kb < kb1; ++kb) {
       if (!__all_sync(0xffffffffu, mbar_wait_to(&empty_bar[stage], phase ^ 1, 41, kb))) break;
       if (elected) {
         uint8_t* sa = smem + stage * Plan::kStage;
-        if (kb >= ahead) {
+        if (!CHAIN || kb >= ahead) {
           mbar_expect_tx(&full_bar[stage], Plan::kStage);
           tma_load_2d(sa, &tmW, &full_bar[stage], kb * BK, n0);
         }

@@ -710,10 +710,10 @@ static bool use_skinny(int M, int N, int K) {
   return tiles <= 128 && tiles <= K / 32;
 }
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool CHAIN>
 static int launch_skinny(const void* A, const void* B, const Params& p, int lda, int ldb, cudaStream_t stream) {
   using Plan = SkinnyPlan<BN, STAGES>;
-  auto kfn = gemm_skinny_kernel<BN, STAGES>;
+  auto kfn = gemm_skinny_kernel<BN, STAGES, CHAIN>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, Plan::kTotal);
@@ -739,17 +739,18 @@ static int launch_skinny(const void* A, const void* B, const Params& p, int lda,
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = chained() ? 2 : 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, tw, tx, p, S, chained() ? 1 : 0);
+  cfg.numAttrs = CHAIN ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kfn, tw, tx, p, S);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
   return SXB_OK;
 }
 
+template <bool CHAIN>
 static int launch_skinny(const void* A, const void* B, const Params& p, int lda, int ldb, cudaStream_t stream) {
-  if (p.M <= 16) return launch_skinny<16, 6>(A, B, p, lda, ldb, stream);
-  if (p.M <= 32) return launch_skinny<32, 5>(A, B, p, lda, ldb, stream);
-  if (p.M <= 64) return launch_skinny<64, 4>(A, B, p, lda, ldb, stream);
-  return launch_skinny<128, 3>(A, B, p, lda, ldb, stream);
+  if (p.M <= 16) return launch_skinny<16, 6, CHAIN>(A, B, p, lda, ldb, stream);
+  if (p.M <= 32) return launch_skinny<32, 5, CHAIN>(A, B, p, lda, ldb, stream);
+  if (p.M <= 64) return launch_skinny<64, 4, CHAIN>(A, B, p, lda, ldb, stream);
+  return launch_skinny<128, 3, CHAIN>(A, B, p, lda, ldb, stream);
 }
 
 }  // namespace gemm
@@ -789,7 +790,7 @@ SXB_API int sxb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
   p.accumulate = accumulate ? 1 : 0; p.direct = tma_c ? 0 : 1; p.C = C; p.ldc = ldc;
   p.alpha = alpha;
   if (layout == NT && (g_gemm_mode == 3 || (g_gemm_mode == 0 && max_ctas <= 0 && use_skinny(M, N, K))))
-    return launch_skinny(A, B, p, lda, ldb, reinterpret_cast<cudaStream_t>(stream));
+    return (chained() ? launch_skinny<true> : launch_skinny<false>)(A, B, p, lda, ldb, reinterpret_cast<cudaStream_t>(stream));
   const int BNsel = (N > 128) ? 256 : 128;
   CUtensorMap ta, tb, tc;
   int rc;
