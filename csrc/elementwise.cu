@@ -251,13 +251,12 @@ bias_act_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* 
 // words of a thread are asked for before the first is used (bf16, us with one word | four: 2048 rows of 128256 254 | 242,
 // 1024 of 50304 61 | 55, 4096 of 32000 127 | 115, 2048 of 32000 72 | 64; one reading and one writing of the first
 // take 158).
-template <typename T, int THREADS, int CTAS>
+template <typename T, int THREADS, int CTAS, int U>
 __global__ void __launch_bounds__(THREADS, CTAS)
 xent_kernel(T* __restrict__ logits, const long long* __restrict__ labels,
             float* __restrict__ loss, float* __restrict__ lse_out, int V, long long ld,
             long long ignore_index, const float* __restrict__ grad_scale, int write_grad) {
   __shared__ float red[32];
-  constexpr int U = 4;
   const long long row = blockIdx.x;
   T* lr = logits + row * ld;
   const long long label = labels[row];
@@ -502,15 +501,18 @@ SXB_API int sxb_cross_entropy(void* logits, const void* labels, void* loss, void
   if (rows <= 0) return SXB_OK;
   if (ld % 8 || (reinterpret_cast<uintptr_t>(logits) & 15)) return SXB_ERR_UNSUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
+  // Rows of at most one word per thread have nothing to ask for ahead, and eight such CTAs fit an SM with the registers of one word
+  // (1024 rows of 256 columns: 4.4 us, 6.5 with four words; 3000 rows: 8.5, 10.1).
   // Short rows: 256 threads.  Long ones 512, two CTAs per SM, so that one reads while the other waits in its reductions;
   // 1024 while no SM has more than one row (64 rows, 128256 columns: 24.6 us, 26.6 with 512; 512 rows: 77.8 and 73.7).
-#define LAUNCH_XENT(THREADS, CTAS)                                                                                            \
-  DISPATCH_16(dtype, (xent_kernel<T, THREADS, CTAS><<<(unsigned)rows, THREADS, 0, s>>>(                                       \
+#define LAUNCH_XENT(THREADS, CTAS, U)                                                                                         \
+  DISPATCH_16(dtype, (xent_kernel<T, THREADS, CTAS, U><<<(unsigned)rows, THREADS, 0, s>>>(                                       \
                          (T*)logits, (const long long*)labels, (float*)loss, (float*)lse, V, ld, ignore_index,                \
                          (const float*)grad_scale, write_grad)))
-  if (V < 32768) LAUNCH_XENT(256, 4);
-  else if (rows > num_sms()) LAUNCH_XENT(512, 2);
-  else LAUNCH_XENT(1024, 1);
+  if (V <= 256 * 8) LAUNCH_XENT(256, 8, 1);
+  else if (V < 32768) LAUNCH_XENT(256, 4, 4);
+  else if (rows > num_sms()) LAUNCH_XENT(512, 2, 4);
+  else LAUNCH_XENT(1024, 1, 4);
 #undef LAUNCH_XENT
   SXB_CHECK_LAUNCH();
   return SXB_OK;
