@@ -89,13 +89,16 @@ class RaggedLlamaModel:
         head = self.lm.head_weight()
         ptrs = 0
 
-        def matrix(w, n, k):
+        def matrix(w, n, k, lds):
             nonlocal ptrs
-            if (w.dtype != bf16 or w.device != dev or w.shape != (n, k) or w.stride(1) != 1 or w.stride(0) % 8
-                    or hasattr(w, "_sxb_gate") or hasattr(w, "_sxb_grad_ready")):
+            if w.dtype != bf16 or w.device != dev or w.shape != (n, k):
+                return None
+            ld, inner = w.stride()
+            if inner != 1 or ld % 8 or hasattr(w, "_sxb_gate") or hasattr(w, "_sxb_grad_ready"):
                 return None
             p = w.data_ptr()
             ptrs |= p
+            lds.append(ld)
             return p
 
         def vector(w):
@@ -108,16 +111,17 @@ class RaggedLlamaModel:
             if (not isinstance(cache, torch.Tensor) or cache.device != dev or not R.atoms_layout_ok(cache, d)
                     or cache.shape[3:] != (nkv, d)):
                 return None
-            wqkv, wo, gu, down = layer.wqkv, layer.wo, layer.w_gate_up, layer.w_down
-            row = [vector(layer.input_layernorm), matrix(wqkv, (nq + 2 * nkv) * d, H), matrix(wo, H, nq * d),
-                   vector(layer.post_attention_layernorm), matrix(gu, 2 * Fw, H), matrix(down, H, Fw), cache.data_ptr()]
+            lds = []
+            row = [vector(layer.input_layernorm), matrix(layer.wqkv, (nq + 2 * nkv) * d, H, lds), matrix(layer.wo, H, nq * d, lds),
+                   vector(layer.post_attention_layernorm), matrix(layer.w_gate_up, 2 * Fw, H, lds),
+                   matrix(layer.w_down, H, Fw, lds), cache.data_ptr()]
             ptrs |= row[-1]
             if None in row:
                 return None
             rows += row
-            rows += [wqkv.stride(0), wo.stride(0), gu.stride(0), down.stride(0)]
+            rows += lds
         emb = m.embed_tokens
-        top = [matrix(emb, emb.shape[0], H), vector(m.norm), matrix(head, head.shape[0], H)]
+        top = [matrix(emb, emb.shape[0], H, []), vector(m.norm), matrix(head, head.shape[0], H, [])]
         if not rows or None in top or not emb.is_contiguous() or head.shape[0] % 8 or ptrs % 16:
             return None
         return rows, top, head, cache
