@@ -28,7 +28,6 @@ struct Params {
   long long q_stride, o_stride;
   float scale;
   int after;                       // launched beside an earlier kernel of the stream: leave only behind it
-  int chain;                       // the kernel's CHAIN
 };
 
 template <int D>
@@ -251,7 +250,8 @@ paged_decode_kernel(const Params p, const int S) {
 
 template <int D>
 static int launch(const Params& p, int n_atoms, int S, bool beside, cudaStream_t stream) {
-  auto k = p.chain ? paged_decode_kernel<D, true> : paged_decode_kernel<D, false>;
+  const bool chain = !beside && chained();
+  auto k = chain ? paged_decode_kernel<D, true> : paged_decode_kernel<D, false>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<D>::kTotal);
   if (e != cudaSuccess) return (int)e;
   cudaLaunchConfig_t cfg = {};
@@ -265,7 +265,7 @@ static int launch(const Params& p, int n_atoms, int S, bool beside, cudaStream_t
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = beside || p.chain ? 2 : 1;
+  cfg.numAttrs = beside || chain ? 2 : 1;
   e = cudaLaunchKernelEx(&cfg, k, p, S);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
   return SXB_OK;
@@ -285,7 +285,6 @@ int paged_decode(const void* q, const void* cache, void* out, const void* atoms,
   p.max_blocks = max_blocks; p.block_size = block_size; p.Hk = Hk; p.group = Hq / Hk;
   p.shift = (block_size & (block_size - 1)) == 0 ? __builtin_ctz(block_size) : -1;
   p.q_stride = q_stride; p.o_stride = o_stride; p.scale = scale; p.after = beside ? 1 : 0;
-  p.chain = !beside && chained() ? 1 : 0;
   // CTAs per sequence: as many as keep the grid within one and a half waves of two per SM, since starting and merging a CTA
   // costs 4 us of a wave (us, up to one and a half | four waves: 61 requests of 2048 80 | 94, 40 of 100 9 | 16, 24 of 6000 93 |
   // 101), and no more than have a step each (4 requests of 40 keys, 32 key/value heads: 4.3 with one, 8.0 with eight).

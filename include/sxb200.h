@@ -418,7 +418,7 @@ int sxb_symm_subset_wsum2(const void* const* bufs, const void* const* sigs, int 
                           void* stream);
 
 /* ---- csrc/attention.cu */
-/* SXB_ATTN_DEBUG=3 cycle accounting of the last dQ launch (8 x uint64, host pointer); see g_attn_prof. */
+/* SXB_ATTN_DEBUG=3 cycle accounting of the last forward or 64-channel dQ launch (8 x uint64, host pointer); see g_attn_prof. */
 int sxb_attn_prof(unsigned long long* out_host);
 
 /* ---- csrc/quantize.cu */
