@@ -3,7 +3,7 @@
 The reference tree does not install (`pip install /root/reference` -> "Neither 'setup.py' nor
 'pyproject.toml' found") and does not import as shipped: ``deepspeed/accelerator``,
 ``deepspeed/ops/op_builder`` and ``deepspeed/ops/csrc`` are 10-16 byte text files (dangling symlink
-stubs), so ``import deepspeed`` dies with ``No module named 'deepspeed.accelerator'`` (SURVEY.md §0.2).
+stubs), so ``import deepspeed`` dies with ``No module named 'deepspeed.accelerator'``.
 
 This script copies every reference file byte-for-byte and puts two tiny *additional* packages where
 the three stubs are:

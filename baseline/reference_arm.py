@@ -8,7 +8,7 @@ gradient checkpointing) through the reference's own public API::
 Same metric, model config, batch, sequence length, optimizer hyper-parameters and timing protocol as
 the product arm.  Nothing from ``shuffle_exchange_b200`` is imported here.  The optimizer is
 ``torch.optim.AdamW`` via the reference's ``torch_adam: true`` switch because the reference's fused-Adam
-CUDA sources are not in its tree (SURVEY.md §0.2).
+CUDA sources are not in its tree.
 """
 from __future__ import annotations
 

@@ -3,7 +3,7 @@
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
-N > 1 is launched by the driver as ``python -m torch.distributed.run --nproc-per-node N ... bench.py
+N > 1 is launched as ``python -m torch.distributed.run --nproc-per-node N ... bench.py
 --gpus N`` (one rank per GPU, NCCL).  Prints ONE JSON line on rank 0.
 
 Timed region = K full training steps (forward + backward with activation recomputation + ZeRO-3

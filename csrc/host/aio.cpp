@@ -1,6 +1,6 @@
 // aio.cpp — asynchronous file IO engine for NVMe offload and fast checkpoint writes.
 //
-// Fresh implementation of the native module behind AsyncIOBuilder (SURVEY §2.3 N15); Python call sites in the
+// Fresh implementation of the native module behind AsyncIOBuilder; Python call sites in the
 // reference: runtime/swap_tensor/utils.py:22-27, partitioned_param_swapper.py:111-122, nvme/test_ds_aio_utils.py:91
 // (aio_handle(block_size, queue_depth, single_submit, overlap_events, intra_op_parallelism) with
 // sync_/async_ pread/pwrite + wait()).

@@ -1,6 +1,6 @@
 // moe_ragged.cu — MoE routing kernels and ragged-batch inference kernels for sm_100a.
 //
-// B200 re-designs of the CUDA kernels shipped under deepspeed/inference/v2/kernels/ragged_ops (SURVEY §2.4):
+// B200 re-designs of the CUDA kernels shipped under deepspeed/inference/v2/kernels/ragged_ops:
 //   top_k_gating      (top_k_gating/top_k_gating_cuda.cu:14-102)
 //   moe_scatter       (moe_scatter/moe_scatter_cuda.cu:23-184)
 //   moe_gather        (moe_gather/moe_gather_cuda.cu:21-138)

@@ -1,7 +1,7 @@
 // quantize.cu — grouped integer and floating-point quantisers, sign packing, random-LTD token movers.
 //
 // Fresh implementations of the native ops the reference loads through op_builder but does not ship
-// (SURVEY §2.3): QuantizerBuilder (N8: ds_quantize / quantize / dequantize / swizzle_quant /
+// in its tree: QuantizerBuilder (N8: ds_quantize / quantize / dequantize / swizzle_quant /
 // quantized_reduction; call sites deepspeed/ops/quantizer/quantizer.py:15-29,
 // runtime/zero/partition_parameters.py:832-862, runtime/comm/coalesced_collectives.py:30-79),
 // FPQuantizerBuilder (N9: ops/fp_quantizer/quantize.py:48-165), PackbitsBuilder (N17:

@@ -377,7 +377,7 @@ constexpr int kMaxVPerLane = 8;      // value head size <= 256
 constexpr int kShortAtom = 16;       // atoms of at most this many queries run one warp per (query, head)
 constexpr int kBQ = 64, kBK = 64;    // query rows / keys per tile of the tiled kernel
 
-// Tiled form for atoms of many queries (prompt portions): one CTA per (64 queries of an atom, query head).  Q (scaled),
+// Tiled form with FMAs for atoms of many queries (prompt portions): one CTA per (64 queries of an atom, query head).  Q (scaled),
 // one 64-key tile of K and V (converted to fp32) and the tile's weights (in the key tile's place, once the scores are
 // done: head sizes up to 128 then leave room for two CTAs per SM) sit in shared memory; 256 threads hold 4x4
 // scores and 4 x (dv/16) outputs each.  Scores, online softmax with the sink logit, and the weighted sum are fp32 FMAs:
@@ -1995,8 +1995,8 @@ static int launch_attention_mma(const void* q, const void* kcache, const void* v
 }
 
 /* The same attention scheduled by attention atoms int32 [n_atoms, 6] = (sequence, first row, queries, first position,
- * -, -), longest first: the first n_long atoms (more than 16 queries, at most 128) run the tiled kernel, 64 queries per
- * CTA; the others one warp per (query, head).  Needs d, dv and both pitches multiples of 4, d and dv at most 256. */
+ * -, -), longest first: the first n_long atoms (more than 16 queries, at most 128) run a tiled kernel, a whole atom per CTA on the
+ * tensor cores or 64 queries per CTA with FMAs; the others one warp per (query, head).  Needs d, dv and both pitches multiples of 4, d and dv at most 256. */
 SXB_API int sxb_sink_attention_atoms(const void* q, const void* kcache, const void* vcache, const void* sink, void* out,
                                      const void* atoms, int n_atoms, int n_long, const void* tables, int max_blocks,
                                      int block_size, int Hq, int G, int d, int dv, float scale, int chunk, int window,

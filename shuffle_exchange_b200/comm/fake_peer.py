@@ -1,4 +1,4 @@
-"""Emulated peers: N logical ranks on ONE GPU (SURVEY §4 (c)).
+"""Emulated peers: N logical ranks on ONE GPU.
 
 The peer-memory kernels only see pointer tables (``bufs[world]``, ``sigs[world]``) and a rank index, so the same
 device code runs when all ``world`` buffers and signal pads live on one device.  The ranks of a collective wait on

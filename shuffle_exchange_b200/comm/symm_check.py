@@ -1,4 +1,4 @@
-"""Flag-protocol checker for the peer-memory collectives (SURVEY §5.2: the reference has no race tooling; its
+"""Flag-protocol checker for the peer-memory collectives (the reference has no race tooling; its
 defences are stream choreography and asserts).
 
 Every symmetric buffer owns a signal pad laid out ``[channel][16 peers]`` of ``uint32`` epochs: peer ``p`` announces

@@ -1,7 +1,7 @@
 """CUDA-only device helper.
 
 The reference routes every device call through a multi-vendor ``get_accelerator()`` object
-(SURVEY.md §2.3 N22 lists the ~60 methods used).  This framework targets B200 only, so the same
+of some 60 methods.  This framework targets B200 only, so the same
 surface is a thin module-level object over ``torch.cuda``; on a machine without a GPU (unit tests
 under gloo) it degrades to CPU so host-side logic stays testable.
 """

@@ -262,8 +262,8 @@ def sink_attention(q: torch.Tensor, kcache: torch.Tensor, vcache: torch.Tensor, 
     ``out_scale`` before it is rounded.
 
     With the batch's attention ``atoms`` (longest first) of which the first ``n_long`` hold more than
-    :data:`SHORT_ATOM` queries, those run the tiled kernel (64 queries per CTA, K/V tiles shared by them) and the rest
-    one warp per (query, head); without atoms every token takes the latter."""
+    :data:`SHORT_ATOM` queries, those run a tiled kernel (K/V tiles shared by an atom's queries on the tensor cores, by
+    64 of them otherwise) and the rest one warp per (query, head); without atoms every token takes the latter."""
     T, Hq, d = q.shape
     bs, G = kcache.shape[1], kcache.shape[2]
     if value_cols > 0:

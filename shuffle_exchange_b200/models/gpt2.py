@@ -1,4 +1,4 @@
-"""GPT-2 ("GPT-2 small ZeRO-1 on CPU/gloo world_size=2").
+"""GPT-2 (trained as GPT-2 small with ZeRO-1 by two gloo ranks on the CPU).
 
 Pre-LN decoder with learned positions, biased projections and tanh-GELU MLP; same fused-op structure
 as ``models/llama.py`` (LayerNorm with fused residual add, bias+GELU kernel, tcgen05 GEMMs and flash

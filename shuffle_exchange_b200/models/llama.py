@@ -1,8 +1,8 @@
 """Llama-family decoder (Llama-2/3, Mistral-style GQA) built on the sm_100a kernels.
 
 The reference does not ship model code for training — users bring a HF/Megatron module and the
-engine wraps it.  This in-tree implementation is what ``bench.py`` trains (BASELINE.json config
-"Llama-3 8B ZeRO-3 bf16") and what the tests use as the flagship model.  Design points:
+engine wraps it.  This in-tree implementation is what ``bench.py`` trains (Llama-3 8B, ZeRO-3, bf16)
+and what the tests use as the flagship model.  Design points:
 
 * fused projections: one ``wqkv`` GEMM ([(Hq+2Hk)·D, H]) and one ``w_gate_up`` GEMM ([2F, H]) so the
   RoPE kernel rotates q|k in place inside the GEMM output and SwiGLU reads one contiguous buffer;

@@ -5,8 +5,8 @@
 * ``libsxb200_host.so`` — ``csrc/host/*.cpp``: AVX-512/AVX2 + OpenMP CPU optimizers, the async
   file-IO engine and host-side schedulers (g++ only, no CUDA).
 
-The reference JIT-builds one pybind module per op through ``op_builder`` (absent from its tree,
-see SURVEY.md §2.3).  Here there is a single C-ABI library per side, built with plain ``nvcc`` /
+The reference JIT-builds one pybind module per op through ``op_builder`` (absent from its
+tree).  Here there is a single C-ABI library per side, built with plain ``nvcc`` /
 ``g++`` in a few seconds, loaded through ``ctypes`` (``native/lib.py``) and declared in
 ``include/sxb200.h``.  Objects are cached on a content hash of the source, every header it can include
 and the compiler flags (``<obj>.sha``), so a stale object cannot outlive a source change whatever the mtimes say.

@@ -2,8 +2,7 @@
 
 Reference: ``deepspeed/ops/fp_quantizer/fp8_gemm.py:23-28`` (dequantise + matmul fallback) and the Triton kernel
 ``fp8_gemm_triton.py:17-165``.  Here the weight is expanded by the grouped dequantise kernel into a bf16 scratch
-tile-set that stays L2-resident for moderate sizes and is consumed by the tcgen05 GEMM (``csrc/gemm_tcgen05.cu``);
-a fully fused dequant-in-the-producer variant is the planned next step.
+tile-set that stays L2-resident for moderate sizes and is consumed by the tcgen05 GEMM (``csrc/gemm_tcgen05.cu``).
 """
 import torch
 

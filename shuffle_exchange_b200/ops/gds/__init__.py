@@ -1,5 +1,5 @@
 """Device-tensor file IO handle (the ``GDSBuilder().load().gds_handle`` of the reference, ``ops/gds`` + the absent
-``csrc/gds`` cuFile binding; SURVEY.md §2.3).
+``csrc/gds`` cuFile binding).
 
 ``gds_handle`` has the ``aio_handle`` method surface but accepts CUDA tensors.  cuFile is not part of this image, so
 transfers take the path cuFile itself uses in compatibility mode: the tensor is streamed through two pinned bounce

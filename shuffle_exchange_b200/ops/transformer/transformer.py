@@ -2,7 +2,7 @@
 
 Reference: ``deepspeed/ops/transformer/transformer.py`` — config (:19-139), the autograd function around the native
 ``forward_fp16/backward_fp16`` entry points (:142-293) and the layer module with its 12 parameters, init rule and
-forward signature (:296-412).  The native module is absent from the reference tree (SURVEY.md §2.3); this is a fresh
+forward signature (:296-412).  The native module is absent from the reference tree; this is a fresh
 B200 implementation on the framework's own kernels:
 
 ==========================  ==============================================================================

@@ -1,7 +1,6 @@
 """Engine checkpoint save / load (bound as methods of :class:`DeepSpeedEngine`).
 
-On-disk layout and key names follow the reference (deepspeed/runtime/engine.py:2826-3959; table in
-SURVEY.md §5.4):
+On-disk layout and key names follow the reference (deepspeed/runtime/engine.py:2826-3959):
 
     <save_dir>/latest                                             text file with the newest tag
     <save_dir>/<tag>/mp_rank_{MP:02d}_model_states.pt              module + bookkeeping
@@ -11,7 +10,7 @@ SURVEY.md §5.4):
     <save_dir>/<tag>/expp_rank_{EP}_mp_rank_{MP:02d}_optim_states.pt            (MoE, non-ZeRO)
     <save_dir>/<tag>/zero_to_fp32.py                               offline consolidation script
 
-One conscious fix (SURVEY.md §2.2-A "side effect"): with replica slices the reference names optimizer
+One conscious fix: with replica slices the reference names optimizer
 files by the rank *inside the slice*, so different replicas overwrite each other.  Here the file index
 is the rank in the full sequence-data-parallel group, and a ``slice_rank`` key is stored inside.
 """

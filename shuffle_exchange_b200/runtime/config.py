@@ -1,5 +1,5 @@
-"""Top-level JSON/HJSON config (reference: deepspeed/runtime/config.py:648-997 ``DeepSpeedConfig``;
-key inventory in SURVEY.md §5.6).
+"""Top-level JSON/HJSON config (reference: deepspeed/runtime/config.py:648-997 ``DeepSpeedConfig``
+and the keys that it reads).
 
 Accepted inputs: a path to a JSON/HJSON file, a dict, or a base64-encoded JSON string.  Duplicate
 keys are rejected.  The batch triad ``train_batch_size = micro_batch x grad_accum x dp_world`` is

@@ -11,7 +11,7 @@ Same user surface as the reference engine (``deepspeed/runtime/pipe/engine.py``:
 * every schedule instruction type maps to one bound handler (``self._handlers``);
 * unlike the reference (which asserts ZeRO stage < 2, :77-78) the stage's data-parallel group may run ZeRO-2 / ZeRO-3:
   every micro-batch backward is one bracketed ``_pre_backward`` / ``_post_backward`` of the sharded optimizer, gradient
-  shards accumulate across micro-batches and the step is taken at the batch boundary (SURVEY §7.2 step 13: parameters are
+  shards accumulate across micro-batches and the step is taken at the batch boundary (parameters are
   gathered per micro-batch pass inside the stage's data-parallel group).
 """
 from __future__ import annotations

@@ -1,6 +1,6 @@
 """``zero_optimization`` config block.
 
-Keys and defaults follow the reference (deepspeed/runtime/zero/config.py; listed in SURVEY.md §5.6)
+Keys and defaults follow the reference (deepspeed/runtime/zero/config.py)
 plus one addition: ``replica_averaging`` carries the fork's four knobs (``method``, ``rings``,
 ``shuffle_step``, ``slice_count``) and an explicit ``seed`` so the shuffle schedule is reproducible;
 the same values are still accepted as ``initialize()`` kwargs for drop-in compatibility.

@@ -12,7 +12,7 @@ notion of **unit**:
   groups), release = dropping the gathered buffer; gradient reduction = ONE reduce-scatter per
   unit launched when the unit's last gradient lands, followed — when no global clipping / overflow
   check forces a deferred step — by the fused Adam update of that unit's shard *inside backward*
-  (kernel K1 of SURVEY.md §8: reduce-scatter ⊕ scale ⊕ Adam ⊕ bf16 write-back, overlapped with the
+  (one kernel: reduce-scatter ⊕ scale ⊕ Adam ⊕ bf16 write-back, overlapped with the
   rest of backward);
 * the fetch order is recorded on the first iteration and replayed as a prefetch schedule on a
   side stream (``prefetch_bucket_size`` / ``max_live_parameters`` bound the look-ahead), forward and

@@ -8,7 +8,7 @@ checkpoint state (:2472-2743), MoE param groups sharded over their expert-data-p
 shuffle_step / slice_count`` decentralised averaging with the user-called trio
 ``shuffle_exchange() / synchronization() / reset_rings()`` (:692-734, :2185-2250).
 
-Design differences (see DESIGN.md): storage is :class:`FlatGroup`; gradients are written by the
+Design differences: storage is :class:`FlatGroup`; gradients are written by the
 wgrad GEMMs directly into the flat gradient buffer ("main grad"), the reduction of a group is ONE
 reduce-scatter launched on a side stream as soon as its last gradient lands, and the update is one
 fused kernel per group that also emits the bf16 shard.  Nothing on this path names a device

@@ -52,8 +52,8 @@ def _entry(rank, world, port, fn, args, errq):
 
 
 def run_dist(fn, world=2, args=()):
-    """Run ``fn(rank, world, *args)`` in ``world`` gloo processes (the reference ships no test harness;
-    this is the CPU multi-process fixture SURVEY.md §4 asks for)."""
+    """Run ``fn(rank, world, *args)`` in ``world`` gloo processes (the reference ships no test harness
+    for several processes on the CPU)."""
     import torch.multiprocessing as mp
     ctx = mp.get_context("spawn")
     errq = ctx.SimpleQueue()

@@ -1,5 +1,5 @@
-"""The compatibility checklist of SURVEY.md §9: names a user of the reference imports or calls must exist here with the
-same spelling (signatures of the entry points are checked where the survey pins them)."""
+"""The compatibility checklist: names a user of the reference imports or calls must exist here with the
+same spelling (signatures of the entry points are checked where callers depend on them)."""
 import inspect
 
 import shuffle_exchange_b200 as sxb

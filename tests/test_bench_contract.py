@@ -1,4 +1,4 @@
-"""What the round driver relies on and can be checked without a GPU: ``bench.py``'s command line and the shape of what
+"""What callers of the benchmark rely on and can be checked without a GPU: ``bench.py``'s command line and the shape of what
 it prints, the reference arm's "unavailable" answer, the entry points of ``__graft_entry__``."""
 import importlib.util
 import json
@@ -25,7 +25,7 @@ def test_bench_flags_and_defaults(monkeypatch):
     monkeypatch.setattr(sys, "argv", ["bench.py", "--gpus", "8", "--steps", "7", "--warmup", "4", "--impl", "reference"])
     a = bench.parse()
     assert (a.gpus, a.steps, a.warmup, a.impl) == (8, 7, 4, "reference")
-    # secondary configurations named by BASELINE.json stay reachable
+    # the secondary configurations stay reachable
     monkeypatch.setattr(sys, "argv", ["bench.py", "--model", "mixtral-8x7b", "--moe-nccl", "--sp", "8", "--seq", "131072"])
     a = bench.parse()
     assert a.model == "mixtral-8x7b" and a.moe_nccl and a.sp == 8 and a.seq == 131072
@@ -34,7 +34,7 @@ def test_bench_flags_and_defaults(monkeypatch):
 def test_reference_arm_answers_unavailable_without_a_gpu():
     import torch
     if torch.cuda.is_available():
-        return                                            # on a GPU box the arm runs for real (driver-measured)
+        return                                            # with a GPU the arm runs for real
     r = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "1",
                         "--warmup", "1"], capture_output=True, text=True, cwd=ROOT, timeout=600)
     assert r.returncode == 0, r.stderr[-1500:]
@@ -55,7 +55,7 @@ def test_graft_entry_points_exist_and_reference_is_staged_by_build():
 
 def test_header_and_library_symbols_agree():
     """Every entry point the Python side registers exists in the built library (a renamed C function would otherwise
-    only fail on the GPU box)."""
+    only fail where there is a GPU)."""
     import re
     so = os.path.join(ROOT, "shuffle_exchange_b200", "native", "libsxb200.so")
     if not os.path.exists(so):

@@ -76,7 +76,7 @@ def test_checkpoint_roundtrip_gpu(tmp_path):
 @pytest.mark.parametrize("stage", [1, 2, 3])
 def test_tied_embedding_gradients_match_fp32_oracle(stage):
     """Llama with ``tie_word_embeddings``: the shared table receives one wgrad (LM head) and one scatter-add
-    (embedding) through the main-grad protocol; the reduced gradient must contain both (ADVICE r1, high)."""
+    (embedding) through the main-grad protocol; the reduced gradient must contain both."""
     import copy
     os.environ.update(MASTER_ADDR="127.0.0.1", MASTER_PORT=str(29600 + stage), RANK="0", WORLD_SIZE="1", LOCAL_RANK="0")
     import shuffle_exchange_b200 as sxb

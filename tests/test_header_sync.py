@@ -69,7 +69,7 @@ def _registered_signatures():
 
 def test_ctypes_signatures_match_the_header():
     """A C entry point that gained or lost a parameter while its ctypes signature did not would corrupt the call's
-    arguments on the GPU box only; the header (kept in step with csrc/ by tools/gen_header.py) is the referee."""
+    arguments on a machine with a GPU only; the header (kept in step with csrc/ by tools/gen_header.py) is the referee."""
     header = _header_params()
     bad = []
     for name, variants in sorted(_registered_signatures().items()):

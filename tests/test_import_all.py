@@ -1,5 +1,5 @@
 """Every module of the package imports on a machine without a GPU (dangling relative imports, missing names and
-modules that touch CUDA at import time show up here rather than on the GPU box)."""
+modules that touch CUDA at import time show up here rather than on a machine with one)."""
 import importlib
 import pkgutil
 

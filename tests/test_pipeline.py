@@ -169,7 +169,7 @@ def test_zero_sharding_inside_pipeline_stages(zero_stage):
 
 
 def test_zero3_with_host_offload_inside_pipeline_stages():
-    """BASELINE config 5 in miniature: ZeRO-3 + pipeline (PP=2) with optimizer state and parameter shards in host
+    """Llama-3 70B's setting in miniature: ZeRO-3 + pipeline (PP=2) with optimizer state and parameter shards in host
     memory, DP=2 per stage."""
     run_dist(_pipe_zero_worker, 4, (3, True))
 

@@ -1,4 +1,4 @@
-"""The fork's decentralised averaging (SURVEY.md §2.2-A): schedule determinism and method semantics."""
+"""The fork's decentralised averaging: schedule determinism and method semantics."""
 import torch
 
 from conftest import run_dist

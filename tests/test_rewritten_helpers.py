@@ -1,4 +1,4 @@
-"""Direct tests of helpers that were re-derived in round 2 and had only indirect coverage: data loader strategies and
+"""Direct tests of helpers that had only indirect coverage: data loader strategies and
 the repeating loader, the write-behind tensor swapper, the sweep job runner, state merging of the checkpoint reshaper,
 and the straight-through quantisers of the compression library."""
 import os

@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Summarise ``.ncu-rep`` files into a small JSON/markdown table (the kept artefacts live in profiles/).
+"""Summarise ``.ncu-rep`` files into a small JSON/markdown table (kept under profiles/).
 
     python tools/ncu_summary.py build/reports/prof_gemm.ncu-rep ... > profiles/ncu_summary_<tag>.md
 """
