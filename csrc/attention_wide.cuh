@@ -5,9 +5,9 @@
 // 128 wide, and an operand that stays for the whole tile is parked in tensor memory where there is room.  Tensor memory then holds
 // every accumulator once: what two buffers of 64 columns did before is done by the order of the work (see each kernel).  K / V tiles
 // shared by clusters (TMA multicast) made no difference to dQ and are not used.
-// Causal, 8192 rows x 32 heads (8 of K, V), blocks of 64 / now, us: dQ 741 / 602, dK and dV 968 / 815; 4096 rows 215 / 171 and
-// 266 / 213; 4 x 1024 rows 98 / 80 and 92 / 76; 2048 rows x 32 heads 71 / 62 and 98 / 83; 2 x 512 rows x 16 heads (4) 13.7 / 11.4 and
-// 41 / 33.
+// Causal, 8192 rows x 32 heads (8 of K, V), blocks of 64 / now, us: dQ 729 / 600, dK and dV 955 / 823; 4096 rows 208 / 170 and
+// 262 / 217; 4 x 1024 rows 91 / 78 and 88 / 76; 2048 rows 68 / 58 and 135 / 110 (begun beside dQ); 2 x 512 rows x 16 heads (4) 12.8 / 10.7
+// and 40 / 32.5.
 #pragma once
 
 namespace sxb {

@@ -15,7 +15,8 @@
 // What bounds it: the row warps (some 25 instructions per score for expf and the split: 2600 cycles a tile) and the 36 MMAs of a tile
 // beside them (2350); 3500 cycles a tile all told.  Against the same three terms on mma.sync, one warp per 16 rows, us: one prompt of 3000
 // rows, 16 heads of 128, chunks of 1024 202 -> 80 (675 with fp32 FMAs); 4096 rows, 32 heads, one chunk 1468 -> 470; four prompts
-// of 750 behind 700, window of 512 201 -> 80; one of 100 rows, 8 heads, 23 both.  K and V in rings of their own matter: 109 with one
+// of 750 behind 700, window of 512 201 -> 80; one of 100 rows, 8 heads, 23 both; 8 heads of 64, portions
+// of 17 / 64 / 128 rows behind 4000 keys 189 / 198 / 262 -> 90 / 91 / 93, heads of 128 258 / 267 / 393 -> 115 / 117 / 119.  K and V in rings of their own matter: 109 with one
 // ring for both.  The error against 64 bits is that of the 16-bit result (1.656e-3) all along.
 #pragma once
 
