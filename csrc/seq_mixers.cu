@@ -967,47 +967,56 @@ channel_decay_gates_kernel(const T* __restrict__ a_raw, long long lda, const T* 
 // State per (slot, head): dv columns of n floats, stored [dv][n].  Each output column evolves on its own:
 //   s <- a s;  u = b (v_c - [delta] s.k);  s <- s + k u;  o_c = s.q (+ D v_c)
 // A column is held by LPC = 8 lanes (the n-vector as 16-byte chunks, chunk i on lane i mod LPC), NC columns per lane,
-// 128 / LPC * NC columns per CTA; the CTA walks its sequence's rows in order, staging k and q of TB tokens at a time in shared memory.  (Spreading
-// a column over a whole warp gives a long sequence four times as many warps, but was measured slower: the work per SM
-// is the same and the longer shuffle trees add instructions.)  The products run as packed pairs (fma.f32x2).
-// What bounds it: with many sequences or heads the words of k and q read from shared memory (halved by NC = 2: 8 sequences,
-// 4096 rows, 32 heads of 128 x 128, 769 us before, 528 now), with few the latency of one token's chain (dot product, three
-// shuffles, update) in the one warp per scheduler.  Taking eight tokens per pass over the state was faster (3 sequences,
-// 2300 rows, 16 heads: 205 us against 277) and is not used: it doubles the rounding error of the read-outs.
-constexpr int kRecThreads = 128, kTB = 8;
+// 128 / LPC * NC columns per CTA; the CTA walks its sequence's rows in order over groups of eight that a warp of its own copies
+// into shared memory.  The products run as packed pairs (fma.f32x2).
+// What bounds it: with few sequences and heads the chain from token to token of the one or two warps of a scheduler, with many
+// the words of k and q that come out of shared memory (a lane reads n / 4 of them for NC columns) and the issue slots.
+// The delta rule's chain was the product S^T k with the shuffles behind it.  It is taken one token ahead, from the state
+// before the update: S_t^T k_{t+1} = a_t (S_{t-1}^T k_{t+1}) + u_t (k_t . k_{t+1}), the last factor being one number for all columns that
+// the copying warp takes; a token then waits for two multiply-adds.  The error against 64 bits is that of the direct form (2300 rows:
+// 9.90e-8 both), since the state itself is stepped as before; eight tokens per pass over the state would double it.
+// DEEP: operands are read one token before their use (keys two), for few warps per scheduler; it costs registers, so with many
+// CTAs they are read where they are used.  Every form takes the same sums in the same order.
+// us, 128 x 128 (sequences, rows in all, heads), before (no look ahead, copies by the walking warps) | now:  delta rule 3, 2300, 16
+// 257 | 205;  1, 4000, 16 816 | 505;  1, 2000, 32 443 | 329;  8, 4096, 32 483 | 482;  decay per channel 386 | 260, 1018 | 670, 637 |
+// 405, 686 | 620;  state space 254 | 149, 717 | 395, 425 | 225, 459 | 331;  64 sequences of one row, 32 heads 53 | 49, 64 | 60, 46 | 46.
+constexpr int kRecThreads = 128, kTB = 8;      // walking threads (one more warp copies), tokens a group
 
-template <int R, bool DELTA, int LPC, bool CHAN, int NC>
-__global__ void __launch_bounds__(kRecThreads)
+// Floats of one group: k [TB][NP] | q [TB][NP] | v [TB][COLS] | (decay, write strength) [TB] | k . previous k [TB] | CHAN: decay [TB][NP].
+template <int R, int LPC, bool CHAN, int NC>
+struct RecStage {
+  static constexpr int NP = R * LPC, COLS = kRecThreads / LPC * NC;
+  static constexpr int kQ = kTB * NP, kV = 2 * kTB * NP, kAB = kV + kTB * COLS, kKK = kAB + 2 * kTB, kG = kKK + kTB;
+  static constexpr int kTotal = kG + (CHAN ? kTB * NP : 0);
+  static constexpr int kBufs = NP > 128 ? 3 : 4;          // groups in shared memory (long rows take long to walk)
+};
+
+template <int R, bool DELTA, int LPC, bool CHAN, int NC, bool DEEP, int MB>
+__global__ void __launch_bounds__(kRecThreads + 32, MB)
 linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict__ qvec, long long ldkq,
                          const float* __restrict__ val, long long ldv, const float* __restrict__ decay,
                          const float* __restrict__ beta, const float* __restrict__ skip, float* __restrict__ state,
                          float* __restrict__ out, const int* __restrict__ seq_info, int H, int G, int n, int dv,
-                         int decay_ld, bool longest_first) {
+                         int decay_ld) {
   // Lane l of a column holds the float4 chunks l, l + LPC, l + 2 LPC, ... of the column's n-vector (padded with zeros
-  // to NP = LPC R), so k, q and the state move as 16-byte words without bank conflicts.  Two staging buffers, each
-  // k [TB][NP] | q [TB][NP] | v [TB][COLS] | decay [TB] | beta [TB]: the next TB tokens are copied in (cp.async) while
-  // the current ones are walked.  CHAN: the decay is a vector over the key channels (decay [rows, H n]) and follows the
-  // scalars as one more [TB][NP] block; the state is multiplied by it chunk by chunk before the delta rule's product.
+  // to NP = LPC R), so k, q and the state move as 16-byte words without bank conflicts.  The last warp copies: behind the
+  // barrier that starts group g it asks for group g + kBufs - 1 (cp.async), then waits for g + 2 and, for the delta rule, takes
+  // the products of neighbouring keys in it.  CHAN: the decay is a vector over the key channels (decay [rows, H n]); the state is
+  // multiplied by it chunk by chunk before the delta rule's product.
   // decay_ld 0: the H decays are the same for every row.  beta null: every write strength is one.
-  constexpr int NP = R * LPC, R4 = R / 4, COLS = kRecThreads / LPC * NC;
+  using Stage = RecStage<R, LPC, CHAN, NC>;
+  constexpr int NP = Stage::NP, kBufs = Stage::kBufs, R4 = R / 4, COLS = Stage::COLS, RP = R / 2;
   extern __shared__ __align__(16) float sm[];
-  constexpr int stage = (CHAN ? 3 : 2) * kTB * NP + kTB * COLS + 2 * kTB;
-  // The plain delta rule at two columns per lane takes up to 32 sequences longest first, whatever their order: a CTA walks its
-  // sequence alone and there are only a few per SM, so a long one that starts late ends late (us as they come | longest
-  // first: 3 sequences, 2300 rows, 16 heads 277 | 254; 4, 1500, 32: 254 | 222; 6, 3000, 32: 449 | 381; 8, 1500, 16: 130 | 111;
-  // 7, 1500, 16: 126 | 126; shortest first 313 for the first).  Not where little more than one CTA per SM is launched, since then
-  // the longest would be the ones that share (5, 1500, 8, 160 CTAs: 101 | 109).  The other forms keep the order of the batch:
-  // they gain as much with 3, 4 and 6 sequences and lose with 5 and 7 (one column, 5 of 8 heads 124 | 135; two, 7 of 16 heads:
-  // state space 103 | 106, channel decay 164 | 166).  Running every second round of CTAs backwards, to pair long with short, was
-  // worse (3 sequences, 32 heads: no gain; 5, 16: none).
-  // A lane holds the four numbers of one sequence.
-  constexpr bool kSorted = DELTA && !CHAN && NC == 2;
+  // Up to 32 sequences are taken longest first, whatever their order: a CTA walks its sequence alone and there are only a few
+  // per SM, so a long one that starts late ends late (us as they come | longest first: delta rule, 3 sequences, 2300 rows, 16 heads 261 | 205; 6,
+  // 3000, 32 440 | 381; 7, 1500, 16 126 | 114; 5, 1500, 8 90 | 91; state space, 3, 2300, 16 177 | 150; decay per channel 306 | 260).  A lane holds the four
+  // numbers of one sequence.
   auto info = [&](int i) {                 // (four words: the table need not start on 16 bytes)
     const int* p = seq_info + 4 * i;
     return make_int4(p[0], p[1], p[2], p[3]);
   };
   int4 si;
-  if (kSorted && longest_first) {         // at most 32 sequences
+  if (gridDim.z > 1 && gridDim.z <= 32) {
     const int i = threadIdx.x % 32, count = gridDim.z;
     si = i < count ? info(i) : make_int4(0, -1, 0, 0);
     int rank = 0;
@@ -1023,18 +1032,127 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
   }
   const int first = si.x, rows = si.y, seen = si.z, slot = si.w;
   const int h = blockIdx.y, g = h / (H / G);
-  const int lc = threadIdx.x / LPC, l = threadIdx.x % LPC;
-  const int col = blockIdx.x * COLS + lc * NC;      // the lane's columns: col .. col + NC - 1
-  constexpr int beta0 = 2 * kTB * NP + kTB * COLS + kTB;
-  for (int i = threadIdx.x; i < 2 * stage; i += blockDim.x) {                 // the padding stays zero
-    const int j = i % stage - beta0;
-    sm[i] = (beta == nullptr && j >= 0 && j < kTB) ? 1.f : 0.f;
-  }
-  float* sp = state + (((long long)slot * H + h) * dv + col) * n;
+  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+  const int groups = (rows + kTB - 1) / kTB;
+  const int col0 = blockIdx.x * COLS;
   const bool n4 = (n & 3) == 0;
-  const bool wide_copy = n4 && (ldkq & 3) == 0 && ((reinterpret_cast<uintptr_t>(kvec) & 15) == 0) &&
-                         ((reinterpret_cast<uintptr_t>(qvec) & 15) == 0);
-  float2 S[NC][R / 2];
+  if (warp == kRecThreads / 32) {
+    // ------------------------------------------------------------------------------------------ copies
+    const bool wide = n4 && (ldkq & 3) == 0 && ((reinterpret_cast<uintptr_t>(kvec) | reinterpret_cast<uintptr_t>(qvec)) & 15) == 0;
+    const bool wide_v = (ldv & 3) == 0 && (dv & 3) == 0 && (reinterpret_cast<uintptr_t>(val) & 15) == 0 && col0 + COLS <= dv;
+    const bool wide_g = n4 && (reinterpret_cast<uintptr_t>(decay) & 15) == 0;
+    auto rows_in = [&](float* to, const float* from, long long ld, int nt, bool by16) {     // [nt][n] -> [nt][NP]
+      if (by16 && n == NP) {
+        constexpr int kLanes = NP < 128 ? NP / 4 : 32, kPass = 32 / kLanes;      // lanes a row, rows at once
+        const float* f = from + lane / kLanes * ld + lane % kLanes * 4;
+        to += lane / kLanes * NP + lane % kLanes * 4;
+        const int left = nt - lane / kLanes;
+#pragma unroll
+        for (int t = 0; t < kTB; t += kPass)
+          if (t < left)
+#pragma unroll
+            for (int c = 0; c < NP; c += 128) __pipeline_memcpy_async(to + t * NP + c, f + t * ld + c, 16);
+      } else if (by16) {
+        const int n16 = n >> 2;
+        for (int i = lane; i < nt * n16; i += 32) {
+          const int t = i / n16, c = (i % n16) * 4;
+          __pipeline_memcpy_async(to + t * NP + c, from + t * ld + c, 16);
+        }
+      } else {
+        for (int i = lane; i < nt * n; i += 32) {
+          const int t = i / n, c = i % n;
+          __pipeline_memcpy_async(to + t * NP + c, from + t * ld + c, 4);
+        }
+      }
+    };
+    auto group_in = [&](int grp) {
+      const int t0 = grp * kTB, nt = min(kTB, rows - t0);
+      if (nt > 0) {
+        float* to = sm + grp % kBufs * Stage::kTotal;
+        const long long row = first + t0;
+        rows_in(to, kvec + row * ldkq + (long long)g * n, ldkq, nt, wide);
+        rows_in(to + Stage::kQ, qvec + row * ldkq + (long long)g * n, ldkq, nt, wide);
+        if (CHAN) rows_in(to + Stage::kG, decay + (row * H + h) * n, (long long)H * n, nt, wide_g);
+        const float* v = val + row * ldv + (long long)h * dv;
+        if (wide_v) {
+          constexpr int kLanes = COLS / 4, kPass = 32 / kLanes;
+          const float* f = v + lane / kLanes * ldv + col0 + lane % kLanes * 4;
+#pragma unroll
+          for (int t = 0; t < kTB; t += kPass)
+            if (t + lane / kLanes < nt) __pipeline_memcpy_async(to + Stage::kV + t * COLS + lane * 4, f + t * ldv, 16);
+        } else {
+          for (int i = lane; i < nt * COLS; i += 32)
+            __pipeline_memcpy_async(to + Stage::kV + i, v + (i / COLS) * ldv + min(col0 + i % COLS, dv - 1), 4);
+        }
+        if (lane < nt) {
+          if (!CHAN) __pipeline_memcpy_async(to + Stage::kAB + 2 * lane, decay + (row + lane) * decay_ld + h, 4);
+          if (beta != nullptr) __pipeline_memcpy_async(to + Stage::kAB + 2 * lane + 1, beta + (row + lane) * H + h, 4);
+        }
+      }
+      __pipeline_commit();
+    };
+    // DELTA: products of every key of a group with the one before it (CHAN: times its own decay), eight lanes a product.
+    auto neighbours = [&](int grp) {
+      const int l8 = lane % 8;
+      float* b = sm + grp % kBufs * Stage::kTotal;
+      const float* before = sm + (grp + kBufs - 1) % kBufs * Stage::kTotal + (kTB - 1) * NP;
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int t = lane / 8 + 4 * r;
+        const float4* x = reinterpret_cast<const float4*>(t == 0 ? before : b + (t - 1) * NP) + l8;
+        const float4* y = reinterpret_cast<const float4*>(b + t * NP) + l8;
+        const float4* d = reinterpret_cast<const float4*>(b + Stage::kG + t * NP) + l8;
+        float2 s01 = make_float2(0.f, 0.f), s23 = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < NP / 32; ++i) {
+          const float4 p = x[8 * i];
+          float4 q = y[8 * i];
+          if (CHAN) {
+            const float4 e = d[8 * i];
+            q = make_float4(q.x * e.x, q.y * e.y, q.z * e.z, q.w * e.w);
+          }
+          s01 = __ffma2_rn(make_float2(p.x, p.y), make_float2(q.x, q.y), s01);
+          s23 = __ffma2_rn(make_float2(p.z, p.w), make_float2(q.z, q.w), s23);
+        }
+        float s = (s01.x + s01.y) + (s23.x + s23.y);
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (l8 == 0) b[Stage::kKK + t] = s;
+      }
+    };
+    for (int i = 0; i < kBufs - 1; ++i) group_in(i);
+    for (int grp = 0; grp < groups; ++grp) {
+      __pipeline_wait_prior(kBufs - 3);   // the group that starts here and the one behind it have landed
+      if (DELTA) {
+        __syncwarp();
+        if (grp == 0 && rows >= kTB) neighbours(0);
+        if (grp + 1 < groups) neighbours(grp + 1);
+      }
+      __syncthreads();                    // the walk of group grp - 1 is over: its buffer is the next one to fill
+      group_in(grp + kBufs - 1);
+    }
+    return;
+  }
+
+  // -------------------------------------------------------------------------------------------- the walk
+  if (n != NP || beta == nullptr) {       // zeros in the padding and ones for absent write strengths, where nothing is copied to
+    const int pad = NP - n, filled = min(rows, kBufs * kTB);
+    for (int i = threadIdx.x; i < filled * (pad + 1); i += kRecThreads) {
+      const int t = i / (pad + 1), c = i % (pad + 1);
+      float* b = sm + t / kTB * Stage::kTotal;
+      if (c == pad) {
+        if (beta == nullptr) b[Stage::kAB + 2 * (t % kTB) + 1] = 1.f;
+      } else {
+        float* x = b + t % kTB * NP + n + c;
+        x[0] = x[Stage::kQ] = 0.f;
+        if (CHAN) x[Stage::kG] = 0.f;
+      }
+    }
+  }
+  const int lc = threadIdx.x / LPC, l = threadIdx.x % LPC;
+  const int col = col0 + lc * NC;          // the lane's columns: col .. col + NC - 1
+  float* sp = state + (((long long)slot * H + h) * dv + col) * n;
+  float2 S[NC][RP];
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
     const float* sc = sp + (long long)c * n;
@@ -1056,200 +1174,192 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
     }
   }
   const float D = skip ? skip[h] : 0.f;
-  __syncthreads();
 
-  auto stage_in = [&](int buf, int t0) {
-    float* sk = sm + buf * stage;
-    float* sq = sk + kTB * NP;
-    float* sv = sq + kTB * NP;
-    float* sa = sv + kTB * COLS;
-    float* sb = sa + kTB;
-    float* sg = sb + kTB;
-    const int nt = min(kTB, rows - t0);
-    if (CHAN) {
-      const long long Hn = (long long)H * n;
-      if (n4) {
-        const int nq4 = n >> 2;
-        for (int i = threadIdx.x; i < nt * nq4; i += blockDim.x) {
-          const int tt = i / nq4, c = (i % nq4) * 4;
-          __pipeline_memcpy_async(sg + tt * NP + c, decay + (long long)(first + t0 + tt) * Hn + (long long)h * n + c, 16);
-        }
-      } else {
-        for (int i = threadIdx.x; i < nt * n; i += blockDim.x) {
-          const int tt = i / n, c = i % n;
-          __pipeline_memcpy_async(sg + tt * NP + c, decay + (long long)(first + t0 + tt) * Hn + (long long)h * n + c, 4);
-        }
-      }
-    }
-    if (wide_copy && n == NP && kRecThreads % (NP / 4) == 0) {     // a thread copies one chunk of every few rows
-      constexpr int kRows = kRecThreads / (NP / 4) > 0 ? kRecThreads / (NP / 4) : 1;
-      const int c = (threadIdx.x % (NP / 4)) * 4;
+  auto words = [&](const float* row, float2 (&w)[RP]) {        // a staged vector's words of this lane
+    const float4* p = reinterpret_cast<const float4*>(row) + l;
 #pragma unroll
-      for (int tt = threadIdx.x / (NP / 4); tt < kTB; tt += kRows) {
-        if (tt < nt) {
-          const long long at = (long long)(first + t0 + tt) * ldkq + g * NP + c;
-          __pipeline_memcpy_async(sk + tt * NP + c, kvec + at, 16);
-          __pipeline_memcpy_async(sq + tt * NP + c, qvec + at, 16);
-        }
-      }
-    } else if (wide_copy) {
-      const int nq4 = n >> 2;
-      for (int i = threadIdx.x; i < nt * nq4; i += blockDim.x) {
-        const int tt = i / nq4, c = (i % nq4) * 4;
-        const long long row = first + t0 + tt;
-        __pipeline_memcpy_async(sk + tt * NP + c, kvec + row * ldkq + g * n + c, 16);
-        __pipeline_memcpy_async(sq + tt * NP + c, qvec + row * ldkq + g * n + c, 16);
-      }
+    for (int r4 = 0; r4 < R4; ++r4) {
+      const float4 x = p[r4 * LPC];
+      w[2 * r4] = make_float2(x.x, x.y), w[2 * r4 + 1] = make_float2(x.z, x.w);
+    }
+  };
+  auto values = [&](const float* row, float (&v)[NC]) {
+#pragma unroll
+    for (int c = 0; c < NC; ++c) v[c] = row[lc * NC + c];
+  };
+  auto lane_dot = [&](const float2 (&x)[RP], const float2 (&w)[RP]) {
+    float2 d01 = make_float2(0.f, 0.f), d23 = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int r4 = 0; r4 < R4; ++r4) {
+      d01 = __ffma2_rn(x[2 * r4], w[2 * r4], d01);
+      d23 = __ffma2_rn(x[2 * r4 + 1], w[2 * r4 + 1], d23);
+    }
+    return (d01.x + d01.y) + (d23.x + d23.y);
+  };
+  // One round of a sum over lanes that differ in bit x: of two numbers, the one that this lane goes on with.
+  auto halve = [&](float lo, float hi, int x) {
+    const bool up = l & x;
+    return (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, x);
+  };
+  // Sums over the columns' lanes, all of them on every lane: first every round halves the numbers a lane carries.
+  auto column_sums = [&](float (&p)[NC]) {
+    float x[NC];
+#pragma unroll
+    for (int c = 0; c < NC; ++c) x[c] = p[c];
+    int w = 1;
+#pragma unroll
+    for (int m = NC / 2; m > 0; m >>= 1, w <<= 1)
+#pragma unroll
+      for (int c = 0; c < m; ++c) x[c] = halve(x[2 * c], x[2 * c + 1], w);
+#pragma unroll
+    for (int o = NC; o < LPC; o <<= 1) x[0] += __shfl_xor_sync(0xffffffffu, x[0], o);
+    if (NC == 1) {
+      p[0] = x[0];
+    } else if (NC == 2) {
+      const float y = __shfl_xor_sync(0xffffffffu, x[0], 1);
+      p[0] = l & 1 ? y : x[0], p[NC - 1] = l & 1 ? x[0] : y;
     } else {
-      for (int i = threadIdx.x; i < nt * n; i += blockDim.x) {
-        const int tt = i / n, c = i % n;
-        const long long row = first + t0 + tt;
-        __pipeline_memcpy_async(sk + tt * NP + c, kvec + row * ldkq + g * n + c, 4);
-        __pipeline_memcpy_async(sq + tt * NP + c, qvec + row * ldkq + g * n + c, 4);
-      }
+#pragma unroll
+      for (int c = 0; c < NC; ++c) p[c] = __shfl_sync(0xffffffffu, x[0], (lane & ~(NC - 1)) | c);
     }
-    for (int i = threadIdx.x; i < nt * COLS; i += blockDim.x) {
-      const int c = min((int)blockIdx.x * COLS + i % COLS, dv - 1);
-      __pipeline_memcpy_async(sv + i, val + (long long)(first + t0 + i / COLS) * ldv + h * dv + c, 4);
+  };
+  auto scaled = [&](const float2 (&x)[RP], const float2 (&d)[RP], float2 (&w)[RP]) {
+#pragma unroll
+    for (int r = 0; r < RP; ++r) w[r] = __fmul2_rn(x[r], d[r]);
+  };
+  // S <- (a) S + u k
+  auto update = [&](const float2 (&k)[RP], float a, const float (&u)[NC]) {
+    const float2 a2 = make_float2(a, a);
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const float2 u2 = make_float2(u[c], u[c]);
+#pragma unroll
+      for (int r = 0; r < RP; ++r) S[c][r] = __ffma2_rn(k[r], u2, CHAN ? S[c][r] : __fmul2_rn(S[c][r], a2));
     }
-    for (int i = threadIdx.x; i < nt; i += blockDim.x) {
-      if (!CHAN) __pipeline_memcpy_async(sa + i, decay + (long long)(first + t0 + i) * decay_ld + h, 4);
-      if (beta != nullptr) __pipeline_memcpy_async(sb + i, beta + (long long)(first + t0 + i) * H + h, 4);
-    }
-    __pipeline_commit();
   };
 
-  stage_in(0, 0);
-  int buf = 0;
-  for (int t0 = 0; t0 < rows; t0 += kTB, buf ^= 1) {
-    const int nt = min(kTB, rows - t0);
-    const bool more = t0 + kTB < rows;
-    if (more) stage_in(buf ^ 1, t0 + kTB);
-    if (more) __pipeline_wait_prior(1);
-    else __pipeline_wait_prior(0);
+  float ahead[NC];                         // DELTA: S^T k of the token to come, before its decay (CHAN: behind it)
+  for (int grp = 0; grp < groups; ++grp) {
+    const int t0 = grp * kTB, nt = min(kTB, rows - t0);
     __syncthreads();
-    const float* sk = sm + buf * stage;
-    const float* sq = sk + kTB * NP;
-    const float* sv = sq + kTB * NP;
-    const float* sa = sv + kTB * COLS;
-    const float* sb = sa + kTB;
-    const float* sg = sb + kTB;
-    // One token.  A full group of TB tokens is walked by straight-line code, so the loads of k and q and the read-out
-    // reductions of neighbouring tokens overlap the serial part (the state update, and the dot product before it for
-    // the delta rule).
-    struct Tok {                      // one token's operands, loaded one token ahead of their use
-      float a, b, v[NC];
-      float4 k[R4], q[R4], g[CHAN ? R4 : 1];
-    };
-    auto fetch = [&](int tt) {
-      Tok t;
-      t.a = CHAN ? 1.f : sa[tt], t.b = sb[tt];
+    const float* b0 = sm + grp % kBufs * Stage::kTotal;
+    const float* b1 = sm + (grp + 1) % kBufs * Stage::kTotal;
+    // (behind the last group the look ahead reads whatever is there; nothing uses it)
+    auto at = [&](int t, int off, int pitch) { return t < kTB ? b0 + off + t * pitch : b1 + off + (t - kTB) * pitch; };
+    if (nt == kTB) {
+      // A full group is walked by straight-line code, a software pipeline: keys are read two tokens ahead of their update, queries,
+      // values and decays one.
+      float2 k[3][RP], q[2][RP], d[2][CHAN ? RP : 1];
+      float v[2][NC];
+      words(at(0, 0, NP), k[0]);
+      if constexpr (DEEP && DELTA) words(at(1, 0, NP), k[1]);
+      if constexpr (DEEP) words(at(0, Stage::kQ, NP), q[0]), values(at(0, Stage::kV, COLS), v[0]);
+      if constexpr (CHAN && (DEEP || DELTA)) words(at(0, Stage::kG, NP), d[0]);
+      if (DELTA && grp == 0) {
+        if constexpr (CHAN) {
+          float2 w[RP];
+          scaled(k[0], d[0], w);
 #pragma unroll
-      for (int c = 0; c < NC; ++c) t.v[c] = sv[tt * COLS + lc * NC + c];
-      const float4* kk = reinterpret_cast<const float4*>(sk + tt * NP) + l;
-      const float4* qq = reinterpret_cast<const float4*>(sq + tt * NP) + l;
+          for (int c = 0; c < NC; ++c) ahead[c] = lane_dot(S[c], w);
+        } else {
 #pragma unroll
-      for (int r4 = 0; r4 < R4; ++r4) t.k[r4] = kk[r4 * LPC], t.q[r4] = qq[r4 * LPC];
-      if (CHAN) {
-        const float4* gg = reinterpret_cast<const float4*>(sg + tt * NP) + l;
-#pragma unroll
-        for (int r4 = 0; r4 < R4; ++r4) t.g[r4] = gg[r4 * LPC];
+          for (int c = 0; c < NC; ++c) ahead[c] = lane_dot(S[c], k[0]);
+        }
+        column_sums(ahead);
       }
-      return t;
-    };
-    auto step = [&](const Tok& t, float (&o_lane)[NC]) {
-      const float a = t.a, b = t.b;
-      const float4* k4 = t.k;
-      float u[NC];
-      if (CHAN) {                      // the decayed state enters the product below: decay first, a stays 1
+      float o1[NC], o2[NC], o4[NC], o[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c)
+      for (int t = 0; t < kTB; ++t) {
+        const float a = CHAN ? 1.f : at(t, Stage::kAB, 2)[0], b = at(t, Stage::kAB, 2)[1];
+        float2 (&kc)[RP] = k[t % 3], (&kn)[RP] = k[(t + 1) % 3];
+        if constexpr (DEEP) {
+          if (DELTA) words(at(t + 2, 0, NP), k[(t + 2) % 3]);
+          else if (t + 1 < kTB) words(at(t + 1, 0, NP), kn);
+          if (t + 1 < kTB) words(at(t + 1, Stage::kQ, NP), q[(t + 1) % 2]), values(at(t + 1, Stage::kV, COLS), v[(t + 1) % 2]);
+        } else {
+          if (DELTA) words(at(t + 1, 0, NP), kn);
+          else if (t > 0) words(at(t, 0, NP), kc);
+          words(at(t, Stage::kQ, NP), q[t % 2]), values(at(t, Stage::kV, COLS), v[t % 2]);
+        }
+        if constexpr (CHAN) {
+          if (DELTA || (DEEP && t + 1 < kTB)) words(at(t + 1, Stage::kG, NP), d[(t + 1) % 2]);
+          if (!DELTA && !DEEP) words(at(t, Stage::kG, NP), d[t % 2]);
 #pragma unroll
-          for (int r4 = 0; r4 < R4; ++r4) {
-            S[c][2 * r4] = __fmul2_rn(S[c][2 * r4], make_float2(t.g[r4].x, t.g[r4].y));
-            S[c][2 * r4 + 1] = __fmul2_rn(S[c][2 * r4 + 1], make_float2(t.g[r4].z, t.g[r4].w));
+          for (int c = 0; c < NC; ++c) scaled(S[c], d[t % 2], S[c]);
+        }
+        float u[NC], p[NC];
+        if (DELTA) {
+          const float kk = at(t + 1, Stage::kKK, 1)[0];
+          if constexpr (CHAN) {
+            float2 w[RP];
+            scaled(kn, d[(t + 1) % 2], w);
+#pragma unroll
+            for (int c = 0; c < NC; ++c) p[c] = lane_dot(S[c], w);
+          } else {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) p[c] = lane_dot(S[c], kn);
           }
-      }
-      if (DELTA) {                     // (a S)^T k = a (S^T k): the decay is folded into the update below
-        float dot[NC];
+#pragma unroll
+          for (int c = 0; c < NC; ++c) u[c] = b * (v[t % 2][c] - (CHAN ? ahead[c] : a * ahead[c]));
+          column_sums(p);
+#pragma unroll
+          for (int c = 0; c < NC; ++c) ahead[c] = fmaf(u[c], kk, CHAN ? p[c] : a * p[c]);
+        } else {
+#pragma unroll
+          for (int c = 0; c < NC; ++c) u[c] = b * v[t % 2][c];
+        }
+        update(kc, a, u);
+        // The read-outs are summed over the lanes as they come, each round halving the tokens that a lane carries.
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-          float2 d01 = make_float2(0.f, 0.f), d23 = make_float2(0.f, 0.f);
-#pragma unroll
-          for (int r4 = 0; r4 < R4; ++r4) {
-            d01 = __ffma2_rn(S[c][2 * r4], make_float2(k4[r4].x, k4[r4].y), d01);
-            d23 = __ffma2_rn(S[c][2 * r4 + 1], make_float2(k4[r4].z, k4[r4].w), d23);
-          }
-          dot[c] = (d01.x + d01.y) + (d23.x + d23.y);
+          o[c] = lane_dot(S[c], q[t % 2]);
+          if (t % 2 == 0) { o1[c] = o[c]; continue; }
+          o[c] = halve(o1[c], o[c], 1);
+          if (t % 4 == 1) { o2[c] = o[c]; continue; }
+          o[c] = halve(o2[c], o[c], 2);
+          if (t % 8 == 3) { o4[c] = o[c]; continue; }
+          o[c] = halve(o4[c], o[c], 4);
         }
-#pragma unroll
-        for (int o = 1; o < LPC; o <<= 1)
-#pragma unroll
-          for (int c = 0; c < NC; ++c) dot[c] += __shfl_xor_sync(0xffffffffu, dot[c], o);
-#pragma unroll
-        for (int c = 0; c < NC; ++c) u[c] = b * (t.v[c] - a * dot[c]);
-      } else {
-#pragma unroll
-        for (int c = 0; c < NC; ++c) u[c] = b * t.v[c];
       }
-      const float2 a2 = make_float2(a, a);
+      // lane l now has token l of every column
+      static_assert(kTB == LPC, "a lane per token");
+      float* to = out + (long long)(first + t0 + l) * H * dv + (long long)h * dv;
+      const float* vt = at(l, Stage::kV, COLS) + lc * NC;
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const float2 u2 = make_float2(u[c], u[c]);
-        float2 o01 = make_float2(0.f, 0.f), o23 = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int r4 = 0; r4 < R4; ++r4) {
-          const float4 q4 = t.q[r4];
-          S[c][2 * r4] = __ffma2_rn(make_float2(k4[r4].x, k4[r4].y), u2, CHAN ? S[c][2 * r4] : __fmul2_rn(S[c][2 * r4], a2));
-          S[c][2 * r4 + 1] = __ffma2_rn(make_float2(k4[r4].z, k4[r4].w), u2,
-                                        CHAN ? S[c][2 * r4 + 1] : __fmul2_rn(S[c][2 * r4 + 1], a2));
-          o01 = __ffma2_rn(S[c][2 * r4], make_float2(q4.x, q4.y), o01);
-          o23 = __ffma2_rn(S[c][2 * r4 + 1], make_float2(q4.z, q4.w), o23);
-        }
-        o_lane[c] = (o01.x + o01.y) + (o23.x + o23.y);       // this lane's part of the read-out
-      }
-    };
-    if (nt == kTB) {
-      // the read-outs of the group are summed over the column's lanes together, off the serial path: TB independent
-      // shuffle trees, then lane t of the column writes token t
-      static_assert(LPC == kTB, "lane t of a column writes token t of the group");
-      float op[kTB][NC];
-      Tok cur = fetch(0);
-#pragma unroll
-      for (int tt = 0; tt < kTB; ++tt) {
-        const Tok nxt = fetch(tt + 1 < kTB ? tt + 1 : tt);
-        step(cur, op[tt]);
-        cur = nxt;
-      }
-#pragma unroll
-      for (int x = 1; x < LPC; x <<= 1)
-#pragma unroll
-        for (int tt = 0; tt < kTB; ++tt)
-#pragma unroll
-          for (int c = 0; c < NC; ++c) op[tt][c] += __shfl_xor_sync(0xffffffffu, op[tt][c], x);
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        float mine = op[0][c];
-#pragma unroll
-        for (int tt = 1; tt < kTB; ++tt) mine = (l == tt) ? op[tt][c] : mine;
-        if (col + c < dv)
-          out[(long long)(first + t0 + l) * H * dv + h * dv + col + c] = mine + D * sv[l * COLS + lc * NC + c];
-      }
+      for (int c = 0; c < NC; ++c)
+        if (col + c < dv) to[col + c] = o[c] + D * vt[c];
     } else {
-      for (int tt = 0; tt < nt; ++tt) {
-        float o[NC];
-        step(fetch(tt), o);
+      for (int t = 0; t < nt; ++t) {
+        const float a = CHAN ? 1.f : at(t, Stage::kAB, 2)[0], b = at(t, Stage::kAB, 2)[1];
+        float2 k[RP], q[RP];
+        float u[NC], o[NC];
+        words(at(t, 0, NP), k), words(at(t, Stage::kQ, NP), q);
+        if (CHAN) {
+          float2 d[RP];
+          words(at(t, Stage::kG, NP), d);
 #pragma unroll
-        for (int x = 1; x < LPC; x <<= 1)
+          for (int c = 0; c < NC; ++c) scaled(S[c], d, S[c]);
+        }
+        if (DELTA) {                       // (a S)^T k = a (S^T k)
 #pragma unroll
-          for (int c = 0; c < NC; ++c) o[c] += __shfl_xor_sync(0xffffffffu, o[c], x);
+          for (int c = 0; c < NC; ++c) u[c] = lane_dot(S[c], k);
+          column_sums(u);
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          const float v = at(t, Stage::kV, COLS)[lc * NC + c];
+          u[c] = b * (DELTA ? v - a * u[c] : v);
+        }
+        update(k, a, u);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) o[c] = lane_dot(S[c], q);
+        column_sums(o);
 #pragma unroll
         for (int c = 0; c < NC; ++c)
           if (col + c < dv && l == 0)
-            out[(long long)(first + t0 + tt) * H * dv + h * dv + col + c] = o[c] + D * sv[tt * COLS + lc * NC + c];
+            out[(long long)(first + t0 + t) * H * dv + (long long)h * dv + col + c] = o[c] + D * at(t, Stage::kV, COLS)[lc * NC + c];
       }
     }
-    __syncthreads();          // the buffer just walked is the target of the next iteration's copies
   }
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
@@ -2133,37 +2243,54 @@ SXB_API int sxb_linear_recurrence(const void* kvec, const void* qvec, long long 
   if (n > 256 || H % G) return SXB_ERR_UNSUPPORTED;
   if (decay_channels && fixed_decay) return SXB_ERR_BAD_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-#define LAUNCH_REC(R, D, LPC, CH, NC)                                                                               \
-  do {                                                                                                              \
-    constexpr int cols = kRecThreads / LPC * NC;                                                                    \
-    const size_t smem = (size_t)2 * ((CH ? 3 : 2) * kTB * (R * LPC) + kTB * cols + 2 * kTB) * sizeof(float);        \
-    if (smem > 48 * 1024)                                                                                           \
-      cudaFuncSetAttribute(linear_recurrence_kernel<R, D, LPC, CH, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize,    \
-                           (int)smem);                                                                              \
-    linear_recurrence_kernel<R, D, LPC, CH, NC><<<dim3((dv + cols - 1) / cols, H, n_seqs), kRecThreads, smem, s>>>(     \
-        (const float*)kvec, (const float*)qvec, ldkq, (const float*)val, ldv, (const float*)decay,                  \
-        (const float*)beta, (const float*)skip, (float*)state, (float*)out, (const int*)seq_info, H, G, n, dv,      \
-        fixed_decay ? 0 : H, n_seqs <= 32 && 4LL * ((dv + cols - 1) / cols) * H * n_seqs >= 5LL * num_sms());       \
+#define LAUNCH_REC(R, D, CH, NC, DEEP, MB)                                                                               \
+  do {                                                                                                                   \
+    constexpr int cols = kRecThreads / 8 * NC;                                                                           \
+    constexpr size_t smem = RecStage<R, 8, CH, NC>::kBufs * RecStage<R, 8, CH, NC>::kTotal * sizeof(float);                                   \
+    if (smem > 48 * 1024)                                                                                                \
+      cudaFuncSetAttribute(linear_recurrence_kernel<R, D, 8, CH, NC, DEEP, MB>,                                          \
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                                      \
+    linear_recurrence_kernel<R, D, 8, CH, NC, DEEP, MB>                                                                  \
+        <<<dim3((dv + cols - 1) / cols, H, n_seqs), kRecThreads + 32, smem, s>>>(                                        \
+            (const float*)kvec, (const float*)qvec, ldkq, (const float*)val, ldv, (const float*)decay,                   \
+            (const float*)beta, (const float*)skip, (float*)state, (float*)out, (const int*)seq_info, H, G, n, dv,       \
+            fixed_decay ? 0 : H);                                                                                        \
   } while (0)
-#define LAUNCH_REC_N(D, CH)                                  \
-  if (n <= 32) LAUNCH_REC(4, D, 8, CH, 1);                   \
-  else if (n <= 64) { if (two) LAUNCH_REC(8, D, 8, CH, 2); else LAUNCH_REC(8, D, 8, CH, 1); }    \
-  else if (n <= 128) { if (two) LAUNCH_REC(16, D, 8, CH, 2); else LAUNCH_REC(16, D, 8, CH, 1); } \
-  else LAUNCH_REC(32, D, 8, CH, 1)
-  // Two columns per lane share every k and q word that is read from shared memory (and every copy into it); with one column
-  // the chip has twice the warps.  Two win once one column would fill the chip one and a half times (us, one | two columns:
-  // delta rule, 8 sequences, 4096 rows, 32 heads 746 | 528; 3, 2300, 16: 303 | 277; 1, 2000, 32: 512 | 440), below that one
-  // does (1, 4096, 16: 833 | 892), and where the columns fill blocks of 32: lanes without a column walk along (16 sequences
-  // of 256 rows, 16 heads, keys of 64: dv = 16 58 | 79, 32 79 | 77, 48 106 | 112).  Every column's sums are taken in the same
-  // order either way.
-  const int blocks = (dv + 15) / 16;
-  const bool two = blocks % 2 == 0 && 2LL * blocks * H * n_seqs >= 3LL * num_sms();
+#define LAUNCH_REC_R(R, D, CH)                                                          \
+  if (form == kOne && n_seqs <= 32) LAUNCH_REC(R, D, CH, 1, true, R == 8 ? 5 : 3);      \
+  else if (form == kOne) LAUNCH_REC(R, D, CH, 1, false, (R == 8 ? 7 : 5) - CH);         \
+  else if (form == kTwoFew) LAUNCH_REC(R, D, CH, 2, D, (R == 8 ? 4 : 3) - D);           \
+  else if (form == kTwo) LAUNCH_REC(R, D, CH, 2, false, (R == 8 ? 6 : 4) - CH);         \
+  else if constexpr (!D && !CH) LAUNCH_REC(R, D, CH, 4, false, R == 8 ? 3 : 2)
+#define LAUNCH_REC_N(D, CH)                                                             \
+  if (n <= 32) LAUNCH_REC(4, D, CH, 1, true, 6);                                        \
+  else if (n <= 64) { LAUNCH_REC_R(8, D, CH); }                                         \
+  else if (n <= 128) { LAUNCH_REC_R(16, D, CH); }                                       \
+  else if (ones <= 2 * sms || (CH && n_seqs <= 32)) LAUNCH_REC(32, D, CH, 1, true, 2);  \
+  else LAUNCH_REC(32, D, CH, 1, false, 3)
+  // Columns per lane, by the CTAs there are of 16 (one column) and of 32 (two).  Columns that share a lane share every word of k
+  // and q; with one each there are twice the warps.
+  // (More than 32 sequences are mostly single rows: there the read ahead only costs warps.)
+  // * One where that is at most a CTA per SM (us, one | two columns: delta rule, 1 sequence of 4000 rows, 16 heads 504 | 647; 1,
+  //   2000, 32, twice the CTAs 421 | 330), and where the columns do not fill blocks of 32: lanes without one walk along.
+  // * Two, for the delta rules read ahead, up to four CTAs per SM, two with a decay per channel (delta rule, read ahead | not:
+  //   3, 2300, 16 205 | 247; 8, 1500, 16 112 | 114; 8, 4096, 32 496 | 482; 64 single rows, 32 heads 74 | 49).
+  // * Beyond, four for a plain decay without the delta rule (two | four: 8, 4096, 32 404 | 334; 64 single
+  //   rows 48 | 46), two for the others (delta rule 8, 4096, 32 482 | 506; 64 single rows 49 | 58; per channel, 128 single rows, 16 heads 64 | 97).
+  enum { kOne, kTwoFew, kTwo, kFour };
+  const int blocks = (dv + 15) / 16, sms = num_sms();
+  const long long ones = (long long)blocks * H * n_seqs;
+  const int form = blocks % 2 || ones <= sms                                          ? kOne
+                   : ones / 2 <= (decay_channels ? 2LL : 4LL) * sms                   ? kTwoFew
+                   : delta || decay_channels || blocks % 4                             ? kTwo
+                                                                                      : kFour;
   if (decay_channels) {
     if (delta) { LAUNCH_REC_N(true, true); } else { LAUNCH_REC_N(false, true); }
   } else {
     if (delta) { LAUNCH_REC_N(true, false); } else { LAUNCH_REC_N(false, false); }
   }
 #undef LAUNCH_REC_N
+#undef LAUNCH_REC_R
 #undef LAUNCH_REC
   SXB_CHECK_LAUNCH();
   return SXB_OK;
