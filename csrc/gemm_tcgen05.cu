@@ -604,38 +604,13 @@ done:
 #include "gemm_skinny.cuh"
 
 // ------------------------------------------------------------------ host side
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn get_encode() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) ==
-            cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
-
 // 2-D bf16 tensor map over a row-major [rows, cols] matrix with row pitch `ld` elements;
 // box = [box_rows, box_cols] with box_cols * 2 == 128 bytes (128B swizzle).
 static int make_map_2d(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint64_t ld,
-                       uint32_t box_rows, uint32_t box_cols, CUtensorMapDataType dt, int esize) {
-  EncodeTiledFn enc = get_encode();
-  if (!enc) return SXB_ERR_DRIVER;
-  cuuint64_t dims[2] = {cols, rows};
-  cuuint64_t strides[1] = {ld * (uint64_t)esize};
-  cuuint32_t box[2] = {box_cols, box_rows};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = enc(m, dt, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? SXB_OK : SXB_ERR_DRIVER;
+                       uint32_t box_rows, uint32_t box_cols) {
+  const unsigned long long dims[2] = {cols, rows}, strides[1] = {ld * 2};
+  const unsigned int box[2] = {box_cols, box_rows};
+  return encode_tensor_map(m, kBF16, 2, ptr, dims, strides, box, 128);
 }
 
 template <int BN, int STAGES>
@@ -721,10 +696,9 @@ static int launch_skinny(const void* A, const void* B, const Params& p, int lda,
     configured = true;
   }
   CUtensorMap tw, tx;
-  const CUtensorMapDataType BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-  int rc = make_map_2d(&tw, B, p.N, p.K, ldb, 128, BK, BF, 2);
+  int rc = make_map_2d(&tw, B, p.N, p.K, ldb, 128, BK);
   if (rc) return rc;
-  rc = make_map_2d(&tx, A, p.M, p.K, lda, BN, BK, BF, 2);
+  rc = make_map_2d(&tx, A, p.M, p.K, lda, BN, BK);
   if (rc) return rc;
   const int tiles_n = (p.N + 127) / 128, tiles_m = (p.M + BN - 1) / BN;
   const int S = skinny_split(tiles_n * tiles_m, (p.K + BK - 1) / BK);
@@ -794,31 +768,30 @@ SXB_API int sxb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
   const int BNsel = (N > 128) ? 256 : 128;
   CUtensorMap ta, tb, tc;
   int rc;
-  const CUtensorMapDataType BF = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const bool big = (M >= 512 && N >= 512 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= 37);
   if (g_gemm_mode == 2 || (g_gemm_mode == 0 && big)) {
-    if (layout == TN) rc = make_map_2d(&ta, A, K, M, lda, BK, 64, BF, 2);
-    else rc = make_map_2d(&ta, A, M, K, lda, 128, BK, BF, 2);
+    if (layout == TN) rc = make_map_2d(&ta, A, K, M, lda, BK, 64);
+    else rc = make_map_2d(&ta, A, M, K, lda, 128, BK);
     if (rc) return rc;
-    if (layout == NT) rc = make_map_2d(&tb, B, N, K, ldb, 128, BK, BF, 2);
-    else rc = make_map_2d(&tb, B, K, N, ldb, BK, 64, BF, 2);
+    if (layout == NT) rc = make_map_2d(&tb, B, N, K, ldb, 128, BK);
+    else rc = make_map_2d(&tb, B, K, N, ldb, BK, 64);
     if (rc) return rc;
     if (tma_c) {
-      rc = make_map_2d(&tc, C, M, N, ldc, 128, 64, BF, 2);
+      rc = make_map_2d(&tc, C, M, N, ldc, 128, 64);
       if (rc) return rc;
     } else {
       tc = ta;
     }
     return launch_pair(ta, tb, tc, p, max_ctas, reinterpret_cast<cudaStream_t>(stream));
   }
-  if (layout == TN) rc = make_map_2d(&ta, A, K, M, lda, BK, 64, BF, 2);
-  else rc = make_map_2d(&ta, A, M, K, lda, BM, BK, BF, 2);
+  if (layout == TN) rc = make_map_2d(&ta, A, K, M, lda, BK, 64);
+  else rc = make_map_2d(&ta, A, M, K, lda, BM, BK);
   if (rc) return rc;
-  if (layout == NT) rc = make_map_2d(&tb, B, N, K, ldb, BNsel, BK, BF, 2);
-  else rc = make_map_2d(&tb, B, K, N, ldb, BK, 64, BF, 2);
+  if (layout == NT) rc = make_map_2d(&tb, B, N, K, ldb, BNsel, BK);
+  else rc = make_map_2d(&tb, B, K, N, ldb, BK, 64);
   if (rc) return rc;
   if (tma_c) {
-    rc = make_map_2d(&tc, C, M, N, ldc, BM, 64, BF, 2);
+    rc = make_map_2d(&tc, C, M, N, ldc, BM, 64);
     if (rc) return rc;
   } else {
     tc = ta;  // never dereferenced by the direct epilogue
