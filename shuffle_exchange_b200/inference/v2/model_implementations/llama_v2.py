@@ -151,7 +151,7 @@ class RaggedLlamaModel:
         n_layers = len(layers) // 11
         _n.attn_call("sxb_ragged_llama_forward", model.buffer_info()[0], table.buffer_info()[0], n_layers,
                      float(c.rms_norm_eps), float(c.rope_theta), 1.0 / math.sqrt(d), _n.stream_ptr())
-        _n.launch_count += 9 * n_layers + 3        # the entry points that the call stands for, itself among them
+        _n.count_launches(9 * n_layers + 3)       # the entry points that the call stands for, itself among them
         return logits
 
     @torch.no_grad()

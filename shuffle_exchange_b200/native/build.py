@@ -2,6 +2,8 @@
 
 * ``libsxb200.so``      — every ``csrc/*.cu`` compiled for ``sm_100a`` (tcgen05/TMEM/TMA kernels,
   fused optimizers, norms, attention, quantisers, MoE/ragged kernels, symmetric-memory collectives).
+* ``_sxb_ops.so``       — ``csrc/torch/*.cpp``: the most called differentiable operators as autograd functions in C++ (g++ against
+  torch's headers; without it they stay in Python, over the same kernels).
 * ``libsxb200_host.so`` — ``csrc/host/*.cpp``: AVX-512/AVX2 + OpenMP CPU optimizers, the async
   file-IO engine and host-side schedulers (g++ only, no CUDA).
 
@@ -126,8 +128,37 @@ def build_host(verbose: bool = False, force: bool = False) -> Path:
     return lib
 
 
+def build_ops(force: bool = False) -> Path:
+    import sysconfig
+
+    import torch
+    from torch.utils.cpp_extension import include_paths
+    OBJ_DIR.mkdir(parents=True, exist_ok=True)
+    gxx = shutil.which("g++") or "g++"
+    cuda = Path(_nvcc()).resolve().parents[1] / "include"
+    inc = [f"-I{d}" for d in (*include_paths(), sysconfig.get_paths()["include"], cuda)]
+    flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    src, obj = CSRC / "torch" / "native_ops.cpp", OBJ_DIR / "ops_native_ops.o"
+    lib = OUT_DIR / "_sxb_ops.so"
+    key = [*flags, torch.__version__, sys.version]
+    if force or _stale(src, obj, [], key) or not lib.exists():
+        digest = _digest(src, [], key)
+        _run([gxx, *flags, *inc, "-c", str(src), "-o", str(obj)])
+        _run([gxx, "-shared", "-o", str(lib), str(obj), f"-L{Path(torch.__file__).parent / 'lib'}", "-ltorch_python", "-ltorch",
+              "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ldl"])
+        _stamp(obj, digest)
+    return lib
+
+
 def build_all(verbose: bool = False, force: bool = False):
-    return build_cuda(verbose, force), build_host(verbose, force)
+    with cf.ThreadPoolExecutor(max_workers=1) as ex:
+        ops = ex.submit(build_ops, force)
+        libs = build_cuda(verbose, force), build_host(verbose, force)
+        try:
+            ops.result()
+        except Exception as e:          # no headers of Python or torch here: the operators stay in Python
+            print(f"WARNING: {OUT_DIR / '_sxb_ops.so'} was not built: {str(e)[-400:]}")
+    return libs
 
 
 if __name__ == "__main__":

@@ -23,8 +23,13 @@ _RANKS = 1                       # ranks of the program as far as known
 _HOST: Optional[ctypes.CDLL] = None
 _LOCK = threading.Lock()
 
-# number of native GPU entry-point calls since the last reset (bench.py reports this)
-launch_count = 0
+try:
+    from . import _sxb_ops as OPS   # differentiable operators in C++ over the same library (csrc/torch); None: they stay in Python
+except ImportError:
+    OPS = None
+
+# native GPU entry-point calls made from Python since the last reset, and those of OPS at that reset (``launch_count`` adds up)
+_calls = _ops_base = 0
 
 F32, F16, BF16, FP8E4M3, I8, U8, I32, I64 = range(8)
 _DT = {
@@ -118,6 +123,8 @@ def load() -> ctypes.CDLL:
                               "shuffle_exchange_b200.native.build`")
         lib = ctypes.CDLL(str(path), mode=ctypes.RTLD_GLOBAL)
         _bind(lib, SIGNATURES)
+        if OPS is not None:
+            OPS.bind(lib._handle, NativeError)
         _LIB = lib
         if _RANKS > 1:                  # behind the line above: a count that arrives meanwhile is told by one side or both
             lib.sxb_attn_note_ranks(_RANKS)
@@ -173,10 +180,10 @@ def no_tape(*tensors: Optional[torch.Tensor]) -> bool:
 
 def call(name: str, *args):
     """Invoke ``name`` and raise on a non-zero status."""
-    global launch_count
+    global _calls
     fn = getattr(load(), name)
     rc = fn(*args)
-    launch_count += 1
+    _calls += 1
     if name in _LONG_RETURN:
         return rc
     if rc != 0:
@@ -189,10 +196,15 @@ def call(name: str, *args):
 
 
 def attn_call(name: str, *args):
-    """:func:`call` of an attention kernel, which has to know of every process group, whoever made it (:func:`note_ranks`)."""
+    """:func:`call` of an attention kernel, which has to know of every process group."""
+    know_ranks()
+    return call(name, *args)
+
+
+def know_ranks() -> None:
+    """:func:`note_ranks` for a process group that exists by now, whoever made it."""
     if _RANKS == 1 and _dist.is_available() and _dist.is_initialized():
         note_ranks(_dist.get_world_size())
-    return call(name, *args)
 
 
 HANG_KINDS = ("attn", "gemm", "gemmx", "moe_ep", "seqmix", "symm")      # kernel families whose waits can give up
@@ -221,9 +233,22 @@ def hang_info(kind: str = "attn"):
     return {"tag": buf[1], "block": (buf[2], buf[3], buf[4]), "thread": buf[5], "parity": buf[6], "aux": buf[7]}
 
 
+def __getattr__(name: str):
+    if name == "launch_count":          # native GPU entry-point calls since the last reset (bench.py reports this)
+        return _calls + (OPS.calls() - _ops_base if OPS is not None else 0)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
+
+
+def count_launches(n: int) -> None:
+    """``n`` entry-point calls that one call stood for."""
+    global _calls
+    _calls += n
+
+
 def reset_launch_count() -> int:
-    global launch_count
-    n, launch_count = launch_count, 0
+    global _calls, _ops_base
+    n = __getattr__("launch_count")
+    _calls, _ops_base = 0, OPS.calls() if OPS is not None else 0
     return n
 
 

@@ -43,6 +43,9 @@ def _torch_act(x, code):
 # ----------------------------------------------------------------------------- GEMM
 GEMM_NT, GEMM_NN, GEMM_TN = 0, 1, 2
 
+# The operators below that most layers call, in C++ (csrc/torch): each returns None for what is not the plain case.
+_ops = _n.OPS
+
 # Set by profiling.flops_profiler while a profile is running: callable(kind: str, flops: float).  The native ops
 # are invisible to torch's dispatcher, so they report their own work.
 flop_sink = None
@@ -244,6 +247,10 @@ def _warn_once(key: str, message: str) -> None:
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``x @ weight.T + bias`` — tcgen05 GEMM for bf16 CUDA tensors (fwd, dgrad and wgrad)."""
+    if _ops is not None and bias is None and flop_sink is None:
+        y = _ops.linear(x, weight)
+        if y is not None:
+            return y
     if x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 \
             and x.shape[-1] % 8 == 0 and weight.shape[0] % 8 == 0:
         if not x.is_contiguous():
@@ -345,6 +352,10 @@ class _RMSNorm(torch.autograd.Function):
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,
              residual: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """Returns ``(norm(x + residual) * weight, x + residual)`` (pre-norm block helper)."""
+    if _ops is not None:
+        y = _ops.rms_norm(x, weight, eps, residual)
+        if y is not None:
+            return y if residual is not None else (y, x)
     if x.is_cuda:
         if not x.is_contiguous():
             x = x.contiguous()
@@ -466,6 +477,10 @@ class _Rope(torch.autograd.Function):
 def rope(x: torch.Tensor, positions: Optional[torch.Tensor], cos: torch.Tensor, sin: torch.Tensor,
          n_heads: int, head_dim: int) -> torch.Tensor:
     """Rotate the first ``n_heads`` heads of every row of ``x`` ([..., C], contiguous); in place on CUDA."""
+    if _ops is not None:
+        y = _ops.rope(x, positions, cos, sin, n_heads, head_dim)
+        if y is not None:
+            return y
     if x.is_cuda:
         if not x.is_contiguous():
             x = x.contiguous()
@@ -512,6 +527,10 @@ class _Gated(torch.autograd.Function):
 def gated_act(x: torch.Tensor, act="silu") -> torch.Tensor:
     """``act(x[..., :F]) * x[..., F:]`` (SwiGLU/GeGLU with concatenated gate|up projection)."""
     code = _act_code(act)
+    if _ops is not None:
+        y = _ops.gated_act(x, code)
+        if y is not None:
+            return y
     if x.is_cuda:
         x = x.contiguous()
         if x.dim() == 2 and x.shape[1] % 2 == 0 and _n.no_tape(x):
@@ -739,6 +758,11 @@ def flash_attention_qkv(qkv: torch.Tensor, n_q: int, n_kv: int, head_dim: int, c
     """``qkv [B, S, (n_q + 2 n_kv) * head_dim]`` (q heads | k heads | v heads) -> ``[B, S, n_q, head_dim]``; the
     gradient comes back as one fused tensor."""
     scale = scale if scale is not None else 1.0 / math.sqrt(head_dim)
+    if _ops is not None and flop_sink is None:
+        _n.know_ranks()
+        y = _ops.attention_qkv(qkv, n_q, n_kv, head_dim, causal, scale)
+        if y is not None:
+            return y
     if qkv.is_cuda:
         if qkv.dtype != torch.bfloat16 or head_dim not in (64, 128):
             # fp16 / fp32 or another head size: the general entry point pads or takes the library path (see there)
