@@ -35,10 +35,73 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t saddr, uint32_t rank) {
   return v;
 }
 
+// The sum of a tile's partial tiles over the cluster's S CTAs, in rank order: [rows of tokens][128 weight rows], `cols` of which exist, to C
+// at `first`.  The CTAs take groups of four columns in turns.  GATED: the tile's first 64 weight rows are gates, the others what they gate:
+// C gets the 64 columns act(gate) * up of the two sums rounded to bf16, as the activation's own kernel would read them.
+template <bool GATED>
+__device__ __forceinline__ void skinny_reduce(const Params& p, int S, int rank, uint32_t sbase, int rows, int cols, size_t first) {
+  constexpr int kWords = GATED ? 16 : 32;
+  auto sum = [&](int at) {
+    float4 part[8];                       // all remote loads in flight before the first is used
+#pragma unroll
+    for (int s = 0; s < 8; ++s)
+      if (s < S) part[s] = ld_cluster_f4(sbase + at * 4, s);
+    float4 a = part[0];
+#pragma unroll
+    for (int s = 1; s < 8; ++s)
+      if (s < S) { a.x += part[s].x; a.y += part[s].y; a.z += part[s].z; a.w += part[s].w; }
+    return make_float4(p.alpha * a.x, p.alpha * a.y, p.alpha * a.z, p.alpha * a.w);
+  };
+  for (int i = rank * kThreads + threadIdx.x; i < rows * kWords; i += S * kThreads) {
+    const int m = i / kWords, c = (i % kWords) * 4;
+    if (c >= cols) continue;
+    const float4 a = sum(m * 128 + c);
+    const size_t at = first + (size_t)m * p.ldc + c;
+    if constexpr (GATED) {
+      const float4 b = sum(m * 128 + 64 + c);
+      const float g[4] = {a.x, a.y, a.z, a.w}, u[4] = {b.x, b.y, b.z, b.w};
+      float r[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        r[j] = ew::act_fwd(__bfloat162float(__float2bfloat16_rn(g[j])), p.act) * __bfloat162float(__float2bfloat16_rn(u[j]));
+      *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.C) + at) = make_uint2(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]));
+      continue;
+    }
+    const float r[4] = {a.x, a.y, a.z, a.w};
+    if (p.c_dtype == kBF16) {
+      __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.C) + at;
+      if (!p.accumulate && c + 4 <= cols && (reinterpret_cast<uintptr_t>(o) & 7) == 0) {
+        *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (c + j < cols) o[j] = __float2bfloat16_rn(p.accumulate ? r[j] + __bfloat162float(o[j]) : r[j]);
+      }
+    } else {
+      float* o = reinterpret_cast<float*>(p.C) + at;
+      if (!p.accumulate && c + 4 <= cols && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
+        *reinterpret_cast<float4*>(o) = make_float4(r[0], r[1], r[2], r[3]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (c + j < cols) o[j] = p.accumulate ? r[j] + o[j] : r[j];
+      }
+    }
+  }
+}
+
+// A stage's 128 weight rows from row n0 of a matrix that starts at `base` (GATED: 64 gates and the 64 rows p.N behind them).
+template <bool GATED>
+__device__ __forceinline__ void load_weights(uint8_t* dst, const CUtensorMap* tm, uint64_t* bar, int k, int base, int n0, const Params& p) {
+  tma_load_2d(dst, tm, bar, k, base + n0);
+  if (GATED) tma_load_2d(dst + 64 * BK * 2, tm, bar, k, base + p.N + n0);
+}
+
 // grid (tiles of 128 weight rows * S, ceil(M / BN)); clusters of S CTAs along x share one tile.
 // CHAIN: launched while the kernel that makes the tokens may still run (its own instance: asked at run time, the question cost a product
 // outside a chain up to half a microsecond, 16 x 768 x 768 7.6 -> 8.2 us).
-template <int BN, int STAGES, bool CHAIN>
+// GATED: B is [2 N, K], gates first, and C the activated product (skinny_reduce).
+template <int BN, int STAGES, bool CHAIN, bool GATED>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p,
                    const int S) {
@@ -51,7 +114,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = blockIdx.x % S, tile = blockIdx.x / S;
-  const int n0 = tile * 128, m0 = blockIdx.y * BN;
+  const int n0 = tile * (GATED ? 64 : 128), m0 = blockIdx.y * BN;
   const int num_kb = (p.K + BK - 1) / BK;
   const int kb0 = (int)((long long)num_kb * rank / S), kb1 = (int)((long long)num_kb * (rank + 1) / S);
 
@@ -88,7 +151,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       if (elected)
         for (int kb = kb0; kb < ahead; ++kb) {
           mbar_expect_tx(&full_bar[kb - kb0], Plan::kStage);
-          tma_load_2d(smem + (kb - kb0) * Plan::kStage, &tmW, &full_bar[kb - kb0], kb * BK, n0);
+          load_weights<GATED>(smem + (kb - kb0) * Plan::kStage, &tmW, &full_bar[kb - kb0], kb * BK, 0, n0, p);
         }
       __syncwarp();
       chain_wait();
@@ -101,7 +164,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         uint8_t* sa = smem + stage * Plan::kStage;
         if (!CHAIN || kb >= ahead) {
           mbar_expect_tx(&full_bar[stage], Plan::kStage);
-          tma_load_2d(sa, &tmW, &full_bar[stage], kb * BK, n0);
+          load_weights<GATED>(sa, &tmW, &full_bar[stage], kb * BK, 0, n0, p);
         }
         tma_load_2d(sa + Plan::kA, &tmX, &full_bar[stage], kb * BK, m0);
       }
@@ -158,42 +221,138 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     tmem_dealloc(tmem_base, Plan::kCols);
   }
   cluster_sync_all();                       // every CTA's partial tile is in its shared memory
-  {
-    const int cols = min(128, p.N - n0);
-    const int items = rows * 32;            // float4 groups of the tile; the cluster's CTAs take them in turn
-    for (int i = rank * kThreads + threadIdx.x; i < items; i += S * kThreads) {
-      const int m = i >> 5, c = (i & 31) * 4;
-      if (c >= cols) continue;
-      float4 part[8];                       // all remote loads in flight before the first is used
-#pragma unroll
-      for (int s = 0; s < 8; ++s)
-        if (s < S) part[s] = ld_cluster_f4(sbase + (m * 128 + c) * 4, s);
-      float4 a = part[0];
-#pragma unroll
-      for (int s = 1; s < 8; ++s)
-        if (s < S) { a.x += part[s].x; a.y += part[s].y; a.z += part[s].z; a.w += part[s].w; }
-      const float r[4] = {p.alpha * a.x, p.alpha * a.y, p.alpha * a.z, p.alpha * a.w};
-      const size_t at = (size_t)(m0 + m) * p.ldc + n0 + c;
-      if (p.c_dtype == kBF16) {
-        __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.C) + at;
-        if (!p.accumulate && c + 4 <= cols && (reinterpret_cast<uintptr_t>(o) & 7) == 0) {
-          *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]));
-        } else {
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (c + j < cols) o[j] = __float2bfloat16_rn(p.accumulate ? r[j] + __bfloat162float(o[j]) : r[j]);
-        }
-      } else {
-        float* o = reinterpret_cast<float*>(p.C) + at;
-        if (!p.accumulate && c + 4 <= cols && (reinterpret_cast<uintptr_t>(o) & 15) == 0) {
-          *reinterpret_cast<float4*>(o) = make_float4(r[0], r[1], r[2], r[3]);
-        } else {
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            if (c + j < cols) o[j] = p.accumulate ? r[j] + o[j] : r[j];
-        }
+  skinny_reduce<GATED>(p, S, rank, sbase, rows, min(GATED ? 64 : 128, p.N - n0), (size_t)m0 * p.ldc + n0);
+  cluster_sync_all();                       // no CTA leaves while a peer still reads its partial tile
+}
+
+// The same product for groups of rows, each against a weight of its own (the experts of a layer): C[rows of g] = A[rows of g] B[g]^T.
+// How many rows a group has is known on the device only; they start at offsets[g], used[g] of them.
+// What bounds it: the weights' bytes.  The persistent pair kernel multiplies 256 rows per tile whatever it has, and its tiles of
+// 256 weight rows leave a last wave nearly empty.  Here a cluster of S CTAs cuts the K of 128 weight rows, the MMA's N is the
+// number of tokens rounded up to 16, and the ring's stages take as much room as the group's tokens need, in boxes of 32.
+// More than 256 tokens are taken in turns of 256 that read the weights again.
+// us, one call after the other so that the chip is at its power limit (the pair kernel's clock falls to 1.05 GHz there, this one's to 1.5),
+// pair kernel | this one: 8 x 28672 x 4096 and 8 x 4096 x 14336, 2 tokens 155 | 118 and 106 | 63; 16 tokens 438 | 301 and 243 | 149; 200 tokens 427 |
+// 327 and 237 | 157 (floors 287 and 144); 400 tokens 440 | 389 and 242 | 177; 1000 tokens 549 | 669 and 340 | 343.
+struct GroupsPlan {
+  static constexpr int kA = 128 * BK * 2, kBox = 32 * BK * 2;
+  static constexpr int kMost = 4, kTurn = 256;                    // stages, tokens
+  static constexpr int kRing = 4 * (kA + 2 * kBox);               // 96 KB: four stages up to 64 tokens, three to 128, two to 256
+  static constexpr int kTotal = kRing + 256 + 1024;               // two CTAs per SM; half of the fp32 tile (64 KB) lies over the ring
+};
+
+template <bool GATED>
+__global__ void __launch_bounds__(kThreads, 2)
+gemm_skinny_groups_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p,
+                          const int S, const int* __restrict__ offsets, const int* __restrict__ used) {
+  using Plan = GroupsPlan;
+  const int g = blockIdx.y;
+  const int rows_all = used[g], row0 = offsets[g];
+  if (rows_all <= 0) return;                                      // the whole cluster
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + Plan::kRing);
+  uint64_t* empty_bar = full_bar + Plan::kMost;
+  uint64_t* done_bar = empty_bar + Plan::kMost;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done_bar + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = blockIdx.x % S, n0 = blockIdx.x / S * (GATED ? 64 : 128);
+  const int num_kb = (p.K + BK - 1) / BK;
+  const int kb0 = (int)((long long)num_kb * rank / S), kb1 = (int)((long long)num_kb * (rank + 1) / S);
+  const int stage_bytes = Plan::kA + (min(rows_all, Plan::kTurn) + 31) / 32 * Plan::kBox;
+  const int stages = min(Plan::kMost, Plan::kRing / stage_bytes), cols = rows_all > 128 ? 256 : 128;
+
+  if (warp == 0 && lane == 0) {
+    tma_prefetch_desc(&tmW);
+    tma_prefetch_desc(&tmX);
+  }
+  if (warp == 1) {
+    if (lane == 0) {
+      for (int s = 0; s < Plan::kMost; ++s) {
+        mbar_init(&full_bar[s], 1);
+        mbar_init(&empty_bar[s], 1);
       }
+      mbar_init(done_bar, 1);
+      mbar_fence_init();
+    }
+    __syncwarp();
+    tmem_alloc(tmem_slot, cols);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t sbase = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
+  const uint32_t tbase = __shfl_sync(0xffffffffu, tmem_base, 0);
+
+  int stage = 0;                                                  // the ring goes on from turn to turn
+  uint32_t phase = 0;
+  for (int turn = 0; turn * Plan::kTurn < rows_all; ++turn) {
+    const int m0 = row0 + turn * Plan::kTurn, rows = min(Plan::kTurn, rows_all - turn * Plan::kTurn);
+    if (warp == 0) {
+      const bool elected = elect_one();
+      const int boxes = (rows + 31) / 32;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!__all_sync(0xffffffffu, mbar_wait_to(&empty_bar[stage], phase ^ 1, 44, kb))) break;
+        if (elected) {
+          uint8_t* sa = smem + stage * stage_bytes;
+          mbar_expect_tx(&full_bar[stage], Plan::kA + boxes * Plan::kBox);
+          load_weights<GATED>(sa, &tmW, &full_bar[stage], kb * BK, g * p.N * (GATED ? 2 : 1), n0, p);
+          for (int i = 0; i < boxes; ++i)
+            tma_load_2d(sa + Plan::kA + i * Plan::kBox, &tmX, &full_bar[stage], kb * BK, m0 + 32 * i);
+        }
+        __syncwarp();
+        if (++stage == stages) { stage = 0; phase ^= 1; }
+      }
+    } else if (warp == 1) {
+      const bool elected = elect_one();
+      const uint32_t idesc = make_idesc(128, (rows + 15) & ~15, 1, 1, 0, 0);
+      constexpr uint32_t kDescHi = (1024u >> 4) | (1u << 14) | (2u << 29);
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!__all_sync(0xffffffffu, mbar_wait_to(&full_bar[stage], phase, 45, kb))) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t at = sbase + stage * stage_bytes;
+        const uint32_t a_lo = ((at >> 4) & 0x3FFFu) | (1u << 16), b_lo = (((at + Plan::kA) >> 4) & 0x3FFFu) | (1u << 16);
+        if (elected) {
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k)
+            umma_f16(tbase, (uint64_t(kDescHi) << 32) | (a_lo + k * 2), (uint64_t(kDescHi) << 32) | (b_lo + k * 2), idesc,
+                     (kb > kb0) || k > 0);
+          umma_commit(&empty_bar[stage]);
+        }
+        __syncwarp();
+        if (++stage == stages) { stage = 0; phase ^= 1; }
+      }
+      if (elected && ok) umma_commit(done_bar);
+      __syncwarp();
+    }
+    bool done = false;
+    if (warp >= 2) done = __all_sync(0xffffffffu, mbar_wait_to(done_bar, turn & 1, 46, turn));
+    for (int half = 0; half < rows; half += 128) {
+      const int part = min(128, rows - half);
+      if (done) {
+        tc_fence_after();
+        const int quad = warp & 3;
+        const uint32_t t_row = tbase + half + (uint32_t(quad * 32) << 16);
+        float* dst = reinterpret_cast<float*>(smem) + quad * 32 + lane;
+#pragma unroll 1
+        for (int c = 0; c < part; c += 16) {
+          uint32_t v[16];
+          tmem_ld_32x16(t_row + c, v);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 16; ++j) dst[(c + j) * 128] = __uint_as_float(v[j]);
+        }
+        tc_fence_before();
+      }
+      __syncthreads();
+      tc_fence_after();
+      cluster_sync_all();                   // every CTA's partial tile is in its shared memory
+      skinny_reduce<GATED>(p, S, rank, sbase, part, min(GATED ? 64 : 128, p.N - n0), (size_t)(m0 + half) * p.ldc + n0);
+      fence_async_smem();                   // read and written here, then by the next turn's copies
+      cluster_sync_all();                   // no CTA leaves, or fills its ring again, while a peer still reads its partial tile
     }
   }
-  cluster_sync_all();                       // no CTA leaves while a peer still reads its partial tile
+  if (warp == 1) tmem_dealloc(tmem_base, cols);
 }

@@ -16,6 +16,10 @@
 // Replaces the cuBLAS calls behind F.linear that the reference relies on
 // (reference: deepspeed/inference/v2/kernels/core_ops/blas_kernels/blas_utils.h:31-41,
 // and every nn.Linear in the training path).
+#include <algorithm>
+#include <climits>
+
+#include "activation.cuh"
 #include "sxb_common.cuh"
 
 namespace sxb {
@@ -50,6 +54,7 @@ struct Params {
   void* C;
   int ldc;
   float alpha;
+  int act;         // products that end in a gated activation: which (ew::Act)
 };
 
 template <int BN, int STAGES>
@@ -685,10 +690,10 @@ static bool use_skinny(int M, int N, int K) {
   return tiles <= 128 && tiles <= K / 32;
 }
 
-template <int BN, int STAGES, bool CHAIN>
+template <int BN, int STAGES, bool CHAIN, bool GATED>
 static int launch_skinny(const void* A, const void* B, const Params& p, int lda, int ldb, cudaStream_t stream) {
   using Plan = SkinnyPlan<BN, STAGES>;
-  auto kfn = gemm_skinny_kernel<BN, STAGES, CHAIN>;
+  auto kfn = gemm_skinny_kernel<BN, STAGES, CHAIN, GATED>;
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, Plan::kTotal);
@@ -696,11 +701,12 @@ static int launch_skinny(const void* A, const void* B, const Params& p, int lda,
     configured = true;
   }
   CUtensorMap tw, tx;
-  int rc = make_map_2d(&tw, B, p.N, p.K, ldb, 128, BK);
+  int rc = make_map_2d(&tw, B, (GATED ? 2 : 1) * (uint64_t)p.N, p.K, ldb, GATED ? 64 : 128, BK);
   if (rc) return rc;
   rc = make_map_2d(&tx, A, p.M, p.K, lda, BN, BK);
   if (rc) return rc;
-  const int tiles_n = (p.N + 127) / 128, tiles_m = (p.M + BN - 1) / BN;
+  constexpr int kTile = GATED ? 64 : 128;
+  const int tiles_n = (p.N + kTile - 1) / kTile, tiles_m = (p.M + BN - 1) / BN;
   const int S = skinny_split(tiles_n * tiles_m, (p.K + BK - 1) / BK);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles_n * S, tiles_m);
@@ -719,12 +725,53 @@ static int launch_skinny(const void* A, const void* B, const Params& p, int lda,
   return SXB_OK;
 }
 
-template <bool CHAIN>
+template <bool CHAIN, bool GATED>
 static int launch_skinny(const void* A, const void* B, const Params& p, int lda, int ldb, cudaStream_t stream) {
-  if (p.M <= 16) return launch_skinny<16, 6, CHAIN>(A, B, p, lda, ldb, stream);
-  if (p.M <= 32) return launch_skinny<32, 5, CHAIN>(A, B, p, lda, ldb, stream);
-  if (p.M <= 64) return launch_skinny<64, 4, CHAIN>(A, B, p, lda, ldb, stream);
-  return launch_skinny<128, 3, CHAIN>(A, B, p, lda, ldb, stream);
+  if (p.M <= 16) return launch_skinny<16, 6, CHAIN, GATED>(A, B, p, lda, ldb, stream);
+  if (p.M <= 32) return launch_skinny<32, 5, CHAIN, GATED>(A, B, p, lda, ldb, stream);
+  if (p.M <= 64) return launch_skinny<64, 4, CHAIN, GATED>(A, B, p, lda, ldb, stream);
+  return launch_skinny<128, 3, CHAIN, GATED>(A, B, p, lda, ldb, stream);
+}
+
+template <bool GATED>
+static int launch_skinny_groups(const void* A, const void* B, const Params& p, long long lda, long long ldb, int groups,
+                                const int* offsets, const int* used, long long total_rows, long long routed, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_skinny_groups_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         GroupsPlan::kTotal);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  CUtensorMap tw, tx;
+  constexpr int kTile = GATED ? 64 : 128;
+  int rc = make_map_2d(&tw, B, (uint64_t)groups * p.N * (GATED ? 2 : 1), p.K, ldb, kTile, BK);
+  if (rc) return rc;
+  rc = make_map_2d(&tx, A, total_rows, p.K, lda, 32, BK);
+  if (rc) return rc;
+  // Cluster size: none while the tiles of the groups that can have rows fill the chip twice over; two CTAs where they do not quite, more
+  // only until they fill it one and a half times, on 32 blocks of K each (8 if more than half of the chip would idle).  us, back to back,
+  // 1 | 2 | 4 CTAs: 8 x 28672 x 4096, 200 tokens 327 | 335 | 392; 8 x 4096 x 14336 164 | 157 | 167; 4 groups of it 75 | 63 | 65; 16 x 1024 x
+  // 4096 35 | 30 | 34.
+  const int num_kb = (p.K + BK - 1) / BK, sms = num_sms();
+  const long long tiles = (long long)((p.N + kTile - 1) / kTile) * std::min<long long>(groups, routed);
+  int S = 1;
+  while (S < 8 && (2 * tiles * S < 3LL * sms || (S == 1 && tiles < 2LL * sms)) &&
+         num_kb / (2 * S) >= (2 * tiles * S < sms ? 8 : 32))
+    S *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((p.N + kTile - 1) / kTile * S, groups);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = GroupsPlan::kTotal;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_skinny_groups_kernel<GATED>, tw, tx, p, S, offsets, used);
+  if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
+  return SXB_OK;
 }
 
 }  // namespace gemm
@@ -764,7 +811,7 @@ SXB_API int sxb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
   p.accumulate = accumulate ? 1 : 0; p.direct = tma_c ? 0 : 1; p.C = C; p.ldc = ldc;
   p.alpha = alpha;
   if (layout == NT && (g_gemm_mode == 3 || (g_gemm_mode == 0 && max_ctas <= 0 && use_skinny(M, N, K))))
-    return (chained() ? launch_skinny<true> : launch_skinny<false>)(A, B, p, lda, ldb, reinterpret_cast<cudaStream_t>(stream));
+    return (chained() ? launch_skinny<true, false> : launch_skinny<false, false>)(A, B, p, lda, ldb, reinterpret_cast<cudaStream_t>(stream));
   const int BNsel = (N > 128) ? 256 : 128;
   CUtensorMap ta, tb, tc;
   int rc;
@@ -799,4 +846,37 @@ SXB_API int sxb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (BNsel == 256) return launch<256, 4>(ta, tb, tc, p, max_ctas, s);
   return launch<128, 6>(ta, tb, tc, p, max_ctas, s);
+}
+
+// C[rows of g] = A[rows of g] B[g]^T in bf16 for `num_groups` groups of few rows: those of group g start at offsets[g] (rows of A and C),
+// used[g] of them (both int32, on the device; `routed` at most in all groups together); B [num_groups][N][K].  act >= 0: B is
+// [num_groups][2 N][K] and C act(first half) * second half of the product's bf16 columns.
+SXB_API int sxb_gemm_grouped_few(const void* A, const void* B, void* C, int N, int K, long long lda, long long ldb, long long ldc,
+                                 int num_groups, const void* offsets, const void* used, long long total_rows, long long routed,
+                                 int act, void* stream) {
+  if (offsets == nullptr || used == nullptr || num_groups < 1 || num_groups > 65535 || total_rows <= 0 || act > ew::kSilu)
+    return SXB_ERR_BAD_ARG;
+  if (N <= 0 || K <= 0 || routed <= 0) return SXB_OK;
+  if ((lda % 8) || (ldb % 8) || (ldc % 8) || (act >= 0 && N % 8) || lda > INT_MAX || ldb > INT_MAX || ldc > INT_MAX ||
+      total_rows > INT_MAX || (long long)num_groups * N > INT_MAX / 2 ||
+      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15))
+    return SXB_ERR_UNSUPPORTED;
+  Params p{};
+  p.N = N; p.K = K; p.layout = NT; p.c_dtype = kBF16; p.direct = 1; p.C = C; p.ldc = (int)ldc; p.alpha = 1.f; p.act = act;
+  return (act >= 0 ? launch_skinny_groups<true> : launch_skinny_groups<false>)(
+      A, B, p, lda, ldb, num_groups, (const int*)offsets, (const int*)used, total_rows, routed, reinterpret_cast<cudaStream_t>(stream));
+}
+
+// C[M, F] = act(A B_0^T) * (A B_1^T) with B [2 F, K] the two halves one after the other and both products rounded to bf16, as the
+// product and the activation's kernel would give it, in one launch; SXB_ERR_UNSUPPORTED where the product has too many rows for it.
+SXB_API int sxb_gemm_gated(const void* A, const void* B, void* C, int M, int F, int K, int lda, int ldb, int ldc, int act,
+                           void* stream) {
+  if (M <= 0 || F <= 0 || K <= 0) return SXB_OK;
+  if (act < 0 || act > ew::kSilu) return SXB_ERR_BAD_ARG;
+  if (F > INT_MAX / 2 || (lda % 8) || (ldb % 8) || (ldc % 8) || (F % 8) || g_gemm_mode != 0 || !use_skinny(M, 2 * F, K) ||
+      ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(C)) & 15))
+    return SXB_ERR_UNSUPPORTED;
+  Params p{};
+  p.M = M; p.N = F; p.K = K; p.layout = NT; p.c_dtype = kBF16; p.direct = 1; p.C = C; p.ldc = ldc; p.alpha = 1.f; p.act = act;
+  return (chained() ? launch_skinny<true, true> : launch_skinny<false, true>)(A, B, p, lda, ldb, reinterpret_cast<cudaStream_t>(stream));
 }

@@ -1,6 +1,7 @@
 // ragged_llama.cu — one forward of a dense Llama over a ragged batch, its kernels issued from here.
 //
-// The kernels are those of the operators' own entry points, in the same order and on the same operands: this entry only takes the
+// The kernels are those of the operators' own entry points, in the same order and on the same operands (a product of few rows takes
+// its activation along, with the same bits): this entry only takes the
 // way from one launch to the next out of Python, which a decode step of a few requests spends its time on (4 layers of 2048, 4
 // requests, prompts and six decode steps: 5.53 ms from Python, 2.88 this way, 2.4 of device work).  Nothing is kept between calls.
 // The launches form a chain (sxb_common.cuh): a kernel comes onto the SMs while the one before it still runs, so that its launch, its
@@ -43,8 +44,12 @@ SXB_API int sxb_ragged_llama_forward(const struct sxb_ragged_llama* m, const str
                                       (int)m->block_size, T, Hq, Hk, D, C, Q, scale, stream))) return rc;
     if ((rc = product(m->ctx, l.wo, l.ld_o, h, T, H, Q))) return rc;
     if ((rc = norm(l.ln2))) return rc;
-    if ((rc = product(m->x, l.w_gate_up, l.ld_gate_up, m->gate_up, T, 2 * F, H))) return rc;
-    if ((rc = sxb_gated_act_fwd(m->gate_up, nullptr, m->act, T, F, 3, kBF16, stream))) return rc;
+    rc = sxb_gemm_gated(m->x, l.w_gate_up, m->act, T, F, H, H, (int)l.ld_gate_up, F, 3, stream);
+    if (rc == SXB_ERR_UNSUPPORTED) {      // many rows: the product and its activation one after the other, the same bits
+      if ((rc = product(m->x, l.w_gate_up, l.ld_gate_up, m->gate_up, T, 2 * F, H))) return rc;
+      rc = sxb_gated_act_fwd(m->gate_up, nullptr, m->act, T, F, 3, kBF16, stream);
+    }
+    if (rc) return rc;
     if ((rc = product(m->act, l.w_down, l.ld_down, h, T, H, F))) return rc;
   }
   if ((rc = norm(m->norm))) return rc;

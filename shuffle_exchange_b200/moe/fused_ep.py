@@ -255,7 +255,7 @@ def grouped_experts_inference(x, scores, assign, offsets, counts, w1, w2, activa
     and return their input: their row groups skip both products and are copied from the receive to the return buffer.
     Replaces the per-expert loop over
     ``cumsum.tolist()`` (reference: ``inference/v2/kernels/cutlass_ops/moe_gemm``)."""
-    from ..ops.gemm_ext import grouped_gemm_nt_used
+    from ..ops.gemm_ext import grouped_gated_nt_few, grouped_gemm_nt_used
     T, H = x.shape
     E = w1.shape[0]
     ep = FusedEP.get(None, H, E + n_identity, T, top_k, 1.0)
@@ -263,16 +263,20 @@ def grouped_experts_inference(x, scores, assign, offsets, counts, w1, w2, activa
     wts = scores.to(torch.float32).contiguous()
     ep.push(x.contiguous(), plan, weights=wts if weight_input else None, zero_pad=False)
     counts = counts.contiguous()
-    h = grouped_gemm_nt_used(ep.recv_rows, w1, plan.group_offsets, counts)
-    if gate_act is not None and h.shape[1] % 16 == 0:
+    h = None
+    if gate_act is not None:
         from ..ops.functional import _act_code
-        a = h.new_empty((h.shape[0], h.shape[1] // 2))
-        _n.call("sxb_gated_act_groups", h.data_ptr(), a.data_ptr(), plan.group_offsets.data_ptr(), counts.data_ptr(), E,
-                T * top_k, a.shape[1], _act_code(gate_act), _n.dtype_code(h.dtype), _n.stream_ptr())
-        h = a
-    else:
-        h = activation(h)
-    grouped_gemm_nt_used(h, w2, plan.group_offsets, counts, out=ep.ret_rows)
+        h = grouped_gated_nt_few(ep.recv_rows, w1, plan.group_offsets, counts, _act_code(gate_act), T * top_k)
+    if h is None:
+        h = grouped_gemm_nt_used(ep.recv_rows, w1, plan.group_offsets, counts, routed=T * top_k)
+        if gate_act is not None and h.shape[1] % 16 == 0:
+            a = h.new_empty((h.shape[0], h.shape[1] // 2))
+            _n.call("sxb_gated_act_groups", h.data_ptr(), a.data_ptr(), plan.group_offsets.data_ptr(), counts.data_ptr(), E,
+                    T * top_k, a.shape[1], _act_code(gate_act), _n.dtype_code(h.dtype), _n.stream_ptr())
+            h = a
+        else:
+            h = activation(h)
+    grouped_gemm_nt_used(h, w2, plan.group_offsets, counts, out=ep.ret_rows, routed=T * top_k)
     if n_identity > 0:
         from ..ops.moe_ops import copy_group_rows_
         copy_group_rows_(ep.ret_rows, ep.recv_rows, plan.group_offsets, E, E + n_identity)

@@ -28,6 +28,8 @@ GROUP_ALIGN_K = 64
 _n.register({
     "sxb_gemm_ext": "ppp" "iiii" "lll" "iii" "f" "pilll" "iipll" "pp" "i" "p",
     "sxb_gemm_grouped_used": "ppp" "ii" "lll" "ipp" "l" "p",
+    "sxb_gemm_grouped_few": "ppp" "ii" "lll" "ipp" "ll" "i" "p",
+    "sxb_gemm_gated": "ppp" "iiiiiii" "p",
     "sxb_gemmx_hang_info": "p",
     "sxb_stream_write_u32": "pip",
     "sxb_fp8_rowwise_quant": "ppp" "li" "ll" "p",
@@ -170,16 +172,39 @@ def grouped_gemm_nt(x, w, offsets, out=None, scale_x=None, qw=None, scale_w=None
     return out
 
 
-def grouped_gemm_nt_used(x, w, offsets, counts, out=None):
+FEW_ROWS = 64           # average rows of a group up to which grouped_gemm_nt_used takes the kernel for few rows
+
+
+def grouped_gemm_nt_used(x, w, offsets, counts, out=None, routed: Optional[int] = None):
     """:func:`grouped_gemm_nt` in bf16 for groups that use only their first ``counts[g]`` rows (int32, device): the rows of
-    padding behind them are neither read nor defined in the result."""
+    padding behind them are neither read nor defined in the result.  ``routed``: how many rows all groups use together, at
+    most.  Up to 64 a group (on average) the product runs with the weights as the MMA's rows and as many columns as there are
+    tokens; the kernel with tiles of 256 rows multiplies padding until the chip reaches its power limit (both products of 8 experts of
+    4096 x 14336, one call after the other, us: 2 tokens 261 | 181, 16 tokens 681 | 450, 200 tokens 663 | 484, 400 tokens 685 | 567; 16 experts of
+    1024 x 4096, 200 tokens 106 | 92, 1000 tokens 113 | 130)."""
     G, N, K = w.shape
     if out is None:
         out = torch.empty((x.shape[0], N), dtype=torch.bfloat16, device=x.device)
     if not x.is_cuda or K == 0 or out.dtype != torch.bfloat16 or out.stride(0) % 8 or out.data_ptr() % 16:
         return grouped_gemm_nt(x, w, offsets, out=out)       # the stores of single elements stay there
+    if routed is not None and routed <= FEW_ROWS * G:
+        _n.call("sxb_gemm_grouped_few", x.data_ptr(), w.data_ptr(), out.data_ptr(), N, K, x.stride(0), w.stride(1), out.stride(0), G,
+                offsets.data_ptr(), counts.data_ptr(), x.shape[0], routed, -1, _n.stream_ptr())
+        return out
     _n.call("sxb_gemm_grouped_used", x.data_ptr(), w.data_ptr(), out.data_ptr(), N, K, x.stride(0), w.stride(1), out.stride(0), G,
             offsets.data_ptr(), counts.data_ptr(), x.shape[0], _n.stream_ptr())
+    return out
+
+
+def grouped_gated_nt_few(x, w, offsets, counts, act: int, routed: int):
+    """``act(x w[g, :F]^T) * (x w[g, F:]^T)`` of the rows that the groups use, ``w`` ``[G, 2 F, K]``: the product and its gated
+    activation in one launch, with the bits of both in turn.  For up to :data:`FEW_ROWS` rows a group; None beyond."""
+    G, N, K = w.shape
+    if not x.is_cuda or K == 0 or N % 16 or routed > FEW_ROWS * G:
+        return None
+    out = torch.empty((x.shape[0], N // 2), dtype=torch.bfloat16, device=x.device)
+    _n.call("sxb_gemm_grouped_few", x.data_ptr(), w.data_ptr(), out.data_ptr(), N // 2, K, x.stride(0), w.stride(1), out.stride(0), G,
+            offsets.data_ptr(), counts.data_ptr(), x.shape[0], routed, act, _n.stream_ptr())
     return out
 
 
