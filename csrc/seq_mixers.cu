@@ -24,6 +24,7 @@
 //   sigmoid_gate_rows, power_norm_act   sigmoid gate per channel or per head in place; p1 z/rms(z) + p2 z^2/rms(z^2) + p3 z^3/rms(z^3) + p0
 #include <algorithm>
 #include <type_traits>
+#include "mma_sync.cuh"
 #include "seq_common.cuh"
 #include <cuda_pipeline.h>
 
@@ -544,6 +545,7 @@ sink_attention_tile_kernel(const float* __restrict__ q, const T* __restrict__ kc
 }
 
 #include "sink_attention_mma.cuh"
+#include "sink_attention_decode.cuh"
 
 // One CTA of kAW warps per (token, key/value head): single decode tokens and short portions.  Keys lo..pos of the token's
 // sequence, lo = start of the token's chunk (chunk > 0) or 0; the warps take 32-key tiles in turn (a lane scores one
@@ -788,6 +790,17 @@ static int attention_rows(int dtype, dim3 grid, const void* q, const void* kcach
                                    float out_scale, cudaStream_t s) {
   const int group = Hq / G;
   int rc = SXB_OK;
+  if (sink_decode_takes(q, kcache, vcache, grid.x, Hq, G, d, dv, kpitch, vpitch, dtype)) {
+    SinkDecodeParams p{};
+    p.q = (const float*)q; p.sink = (const float*)sink; p.dist_bias = (const float*)dist_bias;
+    p.kcache = (const __nv_bfloat16*)kcache; p.vcache = (const __nv_bfloat16*)vcache; p.gate = (const __nv_bfloat16*)gate;
+    p.out = (__nv_bfloat16*)out;
+    p.tok_seq = (const int*)tok_seq; p.tok_pos = (const int*)tok_pos; p.atoms = atoms; p.tables = (const int*)tables;
+    p.max_blocks = max_blocks; p.block_size = block_size; p.Hq = Hq; p.G = G;
+    p.chunk = chunk; p.window = window; p.kpitch = kpitch; p.vpitch = vpitch; p.bias_len = bias_len; p.gate_heads = gate_heads;
+    p.scale = scale; p.out_scale = out_scale; p.gate_ld = gate_ld; p.out_ld = out_ld;
+    return d == 128 ? launch_sink_decode<128>(p, grid.x, s) : launch_sink_decode<64>(p, grid.x, s);
+  }
   // (Taking fewer heads together when a decode batch leaves SMs idle was measured slower: every CTA walks all keys.)
   const int rep = group % 8 == 0 ? 8 : (group % 4 == 0 ? 4 : (group % 2 == 0 ? 2 : 1));
 #define ROWS(REP)                                                                                                      \
