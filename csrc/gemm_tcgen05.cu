@@ -17,6 +17,7 @@
 // (reference: deepspeed/inference/v2/kernels/core_ops/blas_kernels/blas_utils.h:31-41,
 // and every nn.Linear in the training path).
 #include <algorithm>
+#include <atomic>
 #include <climits>
 
 #include "activation.cuh"
@@ -607,6 +608,7 @@ done:
 }
 
 #include "gemm_skinny.cuh"
+#include "gemm_split.cuh"
 
 // ------------------------------------------------------------------ host side
 // 2-D bf16 tensor map over a row-major [rows, cols] matrix with row pitch `ld` elements;
@@ -733,6 +735,75 @@ static int launch_skinny(const void* A, const void* B, const Params& p, int lda,
   return launch_skinny<128, 3, CHAIN, GATED>(A, B, p, lda, ldb, stream);
 }
 
+template <int BN>
+static int launch_split(const CUtensorMap& ta, const CUtensorMap& tb, const Params& p, int S, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_split_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitPlan<BN>::kTotal);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * S);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = SplitPlan<BN>::kTotal;
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_split_kernel<BN>, ta, tb, p, S);
+  if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
+  return SXB_OK;
+}
+
+// Clusters of S CTAs of the split kernel that the device holds at once (an SM each; GPCs that S does not divide leave some idle).
+static int split_clusters(int S) {
+  static std::atomic<int> known[9];
+  int n = known[S].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(S);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = SplitPlan<256>::kTotal;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(gemm_split_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitPlan<256>::kTotal) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, gemm_split_kernel<256>, &cfg) != cudaSuccess || n < 1) {
+      (void)cudaGetLastError();
+      n = -1;
+    }
+    known[S].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+// CTAs that share a tile of 128 x 256 (1: the persistent kernels).  Both are priced in ns and the split is taken where it saves a tenth: a block of
+// K costs a tile 335 (a 256 x 256 tile of a pair 300), a launch of the persistent kernels 4 us beside that, one of clusters 8.5 and 0.8 per
+// CTA that takes part in the sum.  us, measured without | with: gradients of 64 / 200 / 300 / 500 rows through 4096 -> 28672 155 | 52, 156 | 61, 156 | 90,
+// 157 | 98; of 200 rows through 4096 -> 128256 671 | 236, 2048 -> 32000 168 | 56, 768 -> 32000 146 | 33; 200 rows through 2048 -> 3072 19.0 | 15.8.
+// Not taken: 200 rows through 2048 -> 2048 14.4 | 14.7, 662 through 4096 -> 28672 (48 tiles of pairs) 137 | 160.
+static int split_of(int M, int N, int K) {
+  const long long tiles = (long long)((M + BM - 1) / BM) * ((N + 255) / 256), kb = (K + BK - 1) / BK, sms = num_sms();
+  if (tiles >= sms || N <= 128 || kb < 32) return 1;
+  const long long pairs = (long long)((M + 255) / 256) * ((N + 255) / 256);
+  const bool pair = M >= 512 && N >= 512 && pairs >= 37;
+  const long long whole = pair ? (pairs + sms / 2 - 1) / (sms / 2) * kb * 300 + 5000 : kb * 335 + 4000;
+  long long best = whole * 9 / 10;
+  int S = 1;
+  for (int s : {2, 3, 4, 8}) {
+    const int n = split_clusters(s);
+    if (n < 1 || kb < 2 * s) continue;
+    const long long cost = (tiles + n - 1) / n * ((kb + s - 1) / s * 335 + 8500 + 800 * s);
+    if (cost < best) best = cost, S = s;
+  }
+  return S;
+}
+
 template <bool GATED>
 static int launch_skinny_groups(const void* A, const void* B, const Params& p, long long lda, long long ldb, int groups,
                                 const int* offsets, const int* used, long long total_rows, long long routed, cudaStream_t stream) {
@@ -815,6 +886,17 @@ SXB_API int sxb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
   const int BNsel = (N > 128) ? 256 : 128;
   CUtensorMap ta, tb, tc;
   int rc;
+  const int S = g_gemm_mode == 0 && max_ctas <= 0 ? split_of(M, N, K) : 1;
+  if (S > 1) {
+    if (layout == TN) rc = make_map_2d(&ta, A, K, M, lda, BK, 64);
+    else rc = make_map_2d(&ta, A, M, K, lda, BM, BK);
+    if (rc) return rc;
+    if (layout == NT) rc = make_map_2d(&tb, B, N, K, ldb, BNsel, BK);
+    else rc = make_map_2d(&tb, B, K, N, ldb, BK, 64);
+    if (rc) return rc;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    return launch_split<256>(ta, tb, p, S, s);
+  }
   const bool big = (M >= 512 && N >= 512 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= 37);
   if (g_gemm_mode == 2 || (g_gemm_mode == 0 && big)) {
     if (layout == TN) rc = make_map_2d(&ta, A, K, M, lda, BK, 64);
