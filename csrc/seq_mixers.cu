@@ -2030,55 +2030,54 @@ row_gate_add_vec_kernel(T* __restrict__ acc, const T* __restrict__ y, const floa
 }
 
 // Router product in 32-bit: logits[t, r] = bias[r] + sum_c x[t, c] * w[r, c] with x in the activation type (its values
-// taken as they are: no 32-bit copy of the rows is made) and w, bias, logits fp32.  CTAs of eight warps; WPT warps share
-// the columns of one token (prompt batches: one warp per token, eight tokens per CTA, the weights of the few router
-// rows are re-read from L1 by the other warps; few rows: the eight warps of a CTA split one token's columns and add
-// their parts in shared memory).  A lane takes 4 consecutive columns at a time.
+// taken as they are: no 32-bit copy of the rows is made) and w, bias, logits fp32.  A CTA takes 32 / RR tokens, its eight warps split
+// the columns and a lane takes 4 consecutive ones at a time, so that a loaded word of w serves all of the CTA's tokens.  The 32 sums
+// of a warp meet in 31 shuffles, each round halving what a lane carries, and lane i ends up with token i / RR, row i % RR.
+// What bounds it: the latency of its few rounds of loads.  us, one token per CTA, or per warp from 1024 tokens on, before | now: 1 token of 4096
+// columns, 8 rows 7.2 | 3.5; 200 7.9 | 4.0; 700 13.6 | 6.3; 1500 of 2048 21.8 | 6.2; 2048 of 4096 41.7 | 11.0; 2000 of 1024, 16 rows 18.8 | 10.1.
 constexpr int kRouterRows = 16;
 
-template <typename T, int WPT>
+template <typename T, int RR>
 __global__ void __launch_bounds__(256)
 router_logits_kernel(const T* __restrict__ x, long long ld, const float* __restrict__ w, const float* __restrict__ bias,
                      float* __restrict__ out, int n_tokens, int width, int R) {
-  __shared__ float part_sum[8][kRouterRows];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int part = warp % WPT;
-  const int t = blockIdx.x * (8 / WPT) + warp / WPT;
-  const bool active = t < n_tokens;
-  float acc[kRouterRows];
+  constexpr int TT = 32 / RR;
+  __shared__ float part_sum[8][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, t0 = blockIdx.x * TT;
+  float acc[32];
 #pragma unroll
-  for (int r = 0; r < kRouterRows; ++r) acc[r] = 0.f;
-  if (active) {
-    const T* row = x + (long long)t * ld;
-    for (int c = (part * 32 + lane) * 4; c < width; c += 128 * WPT) {
-      float xv[4];
-      load_pack<T, 4>(row + c, xv, true, 4);
+  for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+#pragma unroll 2
+  for (int c = threadIdx.x * 4; c < width; c += 1024) {
+    float xv[TT][4];
 #pragma unroll
-      for (int r = 0; r < kRouterRows; ++r) {
-        if (r < R) {
-          const float4 wv = *reinterpret_cast<const float4*>(w + (long long)r * width + c);
-          acc[r] += (xv[0] * wv.x + xv[1] * wv.y) + (xv[2] * wv.z + xv[3] * wv.w);
-        }
-      }
+    for (int t = 0; t < TT; ++t) load_pack<T, 4>(x + (long long)min(t0 + t, n_tokens - 1) * ld + c, xv[t], true, 4);
+#pragma unroll
+    for (int r = 0; r < RR; ++r) {
+      const float4 wv = *reinterpret_cast<const float4*>(w + (long long)min(r, R - 1) * width + c);
+#pragma unroll
+      for (int t = 0; t < TT; ++t)
+        acc[t * RR + r] += (xv[t][0] * wv.x + xv[t][1] * wv.y) + (xv[t][2] * wv.z + xv[t][3] * wv.w);
     }
   }
 #pragma unroll
-  for (int r = 0; r < kRouterRows; ++r) {
-    if (r < R) {
-      const float v = warp_sum(acc[r]);
-      if (WPT == 1) {
-        if (active && lane == 0) out[(long long)t * R + r] = v + (bias ? bias[r] : 0.f);
-      } else if (lane == 0) {
-        part_sum[warp][r] = v;
-      }
+  for (int b = 1, n = 16; n > 0; b <<= 1, n >>= 1) {
+    const bool up = lane & b;
+#pragma unroll
+    for (int i = 0; i < n; ++i) {
+      const float lo = acc[2 * i], hi = acc[2 * i + 1];
+      acc[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, b);
     }
   }
-  if (WPT > 1) {
-    __syncthreads();
-    if (active && part == 0 && lane < R) {
-      float v = bias ? bias[lane] : 0.f;
-      for (int p = 0; p < WPT; ++p) v += part_sum[warp + p][lane];
-      out[(long long)t * R + lane] = v;
+  part_sum[warp][lane] = acc[0];
+  __syncthreads();
+  if (warp == 0) {
+    const int t = t0 + lane / RR, r = lane % RR;
+    if (t < n_tokens && r < R) {
+      float v = bias ? bias[r] : 0.f;
+#pragma unroll
+      for (int p = 0; p < 8; ++p) v += part_sum[p][lane];
+      out[(long long)t * R + r] = v;
     }
   }
 }
@@ -2556,13 +2555,12 @@ SXB_API int sxb_router_logits(const void* x, long long ld, const void* w, const 
   if (R > kRouterRows || width % 4 || ld % 4 ||
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) != 0)
     return SXB_ERR_UNSUPPORTED;
-  if (n_tokens >= 1024) {
-    SEQMIX_DISPATCH(dtype, (router_logits_kernel<T, 1><<<(n_tokens + 7) / 8, 256, 0, (cudaStream_t)stream>>>(
-                               (const T*)x, ld, (const float*)w, (const float*)bias, (float*)out, n_tokens, width, R)));
-  } else {
-    SEQMIX_DISPATCH(dtype, (router_logits_kernel<T, 8><<<n_tokens, 256, 0, (cudaStream_t)stream>>>(
-                               (const T*)x, ld, (const float*)w, (const float*)bias, (float*)out, n_tokens, width, R)));
-  }
+#define ROUTER(RR)                                                                                                             \
+  SEQMIX_DISPATCH(dtype, (router_logits_kernel<T, RR><<<(n_tokens + 32 / RR - 1) / (32 / RR), 256, 0, (cudaStream_t)stream>>>( \
+                             (const T*)x, ld, (const float*)w, (const float*)bias, (float*)out, n_tokens, width, R)))
+  if (R <= 8) ROUTER(8);
+  else ROUTER(16);
+#undef ROUTER
   SXB_CHECK_LAUNCH();
   return SXB_OK;
 }
