@@ -464,6 +464,52 @@ SXB_API int sxb_bias_act_bwd(const void* dy, const void* x, const void* bias, vo
   return SXB_OK;
 }
 
+// The ends of a mean cross entropy, one CTA each: inv[0] = 1 / max(1, labels that count), out[0] = inv[0] * sum of the rows' losses
+// (summed in 64 bits).  They take the place of eleven launches of elementwise kernels and reductions around the loss kernel.
+namespace sxb {
+namespace ew {
+template <typename V>
+__device__ __forceinline__ V block_total(V v) {
+  __shared__ V part[32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = threadIdx.x < blockDim.x / 32 ? part[threadIdx.x] : V(0);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;                              // on the first warp
+}
+__global__ void __launch_bounds__(1024)
+label_weight_kernel(const long long* __restrict__ labels, long long rows, long long ignore, float* __restrict__ inv) {
+  long long n = 0;
+#pragma unroll 4
+  for (long long i = threadIdx.x; i < rows; i += 1024) n += labels[i] != ignore;
+  n = block_total(n);
+  if (threadIdx.x == 0) inv[0] = 1.f / (float)(n > 1 ? n : 1);
+}
+__global__ void __launch_bounds__(1024)
+mean_loss_kernel(const float* __restrict__ loss, long long rows, const float* __restrict__ inv, float* __restrict__ out) {
+  double a = 0.0;
+#pragma unroll 4
+  for (long long i = threadIdx.x; i < rows; i += 1024) a += loss[i];
+  a = block_total(a);
+  if (threadIdx.x == 0) out[0] = (float)a * inv[0];
+}
+}  // namespace ew
+}  // namespace sxb
+
+SXB_API int sxb_label_weight(const void* labels, long long rows, long long ignore_index, void* inv, void* stream) {
+  label_weight_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>((const long long*)labels, rows, ignore_index, (float*)inv);
+  SXB_CHECK_LAUNCH();
+  return SXB_OK;
+}
+SXB_API int sxb_mean_loss(const void* loss, long long rows, const void* inv, void* out, void* stream) {
+  mean_loss_kernel<<<1, 1024, 0, (cudaStream_t)stream>>>((const float*)loss, rows, (const float*)inv, (float*)out);
+  SXB_CHECK_LAUNCH();
+  return SXB_OK;
+}
+
 // logits [rows, V] (row pitch ld) are overwritten with the gradient when write_grad != 0.
 SXB_API int sxb_cross_entropy(void* logits, const void* labels, void* loss, void* lse,
                               long long rows, int V, long long ld, long long ignore_index,

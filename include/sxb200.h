@@ -105,6 +105,9 @@ int sxb_bias_act_bwd(const void* dy, const void* x, const void* bias, void* dx, 
                      int dtype, void* stream);
 int sxb_cross_entropy(void* logits, const void* labels, void* loss, void* lse, long long rows, int V, long long ld,
                       long long ignore_index, const void* grad_scale, int write_grad, int dtype, void* stream);
+/* inv fp32 [1] = 1 / max(1, labels (int64) other than ignore_index); out fp32 [1] = inv * sum of loss fp32 [rows]. */
+int sxb_label_weight(const void* labels, long long rows, long long ignore_index, void* inv, void* stream);
+int sxb_mean_loss(const void* loss, long long rows, const void* inv, void* out, void* stream);
 int sxb_embedding_fwd(const void* ids, const void* table, void* out, long long ntok, int H, int dtype, void* stream);
 int sxb_embedding_bwd(const void* ids, const void* dout, void* dtable, long long ntok, int H, int dtype, void* stream);
 int sxb_scale_cast(const void* src, void* dst, long long n, int src_dtype, int dst_dtype, float scale,

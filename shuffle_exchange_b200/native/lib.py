@@ -64,6 +64,8 @@ SIGNATURES = {
     "sxb_bias_act": "ppp" "l" "iii" "p",
     "sxb_bias_act_bwd": "pppp" "l" "iii" "p",
     "sxb_cross_entropy": "pppp" "l" "i" "l" "l" "p" "ii" "p",
+    "sxb_label_weight": "p" "ll" "pp",
+    "sxb_mean_loss": "p" "l" "ppp",
     "sxb_scale_by": "p" "l" "p" "i" "p",
     "sxb_embedding_fwd": "ppp" "l" "ii" "p",
     "sxb_embedding_bwd": "ppp" "l" "ii" "p",

@@ -585,14 +585,16 @@ class _CrossEntropy(torch.autograd.Function):
         lab = labels.reshape(-1)
         rows = l2.shape[0]
         loss_rows = torch.empty(rows, dtype=torch.float32, device=logits.device)
-        nvalid = (lab != ignore_index).sum().clamp_(min=1).to(torch.float32)
-        inv = (1.0 / nvalid).reshape(1)
+        inv = torch.empty(1, dtype=torch.float32, device=logits.device)
+        _n.call("sxb_label_weight", lab.data_ptr(), rows, int(ignore_index), inv.data_ptr(), _n.stream_ptr())
         # gradient is written in place of the logits (saves a [T, V] buffer)
         _n.call("sxb_cross_entropy", l2.data_ptr(), lab.data_ptr(), loss_rows.data_ptr(), None, rows, V,
                 l2.stride(0), int(ignore_index), inv.data_ptr(), 1, _n.dtype_code(l2.dtype), _n.stream_ptr())
         ctx.save_for_backward(l2)
         ctx.shape = logits.shape
-        return loss_rows.sum() * inv[0]
+        loss = torch.empty((), dtype=torch.float32, device=logits.device)
+        _n.call("sxb_mean_loss", loss_rows.data_ptr(), rows, inv.data_ptr(), loss.data_ptr(), _n.stream_ptr())
+        return loss
 
     @staticmethod
     def backward(ctx, dloss):
@@ -609,6 +611,8 @@ class _CrossEntropy(torch.autograd.Function):
 def cross_entropy(logits: torch.Tensor, labels: torch.Tensor, ignore_index: int = -100) -> torch.Tensor:
     """Mean token cross entropy.  On CUDA the logits buffer is consumed (overwritten by dlogits)."""
     if logits.is_cuda and logits.dtype in (torch.bfloat16, torch.float16) and logits.shape[-1] % 8 == 0:
+        if labels.dtype != torch.int64 or labels.device != logits.device:
+            labels = labels.to(logits.device, torch.int64)
         return _CrossEntropy.apply(logits.contiguous(), labels.contiguous(), ignore_index)
     if logits.is_cuda:
         raise _n.NativeError("sxb cross_entropy expects bf16/fp16 logits with V % 8 == 0")
