@@ -782,18 +782,33 @@ static int split_clusters(int S) {
   return n;
 }
 
-// CTAs that share a tile of 128 x 256 (1: the persistent kernels).  Both are priced in ns and the split is taken where it saves a tenth: a block of
-// K costs a tile 335 (a 256 x 256 tile of a pair 300), a launch of the persistent kernels 4 us beside that, one of clusters 8.5 and 0.8 per
-// CTA that takes part in the sum.  us, measured without | with: gradients of 64 / 200 / 300 / 500 rows through 4096 -> 28672 155 | 52, 156 | 61, 156 | 90,
-// 157 | 98; of 200 rows through 4096 -> 128256 671 | 236, 2048 -> 32000 168 | 56, 768 -> 32000 146 | 33; 200 rows through 2048 -> 3072 19.0 | 15.8.
-// Not taken: 200 rows through 2048 -> 2048 14.4 | 14.7, 662 through 4096 -> 28672 (48 tiles of pairs) 137 | 160.
+// What a product costs the persistent kernels, in ns: a block of K takes 335 for a CTA's tile of 128 x 256, 300 for a pair's of 256 x 256,
+// and a launch 4 or 5 us beside its waves of tiles.
+static long long price_single(long long M, long long N, long long kb) {
+  const long long tiles = (M + 127) / 128 * ((N + 255) / 256), sms = num_sms();
+  return (tiles + sms - 1) / sms * kb * 335 + 4000;
+}
+static long long price_pair(long long M, long long N, long long kb) {
+  const long long tiles = (M + 255) / 256 * ((N + 255) / 256), pairs = num_sms() / 2;
+  return (tiles + pairs - 1) / pairs * kb * 300 + 5000;
+}
+// Whether pairs of CTAs take a product: from 512 rows on wherever they have half of their tiles or more, below where the prices differ by 4 % (us, weights from HBM, single
+// CTAs | pairs: 200 rows, 4096 -> 12288 32.7 | 28.0, 28672 61.4 | 55.1, 32000 63.2 | 57.0; 400, 2048 -> 16384 31.2 | 27.6, 4096 -> 12288 54.6 | 46.1;
+// 300, 4096 -> 12288, where three tiles of 128 rows meet one wave and two of 256 rows two, 34.6 | 47).
+static bool use_pair(int M, int N, int K) {
+  if (N < 512 || M <= 128) return false;
+  const long long kb = (K + BK - 1) / BK, tiles = (long long)((M + 255) / 256) * ((N + 255) / 256);
+  return tiles >= 37 && (M >= 512 || 100 * price_pair(M, N, kb) < 96 * price_single(M, N, kb));
+}
+
+// CTAs that share a tile of 128 x 256 (1: the persistent kernels).  The split is taken where it saves a tenth: its launch costs 8.5 us and
+// 0.8 per CTA that takes part in the sum.  us, measured without | with: gradients of 64 / 200 / 300 / 500 rows through 4096 -> 28672 155 | 52,
+// 156 | 61, 156 | 90, 157 | 98; of 200 rows through 4096 -> 128256 671 | 236, 2048 -> 32000 168 | 56, 768 -> 32000 146 | 33; 200 rows through
+// 2048 -> 3072 19.0 | 15.8.  Not taken: 200 rows through 2048 -> 2048 14.4 | 14.7, 662 through 4096 -> 28672 (48 tiles of pairs) 137 | 160.
 static int split_of(int M, int N, int K) {
-  const long long tiles = (long long)((M + BM - 1) / BM) * ((N + 255) / 256), kb = (K + BK - 1) / BK, sms = num_sms();
-  if (tiles >= sms || N <= 128 || kb < 32) return 1;
-  const long long pairs = (long long)((M + 255) / 256) * ((N + 255) / 256);
-  const bool pair = M >= 512 && N >= 512 && pairs >= 37;
-  const long long whole = pair ? (pairs + sms / 2 - 1) / (sms / 2) * kb * 300 + 5000 : kb * 335 + 4000;
-  long long best = whole * 9 / 10;
+  const long long tiles = (long long)((M + BM - 1) / BM) * ((N + 255) / 256), kb = (K + BK - 1) / BK;
+  if (tiles >= num_sms() || N <= 128 || kb < 32) return 1;
+  long long best = (use_pair(M, N, K) ? price_pair(M, N, kb) : price_single(M, N, kb)) * 9 / 10;
   int S = 1;
   for (int s : {2, 3, 4, 8}) {
     const int n = split_clusters(s);
@@ -897,8 +912,7 @@ SXB_API int sxb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
     return launch_split<256>(ta, tb, p, S, s);
   }
-  const bool big = (M >= 512 && N >= 512 && (long long)((M + 255) / 256) * ((N + 255) / 256) >= 37);
-  if (g_gemm_mode == 2 || (g_gemm_mode == 0 && big)) {
+  if (g_gemm_mode == 2 || (g_gemm_mode == 0 && use_pair(M, N, K))) {
     if (layout == TN) rc = make_map_2d(&ta, A, K, M, lda, BK, 64);
     else rc = make_map_2d(&ta, A, M, K, lda, 128, BK);
     if (rc) return rc;
