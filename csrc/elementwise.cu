@@ -71,6 +71,23 @@ rope_kernel(T* __restrict__ x, const long long* __restrict__ pos, const float* _
   }
 }
 
+// The vectors that a thread takes of rows of `per` vectors, grid after grid: row and column go on by additions (a 64-bit division per
+// vector was a third of the activation kernels' instructions).
+struct RowWalk {
+  long long at, row, step, drow;
+  int col, dcol, per;
+  __device__ __forceinline__ explicit RowWalk(int per_) : per(per_) {
+    at = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    step = (long long)gridDim.x * blockDim.x;
+    row = at / per, col = (int)(at - row * per);
+    drow = step / per, dcol = (int)(step - drow * per);
+  }
+  __device__ __forceinline__ void next() {
+    at += step, row += drow, col += dcol;
+    if (col >= per) col -= per, ++row;
+  }
+};
+
 // out[T,F] = act(in[:, :F] (+bias)) * (in[:, F:] (+bias))       (concatenated gate|up layout)
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
@@ -80,10 +97,9 @@ gated_fwd_kernel(const T* in, const T* __restrict__ bias, T* __restrict__ out,
   chain_wait();
   const int vpr = F >> 3;
   const long long total = rows * vpr;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / vpr;
-    const int c = (int)(i % vpr) * 8;
+  for (RowWalk i(vpr); i.at < total; i.next()) {
+    const long long r = i.row;
+    const int c = i.col * 8;
     float g[8], u[8], o[8];
     ld8<T>(in + r * 2 * F + c, g);
     ld8<T>(in + r * 2 * F + F + c, u);
@@ -95,7 +111,7 @@ gated_fwd_kernel(const T* in, const T* __restrict__ bias, T* __restrict__ out,
       for (int k = 0; k < 8; ++k) { g[k] += bg[k]; u[k] += bu[k]; }
     }
 #pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = act_fwd(g[k], act) * u[k];
+    for (int k = 0; k < 8; ++k) o[k] = act_fwd<sizeof(T) == 2>(g[k], act) * u[k];
     st8<T>(out + r * F + c, o);
   }
 }
@@ -136,7 +152,7 @@ gated_groups_kernel(const T* __restrict__ in, T* __restrict__ out, const int* __
     ld8<T>(in + r * 2 * F + c, g);
     ld8<T>(in + r * 2 * F + F + c, u);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) o[k] = act_fwd(g[k], act) * u[k];
+    for (int k = 0; k < 8; ++k) o[k] = act_fwd<sizeof(T) == 2>(g[k], act) * u[k];
     st8<T>(out + r * F + c, o);
   }
 }
@@ -146,18 +162,19 @@ gated_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ in, T* __restri
                  long long rows, int F, int act) {
   const int vpr = F >> 3;
   const long long total = rows * vpr;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / vpr;
-    const int c = (int)(i % vpr) * 8;
+  for (RowWalk i(vpr); i.at < total; i.next()) {
+    const long long r = i.row;
+    const int c = i.col * 8;
     float g[8], u[8], d[8], dg[8], du[8];
     ld8<T>(in + r * 2 * F + c, g);
     ld8<T>(in + r * 2 * F + F + c, u);
     ld8<T>(dy + r * F + c, d);
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      dg[k] = d[k] * u[k] * act_bwd(g[k], act);
-      du[k] = d[k] * act_fwd(g[k], act);
+      float f, b;
+      act_both<sizeof(T) == 2>(g[k], act, f, b);
+      dg[k] = d[k] * u[k] * b;
+      du[k] = d[k] * f;
     }
     st8<T>(din + r * 2 * F + c, dg);
     st8<T>(din + r * 2 * F + F + c, du);
@@ -170,10 +187,9 @@ bias_act_kernel(const T* __restrict__ x, const T* __restrict__ bias, T* __restri
                 long long rows, int C, int act) {
   const int vpr = C >> 3;
   const long long total = rows * vpr;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / vpr;
-    const int c = (int)(i % vpr) * 8;
+  for (RowWalk i(vpr); i.at < total; i.next()) {
+    const long long r = i.row;
+    const int c = i.col * 8;
     float v[8];
     ld8<T>(x + r * C + c, v);
     if (bias) {
@@ -183,7 +199,7 @@ bias_act_kernel(const T* __restrict__ x, const T* __restrict__ bias, T* __restri
       for (int k = 0; k < 8; ++k) v[k] += b[k];
     }
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = act_fwd(v[k], act);
+    for (int k = 0; k < 8; ++k) v[k] = act_fwd<sizeof(T) == 2>(v[k], act);
     st8<T>(y + r * C + c, v);
   }
 }
@@ -194,10 +210,9 @@ bias_act_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* 
                     T* __restrict__ dx, long long rows, int C, int act) {
   const int vpr = C >> 3;
   const long long total = rows * vpr;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const long long r = i / vpr;
-    const int c = (int)(i % vpr) * 8;
+  for (RowWalk i(vpr); i.at < total; i.next()) {
+    const long long r = i.row;
+    const int c = i.col * 8;
     float v[8], d[8];
     ld8<T>(x + r * C + c, v);
     ld8<T>(dy + r * C + c, d);
@@ -208,7 +223,11 @@ bias_act_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* 
       for (int k = 0; k < 8; ++k) v[k] += b[k];
     }
 #pragma unroll
-    for (int k = 0; k < 8; ++k) d[k] *= act_bwd(v[k], act);
+    for (int k = 0; k < 8; ++k) {
+      float f, b;
+      act_both<sizeof(T) == 2>(v[k], act, f, b);
+      d[k] *= b;
+    }
     st8<T>(dx + r * C + c, d);
   }
 }
