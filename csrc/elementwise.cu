@@ -32,45 +32,6 @@ __device__ __forceinline__ void st8(T* p, const float (&o)[8]) {
   *reinterpret_cast<uint4*>(p) = t;
 }
 
-// ----------------------------------------------------------------------- RoPE
-// x: [T, row_stride] with n_heads rotated heads of size D at the start of each row.
-// cos/sin: [max_pos, D/2] fp32.  sign = +1 forward, -1 backward (inverse rotation).
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-rope_kernel(T* __restrict__ x, const long long* __restrict__ pos, const float* __restrict__ cs,
-            const float* __restrict__ sn, long long Ttok, int n_heads, int D, long long row_stride,
-            float sign) {
-  const int half = D >> 1;
-  const int vec_per_head = half >> 3;  // 8 elements per thread-iteration
-  const long long total = Ttok * n_heads * vec_per_head;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int v = (int)(i % vec_per_head);
-    const long long th = i / vec_per_head;
-    const int h = (int)(th % n_heads);
-    const long long t = th / n_heads;
-    const long long p = pos ? pos[t] : t;
-    T* base = x + t * row_stride + (long long)h * D + v * 8;
-    float a[8], b[8], c[8], s[8];
-    ld8<T>(base, a);
-    ld8<T>(base + half, b);
-    const float4* cp = reinterpret_cast<const float4*>(cs + p * half + v * 8);
-    const float4* sp = reinterpret_cast<const float4*>(sn + p * half + v * 8);
-    float4 c0 = cp[0], c1 = cp[1], s0 = sp[0], s1 = sp[1];
-    c[0] = c0.x; c[1] = c0.y; c[2] = c0.z; c[3] = c0.w; c[4] = c1.x; c[5] = c1.y; c[6] = c1.z; c[7] = c1.w;
-    s[0] = s0.x; s[1] = s0.y; s[2] = s0.z; s[3] = s0.w; s[4] = s1.x; s[5] = s1.y; s[6] = s1.z; s[7] = s1.w;
-    float oa[8], ob[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float sk = sign * s[k];
-      oa[k] = a[k] * c[k] - b[k] * sk;
-      ob[k] = b[k] * c[k] + a[k] * sk;
-    }
-    st8<T>(base, oa);
-    st8<T>(base + half, ob);
-  }
-}
-
 // The vectors that a thread takes of rows of `per` vectors, grid after grid: row and column go on by additions (a 64-bit division per
 // vector was a third of the activation kernels' instructions).
 struct RowWalk {
@@ -87,6 +48,62 @@ struct RowWalk {
     if (col >= per) col -= per, ++row;
   }
 };
+
+// ----------------------------------------------------------------------- RoPE
+// x: [T, row_stride] with n_heads rotated heads of size D at the start of each row, `rest` columns behind them.
+// cos/sin: [max_pos, D/2] fp32.  sign = +1 forward, -1 backward (inverse rotation).
+// COPY: to y instead of in place, the other columns as they are (a gradient is not rotated in autograd's buffer: 13 us of copying
+// for 4096 rows of 6144, and a launch).
+template <typename T, bool COPY>
+__global__ void __launch_bounds__(kThreads)
+rope_kernel(T* x, T* y, const long long* __restrict__ pos, const float* __restrict__ cs,
+            const float* __restrict__ sn, long long Ttok, int n_heads, int D, long long row_stride, int rest,
+            float sign) {
+  const int half = D >> 1;
+  const int vec_per_head = half >> 3;  // 8 elements per thread-iteration
+  auto turn = [&](long long t, int h, int v) {
+    const long long p = pos ? pos[t] : t;
+    const long long at = t * row_stride + (long long)h * D + v * 8;
+    const T* base = x + at;
+    T* to = (COPY ? y : x) + at;
+    float a[8], b[8], c[8], s[8];
+    ld8<T>(base, a);
+    ld8<T>(base + half, b);
+    const float4* cp = reinterpret_cast<const float4*>(cs + p * half + v * 8);
+    const float4* sp = reinterpret_cast<const float4*>(sn + p * half + v * 8);
+    float4 c0 = cp[0], c1 = cp[1], s0 = sp[0], s1 = sp[1];
+    c[0] = c0.x; c[1] = c0.y; c[2] = c0.z; c[3] = c0.w; c[4] = c1.x; c[5] = c1.y; c[6] = c1.z; c[7] = c1.w;
+    s[0] = s0.x; s[1] = s0.y; s[2] = s0.z; s[3] = s0.w; s[4] = s1.x; s[5] = s1.y; s[6] = s1.z; s[7] = s1.w;
+    float oa[8], ob[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const float sk = sign * s[k];
+      oa[k] = a[k] * c[k] - b[k] * sk;
+      ob[k] = b[k] * c[k] + a[k] * sk;
+    }
+    st8<T>(to, oa);
+    st8<T>(to + half, ob);
+  };
+  if constexpr (COPY) {
+    const int turning = n_heads * vec_per_head, per = turning + rest / 16;
+    for (RowWalk i(per); i.at < Ttok * per; i.next()) {
+      if (i.col < turning) {
+        turn(i.row, i.col / vec_per_head, i.col % vec_per_head);
+      } else {
+        const long long at = i.row * row_stride + (long long)n_heads * D + (i.col - turning) * 16;
+        const uint4 a = *reinterpret_cast<const uint4*>(x + at), b = *reinterpret_cast<const uint4*>(x + at + 8);
+        *reinterpret_cast<uint4*>(y + at) = a;
+        *reinterpret_cast<uint4*>(y + at + 8) = b;
+      }
+    }
+  } else {
+    const long long total = Ttok * n_heads * vec_per_head;
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+      const long long th = i / vec_per_head;
+      turn(th / n_heads, (int)(th % n_heads), (int)(i % vec_per_head));
+    }
+  }
+}
 
 // out[T,F] = act(in[:, :F] (+bias)) * (in[:, F:] (+bias))       (concatenated gate|up layout)
 template <typename T>
@@ -420,10 +437,28 @@ SXB_API int sxb_rope(void* x, const void* positions, const void* cos_tab, const 
   if (head_dim % 16) return SXB_ERR_UNSUPPORTED;
   cudaStream_t s = (cudaStream_t)stream;
   const long long work = tokens * n_heads * (head_dim / 16);
-  DISPATCH_16(dtype, (rope_kernel<T><<<grid_for(work), kThreads, 0, s>>>(
-                         (T*)x, (const long long*)positions, (const float*)cos_tab,
-                         (const float*)sin_tab, tokens, n_heads, head_dim, row_stride,
+  DISPATCH_16(dtype, (rope_kernel<T, false><<<grid_for(work), kThreads, 0, s>>>(
+                         (T*)x, nullptr, (const long long*)positions, (const float*)cos_tab,
+                         (const float*)sin_tab, tokens, n_heads, head_dim, row_stride, 0,
                          inverse ? -1.f : 1.f)));
+  SXB_CHECK_LAUNCH();
+  return SXB_OK;
+}
+
+// y = x with its first n_heads heads rotated, rows of `cols` columns one behind the other; -2 where the columns behind the heads are no
+// multiple of 16.
+SXB_API int sxb_rope_copy(const void* x, void* y, const void* positions, const void* cos_tab, const void* sin_tab, long long tokens,
+                          int n_heads, int head_dim, int cols, int inverse, int dtype, void* stream) {
+  if (tokens <= 0) return SXB_OK;
+  const long long rest = cols - (long long)n_heads * head_dim;
+  if (head_dim % 16 || cols % 8 || rest < 0 || rest % 16 ||
+      ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15))
+    return SXB_ERR_UNSUPPORTED;
+  const long long work = tokens * (cols / 16);
+  cudaStream_t s = (cudaStream_t)stream;
+  DISPATCH_16(dtype, (rope_kernel<T, true><<<grid_for(work), kThreads, 0, s>>>(
+                         (T*)x, (T*)y, (const long long*)positions, (const float*)cos_tab, (const float*)sin_tab, tokens, n_heads,
+                         head_dim, cols, (int)rest, inverse ? -1.f : 1.f)));
   SXB_CHECK_LAUNCH();
   return SXB_OK;
 }

@@ -44,6 +44,7 @@ struct Lib {
                      void*);
   long long (*norm_bwd_scratch_elems)(long long, int, int);
   int (*rope)(void*, const void*, const void*, const void*, long long, int, int, long long, int, int, void*);
+  int (*rope_copy)(const void*, void*, const void*, const void*, const void*, long long, int, int, int, int, int, void*);
   int (*gated_act_fwd)(const void*, const void*, void*, long long, int, int, int, void*);
   int (*gated_act_bwd)(const void*, const void*, void*, long long, int, int, int, void*);
   int (*attn_fwd)(const void*, const void*, const void*, void*, void*, int, int, int, int, int, long long, long long, long long,
@@ -91,6 +92,8 @@ Tensor rows_of(const Tensor& t, int64_t width) {           // [rows, width], con
   Tensor r = t.dim() == 2 ? t : t.reshape({-1, width});
   return r.is_contiguous() ? r : r.contiguous();
 }
+
+bool aligned(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
 
 enum { kNT, kNN, kTN };
 void gemm(const Tensor& a, const Tensor& b, const Tensor& out, int64_t M, int64_t N, int64_t K, int layout) {
@@ -194,8 +197,19 @@ struct Rope : Function<Rope> {                 // in place
   }
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const Tensor dx = grads[0].clone(at::MemoryFormat::Contiguous);       // never rotate autograd's buffer in place
-    rope_kernel(dx, saved[0], saved[1], saved[2], ctx->saved_data["heads"].toInt(), ctx->saved_data["dim"].toInt(), 1);
+    const int64_t heads = ctx->saved_data["heads"].toInt(), dim = ctx->saved_data["dim"].toInt();
+    const Tensor& dy = grads[0];
+    const int64_t C = dy.size(-1);
+    // never rotate autograd's buffer in place
+    if (dy.is_contiguous() && dim % 16 == 0 && C % 8 == 0 && (C - heads * dim) % 16 == 0 && aligned(dy) && C < (int64_t(1) << 31)) {
+      Tensor dx = at::empty(dy.sizes(), dy.options());
+      check("rope_copy", g_lib.rope_copy(dy.data_ptr(), dx.data_ptr(), saved[0].defined() ? saved[0].data_ptr() : nullptr,
+                                         saved[1].data_ptr(), saved[2].data_ptr(), dy.numel() / C, (int)heads, (int)dim, (int)C, 1,
+                                         dtype_code(dy), stream()));
+      return {dx, Variable(), Variable(), Variable(), Variable(), Variable()};
+    }
+    const Tensor dx = dy.clone(at::MemoryFormat::Contiguous);
+    rope_kernel(dx, saved[0], saved[1], saved[2], heads, dim, 1);
     return {dx, Variable(), Variable(), Variable(), Variable(), Variable()};
   }
 };
@@ -293,7 +307,6 @@ bool marked(PyObject* o) {                     // carries the main-grad protocol
     if (PyDict_Contains(*d, m) != 0) return true;
   return false;
 }
-bool aligned(const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) == 0; }
 bool tape(const Tensor& a) { return a.requires_grad(); }
 
 constexpr int64_t kMost = int64_t(1) << 31;
@@ -424,6 +437,7 @@ PyObject* py_bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
   get(l.rmsnorm_bwd, "sxb_rmsnorm_bwd");
   get(l.norm_bwd_scratch_elems, "sxb_norm_bwd_scratch_elems");
   get(l.rope, "sxb_rope");
+  get(l.rope_copy, "sxb_rope_copy");
   get(l.gated_act_fwd, "sxb_gated_act_fwd");
   get(l.gated_act_bwd, "sxb_gated_act_bwd");
   get(l.attn_fwd, "sxb_attn_fwd");

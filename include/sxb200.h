@@ -98,6 +98,9 @@ int sxb_layernorm_bwd(const void* dy, const void* x, const void* w, const void* 
  *      ragged_ops/embed/embed_cuda.cu:19-90) */
 int sxb_rope(void* x, const void* positions, const void* cos_tab, const void* sin_tab, long long tokens,
              int n_heads, int head_dim, long long row_stride, int inverse, int dtype, void* stream);
+/* y [tokens, cols] = x with its first n_heads heads rotated; cols - n_heads * head_dim and head_dim multiples of 16 (else -2). */
+int sxb_rope_copy(const void* x, void* y, const void* positions, const void* cos_tab, const void* sin_tab, long long tokens,
+                  int n_heads, int head_dim, int cols, int inverse, int dtype, void* stream);
 int sxb_gated_act_fwd(const void* in, const void* bias, void* out, long long rows, int F, int act, int dtype, void* stream);
 int sxb_gated_act_bwd(const void* dy, const void* in, void* din, long long rows, int F, int act, int dtype, void* stream);
 int sxb_bias_act(const void* x, const void* bias, void* y, long long rows, int C, int act, int dtype, void* stream);

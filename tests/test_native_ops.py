@@ -19,7 +19,7 @@ def test_nothing_but_plain_gpu_tensors():
     assert F.linear(x, w).shape == (4, 16)
 
 
-OPS = ["linear", "norm", "norm_residual", "gated", "rope", "attention"]
+OPS = ["linear", "norm", "norm_residual", "gated", "rope", "rope_behind", "attention"]
 
 
 def _make(op, shape=(2, 37), grad=True):
@@ -34,9 +34,9 @@ def _make(op, shape=(2, 37), grad=True):
     if op == "gated":
         return [mk(*shape, 128)], lambda x: [F.gated_act(x, "silu")]
     cos, sin = F.rope_tables(64, 64, 10000.0, torch.device("cuda"))
-    if op == "rope":
+    if op.startswith("rope"):                        # behind the heads: sixteen columns at a time, or some that are not
         pos = torch.arange(shape[1], device="cuda").repeat(shape[0])
-        return [mk(*shape, 3 * 64)], lambda x: [F.rope(x * 1, pos, cos, sin, 2, 64)]
+        return [mk(*shape, 3 * 64 if op == "rope" else 2 * 64 + 8)], lambda x: [F.rope(x * 1, pos, cos, sin, 2, 64)]
     return [mk(*shape, 4 * 64)], lambda x: [F.flash_attention_qkv(x, 2, 1, 64)]
 
 
