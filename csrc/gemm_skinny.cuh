@@ -14,6 +14,8 @@
 // launches those, and the first turn of the weight ring, run beside the kernel before (ragged_llama.cu).
 #pragma once
 
+enum ChainForm : int { kBehind = 0, kChained = 1, kEarly = 2 };
+
 template <int BN, int STAGES>
 struct SkinnyPlan {
   static constexpr int kA = 128 * BK * 2;          // weight rows
@@ -98,10 +100,14 @@ __device__ __forceinline__ void load_weights(uint8_t* dst, const CUtensorMap* tm
 }
 
 // grid (tiles of 128 weight rows * S, ceil(M / BN)); clusters of S CTAs along x share one tile.
-// CHAIN: launched while the kernel that makes the tokens may still run (its own instance: asked at run time, the question cost a product
-// outside a chain up to half a microsecond, 16 x 768 x 768 7.6 -> 8.2 us).
+// CHAIN: how the kernel stands to the one before it in its stream.  kChained: within a chain, whose kernels write no weights, so the first
+// weights are fetched while that kernel runs.  kEarly: its set-up (barriers, tensor memory, descriptors) runs beside that kernel's end, every
+// load behind it; its own end lets a successor do the same.  kBehind: an ordinary launch.  (Forms of their own: asked at run time, the
+// question cost a product up to half a microsecond, 16 x 768 x 768 7.6 -> 8.2 us.)
+// us a product, one after the other with weights from HBM, kBehind | kEarly: 1 x 28672 x 4096 40.2 | 39.9, 48 x 4096 x 4096 11.5 | 10.5,
+// 1 x 4096 x 4096 9.6 | 8.6, 5 x 2304 x 768 4.4 | 3.8, 24 x 2048 x 8192 11.8 | 10.1, 33 x 6144 x 4096 14.4 | 13.1, 200 x 4096 x 14336 38.2 | 38.1.
 // GATED: B is [2 N, K], gates first, and C the activated product (skinny_reduce).
-template <int BN, int STAGES, bool CHAIN, bool GATED>
+template <int BN, int STAGES, int CHAIN, bool GATED>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p,
                    const int S) {
@@ -146,7 +152,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if (warp == 0) {
     const bool elected = elect_one();
     int ahead = kb0;
-    if constexpr (CHAIN) {                  // the weights of a first turn of the ring are on their way while that kernel runs
+    if constexpr (CHAIN == kEarly) chain_wait();
+    if constexpr (CHAIN == kChained) {      // the weights of a first turn of the ring are on their way while that kernel runs
       ahead = min(kb1, kb0 + STAGES);
       if (elected)
         for (int kb = kb0; kb < ahead; ++kb) {
@@ -162,7 +169,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       if (!__all_sync(0xffffffffu, mbar_wait_to(&empty_bar[stage], phase ^ 1, 41, kb))) break;
       if (elected) {
         uint8_t* sa = smem + stage * Plan::kStage;
-        if (!CHAIN || kb >= ahead) {
+        if (CHAIN != kChained || kb >= ahead) {
           mbar_expect_tx(&full_bar[stage], Plan::kStage);
           load_weights<GATED>(sa, &tmW, &full_bar[stage], kb * BK, 0, n0, p);
         }

@@ -692,7 +692,7 @@ static bool use_skinny(int M, int N, int K) {
   return tiles <= 128 && tiles <= K / 32;
 }
 
-template <int BN, int STAGES, bool CHAIN, bool GATED>
+template <int BN, int STAGES, int CHAIN, bool GATED>
 static int launch_skinny(const void* A, const void* B, const Params& p, int lda, int ldb, cudaStream_t stream) {
   using Plan = SkinnyPlan<BN, STAGES>;
   auto kfn = gemm_skinny_kernel<BN, STAGES, CHAIN, GATED>;
@@ -727,7 +727,7 @@ static int launch_skinny(const void* A, const void* B, const Params& p, int lda,
   return SXB_OK;
 }
 
-template <bool CHAIN, bool GATED>
+template <int CHAIN, bool GATED>
 static int launch_skinny(const void* A, const void* B, const Params& p, int lda, int ldb, cudaStream_t stream) {
   if (p.M <= 16) return launch_skinny<16, 6, CHAIN, GATED>(A, B, p, lda, ldb, stream);
   if (p.M <= 32) return launch_skinny<32, 5, CHAIN, GATED>(A, B, p, lda, ldb, stream);
@@ -897,7 +897,8 @@ SXB_API int sxb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, i
   p.accumulate = accumulate ? 1 : 0; p.direct = tma_c ? 0 : 1; p.C = C; p.ldc = ldc;
   p.alpha = alpha;
   if (layout == NT && (g_gemm_mode == 3 || (g_gemm_mode == 0 && max_ctas <= 0 && use_skinny(M, N, K))))
-    return (chained() ? launch_skinny<true, false> : launch_skinny<false, false>)(A, B, p, lda, ldb, reinterpret_cast<cudaStream_t>(stream));
+    return (chained() ? launch_skinny<kChained, false> : accumulate ? launch_skinny<kBehind, false> : launch_skinny<kEarly, false>)(
+        A, B, p, lda, ldb, reinterpret_cast<cudaStream_t>(stream));
   const int BNsel = (N > 128) ? 256 : 128;
   CUtensorMap ta, tb, tc;
   int rc;
@@ -974,5 +975,5 @@ SXB_API int sxb_gemm_gated(const void* A, const void* B, void* C, int M, int F, 
     return SXB_ERR_UNSUPPORTED;
   Params p{};
   p.M = M; p.N = F; p.K = K; p.layout = NT; p.c_dtype = kBF16; p.direct = 1; p.C = C; p.ldc = ldc; p.alpha = 1.f; p.act = act;
-  return (chained() ? launch_skinny<true, true> : launch_skinny<false, true>)(A, B, p, lda, ldb, reinterpret_cast<cudaStream_t>(stream));
+  return (chained() ? launch_skinny<kChained, true> : launch_skinny<kEarly, true>)(A, B, p, lda, ldb, reinterpret_cast<cudaStream_t>(stream));
 }
