@@ -251,8 +251,9 @@ struct GroupsPlan {
 template <bool GATED>
 __global__ void __launch_bounds__(kThreads, 2)
 gemm_skinny_groups_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, const Params p,
-                          const int S, const int* __restrict__ offsets, const int* __restrict__ used) {
+                          const int S, const int* offsets, const int* used) {
   using Plan = GroupsPlan;
+  chain_wait();                                                   // rows and their numbers come from earlier kernels
   const int g = blockIdx.y;
   const int rows_all = used[g], row0 = offsets[g];
   if (rows_all <= 0) return;                                      // the whole cluster
@@ -288,6 +289,7 @@ gemm_skinny_groups_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  chain_next();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t sbase = __shfl_sync(0xffffffffu, smem_u32(smem), 0);
   const uint32_t tbase = __shfl_sync(0xffffffffu, tmem_base, 0);

@@ -752,7 +752,7 @@ static int launch_split(const CUtensorMap& ta, const CUtensorMap& tb, const Para
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 1;          // (started early, its clusters find the GPCs in pieces: 200 rows through 2048 -> 32000 163 -> 190 us with the loss around it)
   const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_split_kernel<BN>, ta, tb, p, S);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
   return SXB_OK;
@@ -850,11 +850,13 @@ static int launch_skinny_groups(const void* A, const void* B, const Params& p, l
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = GroupsPlan::kTotal;
   cfg.stream = stream;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_skinny_groups_kernel<GATED>, tw, tx, p, S, offsets, used);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
   return SXB_OK;

@@ -787,7 +787,7 @@ static int attention_rows(int dtype, dim3 grid, const void* q, const void* kcach
                           int max_blocks, int block_size, int Hq, int G, int d, int dv, float scale, int chunk,
                           int window, int kpitch, int vpitch, const int* atoms, const void* dist_bias, int bias_len,
                           const void* gate, long long gate_ld, int gate_heads, long long out_ld,
-                                   float out_scale, cudaStream_t s) {
+                          float out_scale, bool behind_tiles, cudaStream_t s) {
   const int group = Hq / G;
   int rc = SXB_OK;
   if (sink_decode_takes(q, kcache, vcache, grid.x, Hq, G, d, dv, kpitch, vpitch, dtype)) {
@@ -799,6 +799,7 @@ static int attention_rows(int dtype, dim3 grid, const void* q, const void* kcach
     p.max_blocks = max_blocks; p.block_size = block_size; p.Hq = Hq; p.G = G;
     p.chunk = chunk; p.window = window; p.kpitch = kpitch; p.vpitch = vpitch; p.bias_len = bias_len; p.gate_heads = gate_heads;
     p.scale = scale; p.out_scale = out_scale; p.gate_ld = gate_ld; p.out_ld = out_ld;
+    p.early = behind_tiles ? 1 : 0;
     return d == 128 ? launch_sink_decode<128>(p, grid.x, s) : launch_sink_decode<64>(p, grid.x, s);
   }
   // (Taking fewer heads together when a decode batch leaves SMs idle was measured slower: every CTA walks all keys.)
@@ -1967,7 +1968,7 @@ SXB_API int sxb_sink_attention(const void* q, const void* kcache, const void* vc
   if (out_ld <= 0) out_ld = (long long)Hq * dv;
   const int rc = attention_rows(dtype, dim3(n_tokens, 1), q, kcache, vcache, sink, out, tok_seq, tok_pos, tables,
                                 max_blocks, block_size, Hq, G, d, dv, scale, chunk, window, k_pitch, v_pitch, nullptr,
-                                dist_bias, bias_len, gate, gate_ld, gate_heads, out_ld, out_scale, (cudaStream_t)stream);
+                                dist_bias, bias_len, gate, gate_ld, gate_heads, out_ld, out_scale, false, (cudaStream_t)stream);
   if (rc != SXB_OK) return rc;
   SXB_CHECK_LAUNCH();
   return SXB_OK;
@@ -2165,7 +2166,8 @@ SXB_API int sxb_sink_attention_atoms(const void* q, const void* kcache, const vo
   if (n_atoms > n_long) {
     const int rc = attention_rows(dtype, dim3((n_atoms - n_long) * kShortAtom, 1), q, kcache, vcache, sink, out, nullptr,
                                   nullptr, tables, max_blocks, block_size, Hq, G, d, dv, scale, chunk, window, k_pitch,
-                                  v_pitch, (const int*)atoms + 6 * n_long, dist_bias, bias_len, gate, gate_ld, gate_heads, out_ld, out_scale, s);
+                                  v_pitch, (const int*)atoms + 6 * n_long, dist_bias, bias_len, gate, gate_ld, gate_heads, out_ld, out_scale,
+                                  n_long > 0, s);
     if (rc != SXB_OK) return rc;
     SXB_CHECK_LAUNCH();
   }

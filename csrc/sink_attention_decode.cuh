@@ -35,6 +35,7 @@ struct SinkDecodeParams {
   int chunk, window, kpitch, vpitch, bias_len, gate_heads;
   float scale, out_scale;
   long long gate_ld, out_ld;
+  int early;
 };
 
 template <int D>
@@ -43,6 +44,7 @@ sink_decode_kernel(const SinkDecodeParams p, const int S) {
   using L = SinkDecode<D>;
   constexpr int KC = D / 8;                                          // 16-byte chunks of a row
   extern __shared__ __align__(128) uint8_t smem[];
+  if (p.early) chain_wait();                                         // behind the tile kernel, launched while it ends
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = blockIdx.x % S, unit = blockIdx.x / S % (p.G * p.bundles), slot = blockIdx.x / S / (p.G * p.bundles);
   const int g = unit / p.bundles, h0 = g * (p.Hq / p.G) + unit % p.bundles * p.heads;
@@ -304,11 +306,13 @@ static int launch_sink_decode(SinkDecodeParams p, long long n, cudaStream_t s) {
   cfg.blockDim = dim3(32 * kSdWarps);
   cfg.dynamicSmemBytes = SinkDecode<D>::kTotal;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = p.early ? 2 : 1;
   e = cudaLaunchKernelEx(&cfg, sink_decode_kernel<D>, p, S);
   if (e != cudaSuccess) { (void)cudaGetLastError(); return (int)e; }
   return SXB_OK;
