@@ -666,7 +666,7 @@ int sxb_gemm_grouped_used(const void* A, const void* B, void* C, int N, int K, l
 /* The same for groups of few rows (`routed` at most in all groups together): the weights are the MMA's rows.  act >= 0 (0 identity,
  * 1 ReLU, 2 GeLU, 3 SiLU): B [num_groups * 2 N, K], C [total_rows, N] = act(first half) * second half of the bf16 product. */
 int sxb_gemm_grouped_few(const void* A, const void* B, void* C, int N, int K, long long lda, long long ldb, long long ldc,
-                         int num_groups, const void* offsets, const void* counts, long long total_rows, long long routed,
+                         int num_groups, const void* offsets, const void* used, long long total_rows, long long routed,
                          int act, void* stream);
 /* C [M, F] = act(first half) * second half of A B^T in bf16, B [2 F, K]; -2 where the product has too many rows for one launch. */
 int sxb_gemm_gated(const void* A, const void* B, void* C, int M, int F, int K, int lda, int ldb, int ldc, int act,
