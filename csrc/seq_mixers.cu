@@ -1135,6 +1135,7 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
       }
     };
     for (int i = 0; i < kBufs - 1; ++i) group_in(i);
+    if (DELTA && n != NP) __syncthreads();  // the padding is zero: neighbours() reads it ahead of the first group's barrier
     for (int grp = 0; grp < groups; ++grp) {
       __pipeline_wait_prior(kBufs - 3);   // the group that starts here and the one behind it have landed
       if (DELTA) {
@@ -1162,6 +1163,7 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
         if (CHAN) x[Stage::kG] = 0.f;
       }
     }
+    if (DELTA && n != NP) __syncthreads();  // (the copying warp has a barrier to match)
   }
   const int lc = threadIdx.x / LPC, l = threadIdx.x % LPC;
   const int col = col0 + lc * NC;          // the lane's columns: col .. col + NC - 1
