@@ -65,7 +65,7 @@ __device__ __forceinline__ void skinny_reduce(const Params& p, int S, int rank, 
       float r[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        r[j] = ew::act_fwd<true>(__bfloat162float(__float2bfloat16_rn(g[j])), p.act) * __bfloat162float(__float2bfloat16_rn(u[j]));
+        r[j] = ew::act_fwd(__bfloat162float(__float2bfloat16_rn(g[j])), p.act) * __bfloat162float(__float2bfloat16_rn(u[j]));
       *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.C) + at) = make_uint2(pack_bf16(r[0], r[1]), pack_bf16(r[2], r[3]));
       continue;
     }
