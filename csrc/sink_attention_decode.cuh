@@ -8,9 +8,9 @@
 // keys of a (token, key/value head) are dealt out to the four warps of a CTA and to a cluster of up to 8 CTAs, whose partial (maximum,
 // sum, output) are merged in fp32, warps through shared memory, CTAs through distributed shared memory in rank order.
 // What bounds it: the bytes of K and V.  One CTA per (token, key/value head) with fp32 FMAs and a shuffle per key and head, before, was
-// bound by those or, with few tokens, by one CTA's walk.  us, before | now (floor): 1 token behind 3000 keys, 16/4 heads of 128 58 | 10; 8 behind 1000
-// 57 | 11; 40 behind 2000, 32/8 heads 232 | 87 (50); 64 behind 200, 8/2 heads 22 | 10; 64 behind 4000, 32/8 heads 593 | 214 (160); a prompt's last 16
-// rows beside its 384 others 41 | 26.  The error against 64 bits is that of the 16-bit result (1.66e-3) on both sides.
+// bound by those or, with few tokens, by one CTA's walk.  us, before | now (floor): 1 token behind 3000 keys, 16/4 heads of 128 58 | 10.5; 8 behind
+// 1000 57 | 11.4; 40 behind 2000, 32/8 heads 232 | 89 (50); 64 behind 200, 8/2 heads 22 | 10.7; 64 behind 4000, 32/8 heads 593 | 219 (160); a prompt's
+// last 16 rows beside its 384 others 41 | 27.  The error against 64 bits is that of the 16-bit result (1.66e-3) on both sides.
 // Rows that are not finite are taken again by fp32 FMAs (sink_row_plain): three terms do not carry an infinity.
 #pragma once
 
@@ -89,7 +89,6 @@ sink_decode_kernel(const SinkDecodeParams p, const int S) {
   // rows lane / 4 (leading terms, or second ones from lane 16) and lane / 4 + 8 (the rests, or nothing) of head lane / 4 mod 4
   const int t2 = (lane & 3) * 2, mi = lane >> 3, mr = lane & 7, head = (lane >> 2) & 3;
   const bool lead = lane < 16, live = head < p.heads;
-  const float scale2 = p.scale * kSinkLog2e;                         // scores, maxima and sink in units of log 2
   uint32_t qa[D / 16][4];
   {
     const float* src = p.q + ((long long)t * p.Hq + h0 + (live ? head : 0)) * D + t2;
@@ -99,7 +98,7 @@ sink_decode_kernel(const SinkDecodeParams p, const int S) {
       for (int e = 0; e < 2; ++e) {
         const float2 x = *reinterpret_cast<const float2*>(src + kk * 16 + e * 8);
         uint32_t hi, mid, rest;
-        split3<true>(x.x * scale2, x.y * scale2, hi, mid, rest);
+        split3<true>(x.x * p.scale, x.y * p.scale, hi, mid, rest);
         qa[kk][2 * e] = !live ? 0u : lead ? hi : mid;
         qa[kk][2 * e + 1] = live && lead ? rest : 0u;
       }
@@ -131,14 +130,14 @@ sink_decode_kernel(const SinkDecodeParams p, const int S) {
         const float x = __shfl_xor_sync(0xffffffffu, c[n][e], 16), y = __shfl_xor_sync(0xffffffffu, c[n][2 + e], 16);
         const int j = k0 + n * 8 + t2 + e;
         s[n][e] = lead ? (c[n][2 + e] + x) + c[n][e] : (y + c[n][e]) + x;        // the smallest terms first
-        if (bias != nullptr) s[n][e] = fmaf(__ldg(bias + min(max(keys - 1 - j, 0), p.bias_len - 1)), kSinkLog2e, s[n][e]);
+        if (bias != nullptr) s[n][e] += __ldg(bias + min(max(keys - 1 - j, 0), p.bias_len - 1));
         if (j >= keys) s[n][e] = -INFINITY;
         mx = fmaxf(mx, s[n][e]);
       }
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
     mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    if (__any_sync(0xffffffffu, mx > m + 8.f)) {                     // the maximum stays until it grows by more than 2^8
-      const float mn = fmaxf(m, mx), corr = m == -INFINITY ? 0.f : fast_exp2(m - mn);
+    if (__any_sync(0xffffffffu, mx > m + 5.f)) {                     // the maximum stays until it grows by more than e^5
+      const float mn = fmaxf(m, mx), corr = m == -INFINITY ? 0.f : expf(m - mn);
       m = mn;
       l *= corr;
 #pragma unroll
@@ -149,7 +148,7 @@ sink_decode_kernel(const SinkDecodeParams p, const int S) {
     for (int n = 0; n < 2; ++n) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        s[n][e] = fast_exp2(s[n][e] - (m == -INFINITY ? 0.f : m));
+        s[n][e] = expf(s[n][e] - (m == -INFINITY ? 0.f : m));
         l += s[n][e];
       }
       uint32_t hi, mid, rest;
@@ -196,7 +195,7 @@ sink_decode_kernel(const SinkDecodeParams p, const int S) {
 #pragma unroll
     for (int w = 0; w < kSdWarps; ++w) {
       const float2 st = stat[w * kSdHeads + r];
-      const float f = st.x == -INFINITY ? 0.f : fast_exp2(st.x - mm);
+      const float f = st.x == -INFINITY ? 0.f : expf(st.x - mm);
       const float4 x = *reinterpret_cast<const float4*>(smem + w * L::kRing + (r * D + c) * 4);
       ll += st.y * f;
       v.x += x.x * f; v.y += x.y * f; v.z += x.z * f; v.w += x.w * f;
@@ -226,17 +225,17 @@ sink_decode_kernel(const SinkDecodeParams p, const int S) {
         asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
                      : "=f"(x[s].x), "=f"(x[s].y), "=f"(x[s].z), "=f"(x[s].w) : "r"(ax) : "memory");
       }
-    const float sink = p.sink ? p.sink[h0 + r] * kSinkLog2e : -INFINITY;
+    const float sink = p.sink ? p.sink[h0 + r] : -INFINITY;
     float mm = sink;
 #pragma unroll
     for (int s = 0; s < 8; ++s)
       if (s < S) mm = fmaxf(mm, st[s].x);
-    float ll = sink == -INFINITY ? 0.f : fast_exp2(sink - mm);
+    float ll = sink == -INFINITY ? 0.f : expf(sink - mm);
     float v[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
     for (int s = 0; s < 8; ++s)
       if (s < S) {
-        const float f = st[s].x == -INFINITY ? 0.f : fast_exp2(st[s].x - mm);
+        const float f = st[s].x == -INFINITY ? 0.f : expf(st[s].x - mm);
         ll += st[s].y * f;
         v[0] += x[s].x * f; v[1] += x[s].y * f; v[2] += x[s].z * f; v[3] += x[s].w * f;
       }

@@ -12,16 +12,15 @@
 // the MMAs.  Q's three terms take 96 KB of shared memory, a ring of three K/V tiles 96 KB (head size 128).  Tensor memory: scores of
 // even tiles 0..127 (leading term, rests), of odd tiles 128..255, the tile's output 256..383, the weights' three terms 384..479 (A
 // operand).  The scores of the next tile are computed while the rows work on this one, its P V while they work on the next.
-// What bounds it: the 36 MMAs of a tile (2350 cycles) and the row warps beside them (some 19 instructions per score, a third of them for the
-// split; with expf in place of one ex2 of a difference in units of log 2 it was 25 and 2600 cycles); 3200 cycles a tile all told, 3500 with expf
-// (one prompt of 3000 rows 69.6 -> 65.7, 4096 rows, 32 heads, one chunk 466 -> 411; four chunks of Q under way per thread are half of that).  Against the same three terms on mma.sync, one warp per 16 rows, us: one prompt of 3000
+// What bounds it: the row warps (some 25 instructions per score for expf and the split: 2600 cycles a tile) and the 36 MMAs of a tile
+// beside them (2350); 3500 cycles a tile all told.  Four chunks of Q under way per thread: 4096 rows, 32 heads, one chunk 466 -> 449 us, 64 rows,
+// 16 heads 9.3 -> 8.9, one prompt of 3000 rows 70.1 -> 70.9.  (One ex2 of a difference in units of log 2 in place of expf was faster, 412 and 66,
+// and is not used: the 32-bit weights would be less exact, and a bias of the lowest value would leave the range.)  Against the same three terms on mma.sync, one warp per 16 rows, us: one prompt of 3000
 // rows, 16 heads of 128, chunks of 1024 202 -> 80 (675 with fp32 FMAs); 4096 rows, 32 heads, one chunk 1468 -> 470; four prompts
 // of 750 behind 700, window of 512 201 -> 80; one of 100 rows, 8 heads, 23 both; 8 heads of 64, portions
 // of 17 / 64 / 128 rows behind 4000 keys 189 / 198 / 262 -> 90 / 91 / 93, heads of 128 258 / 267 / 393 -> 115 / 117 / 119.  K and V in rings of their own matter: 109 with one
 // ring for both.  The error against 64 bits is that of the 16-bit result (1.656e-3) all along.
 #pragma once
-
-constexpr float kSinkLog2e = 1.4426950408889634f;
 
 // Two fp32 numbers as three packed bf16 pairs whose sum is exact (INF: infinities may occur and keep zero rests).
 template <bool INF>
@@ -266,8 +265,6 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
     const int r = quad * 32 + lane, qp = pos0 + r;              // this thread's row
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
     float* xch = reinterpret_cast<float*>(smb + L::oRow) + r;
-    // scores, maxima and the sink in units of log 2: a weight is one ex2 of a difference
-    const float scale2 = scale * kSinkLog2e;
     // four chunks of Q under way per thread
 #pragma unroll
     for (int i0 = 0; i0 < kSmQ * (D / 8); i0 += 4 * 256) {
@@ -284,7 +281,7 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
         const int i = i0 + u * 256 + tid, qr = i / (D / 8), c = i % (D / 8);
         uint32_t w[3][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) split3<true>(v[u][2 * j] * scale2, v[u][2 * j + 1] * scale2, w[0][j], w[1][j], w[2][j]);
+        for (int j = 0; j < 4; ++j) split3<true>(v[u][2 * j] * scale, v[u][2 * j + 1] * scale, w[0][j], w[1][j], w[2][j]);
 #pragma unroll
         for (int j = 0; j < 3; ++j)
           *reinterpret_cast<uint4*>(smb + j * L::kQ + (c >> 3) * (kSmQ * 128) + qr * 128 + (((c & 7) ^ (qr & 7)) << 4)) =
@@ -296,7 +293,7 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
     if (lane == 0) mbar_arrive(q_full);
 
     constexpr int CV = DV / 2;                                  // value channels of this thread
-    float m = sink ? sink[h] * kSinkLog2e : -INFINITY, l = sink && half == 0 ? 1.f : 0.f, corr_prev = 1.f, acc[CV];
+    float m = sink ? sink[h] : -INFINITY, l = sink && half == 0 ? 1.f : 0.f, corr_prev = 1.f, acc[CV];
 #pragma unroll
     for (int i = 0; i < CV; ++i) acc[i] = 0.f;
     const int lo = first_key(qp, chunk, window), lo_last = first_key(last, chunk, window);
@@ -337,7 +334,7 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
           const float* db = dist_bias + (long long)h * bias_len;
 #pragma unroll
           for (int c = 0; c < 32; ++c)
-            if (c >= c0 && c <= c1) s[c] = fmaf(__ldg(db + min(c1 - c, bias_len - 1)), kSinkLog2e, s[c]);
+            if (c >= c0 && c <= c1) s[c] += __ldg(db + min(c1 - c, bias_len - 1));
         }
 #pragma unroll
         for (int c = 0; c < 32; ++c) s[c] = c >= c0 && c <= c1 ? s[c] : -INFINITY;
@@ -351,11 +348,11 @@ sink_attention_mma_kernel(const float* __restrict__ q, const __nv_bfloat16* __re
       named_bar_sync(1 + quad, 64);
       mt = fmaxf(mt, xm[(half ^ 1) * 128]);
       const float mn = fmaxf(m, mt);
-      const float corr = (mn == -INFINITY) ? 1.f : fast_exp2(m - mn);
+      const float corr = (mn == -INFINITY) ? 1.f : expf(m - mn);
       float ps[4] = {0.f, 0.f, 0.f, 0.f};
-      const float mu = (mn == -INFINITY) ? 0.f : mn;            // what is masked becomes 2^(-inf) = 0 either way
+      const float mu = (mn == -INFINITY) ? 0.f : mn;            // what is masked becomes expf(-inf) = 0 either way
 #pragma unroll
-      for (int c = 0; c < 32; ++c) { s[c] = fast_exp2(s[c] - mu); ps[c & 3] += s[c]; }
+      for (int c = 0; c < 32; ++c) { s[c] = expf(s[c] - mu); ps[c & 3] += s[c]; }
       l = l * corr + ((ps[0] + ps[1]) + (ps[2] + ps[3]));
       m = mn;
       if (j > 0) add_output(j - 1);

@@ -144,3 +144,18 @@ def test_infinite_keys_and_values():
     assert torch.equal(y[want.isinf()].float(), want[want.isinf()])
     ok = want.isfinite()
     assert bool(((y.float() - want)[ok].abs() <= 2.0 ** -8 * want[ok].abs() + 1e-4).all())
+
+
+@pytest.mark.parametrize("with_sink", [True, False])
+def test_biases_of_the_lowest_value_leave_equal_weights(with_sink):
+    """In 32 bits every score is the lowest value, the sink's too: all keys that a row sees weigh the same."""
+    low, plan, page = torch.finfo(torch.float32).min, [(0, 90), (33, 40)], 64
+    b, pages = _batch(plan, page)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    q = torch.randn(130, 4, 128, generator=g, device="cuda")
+    kc, vc = (torch.randn(pages, page, 2, 128, generator=g, device="cuda").bfloat16() for _ in range(2))
+    sink = torch.zeros(4, device="cuda") if with_sink else None
+    y = M.sink_attention(q, kc, vc, sink + low if with_sink else None, b.token_to_seq(), b.token_positions(), b.block_tables(), 0.1, 0,
+                         torch.bfloat16, b.atoms(), b.atoms_longer_than(M.SHORT_ATOM), dist_bias=torch.full((4, 100), low, device="cuda"))
+    want = _oracle(0 * q, kc, vc, b, plan, page, 0.1, 0, 0, sink, None, None)
+    assert bool(((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all())

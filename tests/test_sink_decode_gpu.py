@@ -113,3 +113,15 @@ def test_infinities_come_out_as_from_32_bit_products():
     _close(got[0][:, keep], want[0][:, keep])
     assert bool((~got[1].isfinite()).all()) and bool((~got[2, 1].isfinite()).all())
     _close(got[2, [0, 2, 3]], want[2, [0, 2, 3]])
+
+
+@pytest.mark.parametrize("with_sink", [True, False])
+def test_biases_of_the_lowest_value_leave_equal_weights(with_sink):
+    # in 32 bits every score is the lowest value, the sink's too: all keys weigh the same
+    low = torch.finfo(torch.float32).min
+    q, kc, vc, tables, sink, g = _case([50, 300], 8, 2, 128)
+    poss = [49, 299]
+    ts, tp = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in ([0, 1], poss))
+    got = M.sink_attention(q, kc, vc, torch.full_like(sink, low) if with_sink else None, ts, tp, tables, 0.1, 0, torch.bfloat16,
+                           dist_bias=torch.full((8, 400), low, device="cuda"))
+    _close(got, _walk(0 * q, kc, vc, tables, [0, 1], poss, 0.1, sink=0 * sink if with_sink else None))
