@@ -25,7 +25,6 @@
 #include <torch/csrc/jit/frontend/tracer.h>
 
 #include <atomic>
-#include <stdexcept>
 #include <string>
 
 namespace {
@@ -55,13 +54,18 @@ struct Lib {
 };
 Lib g_lib;
 bool g_bound = false;                          // written once, under the GIL
-PyObject* g_error = nullptr;                   // the exception type of the Python binding
+PyObject* g_error = nullptr;                   // the exception type of the Python binding, once bound
 std::atomic<long long> g_calls{0};             // entry points called since they were last taken
 PyObject* g_marks[3];                          // attributes of the main-grad protocol
 
-struct CallFailed : std::runtime_error {
-  using std::runtime_error::runtime_error;
-};
+// A refused or failed call raises the binding's error, in a backward pass too: as a Python exception that the autograd engine hands on.
+[[noreturn]] void refuse(const std::string& what) {
+  pybind11::gil_scoped_acquire gil;
+  PyErr_SetString(g_error, what.c_str());
+  python_error e;
+  e.persist();
+  throw e;
+}
 
 void check(const char* name, int rc) {
   g_calls.fetch_add(1, std::memory_order_relaxed);
@@ -74,7 +78,7 @@ void check(const char* name, int rc) {
                     : rc == -4 ? "driver entry point unavailable" : "error";
     what += std::string(" rejected the call: ") + why + " (" + std::to_string(rc) + ")";
   }
-  throw CallFailed(what);
+  refuse(what);
 }
 
 void* stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
@@ -311,17 +315,14 @@ bool tape(const Tensor& a) { return a.requires_grad(); }
 
 constexpr int64_t kMost = int64_t(1) << 31;
 
-// Runs f without the GIL and wraps what it returns; a refused call becomes the binding's error.
+// Runs f without the GIL and wraps what it returns.
 template <typename F>
 PyObject* run(F&& f) {
-  HANDLE_TH_ERRORS                             // (hooks on saved tensors may raise: a checkpoint stops its recomputation so)
+  HANDLE_TH_ERRORS                             // (hooks on saved tensors may raise too: a checkpoint stops its recomputation so)
   variable_list out;
-  try {
+  {
     pybind11::gil_scoped_release no_gil;
     out = f();
-  } catch (const CallFailed& e) {
-    PyErr_SetString(g_error ? g_error : PyExc_RuntimeError, e.what());
-    return nullptr;
   }
   if (out.size() == 1) return THPVariable_Wrap(out[0]);
   PyObject* a = THPVariable_Wrap(out[0]);

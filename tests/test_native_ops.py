@@ -160,3 +160,14 @@ def test_changed_operands_are_noticed_and_refusals_are_the_bindings():
     assert out is z and z._version == v + 1
     with pytest.raises(lib.NativeError):
         F.rope(z.detach().requires_grad_() * 1, None, cos, sin, 1, 33)
+
+
+@needs_ops
+@pytest.mark.gpu
+def test_a_call_refused_in_backward_is_the_bindings_error():
+    (x, w), f = _make("linear", shape=(1,))
+    y = f(x, w)[0]
+    calls = lib.OPS.calls()
+    with pytest.raises(lib.NativeError, match="unsupported shape/alignment"):
+        y.backward(torch.zeros(1, 56, dtype=torch.bfloat16, device="cuda")[:, 1:49])       # a row that starts two bytes off
+    assert lib.OPS.calls() == calls + 1 and x.grad is None and w.grad is None
