@@ -6,6 +6,8 @@
 // projection of a decode batch 14.5 us for a kernel of 10.  With these functions the layer
 // takes 440 us, 2 x 300 rows of attention forward and backward 70 (150 before), the host side of a projection 7 (14.5).
 //
+// A weight's marks are read again in backward, where they decide who takes the gradient.
+//
 // Every function here looks at what it is given and returns None for anything that is not the plain case: another device, type or layout,
 // tensor subclasses, forward-mode levels, tracing, function transforms, dispatch modes, weights that carry the main-grad
 // protocol (attributes ops/functional.py reads).  The Python operator then goes its own way, errors included.  Tensors are saved through
@@ -57,6 +59,8 @@ bool g_bound = false;                          // written once, under the GIL
 PyObject* g_error = nullptr;                   // the exception type of the Python binding, once bound
 std::atomic<long long> g_calls{0};             // entry points called since they were last taken
 PyObject* g_marks[3];                          // attributes of the main-grad protocol
+// What backward passes ask of Python: the gradients through marked weights, and the number of ranks told to the library.
+PyObject *g_linear_bwd = nullptr, *g_rms_norm_bwd = nullptr, *g_know_ranks = nullptr;
 
 // A refused or failed call raises the binding's error, in a backward pass too: as a Python exception that the autograd engine hands on.
 [[noreturn]] void refuse(const std::string& what) {
@@ -79,6 +83,40 @@ void check(const char* name, int rc) {
     what += std::string(" rejected the call: ") + why + " (" + std::to_string(rc) + ")";
   }
   refuse(what);
+}
+
+bool marked(PyObject* o) {                     // carries the main-grad protocol, or may
+  PyObject** d = _PyObject_GetDictPtr(o);
+  if (d == nullptr || *d == nullptr) return false;
+  for (PyObject* m : g_marks)
+    if (PyDict_Contains(*d, m) != 0) return true;
+  return false;
+}
+// Calls f of the Python side; what it raises goes on to whoever runs the backward pass.  The GIL is held.
+pybind11::object ask(PyObject* f, const pybind11::tuple& args) {
+  PyObject* r = PyObject_CallObject(f, args.ptr());
+  if (r == nullptr) {
+    python_error e;
+    e.persist();
+    throw e;
+  }
+  return pybind11::reinterpret_steal<pybind11::object>(r);
+}
+pybind11::object py(const Tensor& t) {
+  return t.defined() ? pybind11::reinterpret_steal<pybind11::object>(THPVariable_Wrap(t)) : pybind11::object(pybind11::none());
+}
+// Where the weight has come under the main-grad protocol since the forward pass: the gradients as Python's function f returns or
+// delivers them (a tuple of tensors and None) for what args() gives.  False where it carries no mark.
+template <typename Args>
+bool through_python(PyObject* f, const Tensor& weight, variable_list& grads, Args&& args) {
+  pybind11::gil_scoped_acquire gil;
+  if (!marked(py(weight).ptr())) return false;
+  const pybind11::object r = ask(f, args());
+  for (size_t i = 0; i < grads.size(); ++i) {
+    PyObject* g = PyTuple_GET_ITEM(r.ptr(), i);
+    if (g != Py_None) grads[i] = THPVariable_Unpack(g);
+  }
+  return true;
 }
 
 void* stream() { return (void*)c10::cuda::getCurrentCUDAStream().stream(); }
@@ -129,12 +167,16 @@ struct Linear : Function<Linear> {
     const int64_t K = w.size(1), N = w.size(0);
     const Tensor dy = rows_of(grads[0], N);
     const int64_t M = dy.size(0);
+    const bool want_x = ctx->needs_input_grad(0), want_w = ctx->needs_input_grad(1);
+    variable_list delivered(2);
+    if (through_python(g_linear_bwd, w, delivered, [&] { return pybind11::make_tuple(py(rows_of(x, K)), py(w), py(dy), want_x, want_w); }))
+      return {want_x ? delivered[0].view(x.sizes()) : Tensor(), delivered[1]};
     Tensor dx, dw;
-    if (ctx->needs_input_grad(0)) {
+    if (want_x) {
       dx = at::empty(x.sizes(), dy.options());
       gemm(dy, w, dx, M, K, N, kNN);
     }
-    if (ctx->needs_input_grad(1)) {
+    if (want_w) {
       dw = at::empty({N, K}, w.options());
       const Tensor x2 = rows_of(x, K);
       gemm(dy, x2, dw, N, K, M, kTN);
@@ -173,6 +215,12 @@ struct RmsNorm : Function<RmsNorm> {
     const Tensor dy = grads[0].defined() ? rows_of(grads[0], H) : at::zeros(src.sizes(), src.options());
     Tensor dres;
     if (res && grads[1].defined()) dres = rows_of(grads[1], H);
+    variable_list delivered(2);
+    if (through_python(g_rms_norm_bwd, w, delivered,
+                       [&] { return pybind11::make_tuple(py(rows_of(src, H)), py(w), py(rstd), py(rows_of(dy, H)), py(dres)); })) {
+      const Tensor dx = delivered[0].view(src.sizes());
+      return {dx, delivered[1], Variable(), res ? dx : Variable()};
+    }
     Tensor dx = at::empty(src.sizes(), src.options()), dw = at::empty(w.sizes(), w.options());
     // (its own scratch: passes on other streams may run at the same time)
     const Tensor scratch = at::empty({g_lib.norm_bwd_scratch_elems(rows, (int)H, 0)}, src.options().dtype(at::kFloat));
@@ -283,6 +331,10 @@ struct Attention : Function<Attention> {
     Tensor dqkv = at::empty(qkv.sizes(), qkv.options());
     const Tensor delta = at::empty({B, Hq, S}, qkv.options().dtype(at::kFloat));
     const int64_t k0 = Hq * D, v0 = (Hq + Hk) * D;
+    {
+      pybind11::gil_scoped_acquire gil;        // a process group may have come about since the forward pass
+      ask(g_know_ranks, pybind11::tuple());
+    }
     check("attn_bwd", g_lib.attn_bwd(qkv.data_ptr(), column(qkv, k0), column(qkv, v0), out.data_ptr(), dout.data_ptr(),
                                      lse.data_ptr(), delta.data_ptr(), dqkv.data_ptr(), (void*)column(dqkv, k0),
                                      (void*)column(dqkv, v0), (int)B, (int)S, (int)Hq, (int)Hk, (int)D, C, C, C, out.stride(1),
@@ -295,7 +347,7 @@ struct Attention : Function<Attention> {
 // ------------------------------------------------------------------------------------------------ Python side
 // Nothing but autograd watches what happens here.
 bool unwatched() {
-  return g_bound && torch::autograd::ForwardADLevel::try_get_by_idx(0) == nullptr && !torch::jit::tracer::isTracing() &&
+  return g_bound && g_know_ranks != nullptr && torch::autograd::ForwardADLevel::try_get_by_idx(0) == nullptr && !torch::jit::tracer::isTracing() &&
          !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode) && c10::impl::TorchDispatchModeTLS::stack_len() == 0;
 }
 // A tensor or parameter itself (no subclass), dense and on the GPU; null if it is something else.
@@ -303,13 +355,6 @@ const Tensor* plain(PyObject* o) {
   if (!THPVariable_CheckExact(o)) return nullptr;
   const Tensor& t = THPVariable_Unpack(o);
   return t.defined() && t.is_cuda() && t.layout() == at::kStrided && !t.is_neg() && !t.is_conj() ? &t : nullptr;
-}
-bool marked(PyObject* o) {                     // carries the main-grad protocol, or may
-  PyObject** d = _PyObject_GetDictPtr(o);
-  if (d == nullptr || *d == nullptr) return false;
-  for (PyObject* m : g_marks)
-    if (PyDict_Contains(*d, m) != 0) return true;
-  return false;
 }
 bool tape(const Tensor& a) { return a.requires_grad(); }
 
@@ -452,6 +497,17 @@ PyObject* py_bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
   return PyBool_FromLong(all);
 }
 
+// backward_side(gradients of a product, gradients of a norm, telling the library its ranks): see through_python
+PyObject* py_backward_side(PyObject*, PyObject* const* args, Py_ssize_t n) {
+  if (n != 3) return PyErr_Format(PyExc_TypeError, "backward_side(linear, rms_norm, know_ranks)");
+  PyObject** to[3] = {&g_linear_bwd, &g_rms_norm_bwd, &g_know_ranks};
+  for (int i = 0; i < 3; ++i) {
+    Py_INCREF(args[i]);
+    *to[i] = args[i];
+  }
+  Py_RETURN_NONE;
+}
+
 PyObject* py_calls(PyObject*, PyObject*) { return PyLong_FromLongLong(g_calls.load(std::memory_order_relaxed)); }
 
 PyMethodDef kMethods[] = {
@@ -461,6 +517,7 @@ PyMethodDef kMethods[] = {
     {"gated_act", (PyCFunction)(void*)py_gated, METH_FASTCALL, "gated_act(x, activation code)"},
     {"attention_qkv", (PyCFunction)(void*)py_attention, METH_FASTCALL, "attention_qkv(qkv, hq, hk, d, causal, scale)"},
     {"bind", (PyCFunction)(void*)py_bind, METH_FASTCALL, "bind(handle of libsxb200.so, exception type)"},
+    {"backward_side", (PyCFunction)(void*)py_backward_side, METH_FASTCALL, "backward_side(linear, rms_norm, know_ranks)"},
     {"calls", py_calls, METH_NOARGS, "entry points called so far"},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_sxb_ops", "Differentiable operators over libsxb200.so", -1, kMethods,

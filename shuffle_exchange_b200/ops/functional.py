@@ -204,6 +204,21 @@ def _linear_fwd(x, x2, weight, bias):
     return y
 
 
+def _linear_bwd(x2, weight, dy2, need_x: bool, need_w: bool):
+    """Gradients of rows and weight; None for the weight's where it went to its main-grad view."""
+    dx = dw = None
+    if need_x:
+        gate = getattr(weight, "_sxb_gate", None)
+        if gate is not None:
+            from .gemm_ext import gemm_gated
+            dx = gemm_gated(dy2, weight, GEMM_NN, gate)
+        else:
+            dx = gemm(dy2, weight, GEMM_NN)
+    if need_w:
+        dw = _deliver_wgrad(weight, dy2, x2)
+    return dx, dw
+
+
 class _Linear(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias):
@@ -220,19 +235,9 @@ class _Linear(torch.autograd.Function):
         dy2 = dy.reshape(-1, dy.shape[-1])
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
-        dx = dw = db = None
-        if ctx.needs_input_grad[0]:
-            gate = getattr(weight, "_sxb_gate", None)
-            if gate is not None:
-                from .gemm_ext import gemm_gated
-                dx = gemm_gated(dy2, weight, GEMM_NN, gate).view(ctx.xshape)
-            else:
-                dx = gemm(dy2, weight, GEMM_NN).view(ctx.xshape)
-        if ctx.needs_input_grad[1]:
-            dw = _deliver_wgrad(weight, dy2, x2)
-        if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = dy2.sum(0)
-        return dx, dw, db
+        dx, dw = _linear_bwd(x2, weight, dy2, ctx.needs_input_grad[0], ctx.needs_input_grad[1])
+        db = dy2.sum(0) if ctx.has_bias and ctx.needs_input_grad[2] else None
+        return (None if dx is None else dx.view(ctx.xshape)), dw, db
 
 
 _warned = set()
@@ -299,6 +304,26 @@ def _rms_norm_fwd(x, weight, eps, residual, rstd):
     return y, h
 
 
+def _rms_norm_bwd(src, weight, rstd, dy2, dres):
+    """Gradients of the rows that were normed and of the weight; None for the weight's where it went to its main-grad view."""
+    rows, H = src.shape
+    dx = torch.empty_like(src)
+    mg = getattr(weight, "_sxb_main_grad", None)
+    first = not getattr(weight, "_sxb_grad_written", False)
+    dw = mg if mg is not None else torch.empty_like(weight)
+    scratch = _scratch(src.device, _n.call("sxb_norm_bwd_scratch_elems", rows, H, 0))
+    _n.call("sxb_rmsnorm_bwd", dy2.data_ptr(), src.data_ptr(), weight.data_ptr(), rstd.data_ptr(),
+            _n.ptr(dres), dx.data_ptr(), dw.data_ptr(), scratch.data_ptr(), rows, H,
+            _n.dtype_code(src.dtype), int(mg is not None and not first), _n.stream_ptr())
+    if mg is not None:
+        weight._sxb_grad_written = True
+        hook = getattr(weight, "_sxb_grad_ready", None)
+        if hook is not None:
+            hook(weight)
+        dw = None
+    return dx, dw
+
+
 class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, eps, residual):
@@ -320,7 +345,6 @@ class _RMSNorm(torch.autograd.Function):
     def backward(ctx, dy, dh):
         src, weight, rstd = ctx.saved_tensors
         H = src.shape[-1]
-        rows = src.shape[0]
         if dy is None:
             dy = torch.zeros(ctx.shape, dtype=src.dtype, device=src.device)
         dy2 = dy.reshape(-1, H)
@@ -331,22 +355,13 @@ class _RMSNorm(torch.autograd.Function):
             dres = dh.reshape(-1, H)
             if not dres.is_contiguous():
                 dres = dres.contiguous()
-        dx = torch.empty_like(src)
-        mg = getattr(weight, "_sxb_main_grad", None)
-        first = not getattr(weight, "_sxb_grad_written", False)
-        dw = mg if mg is not None else torch.empty_like(weight)
-        scratch = _scratch(src.device, _n.call("sxb_norm_bwd_scratch_elems", rows, H, 0))
-        _n.call("sxb_rmsnorm_bwd", dy2.data_ptr(), src.data_ptr(), weight.data_ptr(), rstd.data_ptr(),
-                _n.ptr(dres), dx.data_ptr(), dw.data_ptr(), scratch.data_ptr(), rows, H,
-                _n.dtype_code(src.dtype), int(mg is not None and not first), _n.stream_ptr())
-        if mg is not None:
-            weight._sxb_grad_written = True
-            hook = getattr(weight, "_sxb_grad_ready", None)
-            if hook is not None:
-                hook(weight)
-            dw = None
+        dx, dw = _rms_norm_bwd(src, weight, rstd, dy2, dres)
         dxv = dx.view(ctx.shape)
         return dxv, dw, None, (dxv if ctx.has_res else None)
+
+
+if _ops is not None:
+    _ops.backward_side(_linear_bwd, _rms_norm_bwd, _n.know_ranks)
 
 
 def rms_norm(x: torch.Tensor, weight: torch.Tensor, eps: float = 1e-6,

@@ -171,3 +171,40 @@ def test_a_call_refused_in_backward_is_the_bindings_error():
     with pytest.raises(lib.NativeError, match="unsupported shape/alignment"):
         y.backward(torch.zeros(1, 56, dtype=torch.bfloat16, device="cuda")[:, 1:49])       # a row that starts two bytes off
     assert lib.OPS.calls() == calls + 1 and x.grad is None and w.grad is None
+
+
+@needs_ops
+@pytest.mark.gpu
+@pytest.mark.parametrize("op", ["linear", "norm", "norm_residual"])
+def test_a_weight_bound_after_the_forward_delivers_like_pythons(op, monkeypatch):
+    def bound(args, f):
+        w, ready = args[1], []
+        out = f(*args)
+        w._sxb_main_grad = torch.full(w.shape, 2.0, dtype=torch.float32 if op == "linear" else w.dtype, device="cuda")
+        w._sxb_grad_ready, w._sxb_grad_written = lambda p: ready.append(p is w), True          # adds to what is there
+        out[0].backward(torch.ones_like(out[0]))
+        assert ready == [True] and w.grad is None
+        return [w._sxb_main_grad] + [a.grad for a in args if a is not w]
+    a, b = _both(op, monkeypatch, bound)
+    assert all(torch.equal(x, y) for x, y in zip(a, b)) and bool((a[0] != 2).any())
+
+    def refusing(p):
+        raise KeyError("not now")
+    args, f = _make(op)
+    out = f(*args)[0]
+    args[1]._sxb_main_grad, args[1]._sxb_grad_ready = torch.zeros_like(args[1]), refusing
+    with pytest.raises(KeyError, match="not now"):
+        out.backward(torch.ones_like(out))
+
+
+@needs_ops
+@pytest.mark.gpu
+def test_attention_tells_its_ranks_in_both_directions():
+    (x,), f = _make("attention")
+    asked = []
+    lib.OPS.backward_side(F._linear_bwd, F._rms_norm_bwd, lambda: asked.append(1))
+    try:
+        f(x)[0].float().sum().backward()
+    finally:
+        lib.OPS.backward_side(F._linear_bwd, F._rms_norm_bwd, lib.know_ranks)
+    assert asked == [1] and x.grad is not None
