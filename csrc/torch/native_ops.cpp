@@ -29,6 +29,8 @@
 #include <atomic>
 #include <string>
 
+#include "sxb200.h"
+
 namespace {
 
 using at::Tensor;
@@ -38,21 +40,17 @@ using torch::autograd::Variable;
 using torch::autograd::variable_list;
 
 // ------------------------------------------------------------------------------------------------ the C library
-struct Lib {
-  int (*gemm_bf16)(const void*, const void*, void*, int, int, int, int, int, int, int, int, int, float, int, void*);
-  int (*rmsnorm_fwd)(const void*, const void*, const void*, void*, void*, void*, long long, int, float, int, void*);
-  int (*rmsnorm_bwd)(const void*, const void*, const void*, const void*, const void*, void*, void*, void*, long long, int, int, int,
-                     void*);
-  long long (*norm_bwd_scratch_elems)(long long, int, int);
-  int (*rope)(void*, const void*, const void*, const void*, long long, int, int, long long, int, int, void*);
-  int (*rope_copy)(const void*, void*, const void*, const void*, const void*, long long, int, int, int, int, int, void*);
-  int (*gated_act_fwd)(const void*, const void*, void*, long long, int, int, int, void*);
-  int (*gated_act_bwd)(const void*, const void*, void*, long long, int, int, int, void*);
-  int (*attn_fwd)(const void*, const void*, const void*, void*, void*, int, int, int, int, int, long long, long long, long long,
-                  long long, int, float, void*);
-  int (*attn_bwd)(const void*, const void*, const void*, const void*, const void*, const void*, void*, void*, void*, void*, int, int,
-                  int, int, int, long long, long long, long long, long long, long long, long long, long long, long long, int, float,
-                  void*);
+struct Lib {                                   // (typed by the header, which the kernels' sources are checked against)
+  decltype(&sxb_gemm_bf16) gemm_bf16;
+  decltype(&sxb_rmsnorm_fwd) rmsnorm_fwd;
+  decltype(&sxb_rmsnorm_bwd) rmsnorm_bwd;
+  decltype(&sxb_norm_bwd_scratch_elems) norm_bwd_scratch_elems;
+  decltype(&sxb_rope) rope;
+  decltype(&sxb_rope_copy) rope_copy;
+  decltype(&sxb_gated_act_fwd) gated_act_fwd;
+  decltype(&sxb_gated_act_bwd) gated_act_bwd;
+  decltype(&sxb_attn_fwd) attn_fwd;
+  decltype(&sxb_attn_bwd) attn_bwd;
 };
 Lib g_lib;
 bool g_bound = false;                          // written once, under the GIL

@@ -135,14 +135,15 @@ def build_ops(force: bool = False) -> Path:
     from torch.utils.cpp_extension import include_paths
     OBJ_DIR.mkdir(parents=True, exist_ok=True)
     gxx = shutil.which("g++") or "g++"
+    headers = list((ROOT / "include").glob("*.h"))
     cuda = Path(_nvcc()).resolve().parents[1] / "include"
-    inc = [f"-I{d}" for d in (*include_paths(), sysconfig.get_paths()["include"], cuda)]
+    inc = [f"-I{d}" for d in (ROOT / "include", *include_paths(), sysconfig.get_paths()["include"], cuda)]
     flags = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     src, obj = CSRC / "torch" / "native_ops.cpp", OBJ_DIR / "ops_native_ops.o"
     lib = OUT_DIR / "_sxb_ops.so"
     key = [*flags, torch.__version__, sys.version]
-    if force or _stale(src, obj, [], key) or not lib.exists():
-        digest = _digest(src, [], key)
+    if force or _stale(src, obj, headers, key) or not lib.exists():
+        digest = _digest(src, headers, key)
         _run([gxx, *flags, *inc, "-c", str(src), "-o", str(obj)])
         _run([gxx, "-shared", "-o", str(lib), str(obj), f"-L{Path(torch.__file__).parent / 'lib'}", "-ltorch_python", "-ltorch",
               "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ldl"])
@@ -157,6 +158,7 @@ def build_all(verbose: bool = False, force: bool = False):
         try:
             ops.result()
         except Exception as e:          # no headers of Python or torch here: the operators stay in Python
+            (OUT_DIR / "_sxb_ops.so").unlink(missing_ok=True)       # not those of another source, entry point or torch
             print(f"WARNING: {OUT_DIR / '_sxb_ops.so'} was not built: {str(e)[-400:]}")
     return libs
 
