@@ -66,12 +66,14 @@ def test_a_product_may_be_the_first_call_of_a_thread():
     import threading
     lib.load()
     (x, w), f = _make("linear", grad=False)
-    want, got = f(x, w)[0], []
-    t = threading.Thread(target=lambda: got.append(lib.call(
-        "sxb_gemm_bf16", x.data_ptr(), w.data_ptr(), want.data_ptr(), 74, 48, 64, 0, 64, 64, 48, lib.BF16, 0, 1.0, 0, 0)))
+    want, rc = f(x, w)[0], []
+    got = torch.full_like(want, float("nan"))
+    t = threading.Thread(target=lambda: rc.append(lib.call(
+        "sxb_gemm_bf16", x.data_ptr(), w.data_ptr(), got.data_ptr(), 74, 48, 64, 0, 64, 64, 48, lib.BF16, 0, 1.0, 0, 0)))
+    torch.cuda.synchronize()
     t.start(), t.join()
     torch.cuda.synchronize()
-    assert got == [0] and torch.equal(want, f(x, w)[0])
+    assert rc == [0] and torch.equal(got, want)
 
 
 @needs_ops
