@@ -9,13 +9,14 @@
 #include "sxb_common.cuh"
 #include "sxb200.h"
 
-SXB_API int sxb_ragged_llama_forward(const struct sxb_ragged_llama* m, const struct sxb_ragged_llama_layer* layers, int n_layers,
+SXB_API int sxb_ragged_llama_forward(struct sxb_ragged_llama* m, const struct sxb_ragged_llama_layer* layers, int n_layers,
                                      float eps, float theta, float scale, void* stream) {
   using namespace sxb;
   if (m == nullptr || (n_layers > 0 && layers == nullptr)) return SXB_ERR_BAD_ARG;
   const int T = (int)m->T, H = (int)m->H, F = (int)m->F, Hq = (int)m->Hq, Hk = (int)m->Hk, D = (int)m->D;
   const int C = (Hq + 2 * Hk) * D, Q = Hq * D;
   int rc;
+  m->calls = 4;                // embedding, last norm, rows of the last tokens, head; eight or nine a layer
   auto product = [&](const void* x, const void* w, long long ldw, void* y, int rows, int n, int k) {
     return sxb_gemm_bf16(x, w, y, rows, n, k, 0, k, (int)ldw, n, kBF16, 0, 1.0f, 0, stream);
   };
@@ -44,10 +45,12 @@ SXB_API int sxb_ragged_llama_forward(const struct sxb_ragged_llama* m, const str
                                       (int)m->block_size, T, Hq, Hk, D, C, Q, scale, stream))) return rc;
     if ((rc = product(m->ctx, l.wo, l.ld_o, h, T, H, Q))) return rc;
     if ((rc = norm(l.ln2))) return rc;
+    m->calls += 8;
     rc = sxb_gemm_gated(m->x, l.w_gate_up, m->act, T, F, H, H, (int)l.ld_gate_up, F, 3, stream);
     if (rc == SXB_ERR_UNSUPPORTED) {      // many rows: the product and its activation one after the other, the same bits
       if ((rc = product(m->x, l.w_gate_up, l.ld_gate_up, m->gate_up, T, 2 * F, H))) return rc;
       rc = sxb_gated_act_fwd(m->gate_up, nullptr, m->act, T, F, 3, kBF16, stream);
+      ++m->calls;
     }
     if (rc) return rc;
     if ((rc = product(m->act, l.w_down, l.ld_down, h, T, H, F))) return rc;

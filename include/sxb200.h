@@ -299,13 +299,14 @@ struct sxb_ragged_llama {
   void* logits;                                   /* [n_rows, vocab] */
   long long ld_head, T, H, Hq, Hk, D, F, vocab, n_rows, max_blocks, n_blocks, block_size;
   long long n_atoms, n_packed, n_few, few_keys, few_most; /* as for sxb_attn_fwd_atoms_keys */
+  long long calls;                                /* out: entry points that the call stood for */
 };
 struct sxb_ragged_llama_layer {
   const void *ln1, *wqkv, *wo, *ln2, *w_gate_up, *w_down;
   void* cache;                                    /* [n_blocks, block_size, 2, Hk, D] */
   long long ld_qkv, ld_o, ld_gate_up, ld_down;
 };
-int sxb_ragged_llama_forward(const struct sxb_ragged_llama* m, const struct sxb_ragged_llama_layer* layers,
+int sxb_ragged_llama_forward(struct sxb_ragged_llama* m, const struct sxb_ragged_llama_layer* layers,
                              int n_layers, float eps, float theta, float scale, void* stream);
 
 /* ---- csrc/quantize.cu */

@@ -146,12 +146,12 @@ class RaggedLlamaModel:
             batch.input_ids().data_ptr(), batch.token_to_seq().data_ptr(), batch.token_positions().data_ptr(), tables.data_ptr(),
             last.data_ptr(), atoms.data_ptr(), embed, norm, head_ptr, b0, b1, b2, x, qkv, ctx, qkv, qkv + 2 * wide, rows,
             logits.data_ptr(), head.stride(0), T, H, nq, nkv, d, Fw, vocab, n_rows, tables.shape[1], cache.shape[0],
-            cache.shape[1], atoms.shape[0], n_packed, n_few, *few_keys])
+            cache.shape[1], atoms.shape[0], n_packed, n_few, *few_keys, 0])
         table = array.array("q", layers)
         n_layers = len(layers) // 11
         _n.attn_call("sxb_ragged_llama_forward", model.buffer_info()[0], table.buffer_info()[0], n_layers,
                      float(c.rms_norm_eps), float(c.rope_theta), 1.0 / math.sqrt(d), _n.stream_ptr())
-        _n.count_launches(9 * n_layers + 3)       # the entry points that the call stands for, itself among them
+        _n.count_launches(model[-1] - 1)          # the entry points that the call stood for, itself counted as one
         return logits
 
     @torch.no_grad()

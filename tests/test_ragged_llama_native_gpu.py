@@ -190,3 +190,21 @@ def test_operands_that_the_plan_refuses(monkeypatch):
     monkeypatch.setattr(RaggedLlamaModel, "_native_plan", spy)
     eng.put([0, 1], [torch.arange(5, dtype=torch.int32), torch.arange(70, dtype=torch.int32)])
     assert not taken, taken
+
+
+def test_counts_the_entry_points_it_stands_for(monkeypatch):
+    import torch
+    from shuffle_exchange_b200.inference.v2.model_implementations.llama_v2 import RaggedLlamaModel
+    from shuffle_exchange_b200.native import lib
+    model, eng = _engine(512, 4, 2, 1024, 1024, layers=3)
+    real, counts = RaggedLlamaModel._native_forward, []
+
+    def counting(s, b, p):
+        before = lib.launch_count
+        out = real(s, b, p)
+        counts.append(lib.launch_count - before)
+        return out
+    monkeypatch.setattr(RaggedLlamaModel, "_native_forward", counting)
+    for n in (1, 600):                       # one row: the gated product takes its activation along
+        eng.put([n], [torch.ones(n, dtype=torch.int32)])
+    assert counts == [8 * 3 + 4, 9 * 3 + 4]
