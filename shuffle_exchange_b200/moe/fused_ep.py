@@ -266,9 +266,9 @@ def grouped_experts_inference(x, scores, assign, offsets, counts, w1, w2, activa
     h = None
     if gate_act is not None:
         from ..ops.functional import _act_code
-        h = grouped_gated_nt_few(ep.recv_rows, w1, plan.group_offsets, counts, _act_code(gate_act), T * top_k)
+        h = grouped_gated_nt_few(ep.recv_rows, w1, plan.group_offsets, counts, _act_code(gate_act), T * top_k, T)
     if h is None:
-        h = grouped_gemm_nt_used(ep.recv_rows, w1, plan.group_offsets, counts, routed=T * top_k)
+        h = grouped_gemm_nt_used(ep.recv_rows, w1, plan.group_offsets, counts, routed=T * top_k, longest=T)
         if gate_act is not None and h.shape[1] % 16 == 0:
             a = h.new_empty((h.shape[0], h.shape[1] // 2))
             _n.call("sxb_gated_act_groups", h.data_ptr(), a.data_ptr(), plan.group_offsets.data_ptr(), counts.data_ptr(), E,
@@ -276,7 +276,7 @@ def grouped_experts_inference(x, scores, assign, offsets, counts, w1, w2, activa
             h = a
         else:
             h = activation(h)
-    grouped_gemm_nt_used(h, w2, plan.group_offsets, counts, out=ep.ret_rows, routed=T * top_k)
+    grouped_gemm_nt_used(h, w2, plan.group_offsets, counts, out=ep.ret_rows, routed=T * top_k, longest=T)
     if n_identity > 0:
         from ..ops.moe_ops import copy_group_rows_
         copy_group_rows_(ep.ret_rows, ep.recv_rows, plan.group_offsets, E, E + n_identity)

@@ -173,21 +173,31 @@ def grouped_gemm_nt(x, w, offsets, out=None, scale_x=None, qw=None, scale_w=None
 
 
 FEW_ROWS = 64           # average rows of a group up to which grouped_gemm_nt_used takes the kernel for few rows
+ONE_TURN = 256          # and rows that the longest group can have: as many as that kernel takes in one turn over the weights
 
 
-def grouped_gemm_nt_used(x, w, offsets, counts, out=None, routed: Optional[int] = None):
+def _few_rows(groups: int, routed: int, longest: Optional[int]) -> bool:
+    return routed <= FEW_ROWS * groups and (longest is None or longest <= ONE_TURN)
+
+
+def grouped_gemm_nt_used(x, w, offsets, counts, out=None, routed: Optional[int] = None, longest: Optional[int] = None):
     """:func:`grouped_gemm_nt` in bf16 for groups that use only their first ``counts[g]`` rows (int32, device): the rows of
     padding behind them are neither read nor defined in the result.  ``routed``: how many rows all groups use together, at
     most.  Up to 64 a group (on average) the product runs with the weights as the MMA's rows and as many columns as there are
     tokens; the kernel with tiles of 256 rows multiplies padding until the chip reaches its power limit (both products of 8 experts of
     4096 x 14336, one call after the other, us: 2 tokens 261 | 181, 16 tokens 681 | 450, 200 tokens 663 | 484, 400 tokens 685 | 567; 16 experts of
-    1024 x 4096, 200 tokens 106 | 92, 1000 tokens 113 | 130)."""
+    1024 x 4096, 200 tokens 106 | 92, 1000 tokens 113 | 130).
+
+    ``longest``: how many rows one group uses, at most (a router's tokens, each of which goes to an expert once).  That kernel reads the
+    weights again every 256 rows, and how many rows a group has is not known here: where all tokens choose the same experts, a product
+    of 64 experts of 4096 x 2048, each token to one of them, takes 36 | 26 with 256 tokens, 62 | 25 with 512 and 571 | 58 with 4096 (evenly spread 176 |
+    204, 174 | 205, 200 | 199); 8 experts of 28672 x 4096, each token to two, 219 | 157 with 256 (345 | 361), 165 | 129 with 192, 117 | 143 with 128."""
     G, N, K = w.shape
     if out is None:
         out = torch.empty((x.shape[0], N), dtype=torch.bfloat16, device=x.device)
     if not x.is_cuda or K == 0 or out.dtype != torch.bfloat16 or out.stride(0) % 8 or out.data_ptr() % 16:
         return grouped_gemm_nt(x, w, offsets, out=out)       # the stores of single elements stay there
-    if routed is not None and routed <= FEW_ROWS * G:
+    if routed is not None and _few_rows(G, routed, longest):
         _n.call("sxb_gemm_grouped_few", x.data_ptr(), w.data_ptr(), out.data_ptr(), N, K, x.stride(0), w.stride(1), out.stride(0), G,
                 offsets.data_ptr(), counts.data_ptr(), x.shape[0], routed, -1, _n.stream_ptr())
         return out
@@ -196,11 +206,11 @@ def grouped_gemm_nt_used(x, w, offsets, counts, out=None, routed: Optional[int] 
     return out
 
 
-def grouped_gated_nt_few(x, w, offsets, counts, act: int, routed: int):
+def grouped_gated_nt_few(x, w, offsets, counts, act: int, routed: int, longest: Optional[int] = None):
     """``act(x w[g, :F]^T) * (x w[g, F:]^T)`` of the rows that the groups use, ``w`` ``[G, 2 F, K]``: the product and its gated
-    activation in one launch, with the bits of both in turn.  For up to :data:`FEW_ROWS` rows a group; None beyond."""
+    activation in one launch, with the bits of both in turn.  Where :func:`grouped_gemm_nt_used` takes the kernel for few rows; else None."""
     G, N, K = w.shape
-    if not x.is_cuda or K == 0 or N % 16 or routed > FEW_ROWS * G:
+    if not x.is_cuda or K == 0 or N % 16 or not _few_rows(G, routed, longest):
         return None
     out = torch.empty((x.shape[0], N // 2), dtype=torch.bfloat16, device=x.device)
     _n.call("sxb_gemm_grouped_few", x.data_ptr(), w.data_ptr(), out.data_ptr(), N // 2, K, x.stride(0), w.stride(1), out.stride(0), G,

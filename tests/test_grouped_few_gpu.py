@@ -76,6 +76,22 @@ def test_one_product_with_its_activation(M, Fw, K):
     assert rc == 0 and torch.equal(out[:M], F.gated_act(F.linear(x, w), "silu")) and bool((out[M:] == 7).all())
 
 
+@pytest.mark.parametrize("longest,few", [(None, True), (256, True), (257, False)])
+def test_long_groups_keep_to_the_kernel_that_reads_the_weights_once(longest, few, monkeypatch):
+    counts = [250, 3, 0, 5, 7]                                # 53 a group on average
+    x, off, offsets, cnt, g = _groups(counts, 64)
+    w = torch.randn(5, 64, 64, generator=g, device="cuda").to(torch.bfloat16)
+    names, real = [], _n.call
+    monkeypatch.setattr(gemm_ext._n, "call", lambda name, *a: (names.append(name), real(name, *a))[1])
+    y = gemm_ext.grouped_gemm_nt_used(x, w, offsets, cnt, routed=265, longest=longest)
+    assert (names == ["sxb_gemm_grouped_few"]) == few and (names == ["sxb_gemm_grouped_used"]) != few
+    gated = gemm_ext.grouped_gated_nt_few(x, w, offsets, cnt, 3, 265, longest)
+    assert (gated is not None) == few and gemm_ext.grouped_gated_nt_few(x, w, offsets, cnt, 3, 321, longest) is None
+    for e, (o, c) in enumerate(zip(off, counts)):
+        want = x[o:o + c].double() @ w[e].double().t()
+        assert not c or float((y[o:o + c].double() - want).abs().max()) <= 2.0 ** -8 * float(want.abs().max()) + 1e-5
+
+
 def test_refusals():
     x, _, offsets, cnt, g = _groups([3, 4], 64)
     w = torch.zeros(2, 64, 64, device="cuda", dtype=torch.bfloat16)
