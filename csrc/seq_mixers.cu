@@ -2250,11 +2250,11 @@ SXB_API int sxb_recurrence_gates(const void* a_raw, const void* b_raw, long long
  * Per sequence and head, rows in order:  S <- decay S;  u = beta (v - [delta] S^T k);  S <- S + k u^T;
  * o = S^T q (+ skip[h] v).  kvec / qvec fp32 [rows, ldkq] hold G heads of n channels, val fp32 [rows, ldv] H heads of dv,
  * decay / beta fp32 [rows, H] (fixed_decay != 0: decay fp32 [H], the same for every row; beta null: ones), state fp32 [slots, H, dv, n] (taken as zero when the sequence has seen no token), out fp32
- * [rows, H * dv]. */
+ * [rows, H * dv].  n_rows: about how many rows the sequences have together (it chooses between forms with the same bits). */
 SXB_API int sxb_linear_recurrence(const void* kvec, const void* qvec, long long ldkq, const void* val, long long ldv,
                                   const void* decay, const void* beta, const void* skip, void* state, void* out,
                                   const void* seq_info, int n_seqs, int H, int G, int n, int dv, int delta,
-                                  int decay_channels, int fixed_decay, void* stream) {
+                                  int decay_channels, int fixed_decay, long long n_rows, void* stream) {
   if (n_seqs <= 0) return SXB_OK;
   if (n > 256 || H % G) return SXB_ERR_UNSUPPORTED;
   if (decay_channels && fixed_decay) return SXB_ERR_BAD_ARG;
@@ -2273,7 +2273,7 @@ SXB_API int sxb_linear_recurrence(const void* kvec, const void* qvec, long long 
             fixed_decay ? 0 : H);                                                                                        \
   } while (0)
 #define LAUNCH_REC_R(R, D, CH)                                                          \
-  if (form == kOne && n_seqs <= 32) LAUNCH_REC(R, D, CH, 1, true, R == 8 ? 5 : 3);      \
+  if (form == kOne && walks) LAUNCH_REC(R, D, CH, 1, true, R == 8 ? 5 : 3);             \
   else if (form == kOne) LAUNCH_REC(R, D, CH, 1, false, (R == 8 ? 7 : 5) - CH);         \
   else if (form == kTwoFew) LAUNCH_REC(R, D, CH, 2, D, (R == 8 ? 4 : 3) - D);           \
   else if (form == kTwo) LAUNCH_REC(R, D, CH, 2, false, (R == 8 ? 6 : 4) - CH);         \
@@ -2282,18 +2282,23 @@ SXB_API int sxb_linear_recurrence(const void* kvec, const void* qvec, long long 
   if (n <= 32) LAUNCH_REC(4, D, CH, 1, true, 6);                                        \
   else if (n <= 64) { LAUNCH_REC_R(8, D, CH); }                                         \
   else if (n <= 128) { LAUNCH_REC_R(16, D, CH); }                                       \
-  else if (ones <= 2 * sms || (CH && n_seqs <= 32)) LAUNCH_REC(32, D, CH, 1, true, 2);  \
+  else if (ones <= 2 * sms || (CH && walks)) LAUNCH_REC(32, D, CH, 1, true, 2);         \
   else LAUNCH_REC(32, D, CH, 1, false, 3)
   // Columns per lane, by the CTAs there are of 16 (one column) and of 32 (two).  Columns that share a lane share every word of k
   // and q; with one each there are twice the warps.
-  // (More than 32 sequences are mostly single rows: there the read ahead only costs warps.)
+  // (One column is read ahead up to 32 sequences, and beyond where they have 64 rows and more on average: for single rows the read ahead
+  // only costs warps.  us, read ahead | not, heads of 128 x 48, 8 of them: 40 sequences of 200 rows, delta rule 175 | 182, decay per
+  // channel 232 | 266; 100 of 16 57 | 55; 64 single rows 14.3 | 12.3.)
   // * One where that is at most a CTA per SM (us, one | two columns: delta rule, 1 sequence of 4000 rows, 16 heads 504 | 647; 1,
   //   2000, 32, twice the CTAs 421 | 330), and where the columns do not fill blocks of 32: lanes without one walk along.
   // * Two, for the delta rules read ahead, up to four CTAs per SM, two with a decay per channel (delta rule, read ahead | not:
   //   3, 2300, 16 205 | 247; 8, 1500, 16 112 | 114; 8, 4096, 32 496 | 482; 64 single rows, 32 heads 74 | 49).
   // * Beyond, four for a plain decay without the delta rule (two | four: 8, 4096, 32 404 | 334; 64 single
-  //   rows 48 | 46), two for the others (delta rule 8, 4096, 32 482 | 506; 64 single rows 49 | 58; per channel, 128 single rows, 16 heads 64 | 97).
+  //   rows 48 | 46), two for the others.  Without the delta rule the two forms of two columns differ in the registers they are given, which
+  //   decides how far the compiler reads ahead by itself (few CTAs' form | many's: state space, 128 x 128, 16 heads, 2 sequences of 1000 rows
+  //   172 | 235, 8 of 512 205 | 234; decay per channel, 64 x 64, 3 of 766 111 | 154).  (Delta rule 8, 4096, 32 482 | 506; 64 single rows 49 | 58; per channel, 128 single rows, 16 heads 64 | 97).
   enum { kOne, kTwoFew, kTwo, kFour };
+  const bool walks = n_seqs <= 32 || n_rows >= 64LL * n_seqs;
   const int blocks = (dv + 15) / 16, sms = num_sms();
   const long long ones = (long long)blocks * H * n_seqs;
   const int form = blocks % 2 || ones <= sms                                          ? kOne

@@ -513,7 +513,7 @@ int sxb_recurrence_gates(const void* a_raw, const void* b_raw, long long ld, con
 int sxb_linear_recurrence(const void* kvec, const void* qvec, long long ldkq, const void* val, long long ldv,
                           const void* decay, const void* beta, const void* skip, void* state, void* out,
                           const void* seq_info, int n_seqs, int H, int G, int n, int dv, int delta,
-                          int decay_channels, int fixed_decay, void* stream);
+                          int decay_channels, int fixed_decay, long long n_rows, void* stream);
 int sxb_group_norm_gate(const void* y, const void* gate, long long ldg, const void* w, int wlen, void* out,
                         int n_tokens, int C, int gs, float eps, int gate_first, long long out_ld, float out_scale,
                         int dtype, void* stream);

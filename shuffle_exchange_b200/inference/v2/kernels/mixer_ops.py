@@ -27,7 +27,7 @@ _lib.register({
     "sxb_conv_state_update": "p" "l" "pp" "iii" "i" "p",
     "sxb_unit_norm_heads": "p" "l" "iii" "ff" "i" "p",
     "sxb_recurrence_gates": "pp" "l" "pppp" "iii" "i" "p",
-    "sxb_linear_recurrence": "pp" "l" "p" "l" "pppppp" "iiiiii" "ii" "p",
+    "sxb_linear_recurrence": "pp" "l" "p" "l" "pppppp" "iiiiii" "ii" "l" "p",
     "sxb_group_norm_gate": "pp" "l" "p" "i" "p" "iii" "f" "i" "l" "f" "i" "p",
     "sxb_gated_act_rows": "pp" "l" "ii" "i" "f" "p",
     "sxb_conv_residual": "pppppp" "iii" "i" "p",
@@ -452,7 +452,7 @@ def linear_recurrence(kvec: torch.Tensor, qvec: torch.Tensor, val: torch.Tensor,
         _lib.call("sxb_linear_recurrence", _rows(kvec).data_ptr(), _rows(qvec).data_ptr(), kvec.stride(0),
                   _rows(val).data_ptr(), val.stride(0), decay.data_ptr(), _lib.ptr(beta), _lib.ptr(skip),
                   state.data_ptr(), out.data_ptr(), seq_info.data_ptr(), seq_info.shape[0], H, G, n, dv, int(delta),
-                  int(per_channel), int(fixed), _lib.stream_ptr())
+                  int(per_channel), int(fixed), T, _lib.stream_ptr())
         return out
     out = torch.empty(T, H, dv, dtype=torch.float32)
     rep = H // G

@@ -39,6 +39,32 @@ def test_edges_of_groups_in_every_form(rule, n, with_beta):
         assert torch.equal(st.view(copies, N, H, dv, n), first[1][None].expand(copies, -1, -1, -1, -1))
 
 
+@pytest.mark.parametrize("rule", ["delta", "ssd", "channel"])
+@pytest.mark.parametrize("n,dv", [(64, 16), (128, 48), (256, 16), (100, 16)])
+def test_many_sequences_long_and_short(rule, n, dv):
+    """Beyond 32 sequences the rows they have decide on the read ahead; the bits are the same."""
+    H, N = 2, 36
+    g = torch.Generator(device="cuda").manual_seed(n + dv)
+    mk = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    rows = [70 + i % 5 for i in range(N)]
+    T = sum(rows)
+    k, q, v = mk(T, H * n), mk(T, H * n) / n ** 0.5, mk(T, H * dv)
+    k = torch.nn.functional.normalize(k.view(T, H, n), dim=-1).view(T, -1).contiguous()
+    decay = torch.rand(T, H * (n if rule == "channel" else 1), generator=g, device="cuda")
+    beta, state = torch.rand(T, H, generator=g, device="cuda"), mk(N, H, dv, n)
+    info = torch.tensor([[sum(rows[:i]), r, i % 2, i] for i, r in enumerate(rows)], dtype=torch.int32, device="cuda")
+    st = state.clone()
+    out = M.linear_recurrence(k, q, v, decay, beta, None, st, info, H, H, n, dv, rule != "ssd")
+    want, wst = _walk(k, q, v, decay, beta, None, state, info, H, H, n, dv, rule != "ssd")
+    for a, b in ((out, want), (st, wst)):           # sums of n terms over 74 rows, contracting: a few units of the last place
+        assert float((a.double() - b).norm() / b.norm()) < 1e-6
+    # with as many sequences again that have no rows they are short on average
+    both = torch.cat([info, torch.tensor([[0, 0, 0, N + i] for i in range(N)], dtype=torch.int32, device="cuda")])
+    st2 = torch.cat([state, state])
+    assert torch.equal(M.linear_recurrence(k, q, v, decay, beta, None, st2, both, H, H, n, dv, rule != "ssd"), out)
+    assert torch.equal(st2[:N], st)
+
+
 @pytest.mark.parametrize("rule", ["delta", "channel"])
 @pytest.mark.parametrize("n", [16, 40, 72, 96, 100, 200])
 def test_padding_is_zero_before_its_first_reader(rule, n):
