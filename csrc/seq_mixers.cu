@@ -1163,7 +1163,6 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
         if (CHAN) x[Stage::kG] = 0.f;
       }
     }
-    if (DELTA && n != NP) __syncthreads();  // (the copying warp has a barrier to match)
   }
   const int lc = threadIdx.x / LPC, l = threadIdx.x % LPC;
   const int col = col0 + lc * NC;          // the lane's columns: col .. col + NC - 1
@@ -1190,6 +1189,7 @@ linear_recurrence_kernel(const float* __restrict__ kvec, const float* __restrict
     }
   }
   const float D = skip ? skip[h] : 0.f;
+  if (DELTA && n != NP) __syncthreads();   // (with the copying warp; ahead of the state's loads it cost short walks of full rows 4 % by their schedule)
 
   auto words = [&](const float* row, float2 (&w)[RP]) {        // a staged vector's words of this lane
     const float4* p = reinterpret_cast<const float4*>(row) + l;

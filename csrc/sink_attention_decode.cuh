@@ -292,7 +292,8 @@ static int launch_sink_decode(SinkDecodeParams p, long long n, cudaStream_t s) {
   p.bundles = group / p.heads;
   p.shift = (p.block_size & (p.block_size - 1)) == 0 ? __builtin_ctz(p.block_size) : -1;
   // CTAs per token and head: as many as keep the grid within one and a half waves of two per SM, and no more than have a step each
-  // in the longest reach a token can have (us, up to three quarters of a wave | one and a half | three | six: 8 tokens behind 1000 keys, 16/4
+  // in the longest reach a token can have.  n counts tokens, or kShortAtom slots for every short portion, whatever it uses of them: 8 single
+  // tokens in portions behind a prompt count as 128 (us, up to three quarters of a wave | one and a half | three | six: 8 tokens behind 1000 keys, 16/4
   // heads 13.3 | 10.8 | 10.9 | 10.9; 30 behind 1000 29.6 | 21.4 | 25.6 | 37.7; 40 behind 2000, 32/8 87 | 87 | 80 | 92; 40 behind 300 22 | 21 | 27 | 38)
   const long long units = n * p.G * p.bundles, sms = num_sms();
   long long most = (long long)p.max_blocks * p.block_size;
