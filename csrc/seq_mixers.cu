@@ -991,7 +991,7 @@ channel_decay_gates_kernel(const T* __restrict__ a_raw, long long lda, const T* 
 // 9.90e-8 both), since the state itself is stepped as before; eight tokens per pass over the state would double it.
 // DEEP: operands are read one token before their use (keys two), for few warps per scheduler; it costs registers, so with many
 // CTAs they are read where they are used.  Every form takes the same sums in the same order.
-// us, 128 x 128 (sequences, rows in all, heads), before (no look ahead, copies by the walking warps) | now:  delta rule 3, 2300, 16
+// us a call by itself, 128 x 128 (sequences, rows in all, heads), before (no look ahead, copies by the walking warps) | now:  delta rule 3, 2300, 16
 // 257 | 205;  1, 4000, 16 816 | 505;  1, 2000, 32 443 | 329;  8, 4096, 32 483 | 482;  decay per channel 386 | 260, 1018 | 670, 637 |
 // 405, 686 | 620;  state space 254 | 149, 717 | 395, 425 | 225, 459 | 331;  64 sequences of one row, 32 heads 53 | 49, 64 | 60, 46 | 46.
 constexpr int kRecThreads = 128, kTB = 8;      // walking threads (one more warp copies), tokens a group
